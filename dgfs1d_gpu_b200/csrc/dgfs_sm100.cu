@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -183,6 +184,9 @@ struct dgfs_vhs_s {
   // scratch
   float2* rho = nullptr;     // [E][Nrho][Mu][3][N][N] Nyquist-plane transforms
   float2* Fny = nullptr;     // [E][3][N][N] Nyquist planes of F_g
+  double2* rho64 = nullptr;  // FP64 mode: the same of F (null in the
+  double2* Fny64 = nullptr;  //   allocation-free entry), and exp(i N kappa_a)
+  double2* nyq64 = nullptr;
   void* Fg = nullptr;        // [E][n] complex R
   void* H = nullptr;         // [E][Nrho][n] complex R
   double* ReLf = nullptr;    // [E][n]
@@ -209,18 +213,7 @@ struct dgfs_vhs_s {
   cudaEvent_t join_hi = nullptr, join_aux = nullptr;
 };
 
-// FP64-kernel and FP32-terms cluster sizes per N (shared memory per CTA
-// must hold three padded slabs of N^3/C complex elements).
-static int c64_of(int N) {
-  switch (N) {
-    case 8: return 1;
-    case 16: return 2;
-    case 24: return 4;
-    case 32: return 8;
-    case 48: return 16;  // FP64 sums in global memory (vhs_terms_fp64g_kernel)
-    default: return 0;
-  }
-}
+// FP32-terms cluster size per N (0: grid not compiled in)
 static int c32_of(int N) {
   switch (N) {
     case 8: return 1;
@@ -232,17 +225,17 @@ static int c32_of(int N) {
   }
 }
 template <int N> struct VhsClusters;
-// c64: FP64 terms kernel; c32: FP32 terms kernel (default); cpro / cepi:
-// prologue / epilogue (FP64, one slab per CTA up to N=32).  At N=32 an 8-CTA prologue
-// cluster needs 75 KB per CTA and a 16-CTA epilogue cluster 34 KB, so two
-// (four) CTAs share an SM and a 24-point batch runs in one wave of each.
-template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = 1, cepi = 1; };
-template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = 2, cepi = 2; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 4, c32 = 3, cpro = 4, cepi = 4; };
-template <> struct VhsClusters<32> { static constexpr int c64 = 8, c32 = 4, cpro = 8, cepi = 16; };
-// N=48: 16-CTA clusters of 3 planes; the FP64 terms kernel keeps its running
-// sums in global memory (three FP64 slabs would need 331 KB per CTA)
-template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = 16, cepi = 16; };
+// c64, ch32: terms kernel with two lanes per pencil (vhs_termsh_kernel), FP64
+// and FP32 (the default there); c32: FP32 terms kernel with one thread per pencil; cpro / cepi: prologue / epilogue (FP64,
+// one slab per CTA up to N=32).  At N=32 an 8-CTA prologue cluster needs 75 KB
+// per CTA and a 16-CTA epilogue cluster 34 KB, so two (four) CTAs share an SM
+// and a 24-point batch runs in one wave of each.
+template <> struct VhsClusters<8> { static constexpr int c64 = 1, ch32 = 1, c32 = 1, cpro = 1, cepi = 1; };
+template <> struct VhsClusters<16> { static constexpr int c64 = 2, ch32 = 1, c32 = 1, cpro = 2, cepi = 2; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 6, ch32 = 2, c32 = 3, cpro = 4, cepi = 4; };
+template <> struct VhsClusters<32> { static constexpr int c64 = 16, ch32 = 8, c32 = 4, cpro = 8, cepi = 16; };
+// N=48: 16-CTA clusters of 3 planes
+template <> struct VhsClusters<48> { static constexpr int c64 = 16, ch32 = 16, c32 = 16, cpro = 16, cepi = 16; };
 
 static size_t slab_bytes(int N, int C, size_t elem) {
   return (size_t)(N / C) * N * (N + 1) * elem;
@@ -251,7 +244,8 @@ static size_t slab_bytes(int N, int C, size_t elem) {
 static void free_handle(dgfs_vhs_s* h) {
   void* ptrs[] = {h->c0, h->b2, h->b1w64, h->b1w32, h->ph, h->kappa, h->mult,
                   h->Fg, h->H, h->ReLf, h->mhat, h->moments, h->uv, h->hh,
-                  h->GM, h->nyq32, h->rho, h->Fny, h->err};
+                  h->GM, h->nyq32, h->rho, h->Fny, h->err,
+                  h->rho64, h->Fny64, h->nyq64};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (cudaEvent_t e : h->ev)
@@ -286,10 +280,6 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
     return fail(DGFS_ERR_UNSUPPORTED,
                 "velocity grid N=" + std::to_string(d->N) +
                     " is not compiled in (supported: 8, 16, 24, 32, 48)");
-  if (d->precision == DGFS_PREC_FP64 && c64_of(d->N) == 0)
-    return fail(DGFS_ERR_UNSUPPORTED,
-                "velocity grid N=" + std::to_string(d->N) +
-                    " is compiled for the FP32 mode only");
   if (int rc = ensure_twiddles()) return rc;
 
   const int N = d->N, n = N * N * N, Nrho = d->Nrho, M = d->M;
@@ -395,7 +385,13 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
     h->ph = p32;
   } else {
     double2* p64 = nullptr;
-    if ((rc = upload(&p64, ph64))) { free_handle(h); return rc; }
+    std::vector<double2> nyq(kappa.size());
+    for (size_t i = 0; i < kappa.size(); ++i)
+      nyq[i] = make_double2(std::cos(N * kappa[i]), std::sin(N * kappa[i]));
+    if ((rc = upload(&p64, ph64)) || (rc = upload(&h->nyq64, nyq))) {
+      free_handle(h);
+      return rc;
+    }
     h->ph = p64;
   }
 
@@ -408,7 +404,7 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   alloc((void**)&h->err, sizeof(int));
   if (ce_ == cudaSuccess) ce_ = cudaMemset(h->err, 0, sizeof(int));
   alloc(&h->Fg, E * n * ce);
-  alloc(&h->H, E * Nrho * n * ce);
+  alloc(&h->H, E * ((Nrho + 1) / 2) * n * ce);  // packed radial pairs
   alloc((void**)&h->ReLf, E * n * sizeof(double));
   if (fp32) {
     alloc((void**)&h->mhat, E * 3 * N * sizeof(double2));
@@ -418,6 +414,9 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
     alloc((void**)&h->GM, E * n * sizeof(double2));
     alloc((void**)&h->rho, E * Nrho * Mu * 3 * N * N * sizeof(float2));
     alloc((void**)&h->Fny, E * 3 * N * N * sizeof(float2));
+  } else {
+    alloc((void**)&h->rho64, E * Nrho * Mu * 3 * N * N * sizeof(double2));
+    alloc((void**)&h->Fny64, E * 3 * N * N * sizeof(double2));
   }
   if (ce_ != cudaSuccess) {
     free_handle(h);
@@ -512,6 +511,14 @@ static int launch_terms32_c(const VhsTermsArgs& a, int nevals, int Nrho,
                          st, a, map ? *map : none);
 }
 
+// Terms kernel with two lanes per pencil (vhs_termsh_kernel).
+template <typename R, int N, int C>
+static int launch_termsh_c(const VhsTermsArgs& a, int nevals, int Nrho,
+                           cudaStream_t st) {
+  return launch_cluster(vhs_termsh_kernel<R, N, C>, dim3(C, (Nrho + 1) / 2, nevals),
+                        dim3(HalfGeo<N, C>::NT), C, TermsHGeo<R, N, C>::smem, st, a);
+}
+
 // Split-pencil terms kernel (two threads per pencil), same shared memory.
 template <int N, int C>
 static int launch_terms32s_c(const VhsTermsArgs& a, int nevals, int Nrho,
@@ -528,17 +535,30 @@ static int launch_terms32s_c(const VhsTermsArgs& a, int nevals, int Nrho,
 
 // Variant codes: the cluster size C for the one-thread-per-pencil kernel,
 // 100 + C for the split-pencil kernel, 500 + C for the one-thread kernel
-// whose F_g slab and plane transforms arrive by TMA and bulk copies.
+// whose F_g slab and plane transforms arrive by TMA and bulk copies, 600 + C
+// for the kernel with two lanes (l, l ^ 16) per pencil.
 template <int N> struct Terms32Variants;
-template <> struct Terms32Variants<8> { static constexpr int v[3] = {1, 2, 501}; };
-template <> struct Terms32Variants<16> { static constexpr int v[3] = {1, 2, 501}; };
-template <> struct Terms32Variants<24> { static constexpr int v[4] = {3, 4, 6, 503}; };
-template <> struct Terms32Variants<32> { static constexpr int v[5] = {4, 8, 104, 108, 504}; };
-template <> struct Terms32Variants<48> { static constexpr int v[3] = {16, 116, 516}; };
+template <> struct Terms32Variants<8> { static constexpr int v[4] = {1, 2, 501, 601}; };
+template <> struct Terms32Variants<16> { static constexpr int v[5] = {1, 2, 501, 601, 602}; };
+template <> struct Terms32Variants<24> { static constexpr int v[7] = {3, 4, 6, 503, 602, 604, 606}; };
+template <> struct Terms32Variants<32> { static constexpr int v[8] = {4, 8, 104, 108, 504, 604, 608, 616}; };
+template <> struct Terms32Variants<48> { static constexpr int v[4] = {16, 116, 516, 616}; };
 
 template <int N>
 static int launch_terms32(int c, const VhsTermsArgs& a, int nevals, int Nrho,
                           cudaStream_t st, const CUtensorMap* map = nullptr) {
+  if constexpr (N <= 16)
+    if (c == 601) return launch_termsh_c<float, N, 1>(a, nevals, Nrho, st);
+  if constexpr (N == 16 || N == 24)
+    if (c == 602) return launch_termsh_c<float, N, 2>(a, nevals, Nrho, st);
+  if constexpr (N == 24 || N == 32)
+    if (c == 604) return launch_termsh_c<float, N, 4>(a, nevals, Nrho, st);
+  if constexpr (N == 24)
+    if (c == 606) return launch_termsh_c<float, N, 6>(a, nevals, Nrho, st);
+  if constexpr (N == 32)
+    if (c == 608) return launch_termsh_c<float, N, 8>(a, nevals, Nrho, st);
+  if constexpr (N == 32 || N == 48)
+    if (c == 616) return launch_termsh_c<float, N, 16>(a, nevals, Nrho, st);
   if constexpr (N == 8 || N == 16) {
     if (c == 1) return launch_terms32_c<N, 1>(a, nevals, Nrho, st);
     if (c == 2) return launch_terms32_c<N, 2>(a, nevals, Nrho, st);
@@ -576,12 +596,10 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
                    cudaStream_t st, const VhsBilin* bl = nullptr,
                    const void* const* f_list = nullptr,
                    void* const* q_list = nullptr) {
-  constexpr int C64 = VhsClusters<N>::c64 > 0 ? VhsClusters<N>::c64 : 1;
-  constexpr bool HAS64 = VhsClusters<N>::c64 > 0;
+  constexpr int C64 = VhsClusters<N>::c64;
   constexpr int C32 = VhsClusters<N>::c32;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
-  using G64 = Geo<N, C64>;
   using GPRO = Geo<N, CPRO>;
   using GEPI = Geo<N, CEPI>;
   using G32 = Geo<N, C32>;
@@ -599,7 +617,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.src_slots = src_slots; a.src_base = src_base;
     a.c0 = h->c0; a.b2 = h->b2; a.cw = h->cw; a.split = fp32 ? 1 : 0;
     a.Fg = h->Fg; a.ReLf = h->ReLf; a.mhat = h->mhat; a.moments = h->moments;
-    a.Fny = h->Fny;
+    a.Fny = h->Fny; a.Fny64 = h->Fny64;
     if (bl) { a.g = bl->g; a.alpha = bl->alpha; a.beta = bl->beta; }
     const size_t smem = prologue_smem<N, CPRO>();
     if ((rc = launch_cluster(vhs_prologue_kernel<N, CPRO>, dim3(CPRO, nevals),
@@ -625,6 +643,9 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.Fg = h->Fg; a.ph = h->ph; a.uv = h->uv; a.mult = h->mult;
     a.b1w = h->b1w32; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq32; a.rho = h->rho; a.Fny = h->Fny; a.err = h->err;
+    // default: the two-lanes-per-pencil kernel (its own plane format)
+    const int c = h->c32 ? h->c32 : 600 + VhsClusters<N>::ch32;
+    a.pm = c >= 600;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
                            dim3((h->Mu + 1) / 2, h->Nrho, nevals), dim3(6 * N),
@@ -636,9 +657,6 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     DGFS_CUDA(cudaEventRecord(h->fork1, st));
     DGFS_CUDA(cudaStreamWaitEvent(h->hi, h->fork1, 0));
     if (h->profile) cudaEventRecord(h->ev[evi++], h->hi);
-    // default: the TMA variant at the default cluster size, when its map
-    // could be made
-    const int c = h->c32 ? h->c32 : (h->fg_map_ok ? 500 + C32 : C32);
     if ((rc = launch_terms32<N>(c, a, nevals, h->Nrho, h->hi,
                                 h->fg_map_ok ? &h->fg_map : nullptr)))
       return rc;
@@ -663,30 +681,28 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     DGFS_CUDA(cudaStreamWaitEvent(st, h->join_hi, 0));
     DGFS_CUDA(cudaStreamWaitEvent(st, h->join_aux, 0));
   } else {
-    mark(); mark();  // no tables / Maxwellian-gain stages in FP64 mode
-    if constexpr (HAS64) {
-      VhsTermsArgs a{};
-      a.Fg = h->Fg; a.ph = h->ph; a.uv = nullptr; a.mult = h->mult;
-      a.b1w = h->b1w64; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
-      constexpr size_t kSmemMax = 232448;  // 227 KB per CTA
-      constexpr size_t smem3 = 3 * (size_t)G64::SLAB * sizeof(double2) +
-                               9 * N * sizeof(double2);
-      if constexpr (smem3 <= kSmemMax) {
-        if ((rc = launch_cluster(vhs_terms_kernel<double, N, C64, false>,
-                                 dim3(C64, h->Nrho, nevals), dim3(G64::NT), C64,
-                                 smem3, st, a)))
-          return rc;
-      } else {
-        constexpr size_t smem2 = 2 * (size_t)G64::SLAB * sizeof(double2) +
-                                 3 * N * sizeof(double2);
-        static_assert(smem2 <= kSmemMax, "FP64 terms slabs exceed shared memory");
-        if ((rc = launch_cluster(vhs_terms_fp64g_kernel<N, C64>,
-                                 dim3(C64, h->Nrho, nevals), dim3(G64::NT), C64,
-                                 smem2, st, a)))
-          return rc;
-      }
-    } else {
-      return fail(DGFS_ERR_UNSUPPORTED, "no FP64 terms kernel at this N");
+    VhsTermsArgs a{};
+    a.Fg = h->Fg; a.ph = h->ph; a.uv = nullptr; a.mult = h->mult;
+    a.b1w = h->b1w64; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
+    a.nyq = h->nyq64; a.rho = h->rho64; a.Fny = h->Fny64;
+    if (h->rho64) {
+      // packed transforms: Nyquist-plane transforms, then the terms
+      const size_t psmem = (size_t)(3 * N * (N + 1) + 3 * N + 3) * sizeof(double2);
+      if ((rc = launch_plain(vhs_nyq_planes64_kernel<N>, dim3(h->Mu, h->Nrho, nevals),
+                             dim3(3 * N), psmem, st, a)))
+        return rc;
+      mark(); mark();  // no Maxwellian-gain stage in FP64 mode
+      if ((rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st))) return rc;
+    } else if constexpr (N == 8 || N == 16 || N == 32) {
+      // allocation-free entry: its fixed scratch has no room for the plane
+      // transforms, so each term takes a cosine and a sine transform
+      constexpr int CN = N == 32 ? 8 : N / 8;
+      mark(); mark();
+      if ((rc = launch_cluster(vhs_terms_kernel<double, N, CN, false>,
+                               dim3(CN, h->Nrho, nevals), dim3(Geo<N, CN>::NT), CN,
+                               3 * (size_t)Geo<N, CN>::SLAB * sizeof(double2) +
+                                   9 * N * sizeof(double2), st, a)))
+        return rc;
     }
     mark();
   }
@@ -699,7 +715,8 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.Q = Q; a.q_list = q_list; a.q_double = q_double;
     a.dst_slots = dst_slots; a.dst_base = dst_base;
     a.prefac = h->prefac;
-    a.Nrho = fp32 ? (h->Nrho + 1) / 2 : h->Nrho;  // FP32: packed radial pairs
+    // packed radial pairs, except in the allocation-free entry
+    a.Nrho = (fp32 || h->rho64) ? (h->Nrho + 1) / 2 : h->Nrho;
     a.project = h->project; a.c0 = h->c0; a.cw = h->cw;
     for (int i = 0; i < 25; ++i) a.Ginv[i] = h->Ginv[i];
     if (bl) { a.bilinear = 1; a.cg = bl->cg; a.cl = bl->cl; }
@@ -2158,11 +2175,11 @@ extern "C" int dgfs_vhs_variants(int32_t N, int32_t* out, int32_t max) {
   const int* v = nullptr;
   int n = 0;
   switch (N) {
-    case 8: v = Terms32Variants<8>::v; n = 3; break;
-    case 16: v = Terms32Variants<16>::v; n = 3; break;
-    case 24: v = Terms32Variants<24>::v; n = 4; break;
-    case 32: v = Terms32Variants<32>::v; n = 5; break;
-    case 48: v = Terms32Variants<48>::v; n = 3; break;
+    case 8: v = Terms32Variants<8>::v; n = std::size(Terms32Variants<8>::v); break;
+    case 16: v = Terms32Variants<16>::v; n = std::size(Terms32Variants<16>::v); break;
+    case 24: v = Terms32Variants<24>::v; n = std::size(Terms32Variants<24>::v); break;
+    case 32: v = Terms32Variants<32>::v; n = std::size(Terms32Variants<32>::v); break;
+    case 48: v = Terms32Variants<48>::v; n = std::size(Terms32Variants<48>::v); break;
     default: return fail(DGFS_ERR_UNSUPPORTED, "N not compiled in");
   }
   for (int i = 0; i < n && i < max; ++i) out[i] = v[i];

@@ -34,6 +34,7 @@
 
 #include "cluster_slab.cuh"
 #include "fft_reg.cuh"
+#include "half_pencil.cuh"
 
 namespace dgfs {
 
@@ -62,6 +63,7 @@ struct VhsPrologueArgs {
   float2* Fny;                // out (split) [nevals][3][N][N] Nyquist planes of
                               // F_g: [0][ly][lz] at lx=N/2, [1][lx][lz] at
                               // ly=N/2, [2][lx][ly] at lz=N/2
+  double2* Fny64;             // out (not split, may be null): those of F
 };
 
 struct VhsTermsArgs {
@@ -78,6 +80,7 @@ struct VhsTermsArgs {
   int Mu;
   int Nrho;
   int* err;                   // device error flag (a bounded wait gave up)
+  int pm;                     // FP32 plane transforms: 1 stores (Re+Im, Re-Im)
 };
 
 struct VhsTablesArgs {
@@ -335,6 +338,13 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
       }
     } else {
       static_cast<double2*>(a.Fg)[gbase + j] = Fv;
+      if (a.Fny64) {
+        const int lx = rank * G::P + j / (N * N), ly = (j / N) % N, lz = j % N;
+        double2* ny = a.Fny64 + (size_t)e * 3 * N * N;
+        if (lx == N / 2) ny[ly * N + lz] = Fv;
+        if (ly == N / 2) ny[N * N + lx * N + lz] = Fv;
+        if (lz == N / 2) ny[2 * N * N + lx * N + ly] = Fv;
+      }
     }
     if (a.b2c) {
       Fv = cmul(Fv, a.b2c[(size_t)rank * G::P * N * N + j]);
@@ -695,120 +705,6 @@ vhs_terms_kernel(VhsTermsArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 terms for grids whose three FP64 slabs do not fit in shared memory
-// (N = 48: 16-CTA clusters of three planes; the transform slab A and the
-// receive slab take 225.8 KB of the 227 KB).  Same algorithm as
-// vhs_terms_kernel<double, N, C, false>, but each thread's running sum
-// S_p(x, y, z) over the sphere directions lives in global memory at
-// Sg[x * NT + t] (coalesced across the CTA) inside this CTA's own block of H,
-// which the CTA reads back once before the final transform and overwrites
-// with the output only after the cluster barrier that follows.
-// ---------------------------------------------------------------------------
-template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT, 1)
-vhs_terms_fp64g_kernel(VhsTermsArgs a) {
-  using G = Geo<N, C>;
-  using R = double;
-  using T = double2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);
-  T* Rb = A + G::SLAB;
-  T* tab = Rb + G::SLAB;            // [3][N] phase
-  const int t = threadIdx.x;
-  const unsigned rank = cluster_rank();
-  const int p = blockIdx.y, e = blockIdx.z;
-  const T* Fg = static_cast<const T*>(a.Fg) + (size_t)e * G::n;
-  const T* ph = static_cast<const T*>(a.ph);
-  T* H = static_cast<T*>(a.H) + ((size_t)e * a.Nrho + p) * G::n +
-         (size_t)rank * G::P * N * N;
-  T* Sg = H;                        // running sums, then the output block
-  for (int x = 0; x < N; ++x) Sg[(size_t)x * G::NT + t] = T{0, 0};
-
-  bool first = true;
-  for (int q = 0; q < a.Mu; ++q) {
-    __syncthreads();  // previous term's table readers are done
-    for (int i = t; i < 3 * N; i += G::NT)
-      tab[i] = ph[((size_t)p * a.Mu + q) * 3 * N + i];
-    __syncthreads();
-    const R mq = a.mult[q];
-#pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      // z-pass: multiplier cos/sin of a(l), inverse FFT along z
-      {
-        const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-        const T bxy = cmul(tab[lx], tab[N + ly]);
-        T v[N];
-        const T* row = Fg + ((size_t)lx * N + ly) * N;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v[k] = row[k];
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          const T ph3 = cmul(bxy, tab[2 * N + k]);
-          const R m = s == 0 ? ph3.x : ph3.y;
-          v[k].x *= m;
-          v[k].y *= m;
-        }
-        fft<R, N, +1>(v);
-        const int base = pl * G::PLANE + ly * G::ROW;
-#pragma unroll
-        for (int k = 0; k < N; ++k) A[base + k] = v[k];
-      }
-      __syncthreads();
-      {
-        T v[N];
-        slab_col_load_fft<R, N, C, +1>(A, t, v);
-        if (!first) cluster_wait();  // receive buffers are free
-        push_cols_to_yslab<R, N, C>(Rb, t, rank, v);
-      }
-      first = false;
-      cluster_arrive();
-      cluster_wait();
-      T v[N];
-      yslab_load_pencil<R, N, C>(Rb, t, v);
-      cluster_arrive();  // done reading the receive buffer
-      fft<R, N, +1>(v);
-#pragma unroll
-      for (int x = 0; x < N; ++x) {
-        const T h = cmul(v[x], v[x]);
-        T sv = Sg[(size_t)x * G::NT + t];
-        sv.x += mq * h.x;
-        sv.y += mq * h.y;
-        Sg[(size_t)x * G::NT + t] = sv;
-      }
-    }
-  }
-
-  // forward FFT of S_p: x-pass, exchange into X-slabs, y-pass, z-pass
-  T v[N];
-#pragma unroll
-  for (int x = 0; x < N; ++x) v[x] = Sg[(size_t)x * G::NT + t];
-  fft<R, N, -1>(v);
-  if (!first) cluster_wait();
-  push_pencils_to_xslab<R, N, C>(A, t, rank, v);
-  cluster_arrive();
-  cluster_wait();
-  {
-    T w[N];
-    slab_col_load_fft<R, N, C, -1>(A, t, w);
-    const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-    for (int k = 0; k < N; ++k) A[base + k * G::ROW] = w[k];
-  }
-  __syncthreads();
-  slab_row_pass<R, N, C, -1>(A, t);
-  __syncthreads();
-  const R* b1w = static_cast<const R*>(a.b1w) + (size_t)p * G::n +
-                 (size_t)rank * G::P * N * N;
-  for (int j = t; j < G::P * N * N; j += G::NT) {
-    T hv = A[slab_index<N, C>(j)];
-    const R w = b1w[j];
-    hv.x *= w;
-    hv.y *= w;
-    H[j] = hv;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Terms, FP32 Maxwellian-split path with packed real transforms.
 //
 // g = f - M is real, so F_g is Hermitian.  With the phase a(l) = kappa.l the
@@ -995,7 +891,9 @@ vhs_nyq_planes_kernel(VhsTermsArgs a) {
     float2* rho = static_cast<float2*>(a.rho) +
                   ((((size_t)e * a.Nrho + p) * Mu + q) * 3 + P) * N * N;
 #pragma unroll
-    for (int r = 0; r < N; ++r) rho[(size_t)r * N + i] = v[r];
+    for (int r = 0; r < N; ++r)
+      rho[(size_t)r * N + i] =
+          a.pm ? make_float2(v[r].x + v[r].y, v[r].x - v[r].y) : v[r];
   }
 }
 
@@ -1585,6 +1483,327 @@ vhs_terms_fp32s_kernel(VhsTermsArgs a) {
     const float w0 = b1a[j], w1 = b1b ? b1b[j] : 0.f;
     Hout[j] = make_float2(hv.x * w0 + hv.y * w1, hv.y * w0 - hv.x * w1);
   }
+}
+
+// ---------------------------------------------------------------------------
+// Terms with two lanes per pencil (half_pencil.cuh), both precisions: packed
+// real transforms as above, FP32 with the Maxwellian split, FP64 with M = 0.
+// With g+ = C + s, g- = C - s, w+ = s_R + c_I, w- = s_R - c_I the combine of a
+// term is
+//   g+ (g- + u_x) + v_x g- + w- (w+ + u_y) - v_y w+     (FP64: u = v = 0),
+// and the plane transforms are stored as (Re + Im, Re - Im), whose signed sums
+// are w+ and w-.
+//
+// Bound: the exchange between the x- and y-slabs.  Distributed shared memory
+// moves about 8 B per clock and SM whatever the store width, the direction or
+// the cluster size (measured with the exchange alone: 7.2-7.7 remote bytes
+// for C = 4, 8, 16; bulk copies between shared memories are no faster), and
+// a barrier costs 800-1000 clocks, so a lone CTA waits most of the time.  The
+// kernel therefore keeps only the transform slab A (z and y passes in place)
+// and one receive slab R in shared memory, and half the values per lane, so
+// that two or three CTAs of different clusters share an SM and one's exchange
+// runs under another's transforms.  One receive slab needs two cluster
+// barriers per transform (data arrived; buffer read), each split into arrive
+// and wait around a pass that does not depend on it.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double2 nyq_mul(double2 f, double s) {
+  // (1 + s f)(1 - i)/2: s = +1 main multiplier, s = -1 plane multiplier
+  const double ux = 1. + s * f.x, uy = s * f.y;
+  return make_double2(0.5 * (ux + uy), 0.5 * (uy - ux));
+}
+__device__ __forceinline__ float2 nyq_mul(float2 f, float s) {
+  const float ux = 1.f + s * f.x, uy = s * f.y;
+  return make_float2(0.5f * (ux + uy), 0.5f * (uy - ux));
+}
+
+template <typename R, int N, int C> struct TermsHGeo {
+  using G = HalfGeo<N, C>;
+  static constexpr bool SPLIT = sizeof(R) == 4;
+  // tables of one term: phases x, y, z | nu x, y, z | (u | v)
+  static constexpr int TB = (SPLIT ? 9 : 3) * N + 4;
+  static constexpr int RS = G::P * N * N;   // receive slab, no row padding
+  static constexpr size_t smem = (size_t)(G::SLAB + RS + TB) * sizeof(c2_t<R>);
+  // CTAs per SM by shared memory (228 KB, 1 KB reserved per CTA) and by the
+  // registers that a lane's N/2 values and sums need
+  static constexpr int by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
+  static constexpr int max_threads =
+      SPLIT ? (N <= 32 ? 768 : 576)
+            : (N <= 16 ? 640 : N == 24 ? 512 : 384);
+  static constexpr int by_regs = max_threads / G::NT;
+  static constexpr int per_sm =
+      by_smem < by_regs ? (by_smem > 0 ? by_smem : 1) : (by_regs > 0 ? by_regs : 1);
+};
+
+template <typename R, int N, int C>
+__global__ void __launch_bounds__(HalfGeo<N, C>::NT, TermsHGeo<R, N, C>::per_sm)
+vhs_termsh_kernel(VhsTermsArgs a) {
+  using G = HalfGeo<N, C>;
+  using TG = TermsHGeo<R, N, C>;
+  using T = c2_t<R>;
+  constexpr int H = G::H, P = G::P, NT = G::NT;
+  constexpr bool SPLIT = TG::SPLIT;
+  constexpr uint32_t ES = (uint32_t)sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* A = reinterpret_cast<T*>(smem_raw);
+  T* Rb = A + G::SLAB;                 // [P][N x][N z]
+  T* tb = Rb + TG::RS;                 // phases [3N], nu [3]
+  T* ut = tb + 3 * N + 4;              // u [3N], v [3N] (SPLIT)
+  const int t = threadIdx.x, pp = half_pencil(t), h = half_lane(t);
+  const unsigned rank = cluster_rank();
+  const int pair = blockIdx.y, e = blockIdx.z;
+  const int Mu = a.Mu, p0 = 2 * pair;
+  const int npass = (p0 + 1 < a.Nrho ? 2 : 1) * Mu;
+  const int npairs = (a.Nrho + 1) / 2;
+  const T* Fg = static_cast<const T*>(a.Fg) + (size_t)e * G::n +
+                (size_t)rank * P * N * N;
+  const T* phb = static_cast<const T*>(a.ph);
+  const T* uvb = static_cast<const T*>(a.uv);
+  const T* nyb = static_cast<const T*>(a.nyq);
+  // pencil pp: plane pl, row / column c of the X-slab; (yl, z) of the Y-slab
+  const int pl = pp / N, c = pp % N;
+  const int lx = rank * P + pl, yy = lx;
+  auto term = [&](int k) { return (size_t)(p0 + k / Mu) * Mu + k % Mu; };
+  auto load_phases = [&](int k) {      // read by zpass(k)
+    const size_t pq = term(k);
+    for (int i = t; i < 3 * N; i += NT) tb[i] = phb[pq * 3 * N + i];
+    if (t < 3) tb[3 * N + t] = nyb[pq * 3 + t];
+  };
+  auto load_uv = [&](int k) {          // read by the combine of term k
+    const T* uv = uvb + ((size_t)e * a.Nrho * Mu + term(k)) * 6 * N;
+    for (int i = t; i < 6 * N; i += NT) ut[i] = uv[i];
+  };
+  // this CTA's F rows into the padded slab, one asynchronous copy per element
+  auto copy_slab = [&]() {
+    const uint32_t a0 = smem_u32(A);
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+      const int i = j * NT + t;
+      const uint32_t dst = a0 + ES * (uint32_t)((i / N) * G::ROW + i % N);
+      if constexpr (SPLIT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n"
+                     :: "r"(dst), "l"(Fg + i) : "memory");
+      else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n"
+                     :: "r"(dst), "l"(Fg + i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int rowb = pl * G::PLANE + c * G::ROW;   // this lane's row of A
+  const int colb = pl * G::PLANE + c;            // this lane's column of A
+  const int colr = pl * N * N + c;               // this lane's column of R
+  auto zpass = [&]() {
+    const T* nu = tb + 3 * N;
+    const T bxy = cmul(tb[lx], tb[N + c]);
+    T fxy = T{R(1), R(0)};
+    if (lx == H) fxy = nu[0];
+    if (c == H) fxy = cmul(fxy, nu[1]);
+    const T gb = cmul(nyq_mul(fxy, R(1)), bxy);
+    const T gbz = cmul(nyq_mul(cmul(fxy, nu[2]), R(1)), bxy);
+    T v[H];
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      const T bz = tb[2 * N + 2 * m + h];
+      const T f = A[rowb + 2 * m + h];
+      // lz = 2m + h is the Nyquist index H only for m = H/2, h = 0
+      const T g = (2 * m == H && h == 0) ? gbz : gb;
+      const R w = g.x * bz.x - g.y * bz.y;
+      v[m] = T{f.x * w, f.y * w};
+    }
+    fft_half_dit<R, N, +1>(v, h);
+#pragma unroll
+    for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
+  };
+  // CTAs owning this lane's y values, and the offset inside their R
+  uint32_t rdst[G::GRP];
+#pragma unroll
+  for (int g = 0; g < G::GRP; ++g)
+    rdst[g] = mapa_u32(smem_u32(Rb), (uint32_t)((h * H) / P + g)) +
+              ES * (uint32_t)((P > H ? ((h * H) % P) * N * N : 0) + lx * N + c);
+
+  const R sy = (yy & 1) ? R(-1) : R(1), sz = (c & 1) ? R(-1) : R(1);
+  R S[H];
+#pragma unroll
+  for (int m = 0; m < H; ++m) S[m] = R(0);
+  // the first radial point's sums wait in this CTA's own block of H
+  T* Hout = static_cast<T*>(a.H) + ((size_t)e * npairs + pair) * G::n +
+            (size_t)rank * P * N * N;
+  R* stash = reinterpret_cast<R*>(Hout);
+
+  load_phases(0);
+  copy_slab();
+  cp_async_wait_all();
+  __syncthreads();
+  zpass();
+#pragma unroll 1
+  for (int k = 0; k < npass; ++k) {
+    T v[H];
+    __syncthreads();                     // z rows are transformed
+#pragma unroll
+    for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+    __syncthreads();  // A is read; z passes and combines up to k - 1 are done
+    if (k + 1 < npass) {
+      copy_slab();
+      load_phases(k + 1);
+    }
+    if constexpr (SPLIT) load_uv(k);
+    fft_half_dit<R, N, +1>(v, h);
+    if (k) cluster_wait();               // every CTA has read its R
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+      st_cluster(rdst[P > H ? 0 : m / P] + ES * (uint32_t)((P > H ? m : m % P) * N * N),
+                 v[m]);
+    cluster_arrive();
+    if (k + 1 < npass) {
+      cp_async_wait_all();
+      __syncthreads();
+      zpass();
+    }
+    cluster_wait();                      // this transform's columns have arrived
+#pragma unroll
+    for (int m = 0; m < H; ++m) v[m] = Rb[colr + (2 * m + h) * N];
+    cluster_arrive();                    // R is read
+    fft_half_dit<R, N, +1>(v, h);
+    const T* rp = static_cast<const T*>(a.rho) +
+                  ((size_t)e * a.Nrho * Mu + term(k)) * 3 * N * N;
+    const T rx = rp[yy * N + c];
+    const T* rY = rp + N * N + c + h * H * N;
+    const T* rZ = rp + 2 * N * N + yy + h * H * N;
+    if constexpr (SPLIT) {
+      const T* vt = ut + 3 * N;
+      const T uyz = cmul(ut[N + yy], ut[2 * N + c]);
+      const T vyz = cmul(vt[N + yy], vt[2 * N + c]);
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const T ry = rY[m * N], rz = rZ[m * N];
+        const R xs = (m & 1) ? R(-1) : R(1);   // (-1)^x, H is even
+        const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
+        const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
+        const T um = cmul(ut[h * H + m], uyz), vm = cmul(vt[h * H + m], vyz);
+        const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
+        S[m] += gp * (gm + um.x);
+        S[m] += vm.x * gm;
+        S[m] += wm * (wp + um.y);
+        S[m] -= vm.y * wp;
+      }
+    } else {
+      const R mq = a.mult[k % Mu];
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const T ry = rY[m * N], rz = rZ[m * N];
+        const R xs = (m & 1) ? R(-1) : R(1);
+        const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
+        const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
+        const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
+        S[m] += mq * (gp * gm + wm * wp);
+      }
+    }
+    if (k == Mu - 1 && npass > Mu) {
+#pragma unroll
+      for (int m = 0; m < H; ++m) { stash[m * NT + t] = S[m]; S[m] = R(0); }
+    }
+  }
+  // forward transform of S_p0 + i S_p1: x pass, exchange into X-slabs, y, z
+  T v[H];
+#pragma unroll
+  for (int m = 0; m < H; ++m)
+    v[m] = npass > Mu ? T{stash[m * NT + t], S[m]} : T{S[m], R(0)};
+  fft_half_dif<R, N, -1>(v, h);
+  cluster_wait();                        // every CTA is past its last y pass
+  {
+    const uint32_t a0 = smem_u32(A) + ES * (uint32_t)(yy * G::ROW + c);
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      const int l = 2 * m + h;
+      st_cluster(mapa_u32(a0, (uint32_t)(l / P)) + ES * (uint32_t)((l % P) * G::PLANE), v[m]);
+    }
+  }
+  cluster_sync_all();
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+  fft_half_dit<R, N, -1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[colb + (h * H + m) * G::ROW] = v[m];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+  fft_half_dit<R, N, -1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
+  __syncthreads();
+  const R* b1a = static_cast<const R*>(a.b1w) + (size_t)p0 * G::n +
+                 (size_t)rank * P * N * N;
+  const R* b1b = npass > Mu ? b1a + G::n : nullptr;
+#pragma unroll 4
+  for (int j = t; j < P * N * N; j += NT) {
+    const T hv = A[(j / N) * G::ROW + j % N];
+    const R w0 = b1a[j], w1 = b1b ? b1b[j] : R(0);
+    Hout[j] = T{hv.x * w0 + hv.y * w1, hv.y * w0 - hv.x * w1};
+  }
+}
+
+// Plane transforms of the FP64 terms kernel: as vhs_nyq_planes_kernel, one
+// direction per CTA (3N threads, one pencil each) with the planes transformed
+// in place in shared memory; stores (Re + Im, Re - Im), the combinations
+// s_R + c_I and s_R - c_I the terms kernel multiplies.
+template <int N>
+__global__ void __launch_bounds__(3 * N) vhs_nyq_planes64_kernel(VhsTermsArgs a) {
+  constexpr int ROW = N + 1, H = N / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* pls = reinterpret_cast<double2*>(smem_raw);  // [3][N][ROW]
+  double2* tb = pls + 3 * N * ROW;                       // [3N + 3]
+  const int q = blockIdx.x, p = blockIdx.y, e = blockIdx.z, t = threadIdx.x;
+  const int P = t / N, i = t % N, Mu = a.Mu;
+  const size_t pq = (size_t)p * Mu + q;
+  const double2* Fny = static_cast<const double2*>(a.Fny) + (size_t)e * 3 * N * N;
+#pragma unroll 8
+  for (int j = t; j < 3 * N * N; j += 3 * N) pls[(j / N) * ROW + j % N] = Fny[j];
+  tb[t] = static_cast<const double2*>(a.ph)[pq * 3 * N + t];
+  if (t < 3) tb[3 * N + t] = static_cast<const double2*>(a.nyq)[pq * 3 + t];
+  __syncthreads();
+  const double2 nx = tb[3 * N], ny = tb[3 * N + 1], nz = tb[3 * N + 2];
+  // rows: P=0 (lx=H, ly=i, lz=k); P=1 (lx=i, ly=H, lz=k), lx=H excluded;
+  //       P=2 (lx=i, ly=k, lz=H), lx=H and ly=H excluded
+  double2 rowc, f_row, f_rowH;
+  const double2* tk;
+  if (P == 0) {
+    rowc = cmul(tb[H], tb[N + i]);
+    f_row = (i == H) ? cmul(nx, ny) : nx;
+    f_rowH = cmul(f_row, nz);
+    tk = tb + 2 * N;
+  } else if (P == 1) {
+    rowc = cmul(tb[i], tb[N + H]);
+    f_row = ny;
+    f_rowH = cmul(ny, nz);
+    tk = tb + 2 * N;
+  } else {
+    rowc = cmul(tb[i], tb[2 * N + H]);
+    f_row = nz;
+    f_rowH = nz;
+    tk = tb + N;
+  }
+  if (P >= 1 && i == H) rowc = make_double2(0., 0.);
+  const double2 g = cmul(nyq_mul(f_row, -1.), rowc);
+  const double2 gH = (P == 2) ? make_double2(0., 0.) : cmul(nyq_mul(f_rowH, -1.), rowc);
+  double2* row = pls + (P * N + i) * ROW;
+  double2 v[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double2 gk = (k == H) ? gH : g;
+    const double m = gk.x * tk[k].x - gk.y * tk[k].y;
+    v[k] = make_double2(row[k].x * m, row[k].y * m);
+  }
+  fft<double, N, +1>(v);
+#pragma unroll
+  for (int k = 0; k < N; ++k) row[k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < N; ++r) v[r] = pls[(P * N + r) * ROW + i];
+  fft<double, N, +1>(v);
+  double2* rho = static_cast<double2*>(a.rho) +
+                 (((size_t)e * a.Nrho * Mu + pq) * 3 + P) * N * N;
+#pragma unroll
+  for (int r = 0; r < N; ++r)
+    rho[(size_t)r * N + i] = make_double2(v[r].x + v[r].y, v[r].x - v[r].y);
 }
 
 // ---------------------------------------------------------------------------
