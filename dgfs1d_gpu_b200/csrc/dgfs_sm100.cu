@@ -544,6 +544,15 @@ template <> struct Terms32Variants<24> { static constexpr int v[7] = {3, 4, 6, 5
 template <> struct Terms32Variants<32> { static constexpr int v[8] = {4, 8, 104, 108, 504, 604, 608, 616}; };
 template <> struct Terms32Variants<48> { static constexpr int v[4] = {16, 116, 516, 616}; };
 
+// Default variant: two lanes per pencil where two CTAs of different clusters
+// fit an SM and so hide each other's exchanges (N=24: 275 against 329 us for a
+// 24-point evaluation; N=48: 42.3 against 63.9 ms for 96 points); below, the
+// one-thread kernel with TMA staging (N=32: 666 against 719 us).
+template <int N> static int default_terms32(bool tma) {
+  if (N == 24 || N == 48) return 600 + VhsClusters<N>::ch32;
+  return (tma ? 500 : 0) + VhsClusters<N>::c32;
+}
+
 template <int N>
 static int launch_terms32(int c, const VhsTermsArgs& a, int nevals, int Nrho,
                           cudaStream_t st, const CUtensorMap* map = nullptr) {
@@ -644,7 +653,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.b1w = h->b1w32; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq32; a.rho = h->rho; a.Fny = h->Fny; a.err = h->err;
     // default: the two-lanes-per-pencil kernel (its own plane format)
-    const int c = h->c32 ? h->c32 : 600 + VhsClusters<N>::ch32;
+    const int c = h->c32 ? h->c32 : default_terms32<N>(h->fg_map_ok);
     a.pm = c >= 600;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
@@ -2223,9 +2232,10 @@ struct dgfs_fno_s {
   float* out = nullptr;
   double* qs = nullptr;
   double* fpart = nullptr;           // [maxB][FCH][6] partial sums
-  float *dout = nullptr, *dz = nullptr, *aw = nullptr, *dvA = nullptr,
-        *dvB = nullptr, *dy = nullptr, *part = nullptr;
-  float2 *gUh = nullptr, *gVh = nullptr;
+  // backward: dL/dout, dL/dy_l of two successive layers, the spectral part of
+  // dL/dv_l, partial weight gradients
+  float *dout = nullptr, *dyA = nullptr, *dyB = nullptr, *Ug = nullptr,
+        *part = nullptr;
   double* loss = nullptr;
   int* err = nullptr;                // device error flag (bounded waits)
   int use_tc = 1;                    // dense layers on tcgen05 tensor cores
@@ -2328,8 +2338,6 @@ extern "C" int dgfs_fno_create(const dgfs_fno_desc* d, dgfs_fno_handle* out) {
   const long nm = (long)K * K * K;
   for (int l = 0; l < 4; ++l) A(&h->Vh[l], B * nm * fno::WD);
   A(&h->Uh, B * nm * fno::WD);
-  A(&h->gUh, B * nm * fno::WD);
-  A(&h->gVh, B * nm * fno::WD);
   A(&h->Yp, B * N * K * K * fno::WD);
   A(&h->Sp, B * N * K * K * fno::WD);
   A(&h->T1, B * K * N * N * fno::WD);
@@ -2339,12 +2347,10 @@ extern "C" int dgfs_fno_create(const dgfs_fno_desc* d, dgfs_fno_handle* out) {
   A(&h->qs, B);
   A(&h->fpart, B * fno::FCH * 6);
   A(&h->dout, B * n);
-  A(&h->dz, B * n * fno::PJ);
-  A(&h->aw, B * n * fno::PJ);
-  A(&h->dvA, B * n * fno::WD);
-  A(&h->dvB, B * n * fno::WD);
-  A(&h->dy, B * n * fno::WD);
-  A(&h->part, (size_t)kFnoWgradGrid * fno::WD * fno::PJ);
+  A(&h->dyA, B * n * fno::WD);
+  A(&h->dyB, B * n * fno::WD);
+  A(&h->Ug, B * n * fno::WD);
+  A(&h->part, (size_t)kFnoWgradGrid * fno::kProjPart);
   A(&h->loss, B);
   A(&h->err, 1);
   if (e == cudaSuccess) e = cudaMemcpy(h->c0, c0.data(), N * sizeof(double), cudaMemcpyHostToDevice);
@@ -2410,23 +2416,23 @@ static int fno_dft(const void* in, void* out, const float2* table, long outer,
   return DGFS_OK;
 }
 
-// forward DFT of a real field [B][n][WD] (IN: 0 BF16, 1 FP32) into [B][K^3][WD]:
+// forward DFT of a BF16 field [B][n][WD] into [B][K^3][WD]:
 // one pass per axis (the y and z passes read 32 complex values per pencil,
 // which keeps every thread busy; a fused y/z kernel idles 60% of its
 // threads in the y pass and measured slower)
-template <int N, int K, int IN>
+template <int N, int K>
 static int fno_dft3(dgfs_fno_s* h, const void* in, const float2* tab, float2* out,
                     int B, cudaStream_t st) {
   constexpr int WD = fno::WD;
   int rc;
-  if ((rc = fno_dft<N, K, IN, 0>(in, h->T1, tab, B, N * N * WD, st))) return rc;
+  if ((rc = fno_dft<N, K, 0, 0>(in, h->T1, tab, B, N * N * WD, st))) return rc;
   if ((rc = fno_dft<N, K, 2, 0>(h->T1, h->T2, tab, (long)B * K, N * WD, st))) return rc;
   return fno_dft<N, K, 2, 0>(h->T2, out, tab, (long)B * K * K, WD, st);
 }
 
-// expand [B][K^3][WD] complex to the real part on the grid: fused z/y
-// passes, then the x pass (OUT: 2 FP32 add, 3 BF16 store)
-template <int N, int K, int OUT>
+// expand [B][K^3][WD] complex to the real part on the grid (BF16): fused z/y
+// passes, then the x pass
+template <int N, int K>
 static int fno_idft3(dgfs_fno_s* h, const float2* in, const float2* tab, void* out,
                      int B, cudaStream_t st) {
   constexpr int WD = fno::WD;
@@ -2437,7 +2443,7 @@ static int fno_idft3(dgfs_fno_s* h, const float2* in, const float2* tab, void* o
   fno::fno_dft_zy_inv_kernel<N, K><<<dim3(WD / fno::DCG, K, B), 256, smem, st>>>(
       in, h->T1, tab);
   DGFS_CUDA(cudaGetLastError());
-  return fno_dft<K, N, 2, OUT>(h->T1, out, tab, B, N * N * WD, st);
+  return fno_dft<K, N, 2, 3>(h->T1, out, tab, B, N * N * WD, st);
 }
 
 // Dense layer / projection on the tensor cores: persistent 128-row tiles.
@@ -2476,11 +2482,11 @@ static int fno_forward(dgfs_fno_s* h, const void* f, int f_double,
   fno_features_kernel<2><<<fg, 256, 0, st>>>(fa);
   DGFS_CUDA(cudaGetLastError());
   for (int l = 0; l < 4; ++l) {
-    if ((rc = fno_dft3<N, K, 0>(h, h->v[l], h->tF, h->Vh[l], B, st))) return rc;
-    fno_mix_kernel<0><<<(unsigned)nm, dim3(32, 8), 0, st>>>(
-        h->Vh[l], nullptr, h->p16 + h->L.W[l], h->Uh, nullptr, B, (int)nm);
+    if ((rc = fno_dft3<N, K>(h, h->v[l], h->tF, h->Vh[l], B, st))) return rc;
+    fno_mix_kernel<<<(unsigned)nm, dim3(32, 8), 0, st>>>(
+        h->Vh[l], h->p16 + h->L.W[l], h->Uh, B, (int)nm);
     DGFS_CUDA(cudaGetLastError());
-    if ((rc = fno_idft3<N, K, 3>(h, h->Uh, h->tG, h->U, B, st))) return rc;
+    if ((rc = fno_idft3<N, K>(h, h->Uh, h->tG, h->U, B, st))) return rc;
     if (h->use_tc) {
       TcArgs ta{};
       ta.x = h->v[l]; ta.w16 = h->p16; ta.offW = h->L.D[l]; ta.offb = h->L.d[l];
@@ -2508,13 +2514,13 @@ static int fno_forward(dgfs_fno_s* h, const void* f, int f_double,
   return DGFS_OK;
 }
 
-// Inference forward with the fused spectral passes (see fno_kernels.cuh):
-// per layer one x-mix launch and one yz-inverse + dense launch, and one
-// yz-forward launch for the next layer's spectra.
+// Forward with the fused spectral passes (see fno_kernels.cuh): per layer one
+// x-mix launch and one yz-inverse + dense launch, and one yz-forward launch
+// for the next layer's spectra.  Training also keeps y_l and the spectra Vh.
 template <int N, int K>
 static int fno_forward_fused(dgfs_fno_s* h, const void* f, int f_double,
                              const int32_t* src_slots, int src_base, int B,
-                             cudaStream_t st) {
+                             cudaStream_t st, bool train = false) {
   using namespace fno;
   const long R = (long)B * h->n;
   FeatArgs fa{};
@@ -2529,25 +2535,27 @@ static int fno_forward_fused(dgfs_fno_s* h, const void* f, int f_double,
   const int fsm = N * K * WD * (int)sizeof(float2);
   const int xsm = 2 * K * K * WD * (int)sizeof(float2);
   const int ism = YzInvGeo<N, K>::SMEM;
-  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K>,
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, __nv_bfloat16>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   DGFS_CUDA(cudaFuncSetAttribute(fno_xmix_kernel<N, K>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
   DGFS_CUDA(cudaFuncSetAttribute(fno_yzinv_dense_kernel<N, K>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, ism));
   const dim3 pg(N, B);
-  fno_yzfwd_kernel<N, K><<<pg, 256, fsm, st>>>(h->v[0], h->Yp);
+  fno_yzfwd_kernel<N, K, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[0], h->Yp);
   DGFS_CUDA(cudaGetLastError());
   for (int l = 0; l < 4; ++l) {
     fno_xmix_kernel<N, K><<<dim3(K * K, (B + K - 1) / K), K * 32, xsm, st>>>(
-        h->Yp, h->p16 + h->L.W[l], h->Sp, B);
+        h->Yp, h->p16 + h->L.W[l], h->Sp, train ? h->Vh[l] : nullptr, B);
     YzInvArgs ya{};
     ya.S = h->Sp; ya.v = h->v[l]; ya.w16 = h->p16; ya.offD = h->L.D[l];
     ya.offd = h->L.d[l]; ya.vout = h->v[l + 1]; ya.act = l < 3 ? 1 : 0;
+    ya.y = train ? h->y[l] : nullptr;
     ya.err = h->err;
     fno_yzinv_dense_kernel<N, K><<<dim3(N * YzInvGeo<N, K>::ZP, B),
                                    YzInvGeo<N, K>::NT, ism, st>>>(ya);
-    if (l < 3) fno_yzfwd_kernel<N, K><<<pg, 256, fsm, st>>>(h->v[l + 1], h->Yp);
+    if (l < 3)
+      fno_yzfwd_kernel<N, K, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[l + 1], h->Yp);
     DGFS_CUDA(cudaGetLastError());
   }
   TcArgs ta{};
@@ -2557,28 +2565,24 @@ static int fno_forward_fused(dgfs_fno_s* h, const void* f, int f_double,
   return fno_tc<PJ, 1>(h, ta, st);
 }
 
-template <int KA, int KB>
-static int fno_wgrad(dgfs_fno_s* h, const __nv_bfloat16* A, const float* Bm,
-                     long R, long off, cudaStream_t st) {
-  constexpr int RI = KA < 4 ? KA : 4;
-  constexpr int NTH = (KA / RI) * (KB / 4);
-  fno::fno_wgrad_kernel<KA, KB><<<kFnoWgradGrid, NTH, 0, st>>>(A, Bm, R, h->part);
-  DGFS_CUDA(cudaGetLastError());
-  fno::fno_reduce_kernel<<<(KA * KB + 255) / 256, 256, 0, st>>>(
-      h->part, kFnoWgradGrid, KA * KB, h->grad + off);
+// sum of G partial gradient records of n values into grad + off
+static int fno_reduce(dgfs_fno_s* h, int G, int n, long off, cudaStream_t st) {
+  fno::fno_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(h->part, G, n, h->grad + off);
   DGFS_CUDA(cudaGetLastError());
   return DGFS_OK;
 }
 
-template <int KB>
-static int fno_colsum(dgfs_fno_s* h, const float* Bm, long R, long off,
-                      cudaStream_t st) {
-  fno::fno_colsum_kernel<KB><<<kFnoWgradGrid, 256, 0, st>>>(Bm, R, h->part);
+template <int MODE>
+static int fno_layer_bwd(dgfs_fno_s* h, const fno::LayerBwdArgs& a, long off,
+                         cudaStream_t st) {
+  constexpr int n = MODE == 2 ? fno::CIN * fno::WD + fno::WD : fno::kLayerPart;
+  const int grid = (int)std::min<long>((a.R + fno::LBT - 1) / fno::LBT, kFnoWgradGrid);
+  DGFS_CUDA(cudaFuncSetAttribute(fno::fno_layer_bwd_kernel<MODE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)fno::kLayerBwdSmem));
+  fno::fno_layer_bwd_kernel<MODE><<<grid, 256, fno::kLayerBwdSmem, st>>>(a);
   DGFS_CUDA(cudaGetLastError());
-  fno::fno_reduce_kernel<<<(KB + 255) / 256, 256, 0, st>>>(h->part, kFnoWgradGrid,
-                                                           KB, h->grad + off);
-  DGFS_CUDA(cudaGetLastError());
-  return DGFS_OK;
+  return fno_reduce(h, grid, n, off, st);   // weight and bias are adjacent
 }
 
 // gradients of the loss (dout already set) w.r.t. every parameter
@@ -2586,45 +2590,51 @@ template <int N, int K>
 static int fno_backward(dgfs_fno_s* h, int B, cudaStream_t st) {
   using namespace fno;
   const long R = (long)B * h->n;
-  const long nm = (long)K * K * K;
-  const unsigned gR = (unsigned)((R + 255) / 256);
   int rc;
-  // projection
-  fno_proj_bwd_kernel<<<gR, 256, 0, st>>>(h->v[4], h->p16, h->L, h->dout, h->dz,
-                                          h->aw, h->dvA, R);
-  DGFS_CUDA(cudaGetLastError());
-  if ((rc = fno_wgrad<WD, PJ>(h, h->v[4], h->dz, R, h->L.Q1, st))) return rc;
-  if ((rc = fno_colsum<PJ>(h, h->dz, R, h->L.q1, st))) return rc;
-  if ((rc = fno_colsum<PJ>(h, h->aw, R, h->L.q2, st))) return rc;
-  if ((rc = fno_colsum<1>(h, h->dout, R, h->L.q2b, st))) return rc;
-  float* dv = h->dvA;     // gradient w.r.t. v_{l+1}
-  float* dvn = h->dvB;
-  for (int l = 3; l >= 0; --l) {
-    const float* dyl = dv;
-    if (l < 3) {
-      fno_gelu_bwd_kernel<<<(unsigned)((R * WD + 255) / 256), 256, 0, st>>>(
-          dv, h->y[l], h->dy, R * WD);
-      DGFS_CUDA(cudaGetLastError());
-      dyl = h->dy;
-    }
-    if ((rc = fno_wgrad<WD, WD>(h, h->v[l], dyl, R, h->L.D[l], st))) return rc;
-    if ((rc = fno_colsum<WD>(h, dyl, R, h->L.d[l], st))) return rc;
-    fno_dense_bwd_kernel<<<gR, 256, 0, st>>>(dyl, h->p16, h->L.D[l], dvn, R);
+  // projection: dL/dv_4 = dL/dy_3, gradients of Q1, q1, q2, q2b (adjacent)
+  {
+    const int grid = (int)std::min<long>((R + PBT - 1) / PBT, kFnoWgradGrid);
+    DGFS_CUDA(cudaFuncSetAttribute(fno_proj_bwd_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kProjBwdSmem));
+    fno_proj_bwd_kernel<<<grid, 256, kProjBwdSmem, st>>>(
+        h->v[4], h->p16, h->L, h->dout, h->dyA, h->part, R);
     DGFS_CUDA(cudaGetLastError());
-    // spectral path: gUh = B^H dy, gW, gVh = gUh W^H, dv += Re(A^H gVh)
-    if ((rc = fno_dft3<N, K, 1>(h, dyl, h->tFs, h->gUh, B, st))) return rc;
-    fno_mix_kernel<2><<<(unsigned)nm, dim3(32, 8), 0, st>>>(
-        h->Vh[l], h->gUh, nullptr, nullptr, h->grad + h->L.W[l], B, (int)nm);
-    DGFS_CUDA(cudaGetLastError());
-    fno_mix_kernel<1><<<(unsigned)nm, dim3(32, 8), 0, st>>>(
-        h->gUh, nullptr, h->p16 + h->L.W[l], h->gVh, nullptr, B, (int)nm);
-    DGFS_CUDA(cudaGetLastError());
-    if ((rc = fno_idft3<N, K, 2>(h, h->gVh, h->tGs, dvn, B, st))) return rc;
-    std::swap(dv, dvn);
+    if ((rc = fno_reduce(h, grid, kProjPart, h->L.Q1, st))) return rc;
   }
-  // lift
-  if ((rc = fno_wgrad<CIN, WD>(h, h->x0, dv, R, h->L.P, st))) return rc;
-  return fno_colsum<WD>(h, dv, R, h->L.p, st);
+  const int fsm = N * K * WD * (int)sizeof(float2);
+  const int xsm = 2 * K * K * WD * (int)sizeof(float2);
+  const int ism = YzInvGeo<N, K>::T_BYTES;
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, float>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  DGFS_CUDA(cudaFuncSetAttribute(fno_xmix_bwd_kernel<N, K>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzinv_bwd_kernel<N, K>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, ism));
+  float *dy = h->dyA, *dyn = h->dyB;
+  LayerBwdArgs la{};
+  la.w16 = h->p16; la.partial = h->part; la.R = R; la.U = h->Ug;
+  la.dy = dy; la.v = h->v[3];
+  if ((rc = fno_layer_bwd<0>(h, la, h->L.D[3], st))) return rc;
+  for (int l = 3; l >= 0; --l) {
+    fno_yzfwd_kernel<N, K, float><<<dim3(N, B), 256, fsm, st>>>(dy, h->Yp);
+    fno_xmix_bwd_kernel<N, K><<<K * K, K * 32, xsm, st>>>(
+        h->Yp, h->Vh[l], h->p16 + h->L.W[l], h->Sp,
+        reinterpret_cast<float2*>(h->grad + h->L.W[l]), B);
+    fno_yzinv_bwd_kernel<N, K><<<dim3(N * YzInvGeo<N, K>::ZP, B), 256, ism, st>>>(
+        h->Sp, h->Ug);
+    DGFS_CUDA(cudaGetLastError());
+    la.dy = dy; la.offD = h->L.D[l];
+    if (l > 0) {
+      la.y = h->y[l - 1]; la.v = h->v[l - 1]; la.dyo = dyn;
+      if ((rc = fno_layer_bwd<1>(h, la, h->L.D[l - 1], st))) return rc;
+    } else {
+      la.v = h->x0;
+      if ((rc = fno_layer_bwd<2>(h, la, h->L.P, st))) return rc;
+    }
+    std::swap(dy, dyn);
+  }
+  return DGFS_OK;
 }
 
 template <int N, int K>
@@ -2680,7 +2690,10 @@ template <int N, int K>
 static int fno_train_t(dgfs_fno_s* h, const double* f, const double* Qt, int B,
                        float lr, int step, int update, cudaStream_t st) {
   int rc;
-  if ((rc = fno_forward<N, K>(h, f, 1, nullptr, 0, B, st))) return rc;
+  if ((rc = (h->use_fused && h->use_tc)
+                ? fno_forward_fused<N, K>(h, f, 1, nullptr, 0, B, st, true)
+                : fno_forward<N, K>(h, f, 1, nullptr, 0, B, st)))
+    return rc;
   fno::fno_loss_kernel<512><<<B, 512, 0, st>>>(h->out, Qt, h->qs, h->sQ, h->n,
                                                 B, h->dout, h->loss);
   DGFS_CUDA(cudaGetLastError());

@@ -406,62 +406,31 @@ fno_dft_zy_inv_kernel(const float2* in, float2* out, const float2* table) {
 }
 
 // ---------------------------------------------------------------------------
-// Per-mode channel mixing, one CTA per mode m, block (32, 8).
-//   MODE 0 (forward):      out[b][i'] = sum_i in[b][i] W[i][i']
-//   MODE 1 (data grad):    out[b][i]  = sum_o g[b][o] conj(W[i][o])
-//   MODE 2 (weight grad):  gW[i][o]   = sum_b conj(V[b][i]) g[b][o]
+// Per-mode channel mixing, one CTA per mode m, block (32, 8):
+//   out[b][i'] = sum_i in[b][i] W[i][i']
 // W: BF16 complex [K^3][WD][WD] (re, im interleaved); in/out [B][K^3][WD].
 // ---------------------------------------------------------------------------
-template <int MODE>
 __global__ void __launch_bounds__(256)
-fno_mix_kernel(const float2* in, const float2* in2, const __nv_bfloat16* W,
-               float2* out, float* gW, int B, int nm) {
+fno_mix_kernel(const float2* in, const __nv_bfloat16* W, float2* out, int B, int nm) {
   __shared__ float2 ws[WD * WD];
   __shared__ float2 xs[32 * WD];   // up to 32 samples
-  __shared__ float2 gs[32 * WD];
   const int m = blockIdx.x, tx = threadIdx.x, ty = threadIdx.y;
   const int t = ty * 32 + tx;
-  if (MODE != 2) {
-    const __nv_bfloat162* wm =
-        reinterpret_cast<const __nv_bfloat162*>(W) + (long)m * WD * WD;
-    for (int i = t; i < WD * WD; i += 256) ws[i] = __bfloat1622float2(wm[i]);
-  }
-  for (int i = t; i < B * WD; i += 256) {
-    const int b = i / WD, c = i % WD;
-    xs[i] = in[((long)b * nm + m) * WD + c];
-    if (MODE == 2) gs[i] = in2[((long)b * nm + m) * WD + c];
-  }
+  const __nv_bfloat162* wm =
+      reinterpret_cast<const __nv_bfloat162*>(W) + (long)m * WD * WD;
+  for (int i = t; i < WD * WD; i += 256) ws[i] = __bfloat1622float2(wm[i]);
+  for (int i = t; i < B * WD; i += 256)
+    xs[i] = in[((long)(i / WD) * nm + m) * WD + i % WD];
   __syncthreads();
-  if (MODE == 0 || MODE == 1) {
-    for (int b = ty; b < B; b += 8) {
-      float re = 0.f, im = 0.f;
+  for (int b = ty; b < B; b += 8) {
+    float re = 0.f, im = 0.f;
 #pragma unroll 8
-      for (int i = 0; i < WD; ++i) {
-        const float2 x = xs[b * WD + i];
-        if (MODE == 0) {
-          const float2 w = ws[i * WD + tx];
-          re += x.x * w.x - x.y * w.y;
-          im += x.x * w.y + x.y * w.x;
-        } else {
-          const float2 w = ws[tx * WD + i];  // conj(W[tx][i])
-          re += x.x * w.x + x.y * w.y;
-          im += x.y * w.x - x.x * w.y;
-        }
-      }
-      out[((long)b * nm + m) * WD + tx] = make_float2(re, im);
+    for (int i = 0; i < WD; ++i) {
+      const float2 x = xs[b * WD + i], w = ws[i * WD + tx];
+      re += x.x * w.x - x.y * w.y;
+      im += x.x * w.y + x.y * w.x;
     }
-  } else {
-    for (int i = ty; i < WD; i += 8) {
-      float re = 0.f, im = 0.f;
-      for (int b = 0; b < B; ++b) {
-        const float2 v = xs[b * WD + i], g = gs[b * WD + tx];
-        re += v.x * g.x + v.y * g.y;
-        im += v.x * g.y - v.y * g.x;
-      }
-      float* o = gW + 2 * (((long)m * WD + i) * WD + tx);
-      o[0] = re;
-      o[1] = im;
-    }
+    out[((long)b * nm + m) * WD + tx] = make_float2(re, im);
   }
 }
 
@@ -509,42 +478,6 @@ fno_dense_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w16, long offD
   }
 }
 
-// Dense layer, data gradient: dx = dy D^T (FP32 in/out).
-__global__ void __launch_bounds__(256)
-fno_dense_bwd_kernel(const float* dy, const __nv_bfloat16* w16, long offD,
-                     float* dx, long R) {
-  __shared__ float Ds[WD * WD];
-  for (int i = threadIdx.x; i < WD * WD; i += blockDim.x) Ds[i] = bf(w16[offD + i]);
-  __syncthreads();
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  float g[WD];
-  const float4* gp = reinterpret_cast<const float4*>(dy + r * WD);
-#pragma unroll
-  for (int q = 0; q < WD / 4; ++q) {
-    const float4 u = gp[q];
-    g[4 * q] = u.x; g[4 * q + 1] = u.y; g[4 * q + 2] = u.z; g[4 * q + 3] = u.w;
-  }
-  float4* op = reinterpret_cast<float4*>(dx + r * WD);
-#pragma unroll 2
-  for (int i = 0; i < WD; i += 4) {
-    float a[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int o = 0; o < WD; ++o) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) a[k] += g[o] * Ds[(i + k) * WD + o];
-    }
-    op[i / 4] = make_float4(a[0], a[1], a[2], a[3]);
-  }
-}
-
-// dy = dv * GELU'(y)
-__global__ void fno_gelu_bwd_kernel(const float* dv, const __nv_bfloat16* y,
-                                    float* dy, long total) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < total) dy[i] = dv[i] * gelu_d(bf(y[i]));
-}
-
 // ---------------------------------------------------------------------------
 // Projection, forward: out = sum_j q2[j] GELU(x Q1[:, j] + q1[j]) + q2b.
 // ---------------------------------------------------------------------------
@@ -585,127 +518,313 @@ fno_proj_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w16, Layout L,
   out[r] = acc;
 }
 
-// Projection, backward: dz = dout q2 GELU'(z), aw = dout GELU(z) (for dq2),
-// dx = dz Q1^T.
-__global__ void __launch_bounds__(256)
-fno_proj_bwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w16, Layout L,
-                    const float* dout, float* dz, float* aw, float* dx, long R) {
-  __shared__ float Qs[WD * PJ + 2 * PJ];
-  for (int i = threadIdx.x; i < WD * PJ; i += blockDim.x) Qs[i] = bf(w16[L.Q1 + i]);
-  for (int i = threadIdx.x; i < PJ; i += blockDim.x) {
-    Qs[WD * PJ + i] = bf(w16[L.q1 + i]);
-    Qs[WD * PJ + PJ + i] = bf(w16[L.q2 + i]);
-  }
-  __syncthreads();
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  float xi[WD], gx[WD];
-  const uint4* xp = reinterpret_cast<const uint4*>(x + r * WD);
-#pragma unroll
-  for (int q = 0; q < WD / 8; ++q) {
-    const uint4 u = xp[q];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 f = __bfloat1622float2(h[k]);
-      xi[q * 8 + 2 * k] = f.x;
-      xi[q * 8 + 2 * k + 1] = f.y;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < WD; ++i) gx[i] = 0.f;
-  const float go = dout[r];
-#pragma unroll 2
-  for (int j = 0; j < PJ; ++j) {
-    float z = Qs[WD * PJ + j];
-#pragma unroll
-    for (int i = 0; i < WD; ++i) z += xi[i] * Qs[i * PJ + j];
-    const float g = go * Qs[WD * PJ + PJ + j] * gelu_d(z);
-    dz[r * PJ + j] = g;
-    aw[r * PJ + j] = go * gelu(z);
-#pragma unroll
-    for (int i = 0; i < WD; ++i) gx[i] += g * Qs[i * PJ + j];
-  }
-  float4* op = reinterpret_cast<float4*>(dx + r * WD);
-#pragma unroll
-  for (int i = 0; i < WD; i += 4) op[i / 4] = make_float4(gx[i], gx[i + 1], gx[i + 2], gx[i + 3]);
+// ---------------------------------------------------------------------------
+// Backward of the pointwise parts.  The weight gradients are sums over every
+// grid point, so each persistent CTA keeps its share of them in registers over
+// all its tiles and writes one partial record; fno_reduce_kernel adds the
+// records in a fixed order (deterministic).  Nothing of width PJ reaches
+// global memory.
+//
+// Bound: FP32 FMAs and shared-memory reads, about equal.  Against separate
+// kernels for dz, its products and its column sums (which moved 2 x 4 B x PJ
+// per point through global memory twice) a step's projection backward went
+// from 2.0 to 0.5 ms on 24 samples at N=32, and the four layers' pointwise
+// parts from 2.5 to 0.6 ms.
+// ---------------------------------------------------------------------------
+constexpr int PBT = 64;                    // points per tile (projection)
+constexpr int PBX = WD + 4, PBZ = PJ + 4;  // row pitches (floats)
+constexpr int kProjPart = WD * PJ + 2 * PJ + 1;  // gQ1 | gq1 | gq2 | gq2b
+constexpr size_t kProjBwdSmem =
+    (size_t)(PBT * PBX + PJ * PBX + WD * PBZ + PBT * PBZ + 2 * PJ + PBT) * sizeof(float);
+
+__device__ __forceinline__ float4 bf4(uint2 u) {
+  const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.x));
+  const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// ---------------------------------------------------------------------------
-// Weight gradient G[i][j] = sum_r A[r][i] Bm[r][j] (A: BF16 [R][KA], Bm: FP32
-// [R][KB]).  Persistent CTAs over 64-row tiles; thread owns an RI x 4 block;
-// per-CTA partials [gridDim][KA][KB], summed by fno_reduce_kernel in a fixed
-// order (deterministic).
-// ---------------------------------------------------------------------------
-template <int KA, int KB>
-__global__ void fno_wgrad_kernel(const __nv_bfloat16* A, const float* Bm, long R,
-                                 float* partial) {
-  constexpr int RI = KA < 4 ? KA : 4;
-  constexpr int NTH = (KA / RI) * (KB / 4);
-  constexpr int TR = 64;
-  __shared__ __align__(16) float As[TR * KA];
-  __shared__ __align__(16) float Bs[TR * KB];
+// z = x Q1 + q1, dz = dout q2 GELU'(z), dx = dz Q1^T; gQ1 = x^T dz,
+// gq1 = sum dz, gq2 = sum dout GELU(z), gq2b = sum dout.
+__global__ void __launch_bounds__(256, 2)
+fno_proj_bwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w16, Layout L,
+                    const float* dout, float* dx, float* partial, long R) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* xs = reinterpret_cast<float*>(smem_raw);  // [PBT][PBX]
+  float* qt = xs + PBT * PBX;                      // Q1^T [PJ][PBX]
+  float* qs = qt + PJ * PBX;                       // Q1 [WD][PBZ]
+  float* zs = qs + WD * PBZ;                       // dz [PBT][PBZ]
+  float* b1 = zs + PBT * PBZ;                      // q1 [PJ]
+  float* b2 = b1 + PJ;                             // q2 [PJ]
+  float* go = b2 + PJ;                             // dout [PBT]
   const int t = threadIdx.x;
-  const int i0 = (t / (KB / 4)) * RI, j0 = (t % (KB / 4)) * 4;
-  float acc[RI][4];
-#pragma unroll
-  for (int a = 0; a < RI; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = 0.f;
-  for (long r0 = (long)blockIdx.x * TR; r0 < R; r0 += (long)gridDim.x * TR) {
-    const int nr = (int)min((long)TR, R - r0);
+  for (int i = t; i < WD * PJ; i += 256) {
+    const float w = bf(w16[L.Q1 + i]);
+    qt[(i % PJ) * PBX + i / PJ] = w;
+    qs[(i / PJ) * PBZ + i % PJ] = w;
+  }
+  for (int i = t; i < PJ; i += 256) {
+    b1[i] = bf(w16[L.q1 + i]);
+    b2[i] = bf(w16[L.q2 + i]);
+  }
+  const int lo = t % 16, pg = t / 16;      // column group; points 4 pg .. + 3
+  const int gi = (t / 32) * 4, gj = (t % 32) * 4;  // block of gQ1
+  float gw[4][4] = {}, gq1[8] = {}, gq2[8] = {}, gb = 0.f;
+  for (long r0 = (long)blockIdx.x * PBT; r0 < R; r0 += (long)gridDim.x * PBT) {
+    __syncthreads();                       // the previous tile is consumed
+    for (int i = t; i < PBT * WD / 4; i += 256) {
+      const long r = r0 + i / 8;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < R) v = bf4(*reinterpret_cast<const uint2*>(x + r * WD + (i % 8) * 4));
+      *reinterpret_cast<float4*>(xs + (i / 8) * PBX + (i % 8) * 4) = v;
+    }
+    if (t < PBT) {
+      go[t] = r0 + t < R ? dout[r0 + t] : 0.f;
+      gb += go[t];
+    }
     __syncthreads();
-    for (int k = t; k < TR * KA; k += NTH)
-      As[k] = (k / KA < nr) ? bf(A[r0 * KA + k]) : 0.f;
-    for (int k = t; k < TR * KB; k += NTH)
-      Bs[k] = (k / KB < nr) ? Bm[r0 * KB + k] : 0.f;
+    {
+      float z[4][8];
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const float v = b1[lo + 16 * b];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) z[a][b] = v;
+      }
+#pragma unroll 2
+      for (int k = 0; k < WD; k += 4) {
+        float4 xv[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          xv[a] = *reinterpret_cast<const float4*>(xs + (4 * pg + a) * PBX + k);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const float4 q = *reinterpret_cast<const float4*>(qt + (lo + 16 * b) * PBX + k);
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            z[a][b] += xv[a].x * q.x; z[a][b] += xv[a].y * q.y;
+            z[a][b] += xv[a].z * q.z; z[a][b] += xv[a].w * q.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float g = go[4 * pg + a];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const int j = lo + 16 * b;
+          const float d = g * b2[j] * gelu_d(z[a][b]);
+          zs[(4 * pg + a) * PBZ + j] = d;
+          gq1[b] += d;
+          gq2[b] += g * gelu(z[a][b]);
+        }
+      }
+    }
     __syncthreads();
+    {  // dx: points 4 pg + a, channels lo + 16 b
+      float d[4][2] = {};
 #pragma unroll 4
-    for (int r = 0; r < TR; ++r) {
-      float av[RI];
+      for (int j = 0; j < PJ; j += 4) {
+        float4 zv[4];
 #pragma unroll
-      for (int a = 0; a < RI; ++a) av[a] = As[r * KA + i0 + a];
-      const float4 bv = *reinterpret_cast<const float4*>(&Bs[r * KB + j0]);
+        for (int a = 0; a < 4; ++a)
+          zv[a] = *reinterpret_cast<const float4*>(zs + (4 * pg + a) * PBZ + j);
 #pragma unroll
-      for (int a = 0; a < RI; ++a) {
-        acc[a][0] += av[a] * bv.x; acc[a][1] += av[a] * bv.y;
-        acc[a][2] += av[a] * bv.z; acc[a][3] += av[a] * bv.w;
+        for (int b = 0; b < 2; ++b) {
+          const float4 q = *reinterpret_cast<const float4*>(qs + (lo + 16 * b) * PBZ + j);
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            d[a][b] += zv[a].x * q.x; d[a][b] += zv[a].y * q.y;
+            d[a][b] += zv[a].z * q.z; d[a][b] += zv[a].w * q.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        if (r0 + 4 * pg + a < R) {
+          dx[(r0 + 4 * pg + a) * WD + lo] = d[a][0];
+          dx[(r0 + 4 * pg + a) * WD + lo + 16] = d[a][1];
+        }
+    }
+#pragma unroll 4
+    for (int r = 0; r < PBT; ++r) {
+      const float4 a = *reinterpret_cast<const float4*>(xs + r * PBX + gi);
+      const float4 b = *reinterpret_cast<const float4*>(zs + r * PBZ + gj);
+      gw[0][0] += a.x * b.x; gw[0][1] += a.x * b.y; gw[0][2] += a.x * b.z; gw[0][3] += a.x * b.w;
+      gw[1][0] += a.y * b.x; gw[1][1] += a.y * b.y; gw[1][2] += a.y * b.z; gw[1][3] += a.y * b.w;
+      gw[2][0] += a.z * b.x; gw[2][1] += a.z * b.y; gw[2][2] += a.z * b.z; gw[2][3] += a.z * b.w;
+      gw[3][0] += a.w * b.x; gw[3][1] += a.w * b.y; gw[3][2] += a.w * b.z; gw[3][3] += a.w * b.w;
+    }
+  }
+  float* P = partial + (long)blockIdx.x * kProjPart;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) P[(gi + a) * PJ + gj + c] = gw[a][c];
+  // column sums: the 16 point groups of each column in order
+  __syncthreads();
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    zs[pg * PJ + lo + 16 * b] = gq1[b];
+    zs[(16 + pg) * PJ + lo + 16 * b] = gq2[b];
+  }
+  if (t < PBT) go[t] = gb;
+  __syncthreads();
+  {
+    const int j = t % PJ, which = t / PJ;
+    float v = 0.f;
+    for (int k = 0; k < 16; ++k) v += zs[(16 * which + k) * PJ + j];
+    P[WD * PJ + which * PJ + j] = v;
+  }
+  if (t == 0) {
+    float v = 0.f;
+    for (int k = 0; k < PBT; ++k) v += go[k];
+    P[WD * PJ + 2 * PJ] = v;
+  }
+}
+
+struct LayerBwdArgs {
+  const float* dy;          // [R][WD] gradient w.r.t. y_l
+  const float* U;           // [R][WD] spectral part of the gradient w.r.t. v_l
+  const __nv_bfloat16* w16;
+  long offD;                // D_l
+  const __nv_bfloat16* y;   // y_{l-1} (MODE 1)
+  const __nv_bfloat16* v;   // v_{l-1} (MODE 1), v_3 (MODE 0), x0 (MODE 2)
+  float* dyo;               // [R][WD] gradient w.r.t. y_{l-1} (MODE 1)
+  float* partial;           // [grid][KV * WD + WD]: weight | bias gradients
+  long R;
+};
+
+constexpr int LBT = 128;                 // points per tile
+constexpr int LBP = WD + 4;              // row pitch (floats)
+constexpr int kLayerPart = WD * WD + WD;
+constexpr size_t kLayerBwdSmem =
+    (size_t)(3 * LBT * LBP + WD * LBP) * sizeof(float);
+
+// MODE 0: gD = v^T dy, gd = sum dy (the last layer: y_3 = v_4).
+// MODE 1: dv_l = dy D_l^T + U, dy' = dv_l GELU'(y_{l-1}), gradients of layer
+//         l-1 from dy' and v_{l-1}.
+// MODE 2: dv_0 as in MODE 1, gradients of the lift from dv_0 and x0.
+template <int MODE>
+__global__ void __launch_bounds__(256) fno_layer_bwd_kernel(LayerBwdArgs a) {
+  constexpr int KV = MODE == 2 ? CIN : WD;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* dys = reinterpret_cast<float*>(smem_raw);  // [LBT][LBP] dy in
+  float* gs = dys + LBT * LBP;                      // [LBT][LBP] dv_l, then dy out
+  float* vs = gs + LBT * LBP;                       // [LBT][LBP] v
+  float* Ds = vs + LBT * LBP;                       // D_l [WD][LBP]
+  const int t = threadIdx.x;
+  if (MODE != 0)
+    for (int i = t; i < WD * WD; i += 256) Ds[(i / WD) * LBP + i % WD] = bf(a.w16[a.offD + i]);
+  const int ig = t % 8, pg = t / 8;               // channels ig + 8 b; points 4 pg + .
+  const int sl = t / 64, gi = ((t % 64) / 8) * 4, gj = (t % 8) * 4;  // weight block
+  float gw[4][4] = {}, gb[4] = {};
+  const float* G = MODE == 0 ? dys : gs;
+  for (long r0 = (long)blockIdx.x * LBT; r0 < a.R; r0 += (long)gridDim.x * LBT) {
+    __syncthreads();
+    for (int i = t; i < LBT * 8; i += 256) {
+      const long r = r0 + i / 8;
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f), v = d;
+      if (r < a.R) {
+        d = *reinterpret_cast<const float4*>(a.dy + r * WD + (i % 8) * 4);
+        if (MODE != 2) v = bf4(*reinterpret_cast<const uint2*>(a.v + r * WD + (i % 8) * 4));
+        else if (i % 8 == 0) v = bf4(*reinterpret_cast<const uint2*>(a.v + r * CIN));
+      }
+      *reinterpret_cast<float4*>(dys + (i / 8) * LBP + (i % 8) * 4) = d;
+      if (MODE != 2 || i % 8 == 0)
+        *reinterpret_cast<float4*>(vs + (i / 8) * LBP + (i % 8) * 4) = v;
+    }
+    __syncthreads();
+    if (MODE != 0) {
+      float d[4][4] = {};
+#pragma unroll 2
+      for (int o = 0; o < WD; o += 4) {
+        float4 yv[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+          yv[p] = *reinterpret_cast<const float4*>(dys + (4 * pg + p) * LBP + o);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float4 w = *reinterpret_cast<const float4*>(Ds + (ig + 8 * b) * LBP + o);
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            d[p][b] += yv[p].x * w.x; d[p][b] += yv[p].y * w.y;
+            d[p][b] += yv[p].z * w.z; d[p][b] += yv[p].w * w.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) gs[(4 * pg + p) * LBP + ig + 8 * b] = d[p][b];
+      __syncthreads();
+      for (int i = t; i < LBT * 8; i += 256) {
+        const long r = r0 + i / 8;
+        float4* g = reinterpret_cast<float4*>(gs + (i / 8) * LBP + (i % 8) * 4);
+        float4 d4 = *g;
+        if (r < a.R) {
+          const float4 u = *reinterpret_cast<const float4*>(a.U + r * WD + (i % 8) * 4);
+          d4.x += u.x; d4.y += u.y; d4.z += u.z; d4.w += u.w;
+          if (MODE == 1) {
+            const float4 y = bf4(*reinterpret_cast<const uint2*>(a.y + r * WD + (i % 8) * 4));
+            d4.x *= gelu_d(y.x); d4.y *= gelu_d(y.y);
+            d4.z *= gelu_d(y.z); d4.w *= gelu_d(y.w);
+            *reinterpret_cast<float4*>(a.dyo + r * WD + (i % 8) * 4) = d4;
+          }
+        }
+        *g = d4;       // rows past R hold zeros (dy = 0 there)
+      }
+      __syncthreads();
+    }
+    // weight block (gi, gj) over the points of slice sl
+    if (gi < KV) {
+#pragma unroll 4
+      for (int r = 32 * sl; r < 32 * sl + 32; ++r) {
+        const float4 v = *reinterpret_cast<const float4*>(vs + r * LBP + gi);
+        const float4 g = *reinterpret_cast<const float4*>(G + r * LBP + gj);
+        gw[0][0] += v.x * g.x; gw[0][1] += v.x * g.y; gw[0][2] += v.x * g.z; gw[0][3] += v.x * g.w;
+        gw[1][0] += v.y * g.x; gw[1][1] += v.y * g.y; gw[1][2] += v.y * g.z; gw[1][3] += v.y * g.w;
+        gw[2][0] += v.z * g.x; gw[2][1] += v.z * g.y; gw[2][2] += v.z * g.z; gw[2][3] += v.z * g.w;
+        gw[3][0] += v.w * g.x; gw[3][1] += v.w * g.y; gw[3][2] += v.w * g.z; gw[3][3] += v.w * g.w;
+        if (gi == 0) { gb[0] += g.x; gb[1] += g.y; gb[2] += g.z; gb[3] += g.w; }
       }
     }
   }
-  float* P = partial + (long)blockIdx.x * KA * KB;
-#pragma unroll
-  for (int a = 0; a < RI; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) P[(i0 + a) * KB + j0 + c] = acc[a][c];
-}
-
-// Column sums S[j] = sum_r Bm[r][j] (bias gradients); partials per CTA.
-template <int KB>
-__global__ void __launch_bounds__(256)
-fno_colsum_kernel(const float* Bm, long R, float* partial) {
-  constexpr int RPT = 256 / KB;  // rows per pass
-  __shared__ float red[256];
-  const int t = threadIdx.x, j = t % KB, rr = t / KB;
-  float s = 0.f;
-  for (long r = (long)blockIdx.x * RPT + rr; r < R; r += (long)gridDim.x * RPT)
-    s += Bm[r * KB + j];
-  red[t] = s;
+  // the four slices of each block in order
   __syncthreads();
-  if (t < KB) {
+  float* red = dys;   // [4][KV * WD + WD] fits the three tiles
+  if (gi < KV) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) red[sl * (KV * WD + WD) + (gi + p) * WD + gj + c] = gw[p][c];
+    if (gi == 0)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) red[sl * (KV * WD + WD) + KV * WD + gj + c] = gb[c];
+  }
+  __syncthreads();
+  for (int i = t; i < KV * WD + WD; i += 256) {
     float v = 0.f;
-    for (int k = 0; k < RPT; ++k) v += red[k * KB + t];
-    partial[(long)blockIdx.x * KB + t] = v;
+    for (int k = 0; k < 4; ++k) v += red[k * (KV * WD + WD) + i];
+    a.partial[(long)blockIdx.x * (KV * WD + WD) + i] = v;
   }
 }
 
-// out[i] = sum_g partial[g][i] (fixed order)
-__global__ void fno_reduce_kernel(const float* partial, int G, int n, float* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int g = 0; g < G; ++g) s += partial[(long)g * n + i];
-  out[i] = s;
+// out[i] = sum_g partial[g][i]: 32 outputs per CTA, eight strided slices of g
+// per output, added in a fixed order.
+__global__ void __launch_bounds__(256)
+fno_reduce_kernel(const float* partial, int G, int n, float* out) {
+  __shared__ float red[8][33];
+  const int c = threadIdx.x % 32, s = threadIdx.x / 32, i = blockIdx.x * 32 + c;
+  float v = 0.f;
+  if (i < n)
+#pragma unroll 8
+    for (int g = s; g < G; g += 8) v += partial[(long)g * n + i];
+  red[s][c] = v;
+  __syncthreads();
+  if (s == 0 && i < n) {
+    for (int k = 1; k < 8; ++k) v += red[k][c];
+    out[i] = v;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1042,7 +1161,7 @@ __host__ __device__ constexpr int fbin(int kk) {
 template <int N, int K>
 __global__ void __launch_bounds__(K * 32)
 fno_xmix_kernel(const float2* __restrict__ Y, const __nv_bfloat16* __restrict__ W,
-                float2* __restrict__ S, int B) {
+                float2* __restrict__ S, float2* __restrict__ Vh, int B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* Vs = reinterpret_cast<float2*>(smem_raw);  // [K samples][K][WD]
   float2* Us = Vs + K * K * WD;                       // [K samples][K][WD]
@@ -1058,6 +1177,10 @@ fno_xmix_kernel(const float2* __restrict__ Y, const __nv_bfloat16* __restrict__ 
     fft<float, N, -1>(v);
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) Vs[(w * K + kk) * WD + lane] = v[fbin<N, K>(kk)];
+    if (Vh)  // training: the full spectrum, for the weight gradient
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk)
+        Vh[(((long)(b0 + w) * K + kk) * K * K + kyz) * WD + lane] = v[fbin<N, K>(kk)];
   }
   __syncthreads();
   {  // mix: thread (kx = w, o = lane) with the column W[m][.][o] in registers,
@@ -1105,15 +1228,24 @@ fno_xmix_kernel(const float2* __restrict__ Y, const __nv_bfloat16* __restrict__ 
   }
 }
 
-// yz spectra of one (b, x) plane of a BF16 field [B][N][N][N][WD].
-template <int N, int K>
+// Two adjacent channels of a BF16 or FP32 field.
+__device__ __forceinline__ float2 chan2(const __nv_bfloat16* p) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+}
+__device__ __forceinline__ float2 chan2(const float* p) {
+  return *reinterpret_cast<const float2*>(p);
+}
+
+// yz spectra of one (b, x) plane of a BF16 (activations) or FP32 (gradients)
+// field [B][N][N][N][WD].
+template <int N, int K, typename TV>
 __global__ void __launch_bounds__(256)
-fno_yzfwd_kernel(const __nv_bfloat16* __restrict__ v, float2* __restrict__ Y) {
+fno_yzfwd_kernel(const TV* __restrict__ v, float2* __restrict__ Y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* T2 = reinterpret_cast<float2*>(smem_raw);  // [N y][K kz][WD]
   const int x = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
   const long plane = (long)b * N + x;
-  const __nv_bfloat16* vp = v + plane * N * N * WD;
+  const TV* vp = v + plane * N * N * WD;
   // z pass: pencil (y, channel pair cp); the two channels are the real and
   // imaginary parts of one FFT, separated by Hermitian symmetry
   for (int p = t; p < N * (WD / 2); p += 256) {
@@ -1121,8 +1253,7 @@ fno_yzfwd_kernel(const __nv_bfloat16* __restrict__ v, float2* __restrict__ Y) {
     float2 c[N];
 #pragma unroll
     for (int z = 0; z < N; ++z)
-      c[z] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(
-          vp + ((long)y * N + z) * WD + 2 * cp));
+      c[z] = chan2(vp + ((long)y * N + z) * WD + 2 * cp);
     fft<float, N, -1>(c);
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
@@ -1154,6 +1285,7 @@ struct YzInvArgs {
   const __nv_bfloat16* w16;  // BF16 parameters
   long offD, offd;           // D_l [WD][WD], d_l [WD]
   __nv_bfloat16* vout;       // v_{l+1} [B][N^3][WD]
+  __nv_bfloat16* y;          // pre-activation out (training; may be null)
   int act;                   // GELU (layers 0..2) or identity (last layer)
   int* err;                  // device error flag
 };
@@ -1181,8 +1313,7 @@ struct YzInvGeo {
 // kz -> z inverse of one (ky, channel) pencil, keeping the slab's z values.
 template <int N, int K, int Z0, int NZ>
 __device__ __forceinline__ void yzinv_zpass(const float2* src, float2* T, int ky,
-                                            int ch) {
-  constexpr float inv = 1.f / N;
+                                            int ch, float inv) {
   float2 c[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) c[j] = make_float2(0.f, 0.f);
@@ -1192,6 +1323,24 @@ __device__ __forceinline__ void yzinv_zpass(const float2* src, float2* T, int ky
 #pragma unroll
   for (int zl = 0; zl < NZ; ++zl)
     T[(ky * NZ + zl) * WD + ch] = make_float2(c[Z0 + zl].x * inv, c[Z0 + zl].y * inv);
+}
+
+// Spectrum along y of two real pencils as one complex one: with sym(a)(k) =
+// (a(k) + conj a(-k))/2, c = sym(a) + i sym(b), so that IFFT(c) = Re IFFT(a) +
+// i Re IFFT(b).  src: the two channels' values at ky = 0, `pitch` apart per ky.
+template <int N, int K>
+__device__ __forceinline__ void yzinv_sym(const float2* src, int pitch, float2* c) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) c[j] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int ky = 0; ky < K; ++ky) {
+    const float4 ab = *reinterpret_cast<const float4*>(src + ky * pitch);
+    const int k = fbin<N, K>(ky), nk = (N - k) % N;
+    c[k].x += 0.5f * (ab.x - ab.w);
+    c[k].y += 0.5f * (ab.y + ab.z);
+    c[nk].x += 0.5f * (ab.x + ab.w);
+    c[nk].y += 0.5f * (ab.z - ab.y);
+  }
 }
 
 // Grid (N ZP, B): blockIdx.x = x ZP + slab.  The rows' BF16 activations load
@@ -1250,8 +1399,8 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
   for (int p = t; p < K * WD; p += NT) {
     const int ky = p / WD, ch = p % WD;
     const float2* src = a.S + (plane * K + ky) * K * WD + ch;
-    if (zh == 0) yzinv_zpass<N, K, 0, NZ>(src, T, ky, ch);
-    else yzinv_zpass<N, K, NZ, NZ>(src, T, ky, ch);
+    if (zh == 0) yzinv_zpass<N, K, 0, NZ>(src, T, ky, ch, 1.f / N);
+    else yzinv_zpass<N, K, NZ, NZ>(src, T, ky, ch, 1.f / N);
   }
   cp_async_wait_all();
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -1293,24 +1442,13 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
   __syncthreads();
   const bool ok = *abort_flag == 0;
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  // ky -> y, real part: pencil (zl, channel pair); c = sym(a) + i sym(b) with
-  // sym(a)(k) = (a(k) + conj a(-k))/2, so that IFFT(c) = Re IFFT(a) + i Re IFFT(b)
+  // ky -> y, real part: pencil (zl, channel pair)
   if (ok) {
     constexpr float inv = 1.f / N;
     for (int p = t; p < NZ * (WD / 2); p += NT) {
       const int zl = p / (WD / 2), cp = p % (WD / 2);
       float2 c[N];
-#pragma unroll
-      for (int j = 0; j < N; ++j) c[j] = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int ky = 0; ky < K; ++ky) {
-        const float4 ab = *reinterpret_cast<const float4*>(T + (ky * NZ + zl) * WD + 2 * cp);
-        const int k = fbin<N, K>(ky), nk = (N - k) % N;
-        c[k].x += 0.5f * (ab.x - ab.w);
-        c[k].y += 0.5f * (ab.y + ab.z);
-        c[nk].x += 0.5f * (ab.x + ab.w);
-        c[nk].y += 0.5f * (ab.z - ab.y);
-      }
+      yzinv_sym<N, K>(T + zl * WD + 2 * cp, NZ * WD, c);
       fft<float, N, +1>(c);
 #pragma unroll
       for (int y = 0; y < N; ++y)
@@ -1339,7 +1477,7 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
           : "r"(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(tile * WD)));
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
       const uint4* Ur = reinterpret_cast<const uint4*>(Us + (long)r * WD);
-      uint4 vo[4];
+      uint4 vo[4], yo[4];
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) {
         const uint4 u = Ur[c4];
@@ -1352,6 +1490,7 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
           const __nv_bfloat162 yy = __floats2bfloat162_rn(
               __uint_as_float(rg[j]) + ep[j] + uf.x,
               __uint_as_float(rg[j + 1]) + ep[j + 1] + uf.y);
+          reinterpret_cast<__nv_bfloat162*>(&yo[c4])[h] = yy;
           if (a.act) {
             const float2 yf = __bfloat1622float2(yy);
             o2[h] = __floats2bfloat162_rn(gelu(yf.x), gelu(yf.y));
@@ -1363,6 +1502,11 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
       uint4* vd = reinterpret_cast<uint4*>(a.vout + (plane * N * N + pt) * WD);
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) vd[c4] = vo[c4];
+      if (a.y) {
+        uint4* yd = reinterpret_cast<uint4*>(a.y + (plane * N * N + pt) * WD);
+#pragma unroll
+        for (int c4 = 0; c4 < 4; ++c4) yd[c4] = yo[c4];
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1371,6 +1515,136 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n"
                  ::"r"(tmem), "r"(G::NCOL));
   if (!ok && t == 0) atomicExch(a.err, 1);
+}
+
+// ---------------------------------------------------------------------------
+// Backward of the spectral part, from the yz spectra Y of dy (fno_yzfwd):
+//   g = x transform of Y / N^3 (adjoint of the inverse transform),
+//   gW[m][i][o] = sum_b conj(Vh[b][m][i]) g[b][m][o],
+//   S = inverse x transform of gV[b][m][i] = sum_o g[b][m][o] conj(W[m][i][o]).
+// Grid K*K (blockIdx.x = ky K + kz), one warp per kx; the samples pass in
+// chunks of K, and a lane keeps its column gW[m][.][o] in registers over all
+// of them.  Bound: reading Y and Vh and writing gW and S once (about 0.5 GB
+// per step of 24 samples at N=32).
+// ---------------------------------------------------------------------------
+template <int N, int K>
+__global__ void __launch_bounds__(K * 32)
+fno_xmix_bwd_kernel(const float2* __restrict__ Y, const float2* __restrict__ Vh,
+                    const __nv_bfloat16* __restrict__ W, float2* __restrict__ S,
+                    float2* __restrict__ gW, int B) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* Gs = reinterpret_cast<float2*>(smem_raw);  // [K samples][K][WD] g
+  float2* Vs = Gs + K * K * WD;                       // the same of Vh, then gV
+  const int kyz = blockIdx.x, ky = kyz / K, kz = kyz % K;
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const long xs = (long)K * K * WD;
+  const long m = ((long)w * K + ky) * K + kz;
+  constexpr float scale = 1.f / ((float)N * N * N);
+  float2 gw[WD];
+#pragma unroll
+  for (int i = 0; i < WD; ++i) gw[i] = make_float2(0.f, 0.f);
+  for (int b0 = 0; b0 < B; b0 += K) {
+    const int nb = min(K, B - b0);
+    __syncthreads();
+    if (w < nb) {
+      const float2* src = Y + ((long)(b0 + w) * N * K * K + kyz) * WD + lane;
+      float2 v[N];
+#pragma unroll
+      for (int x = 0; x < N; ++x) v[x] = src[x * xs];
+      fft<float, N, -1>(v);
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk) {
+        const float2 c = v[fbin<N, K>(kk)];
+        Gs[(w * K + kk) * WD + lane] = make_float2(c.x * scale, c.y * scale);
+        Vs[(w * K + kk) * WD + lane] =
+            Vh[(((long)(b0 + w) * K + kk) * K * K + kyz) * WD + lane];
+      }
+    }
+    __syncthreads();
+    for (int s = 0; s < nb; ++s) {       // weight gradient: o = lane
+      const float2 g = Gs[(s * K + w) * WD + lane];
+      const float4* vr = reinterpret_cast<const float4*>(Vs + (s * K + w) * WD);
+#pragma unroll
+      for (int q = 0; q < WD / 2; ++q) {
+        const float4 c = vr[q];
+        gw[2 * q].x += c.x * g.x; gw[2 * q].x += c.y * g.y;
+        gw[2 * q].y += c.x * g.y; gw[2 * q].y -= c.y * g.x;
+        gw[2 * q + 1].x += c.z * g.x; gw[2 * q + 1].x += c.w * g.y;
+        gw[2 * q + 1].y += c.z * g.y; gw[2 * q + 1].y -= c.w * g.x;
+      }
+    }
+    __syncthreads();                     // Vs is consumed
+    {                                    // data gradient: i = lane
+      float2 wr[WD];
+      const uint4* wm = reinterpret_cast<const uint4*>(
+          reinterpret_cast<const __nv_bfloat162*>(W) + (m * WD + lane) * WD);
+#pragma unroll
+      for (int q = 0; q < WD / 4; ++q) {
+        const uint4 u = wm[q];
+        wr[4 * q] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.x));
+        wr[4 * q + 1] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.y));
+        wr[4 * q + 2] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.z));
+        wr[4 * q + 3] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.w));
+      }
+      for (int s = 0; s < nb; ++s) {
+        const float4* gr = reinterpret_cast<const float4*>(Gs + (s * K + w) * WD);
+        float re = 0.f, im = 0.f;
+#pragma unroll
+        for (int q = 0; q < WD / 2; ++q) {
+          const float4 g = gr[q];
+          re += g.x * wr[2 * q].x; re += g.y * wr[2 * q].y;
+          im += g.y * wr[2 * q].x; im -= g.x * wr[2 * q].y;
+          re += g.z * wr[2 * q + 1].x; re += g.w * wr[2 * q + 1].y;
+          im += g.w * wr[2 * q + 1].x; im -= g.z * wr[2 * q + 1].y;
+        }
+        Vs[(s * K + w) * WD + lane] = make_float2(re, im);
+      }
+    }
+    __syncthreads();
+    if (w < nb) {
+      float2 v[N];
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk) v[fbin<N, K>(kk)] = Vs[(w * K + kk) * WD + lane];
+      fft<float, N, +1>(v);
+      float2* dst = S + ((long)(b0 + w) * N * K * K + kyz) * WD + lane;
+#pragma unroll
+      for (int x = 0; x < N; ++x) dst[x * xs] = v[x];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < WD; ++i) gW[(m * WD + i) * WD + lane] = gw[i];
+}
+
+// U = Re of the (unscaled) yz inverse of S, FP32, one z-slab of a (b, x) plane
+// per CTA as in fno_yzinv_dense_kernel.
+template <int N, int K>
+__global__ void __launch_bounds__(256, 2)
+fno_yzinv_bwd_kernel(const float2* __restrict__ S, float* __restrict__ U) {
+  using G = YzInvGeo<N, K>;
+  constexpr int NZ = G::NZ;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* T = reinterpret_cast<float2*>(smem_raw);  // [K][NZ][WD]
+  const int x = blockIdx.x / G::ZP, zh = blockIdx.x % G::ZP, z0 = zh * NZ;
+  const int b = blockIdx.y, t = threadIdx.x;
+  const long plane = (long)b * N + x;
+  for (int p = t; p < K * WD; p += 256) {
+    const int ky = p / WD, ch = p % WD;
+    const float2* src = S + (plane * K + ky) * K * WD + ch;
+    if (zh == 0) yzinv_zpass<N, K, 0, NZ>(src, T, ky, ch, 1.f);
+    else yzinv_zpass<N, K, NZ, NZ>(src, T, ky, ch, 1.f);
+  }
+  __syncthreads();
+  for (int p = t; p < NZ * (WD / 2); p += 256) {
+    const int zl = p / (WD / 2), cp = p % (WD / 2);
+    float2 c[N];
+    yzinv_sym<N, K>(T + zl * WD + 2 * cp, NZ * WD, c);
+    fft<float, N, +1>(c);
+    float* dst = U + (plane * N * N + z0 + zl) * WD + 2 * cp;
+#pragma unroll
+    for (int y = 0; y < N; ++y) *reinterpret_cast<float2*>(dst + (long)y * N * WD) = c[y];
+  }
 }
 
 // Adam on the FP32 master parameters; refreshes the BF16 copy.
