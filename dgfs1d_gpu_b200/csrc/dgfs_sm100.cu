@@ -1414,66 +1414,68 @@ struct dgfs_vss_s {
   int precision = DGFS_PREC_FP64;
   double* w = nullptr;     // [Nrho] w_r s_w / n
   VssPair pair[16];
-  double2* F[2] = {nullptr, nullptr};  // [E][n] spectra of the two inputs
-  // FP32 mode scratch (Maxwellian split): per input slot s (the two inputs
-  // of a pair, or every species of dgfs_vss_eval_species) F_g, spectra and
-  // moments; per partner q of a species (slice q) the loss, tables, FP64
-  // Maxwellian gain and the FP32 terms
+  // direction lists: every direction, and (for a species with itself) one of
+  // each antipodal pair with its antipode
+  int2 *dirs = nullptr, *dirsm = nullptr;
+  int nd = 0, ndm = 0;
+  // scratch.  Per input slot s (the two inputs of a pair, or every species of
+  // dgfs_vss_eval_species): F (FP32 mode: F_g) and its Nyquist planes, and in
+  // the FP32 mode the Maxwellian spectra and moments; per partner (slice) the
+  // loss, the plane transforms, in the FP32 mode the tables and the FP64
+  // Maxwellian gain; the terms' spectra H
   double* c0 = nullptr;                // [N]
-  double* b2dummy = nullptr;           // [n] unused real loss kernel
-  float2* Fg[4] = {};                  // [E][n]
+  void* F[4] = {};                     // [E][n] complex R
+  void* Fny[4] = {};                   // [E][3][N][N] complex R
   double2* mhat[4] = {};               // [E][3][N]
   double* mom[4] = {};                 // [E][5]
   double* ReLf = nullptr;              // [nspcs][E][n]
+  void* rho = nullptr;                 // [nspcs][E][T][3][N][N] complex R
   float2* uv = nullptr;                // [nspcs][E][T][2][3][N]
   double2* hh = nullptr;               // [nspcs][E][T][3][N]
   double2* GM = nullptr;               // [nspcs][E][n]
-  float2* H = nullptr;                 // [nspcs][E][Nrho][n]
+  void* H = nullptr;                   // [hslots][n] complex R
+  size_t hslots = 0;                   // spectra of one evaluation: pairs x
+                                       // points x radial slices
   double cw = 0;
-  // the FP64 Maxwellian gain of dgfs_vss_eval_species runs on `aux` (low
-  // priority) beside the FP32 terms kernel
+  // the FP64 Maxwellian gain of the FP32 mode runs on `aux` (low priority)
+  // beside the terms kernel
   cudaStream_t aux = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 static void free_vss(dgfs_vss_s* h) {
-  for (auto& p : h->pair) {
-    if (p.b) cudaFree(p.b);
-    if (p.c) cudaFree(p.c);
-    if (p.ph) cudaFree(p.ph);
-    if (p.b32) cudaFree(p.b32);
-    if (p.ph32) cudaFree(p.ph32);
-  }
-  void* ptrs[] = {h->w, h->F[0], h->F[1], h->c0, h->b2dummy, h->ReLf, h->uv,
-                  h->hh, h->GM, h->H};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
-  for (int s = 0; s < 4; ++s)
-    for (void* q : {(void*)h->Fg[s], (void*)h->mhat[s], (void*)h->mom[s]})
+  for (auto& p : h->pair)
+    for (void* q : {(void*)p.b, (void*)p.c, (void*)p.ph, (void*)p.b32, (void*)p.ph32})
       if (q) cudaFree(q);
+  for (int i = 0; i < 4; ++i)
+    for (void* q : {h->F[i], h->Fny[i], (void*)h->mhat[i], (void*)h->mom[i]})
+      if (q) cudaFree(q);
+  for (void* q : {(void*)h->w, (void*)h->dirs, (void*)h->dirsm, (void*)h->c0,
+                  (void*)h->ReLf, h->rho, (void*)h->uv, (void*)h->hh, (void*)h->GM, h->H})
+    if (q) cudaFree(q);
   if (h->fork) cudaEventDestroy(h->fork);
   if (h->join) cudaEventDestroy(h->join);
   if (h->aux) cudaStreamDestroy(h->aux);
   delete h;
 }
 
-// FP32 copies of a pair's weights and phases
 __global__ void vss_to_fp32_kernel(const double2* in, float2* out, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = make_float2((float)in[i].x, (float)in[i].y);
 }
 
+// cluster sizes of the terms kernel (vss_terms_kernel), FP64 and FP32
 template <int N> struct VssClusters;
-template <> struct VssClusters<8> { static constexpr int c = 1; };
-template <> struct VssClusters<16> { static constexpr int c = 2; };
-template <> struct VssClusters<24> { static constexpr int c = 6; };
-template <> struct VssClusters<32> { static constexpr int c = 16; };
-// FP32 terms kernel: five FP32 slabs per CTA
-template <int N> struct VssClusters32;
-template <> struct VssClusters32<8> { static constexpr int c = 1; };
-template <> struct VssClusters32<16> { static constexpr int c = 2; };
-template <> struct VssClusters32<24> { static constexpr int c = 3; };
-template <> struct VssClusters32<32> { static constexpr int c = 8; };
+template <> struct VssClusters<8> { static constexpr int c64 = 1, c32 = 1; };
+template <> struct VssClusters<16> { static constexpr int c64 = 2, c32 = 2; };
+#ifndef VC64
+#define VC64 6
+#endif
+#ifndef VC32
+#define VC32 6
+#endif
+template <> struct VssClusters<24> { static constexpr int c64 = VC64, c32 = VC32; };
+template <> struct VssClusters<32> { static constexpr int c64 = 16, c32 = 8; };
 
 template <int N>
 static int vss_setup_pair(dgfs_vss_s* h, const dgfs_vss_desc* d, int p, int q,
@@ -1568,51 +1570,78 @@ extern "C" int dgfs_vss_create(const dgfs_vss_desc* d, dgfs_vss_handle* out) {
         default: rc = vss_setup_pair<32>(h, d, p, q, 0); break;
       }
     }
-  if (!rc) {
-    cudaError_t e1 = cudaMalloc(&h->F[0], sizeof(double2) * (size_t)h->max_evals * h->n);
-    if (e1 == cudaSuccess)
-      e1 = cudaMalloc(&h->F[1], sizeof(double2) * (size_t)h->max_evals * h->n);
-    if (e1 != cudaSuccess)
-      rc = fail(DGFS_ERR_CUDA, std::string("allocation: ") + cudaGetErrorString(e1));
+  // direction lists
+  std::vector<int2> dirs(d->M), dirsm;
+  std::vector<char> used(d->M, 0);
+  for (int m = 0; m < d->M; ++m) dirs[m] = make_int2(m, -1);
+  for (int m = 0; m < d->M; ++m) {
+    if (used[m]) continue;
+    int anti = -1;
+    for (int q = m + 1; q < d->M && anti < 0; ++q)
+      if (!used[q] && d->sz[3 * q] == -d->sz[3 * m] &&
+          d->sz[3 * q + 1] == -d->sz[3 * m + 1] && d->sz[3 * q + 2] == -d->sz[3 * m + 2])
+        anti = q;
+    if (anti >= 0) used[anti] = 1;
+    dirsm.push_back(make_int2(m, anti));
   }
-  if (!rc && h->precision == DGFS_PREC_FP32) {
+  h->nd = d->M; h->ndm = (int)dirsm.size();
+  if (!rc) rc = upload(&h->dirs, dirs);
+  if (!rc) rc = upload(&h->dirsm, dirsm);
+  const bool fp32 = h->precision == DGFS_PREC_FP32;
+  if (!rc) {
     const size_t E = h->max_evals, n = h->n, N = h->N, T = (size_t)h->Nrho * h->M;
+    const size_t ns = h->nspcs, ce = fp32 ? sizeof(float2) : sizeof(double2);
     cudaError_t e1 = cudaSuccess;
-    auto A = [&](auto** q, size_t cnt) {
-      if (e1 == cudaSuccess) e1 = cudaMalloc((void**)q, cnt * sizeof(**q));
+    auto A = [&](auto** q, size_t bytes) {
+      if (e1 == cudaSuccess) e1 = cudaMalloc((void**)q, bytes);
     };
-    const size_t ns = h->nspcs;
     for (int s2 = 0; s2 < std::max(2, h->nspcs); ++s2) {
-      A(&h->Fg[s2], E * n); A(&h->mhat[s2], E * 3 * N); A(&h->mom[s2], E * 5);
-    }
-    A(&h->ReLf, ns * E * n); A(&h->uv, ns * E * T * 6 * N);
-    A(&h->hh, ns * E * T * 3 * N); A(&h->GM, ns * E * n);
-    A(&h->H, ns * E * h->Nrho * n); A(&h->b2dummy, n);
-    if (e1 == cudaSuccess) {
-      int lo = 0, hi = 0;
-      e1 = cudaDeviceGetStreamPriorityRange(&lo, &hi);
-      if (e1 == cudaSuccess)
-        e1 = cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, lo);
-      if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
-      if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming);
-    }
-    for (int pq = 0; pq < h->nspcs * h->nspcs; ++pq) {
-      A(&h->pair[pq].b32, T * n); A(&h->pair[pq].ph32, T * 6 * N);
-    }
-    if (e1 == cudaSuccess) {
-      for (int pq = 0; pq < h->nspcs * h->nspcs; ++pq) {
-        vss_to_fp32_kernel<<<(unsigned)((T * n + 255) / 256), 256>>>(
-            h->pair[pq].b, h->pair[pq].b32, T * n);
-        vss_to_fp32_kernel<<<(unsigned)((T * 6 * N + 255) / 256), 256>>>(
-            h->pair[pq].ph, h->pair[pq].ph32, T * 6 * N);
+      A(&h->F[s2], E * n * ce);
+      A(&h->Fny[s2], E * 3 * N * N * ce);
+      if (fp32) {
+        A(&h->mhat[s2], E * 3 * N * sizeof(double2));
+        A(&h->mom[s2], E * 5 * sizeof(double));
       }
-      e1 = cudaDeviceSynchronize();
+    }
+    A(&h->ReLf, ns * E * n * sizeof(double));
+    A(&h->rho, ns * E * T * 3 * N * N * ce);
+    // FP32: one spectrum per pair, point and radial point (their sum is FP64,
+    // in the epilogue); FP64: as many radial slices as give 256 clusters, so
+    // that a few points fill the GPU and many do not need one per radial point
+    h->hslots = fp32 ? ns * E * h->Nrho
+                     : std::max(ns * E, std::min<size_t>(ns * E * h->Nrho, 256));
+    A(&h->H, h->hslots * n * ce);
+    if (fp32) {
+      A(&h->uv, ns * E * T * 6 * N * sizeof(float2));
+      A(&h->hh, ns * E * T * 3 * N * sizeof(double2));
+      A(&h->GM, ns * E * n * sizeof(double2));
+      if (e1 == cudaSuccess) {
+        int lo = 0, hi = 0;
+        e1 = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+        if (e1 == cudaSuccess)
+          e1 = cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, lo);
+        if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
+        if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming);
+      }
+      for (int pq = 0; pq < h->nspcs * h->nspcs; ++pq) {
+        A(&h->pair[pq].b32, T * n * sizeof(float2));
+        A(&h->pair[pq].ph32, T * 6 * N * sizeof(float2));
+      }
+      if (e1 == cudaSuccess) {
+        for (int pq = 0; pq < h->nspcs * h->nspcs; ++pq) {
+          vss_to_fp32_kernel<<<(unsigned)((T * n + 255) / 256), 256>>>(
+              h->pair[pq].b, h->pair[pq].b32, T * n);
+          vss_to_fp32_kernel<<<(unsigned)((T * 6 * N + 255) / 256), 256>>>(
+              h->pair[pq].ph, h->pair[pq].ph32, T * 6 * N);
+        }
+        e1 = cudaDeviceSynchronize();
+      }
     }
     std::vector<double> c0(N);
     for (size_t i = 0; i < N; ++i) c0[i] = -d->L + d->L / N + i * (2.0 * d->L / N);
     h->cw = std::pow(2.0 * d->L / N, 3);
     if (e1 == cudaSuccess) rc = upload(&h->c0, c0);
-    else rc = fail(DGFS_ERR_CUDA, std::string("FP32 scratch: ") + cudaGetErrorString(e1));
+    else rc = fail(DGFS_ERR_CUDA, std::string("scratch allocation: ") + cudaGetErrorString(e1));
   }
   if (rc) { free_vss(h); return rc; }
   if (int rc_s = settle_uploads()) { free_vss(h); return rc_s; }
@@ -1625,174 +1654,153 @@ extern "C" int dgfs_vss_destroy(dgfs_vss_handle h) {
   return DGFS_OK;
 }
 
-template <int N>
-static int vss_run(dgfs_vss_s* h, int p, int q, const void* fp, const void* fq,
-                   int f_double, void* Q, int q_double, const int32_t* ss,
-                   int sb, const int32_t* ds, int db, int nevals,
-                   cudaStream_t st) {
-  constexpr int C = VssClusters<N>::c;
-  using G = Geo<N, C>;
-  int rc;
-  const VssPair& P = h->pair[p * h->nspcs + q];
-  if (h->precision == DGFS_PREC_FP32) {
-    constexpr int CPRO = VhsClusters<N>::cpro;
-    constexpr int CEPI = VhsClusters<N>::cepi;
-    constexpr int C3 = VssClusters32<N>::c;
-    using GPRO = Geo<N, CPRO>;
-    using GEPI = Geo<N, CEPI>;
-    using G3 = Geo<N, C3>;
-    const int T = h->Nrho * h->M;
-    // prologues: F_g, Maxwellian spectra of f_p and f_q; the f_q pass also
-    // leaves the loss Re IFFT(c G) (complex loss kernel)
-    for (int s2 = 0; s2 < 2; ++s2) {
-      VhsPrologueArgs a{};
-      a.f = s2 == 0 ? fp : fq; a.f_double = f_double; a.src_slots = ss; a.src_base = sb;
-      a.c0 = h->c0; a.b2 = h->b2dummy; a.b2c = P.c; a.cw = h->cw; a.split = 1;
-      a.Fg = h->Fg[s2]; a.ReLf = h->ReLf; a.mhat = h->mhat[s2]; a.moments = h->mom[s2];
-      a.Fny = nullptr;
-      const size_t smem = prologue_smem<N, CPRO>();
-      if ((rc = launch_cluster(vhs_prologue_kernel<N, CPRO>, dim3(CPRO, nevals),
-                               dim3(GPRO::NT), CPRO, smem, st, a)))
-        return rc;
-    }
-    VssTablesArgs ta{};
-    ta.mhat_p = h->mhat[0]; ta.mhat_q = h->mhat[1]; ta.ph = P.ph; ta.uv = h->uv;
-    ta.hh = h->hh; ta.T = T; ta.nevals = nevals;
-    if ((rc = launch_plain(vss_tables_kernel<N>, dim3((nevals * T * 3 + 127) / 128),
-                           dim3(128), 0, st, ta)))
-      return rc;
-    VssGainArgs ga{};
-    ga.hh = h->hh; ga.b = P.b; ga.w = h->w; ga.GM = h->GM; ga.Nrho = h->Nrho; ga.M = h->M;
-    if ((rc = launch_plain(vss_maxwell_gain_kernel<N>,
-                           dim3((h->n + 255) / 256, nevals), dim3(256), 0, st, ga)))
-      return rc;
-    VssTerms32Args tt{};
-    tt.pr[0] = {h->Fg[0], h->Fg[1], P.ph32, h->uv, P.b32, h->H};
-    tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals;
-    const size_t smem3 = 5 * slab_bytes(N, C3, sizeof(float2)) + 24 * N * sizeof(float2);
-    if ((rc = launch_cluster(vss_terms32_kernel<N, C3>, dim3(C3, h->Nrho, nevals),
-                             dim3(G3::NT), C3, smem3, st, tt)))
-      return rc;
-    VhsEpilogueArgs ea{};
-    ea.H = h->H; ea.h_double = 0; ea.GM = h->GM; ea.ReLf = h->ReLf; ea.f = fp;
-    ea.f_double = f_double; ea.src_slots = ss; ea.src_base = sb; ea.Q = Q;
-    ea.q_double = q_double; ea.dst_slots = ds; ea.dst_base = db;
-    ea.prefac = P.prefac; ea.Nrho = h->Nrho; ea.project = 0; ea.c0 = h->c0; ea.cw = h->cw;
-    const size_t smemE = epilogue_smem<N, CEPI>();
-    return launch_cluster(vhs_epilogue_kernel<N, CEPI>, dim3(CEPI, nevals),
-                          dim3(GEPI::NT), CEPI, smemE, st, ea);
-  }
-  for (int s = 0; s < 2; ++s) {
-    Fft3Args fa{};
-    fa.f = s == 0 ? fp : fq; fa.f_double = f_double; fa.slots = ss; fa.base = sb;
-    fa.out = h->F[s];
-    if ((rc = launch_cluster(fft3_forward_kernel<N, C>, dim3(C, nevals),
-                             dim3(G::NT), C, slab_bytes(N, C, sizeof(double2)),
-                             st, fa)))
-      return rc;
-  }
-  VssPairArgs a{};
-  a.Fp = h->F[0]; a.Fq = h->F[1]; a.b = P.b; a.c = P.c; a.ph = P.ph; a.w = h->w;
-  a.fp = fp; a.f_double = f_double; a.src_slots = ss; a.src_base = sb;
-  a.Q = Q; a.q_double = q_double; a.dst_slots = ds; a.dst_base = db;
-  a.prefac = P.prefac; a.Nrho = h->Nrho; a.M = h->M;
-  const size_t smem = 4 * slab_bytes(N, C, sizeof(double2)) + 6 * N * sizeof(double2);
-  return launch_cluster(vss_pair_kernel<N, C>, dim3(C, nevals), dim3(G::NT), C,
-                        smem, st, a);
-}
+// Inputs of one evaluation: nin input arrays (slot s: fin[s], or one array per
+// evaluation from the device list fl[s]), the slot of f_p, and nq partners
+// (partner k: pair index p * nspcs + q[k], slot sq[k]).
+struct VssCall {
+  int p, nin, sp, nq;
+  const void* fin[4];
+  const void* const* fl[4];
+  int q[4], sq[4];
+};
 
-extern "C" int dgfs_vss_eval(dgfs_vss_handle h, int32_t p, int32_t q,
-                             const void* fp, const void* fq, int32_t f_dtype,
-                             void* Q, int32_t q_dtype, const int32_t* src_slots,
-                             int32_t src_base, const int32_t* dst_slots,
-                             int32_t dst_base, int32_t nevals, void* stream);
-
-// All pairs (p, q), q < nspcs, of one species p in FP32 mode:
-//   Q_p[dst] += sum_q Q_pq(f_p[src], f_q[src])
-// with one prologue per input species q (its F_g, Maxwellian spectra and
-// the loss of the pair, Re IFFT(c_pq F_q)), the 1-D tables per pair, the
-// FP64 Maxwellian gain per pair on the low-priority stream beside one FP32
-// terms launch over every pair, and one epilogue that sums the pairs'
-// spectra with their prefactors before a single inverse transform
-// (Re IFFT is linear: sum_q pref_pq Re IFFT(Ghat_pq) = Re IFFT(sum ...)).
-template <int N>
-static int vss_run_species(dgfs_vss_s* h, int p, const void* const* f,
-                           int f_double, void* Qp, int q_double,
-                           const int32_t* ss, int sb, const int32_t* ds,
-                           int db, int nevals, cudaStream_t st,
-                           const void* const* fl = nullptr, size_t fl_stride = 0,
-                           void* const* ql = nullptr) {
+//   Q_p[dst] += sum_k Q_p,q[k](f_p[src], f_q[k][src])
+// with one prologue per input array (F, its Nyquist planes and, for a partner,
+// the loss of the pair), the plane transforms, one terms launch over every
+// pair and one epilogue that sums the pairs' spectra with their prefactors
+// before a single inverse transform (Re IFFT is linear); in the FP32 mode also
+// the 1-D tables per pair and the FP64 Maxwellian gain on the low-priority
+// stream beside the terms.
+template <typename R, int N>
+static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int q_double,
+                   const int32_t* ss, int sb, const int32_t* ds, int db, int nevals,
+                   cudaStream_t st, void* const* ql = nullptr) {
+  constexpr bool FP32 = sizeof(R) == 4;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
-  constexpr int C3 = VssClusters32<N>::c;
-  using GPRO = Geo<N, CPRO>;
-  using GEPI = Geo<N, CEPI>;
-  using G3 = Geo<N, C3>;
-  const int ns = h->nspcs, T = h->Nrho * h->M;
-  const size_t E = h->max_evals, n = h->n;
-  auto ReLf = [&](int q) { return h->ReLf + q * E * n; };
-  auto uv = [&](int q) { return h->uv + q * E * T * 6 * N; };
-  auto hh = [&](int q) { return h->hh + q * E * T * 3 * N; };
-  auto GM = [&](int q) { return h->GM + q * E * n; };
-  auto H = [&](int q) { return h->H + q * E * h->Nrho * n; };
+  constexpr int C = FP32 ? VssClusters<N>::c32 : VssClusters<N>::c64;
+  using T = c2_t<R>;
+  const size_t E = h->max_evals, n = h->n, Tt = (size_t)h->Nrho * h->M;
+  auto ReLf = [&](int k) { return h->ReLf + k * E * n; };
+  auto pair = [&](int k) -> const VssPair& { return h->pair[c.p * h->nspcs + c.q[k]]; };
   int rc;
-  for (int q = 0; q < ns; ++q) {
-    const VssPair& P = h->pair[p * ns + q];
+  for (int s = 0; s < c.nin; ++s) {
+    int k = 0;                      // the partner whose loss this input gives
+    while (k < c.nq && c.sq[k] != s) ++k;
     VhsPrologueArgs a{};
-    a.f = fl ? nullptr : f[q]; a.f_list = fl ? fl + q * fl_stride : nullptr;
-    a.f_double = f_double; a.src_slots = ss; a.src_base = sb;
-    a.c0 = h->c0; a.b2 = h->b2dummy; a.b2c = P.c; a.cw = h->cw; a.split = 1;
-    a.Fg = h->Fg[q]; a.ReLf = ReLf(q); a.mhat = h->mhat[q]; a.moments = h->mom[q];
+    a.f = c.fin[s]; a.f_list = c.fl[s]; a.f_double = f_double;
+    a.src_slots = ss; a.src_base = sb; a.c0 = h->c0; a.cw = h->cw;
+    a.b2c = pair(k < c.nq ? k : 0).c; a.ReLf = k < c.nq ? ReLf(k) : nullptr;
+    a.Fg = h->F[s];
+    if (FP32) {
+      a.split = 1; a.Fny = static_cast<float2*>(h->Fny[s]);
+      a.mhat = h->mhat[s]; a.moments = h->mom[s];
+    } else {
+      a.Fny64 = static_cast<double2*>(h->Fny[s]);
+    }
     if ((rc = launch_cluster(vhs_prologue_kernel<N, CPRO>, dim3(CPRO, nevals),
-                             dim3(GPRO::NT), CPRO, prologue_smem<N, CPRO>(), st,
+                             dim3(Geo<N, CPRO>::NT), CPRO, prologue_smem<N, CPRO>(), st,
                              a)))
       return rc;
   }
-  for (int q = 0; q < ns; ++q) {
-    VssTablesArgs ta{};
-    ta.mhat_p = h->mhat[p]; ta.mhat_q = h->mhat[q];
-    ta.ph = h->pair[p * ns + q].ph; ta.uv = uv(q); ta.hh = hh(q);
-    ta.T = T; ta.nevals = nevals;
-    if ((rc = launch_plain(vss_tables_kernel<N>, dim3((nevals * T * 3 + 127) / 128),
-                           dim3(128), 0, st, ta)))
-      return rc;
-  }
-  DGFS_CUDA(cudaEventRecord(h->fork, st));
-  DGFS_CUDA(cudaStreamWaitEvent(h->aux, h->fork, 0));
-  VssTerms32Args tt{};
-  for (int q = 0; q < ns; ++q) {
-    const VssPair& P = h->pair[p * ns + q];
-    tt.pr[q] = {h->Fg[p], h->Fg[q], P.ph32, uv(q), P.b32, H(q)};
-  }
+  VssTermsArgs tt{};
   tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals;
-  const size_t smem3 = 5 * slab_bytes(N, C3, sizeof(float2)) + 24 * N * sizeof(float2);
-  if ((rc = launch_cluster(vss_terms32_kernel<N, C3>, dim3(C3, h->Nrho, nevals * ns),
-                           dim3(G3::NT), C3, smem3, st, tt)))
-    return rc;
-  for (int q = 0; q < ns; ++q) {
-    VssGainArgs ga{};
-    ga.hh = hh(q); ga.b = h->pair[p * ns + q].b; ga.w = h->w; ga.GM = GM(q);
-    ga.Nrho = h->Nrho; ga.M = h->M;
-    if ((rc = launch_plain(vss_maxwell_gain_kernel<N>,
-                           dim3((h->n + 255) / 256, nevals), dim3(256), 0,
-                           h->aux, ga)))
-      return rc;
+  tt.NS = FP32 ? h->Nrho
+               : (int)std::max<size_t>(1, std::min<size_t>(
+                     h->Nrho, h->hslots / ((size_t)c.nq * nevals)));
+  for (int k = 0; k < c.nq; ++k) {
+    const VssPair& P = pair(k);
+    // a species with itself: antipodal directions share their transforms
+    const bool merge = c.q[k] == c.p && c.sq[k] == c.sp;
+    VssTermsPair& pr = tt.pr[k];
+    pr.Fp = h->F[c.sp]; pr.Fq = h->F[c.sq[k]];
+    pr.Fnyp = h->Fny[c.sp]; pr.Fnyq = h->Fny[c.sq[k]];
+    pr.ph = FP32 ? (const void*)P.ph32 : (const void*)P.ph;
+    pr.b = FP32 ? (const void*)P.b32 : (const void*)P.b;
+    pr.uv = FP32 ? h->uv + k * E * Tt * 6 * N : nullptr;
+    pr.rho = static_cast<T*>(h->rho) + k * E * Tt * 3 * N * N;
+    pr.H = static_cast<T*>(h->H) + (size_t)k * nevals * tt.NS * n;
+    pr.dirs = merge ? h->dirsm : h->dirs;
+    pr.nd = merge ? h->ndm : h->nd;
   }
-  DGFS_CUDA(cudaEventRecord(h->join, h->aux));
-  DGFS_CUDA(cudaStreamWaitEvent(st, h->join, 0));
+  const size_t psmem = (size_t)(6 * N * (N + 1) + 6 * N) * sizeof(T);
+  if (FP32) {
+    for (int k = 0; k < c.nq; ++k) {
+      VssTablesArgs ta{};
+      ta.mhat_p = h->mhat[c.sp]; ta.mhat_q = h->mhat[c.sq[k]];
+      ta.ph = pair(k).ph; ta.uv = const_cast<float2*>(tt.pr[k].uv);
+      ta.hh = h->hh + k * E * Tt * 3 * N; ta.T = (int)Tt; ta.nevals = nevals;
+      if ((rc = launch_plain(vss_tables_kernel<N>,
+                             dim3((unsigned)((nevals * Tt * 3 + 127) / 128)), dim3(128), 0,
+                             st, ta)))
+        return rc;
+    }
+    DGFS_CUDA(cudaEventRecord(h->fork, st));
+    DGFS_CUDA(cudaStreamWaitEvent(h->aux, h->fork, 0));
+  }
+  if ((rc = launch_plain(vss_planes_kernel<R, N>, dim3((unsigned)Tt, 1, nevals * c.nq),
+                         dim3(3 * N), psmem, st, tt)))
+    return rc;
+  if ((rc = launch_cluster(vss_terms_kernel<R, N, C>, dim3(C, tt.NS, nevals * c.nq),
+                           dim3(HalfGeo<N, C>::NT), C, VssHGeo<R, N, C>::smem, st, tt)))
+    return rc;
+  if (FP32) {
+    for (int k = 0; k < c.nq; ++k) {
+      VssGainArgs ga{};
+      ga.hh = h->hh + k * E * Tt * 3 * N; ga.b = pair(k).b; ga.w = h->w;
+      ga.GM = h->GM + k * E * n; ga.dirs = tt.pr[k].dirs; ga.nd = tt.pr[k].nd;
+      ga.Nrho = h->Nrho; ga.M = h->M; ga.nevals = nevals;
+      using GG = VssGainGeo<N>;
+      if ((rc = launch_plain(vss_maxwell_gain_kernel<N>,
+                             dim3(N, N / GG::NYB, (nevals + GG::EP - 1) / GG::EP),
+                             dim3(GG::NT), 0, h->aux, ga)))
+        return rc;
+    }
+    DGFS_CUDA(cudaEventRecord(h->join, h->aux));
+    DGFS_CUDA(cudaStreamWaitEvent(st, h->join, 0));
+  }
   VhsEpilogueArgs ea{};
-  ea.f = fl ? nullptr : f[p]; ea.f_list = fl ? fl + p * fl_stride : nullptr;
+  ea.f = c.fin[c.sp]; ea.f_list = c.fl[c.sp];
   ea.f_double = f_double; ea.src_slots = ss; ea.src_base = sb;
   ea.Q = Qp; ea.q_list = ql; ea.q_double = q_double;
-  ea.dst_slots = ds; ea.dst_base = db;
-  ea.Nrho = h->Nrho; ea.project = 0; ea.c0 = h->c0; ea.cw = h->cw;
-  ea.nt = ns;
-  for (int q = 0; q < ns; ++q) {
-    ea.Ht[q] = H(q); ea.GMt[q] = GM(q); ea.ReLft[q] = ReLf(q);
-    ea.pref[q] = h->pair[p * ns + q].prefac;
+  ea.dst_slots = ds; ea.dst_base = db; ea.h_double = FP32 ? 0 : 1;
+  ea.Nrho = tt.NS; ea.c0 = h->c0; ea.cw = h->cw; ea.nt = c.nq;
+  for (int k = 0; k < c.nq; ++k) {
+    ea.Ht[k] = tt.pr[k].H; ea.GMt[k] = FP32 ? h->GM + k * E * n : nullptr;
+    ea.ReLft[k] = ReLf(k); ea.pref[k] = pair(k).prefac;
   }
   return launch_cluster(vhs_epilogue_kernel<N, CEPI>, dim3(CEPI, nevals),
-                        dim3(GEPI::NT), CEPI, epilogue_smem<N, CEPI>(), st, ea);
+                        dim3(Geo<N, CEPI>::NT), CEPI, epilogue_smem<N, CEPI>(), st, ea);
+}
+
+// Every point of a call, max_evals at a time.
+static int vss_eval_impl(dgfs_vss_s* h, VssCall c, int f_double, void* Qp, int q_double,
+                         const int32_t* src_slots, int src_base, const int32_t* dst_slots,
+                         int dst_base, int nevals, cudaStream_t st,
+                         void* const* q_list = nullptr) {
+  const bool fp32 = h->precision == DGFS_PREC_FP32;
+  for (int off = 0; off < nevals; off += h->max_evals) {
+    const int cnt = std::min(h->max_evals, nevals - off);
+    const int32_t* ss = src_slots ? src_slots + off : nullptr;
+    const int32_t* ds = dst_slots ? dst_slots + off : nullptr;
+    void* const* ql = q_list ? q_list + off : nullptr;
+    VssCall cc = c;
+    for (int s = 0; s < c.nin; ++s)
+      if (c.fl[s]) cc.fl[s] = c.fl[s] + off;
+    int rc;
+#define DGFS_VSS_RUN(R, N)                                                          \
+  vss_run<R, N>(h, cc, f_double, Qp, q_double, ss, src_base + off, ds, dst_base + off, \
+                cnt, st, ql)
+    switch (h->N) {
+      case 8: rc = fp32 ? DGFS_VSS_RUN(float, 8) : DGFS_VSS_RUN(double, 8); break;
+      case 16: rc = fp32 ? DGFS_VSS_RUN(float, 16) : DGFS_VSS_RUN(double, 16); break;
+      case 24: rc = fp32 ? DGFS_VSS_RUN(float, 24) : DGFS_VSS_RUN(double, 24); break;
+      default: rc = fp32 ? DGFS_VSS_RUN(float, 32) : DGFS_VSS_RUN(double, 32); break;
+    }
+#undef DGFS_VSS_RUN
+    if (rc) return rc;
+  }
+  return DGFS_OK;
 }
 
 extern "C" int dgfs_vss_eval_species(dgfs_vss_handle h, int32_t p,
@@ -1814,29 +1822,14 @@ extern "C" int dgfs_vss_eval_species(dgfs_vss_handle h, int32_t p,
     return fail(DGFS_ERR_INVALID, "dtype must be DGFS_F32 or DGFS_F64");
   if (nevals == 0) return DGFS_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (h->precision != DGFS_PREC_FP32) {
-    // the FP64 mode (the reference's) evaluates the pairs one by one
-    for (int q = 0; q < h->nspcs; ++q)
-      if (int rc = dgfs_vss_eval(h, p, q, f[p], f[q], f_dtype, Qp, q_dtype,
-                                 src_slots, src_base, dst_slots, dst_base,
-                                 nevals, stream))
-        return rc;
-    return DGFS_OK;
+  VssCall c{};
+  c.p = c.sp = p; c.nin = c.nq = h->nspcs;
+  for (int q = 0; q < h->nspcs; ++q) {
+    c.fin[q] = f[q];
+    c.q[q] = c.sq[q] = q;
   }
-  for (int off = 0; off < nevals; off += h->max_evals) {
-    const int cnt = std::min(h->max_evals, nevals - off);
-    const int32_t* ss = src_slots ? src_slots + off : nullptr;
-    const int32_t* ds = dst_slots ? dst_slots + off : nullptr;
-    int rc;
-    switch (h->N) {
-      case 8: rc = vss_run_species<8>(h, p, f, f_dtype, Qp, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      case 16: rc = vss_run_species<16>(h, p, f, f_dtype, Qp, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      case 24: rc = vss_run_species<24>(h, p, f, f_dtype, Qp, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      default: rc = vss_run_species<32>(h, p, f, f_dtype, Qp, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-    }
-    if (rc) return rc;
-  }
-  return DGFS_OK;
+  return vss_eval_impl(h, c, f_dtype == DGFS_F64, Qp, q_dtype == DGFS_F64, src_slots,
+                       src_base, dst_slots, dst_base, nevals, st);
 }
 
 // Every pair of species p for a list of points of several mixtures that
@@ -1864,23 +1857,14 @@ extern "C" int dgfs_vss_eval_species_multi(dgfs_vss_handle h, int32_t p,
       (q_dtype != DGFS_F32 && q_dtype != DGFS_F64))
     return fail(DGFS_ERR_INVALID, "dtype must be DGFS_F32 or DGFS_F64");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const void* none[4] = {};
-  for (int off = 0; off < nevals; off += h->max_evals) {
-    const int cnt = std::min(h->max_evals, nevals - off);
-    const int32_t* ss = src_slots ? src_slots + off : nullptr;
-    const int32_t* ds = dst_slots ? dst_slots + off : nullptr;
-    const void* const* fl = f_lists + off;
-    void* const* ql = q_list + off;
-    int rc;
-    switch (h->N) {
-      case 8: rc = vss_run_species<8>(h, p, none, f_dtype, nullptr, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st, fl, nevals, ql); break;
-      case 16: rc = vss_run_species<16>(h, p, none, f_dtype, nullptr, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st, fl, nevals, ql); break;
-      case 24: rc = vss_run_species<24>(h, p, none, f_dtype, nullptr, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st, fl, nevals, ql); break;
-      default: rc = vss_run_species<32>(h, p, none, f_dtype, nullptr, q_dtype, ss, src_base + off, ds, dst_base + off, cnt, st, fl, nevals, ql); break;
-    }
-    if (rc) return rc;
+  VssCall c{};
+  c.p = c.sp = p; c.nin = c.nq = h->nspcs;
+  for (int q = 0; q < h->nspcs; ++q) {
+    c.fl[q] = f_lists + (size_t)q * nevals;
+    c.q[q] = c.sq[q] = q;
   }
-  return DGFS_OK;
+  return vss_eval_impl(h, c, f_dtype == DGFS_F64, nullptr, q_dtype == DGFS_F64, src_slots,
+                       src_base, dst_slots, dst_base, nevals, st, q_list);
 }
 
 extern "C" int dgfs_vss_eval(dgfs_vss_handle h, int32_t p, int32_t q,
@@ -1900,21 +1884,12 @@ extern "C" int dgfs_vss_eval(dgfs_vss_handle h, int32_t p, int32_t q,
   if ((f_dtype != DGFS_F32 && f_dtype != DGFS_F64) ||
       (q_dtype != DGFS_F32 && q_dtype != DGFS_F64))
     return fail(DGFS_ERR_INVALID, "dtype must be DGFS_F32 or DGFS_F64");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  for (int off = 0; off < nevals; off += h->max_evals) {
-    const int cnt = std::min(h->max_evals, nevals - off);
-    const int32_t* ss = src_slots ? src_slots + off : nullptr;
-    const int32_t* ds = dst_slots ? dst_slots + off : nullptr;
-    int rc;
-    switch (h->N) {
-      case 8: rc = vss_run<8>(h, p, q, f_p, f_q, f_dtype == DGFS_F64, Q_p, q_dtype == DGFS_F64, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      case 16: rc = vss_run<16>(h, p, q, f_p, f_q, f_dtype == DGFS_F64, Q_p, q_dtype == DGFS_F64, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      case 24: rc = vss_run<24>(h, p, q, f_p, f_q, f_dtype == DGFS_F64, Q_p, q_dtype == DGFS_F64, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-      default: rc = vss_run<32>(h, p, q, f_p, f_q, f_dtype == DGFS_F64, Q_p, q_dtype == DGFS_F64, ss, src_base + off, ds, dst_base + off, cnt, st); break;
-    }
-    if (rc) return rc;
-  }
-  return DGFS_OK;
+  VssCall c{};
+  c.p = p; c.nq = 1; c.q[0] = q; c.fin[0] = f_p; c.nin = 1;
+  if (f_q != f_p) { c.fin[1] = f_q; c.nin = 2; c.sq[0] = 1; }
+  return vss_eval_impl(h, c, f_dtype == DGFS_F64, Q_p, q_dtype == DGFS_F64, src_slots,
+                       src_base, dst_slots, dst_base, nevals,
+                       static_cast<cudaStream_t>(stream));
 }
 
 // Conservation projection of Q (no counterpart in the reference): after it,

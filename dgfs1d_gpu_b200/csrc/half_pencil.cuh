@@ -37,8 +37,7 @@ __device__ __forceinline__ void half_butterfly(c2_t<R>* v, R sgn) {
 #pragma unroll
   for (int k = 0; k < H; ++k) {
     const c2_t<R> o = pair_swap(v[k]);
-    v[k].x = sgn * v[k].x + o.x;
-    v[k].y = sgn * v[k].y + o.y;
+    v[k] = cfma(sgn, v[k], o);
   }
 }
 

@@ -55,7 +55,7 @@ struct VhsPrologueArgs {
   double cw;                  // velocity cell volume
   int split;                  // 1: Maxwellian split (FP32 mode)
   void* Fg;                   // out [nevals][n] complex (float2 if split else double2)
-  double* ReLf;               // out [nevals][n] Re IFFT(b2 F)
+  double* ReLf;               // out [nevals][n] Re IFFT(b2 F) (null: skipped)
   double2* mhat;              // out [nevals][3][N] Maxwellian 1-D spectra (split)
   double* moments;            // out [nevals][5] rho, ux, uy, uz, T (split)
                               // Fg, mhat and moments may be null (split):
@@ -135,7 +135,8 @@ struct VhsEpilogueArgs {
   double cg, cl;
   // several pair operators into one output (the VSS species sum): when
   // nt > 0, Ghat = sum_t pref[t] (GMt[t] + sum_p Ht[t][p]) and the loss is
-  // f sum_t pref[t] ReLft[t] (FP32 H); H, GM, ReLf and prefac are unused
+  // f sum_t pref[t] ReLft[t] (GMt[t] may be null); H, GM, ReLf and prefac are
+  // unused
   int nt;
   const void* Ht[4];
   const double2* GMt[4];
@@ -358,6 +359,7 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
   if (a.split && rank == 0)
     if (a.mhat)
       for (int i = t; i < 3 * N; i += G::NT) a.mhat[(size_t)e * 3 * N + i] = mh[i];
+  if (!a.ReLf) return;   // (no CTA writes to a peer past this point)
   __syncthreads();
   // loss: Re IFFT(b2 F); the Y-slab exchange reuses the slab once every CTA
   // of the cluster has read its own
@@ -1652,49 +1654,55 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     for (int m = 0; m < H; ++m)
       st_cluster(rdst[P > H ? 0 : m / P] + ES * (uint32_t)((P > H ? m : m % P) * N * N),
                  v[m]);
-    cluster_arrive();
-    if (k + 1 < npass) {
-      cp_async_wait_all();
-      __syncthreads();
-      zpass();
+    cp_async_wait_all();
+    __syncthreads();                     // next F slab and tables are in place
+    if (k + 1 < npass) zpass();
+    cluster_arrive();                    // (the stores land during the z pass)
+    // the part of the combine that needs the plane transforms only, while the
+    // exchange completes
+    const T* rp = static_cast<const T*>(a.rho) +
+                  ((size_t)e * a.Nrho * Mu + term(k)) * 3 * N * N;
+    const T rx = rp[yy * N + c];
+    const T* rY = rp + N * N + c + h * H * N;
+    const T* rZ = rp + 2 * N * N + yy + h * H * N;
+    const R mq = SPLIT ? R(1) : (R)a.mult[k % Mu];
+    T uyz{}, vyz{};
+    if constexpr (SPLIT) {
+      uyz = cmul(ut[N + yy], ut[2 * N + c]);
+      vyz = cmul(ut[4 * N + yy], ut[5 * N + c]);
+    }
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      const T ry = rY[m * N], rz = rZ[m * N];
+      const R xs = (m & 1) ? R(-1) : R(1);   // (-1)^x, H is even
+      const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
+      const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
+      if constexpr (SPLIT) {
+        const T ux = ut[h * H + m], vx = ut[3 * N + h * H + m];
+        const R uy = ux.x * uyz.y + ux.y * uyz.x;
+        const R vy = vx.x * vyz.y + vx.y * vyz.x;
+        S[m] += wm * (wp + uy);
+        S[m] -= vy * wp;
+      } else {
+        S[m] += mq * (wm * wp);
+      }
     }
     cluster_wait();                      // this transform's columns have arrived
 #pragma unroll
     for (int m = 0; m < H; ++m) v[m] = Rb[colr + (2 * m + h) * N];
     cluster_arrive();                    // R is read
     fft_half_dit<R, N, +1>(v, h);
-    const T* rp = static_cast<const T*>(a.rho) +
-                  ((size_t)e * a.Nrho * Mu + term(k)) * 3 * N * N;
-    const T rx = rp[yy * N + c];
-    const T* rY = rp + N * N + c + h * H * N;
-    const T* rZ = rp + 2 * N * N + yy + h * H * N;
-    if constexpr (SPLIT) {
-      const T* vt = ut + 3 * N;
-      const T uyz = cmul(ut[N + yy], ut[2 * N + c]);
-      const T vyz = cmul(vt[N + yy], vt[2 * N + c]);
 #pragma unroll
-      for (int m = 0; m < H; ++m) {
-        const T ry = rY[m * N], rz = rZ[m * N];
-        const R xs = (m & 1) ? R(-1) : R(1);   // (-1)^x, H is even
-        const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
-        const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
-        const T um = cmul(ut[h * H + m], uyz), vm = cmul(vt[h * H + m], vyz);
-        const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
-        S[m] += gp * (gm + um.x);
-        S[m] += vm.x * gm;
-        S[m] += wm * (wp + um.y);
-        S[m] -= vm.y * wp;
-      }
-    } else {
-      const R mq = a.mult[k % Mu];
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        const T ry = rY[m * N], rz = rZ[m * N];
-        const R xs = (m & 1) ? R(-1) : R(1);
-        const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
-        const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
-        const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
-        S[m] += mq * (gp * gm + wm * wp);
+    for (int m = 0; m < H; ++m) {
+      const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
+      if constexpr (SPLIT) {
+        const T ux = ut[h * H + m], vx = ut[3 * N + h * H + m];
+        const R u = ux.x * uyz.x - ux.y * uyz.y;
+        const R w = vx.x * vyz.x - vx.y * vyz.y;
+        S[m] += gp * (gm + u);
+        S[m] += w * gm;
+      } else {
+        S[m] += mq * (gp * gm);
       }
     }
     if (k == Mu - 1 && npass > Mu) {
@@ -1839,9 +1847,19 @@ vhs_epilogue_kernel(VhsEpilogueArgs a) {
       for (int u = 0; u < UNR; ++u) {
         const int j2 = b0 + u * G::NT;
         if (j2 < TOT2) {
-          T g0 = a.GMt[it][(size_t)e * G::n + off + 2 * j2];
-          T g1 = a.GMt[it][(size_t)e * G::n + off + 2 * j2 + 1];
-          for (int p = 0; p < a.Nrho; ++p) {
+          T g0 = T{0, 0}, g1 = T{0, 0};
+          if (a.GMt[it]) {
+            g0 = a.GMt[it][(size_t)e * G::n + off + 2 * j2];
+            g1 = a.GMt[it][(size_t)e * G::n + off + 2 * j2 + 1];
+          }
+          if (a.h_double) {
+            for (int p = 0; p < a.Nrho; ++p) {
+              const double2* h = static_cast<const double2*>(a.Ht[it]) +
+                                 ((size_t)e * a.Nrho + p) * G::n + off + 2 * j2;
+              const double2 h0 = h[0], h1 = h[1];
+              g0.x += h0.x; g0.y += h0.y; g1.x += h1.x; g1.y += h1.y;
+            }
+          } else for (int p = 0; p < a.Nrho; ++p) {
             const float4 h = reinterpret_cast<const float4*>(
                 static_cast<const float2*>(a.Ht[it]) +
                 ((size_t)e * a.Nrho + p) * G::n + off)[j2];

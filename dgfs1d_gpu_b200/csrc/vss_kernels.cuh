@@ -7,12 +7,12 @@
 //   t1 = e^{+i a m_q/(m_p+m_q)} F,  t2 = e^{-i a m_p/(m_p+m_q)} G,
 //   Qhat = sum_{r,m} (w_r s_w / n) b_{pq,rm}(l) FFT(IFFT(t1) IFFT(t2)),
 //   Q_p += prefac_pq (Re IFFT(Qhat) - f_p Re IFFT(c_pq G)).
-// The weights b_{pq,rm} depend on both r and m, so every term needs its own
-// forward transform (3 transforms per term).  Here one thread-block cluster
-// evaluates one point completely: per term the two inverse transforms and
-// the forward transform exchange through distributed shared memory, the
-// spectral accumulator stays in shared memory, and the final inverse
-// transform, the loss and the output run in the same kernel.  FP64.
+// f_p and f_q are real, so (Nyquist planes apart) u = IFFT(t1) and
+// v = IFFT(t2) are real and one complex inverse transform of t1 + i t2 gives
+// both; the weights b_{pq,rm} depend on both r and m, so every term has its own
+// forward transform: two transforms per term instead of three.  For a species
+// with itself the product u v is the same for sigma and -sigma, so antipodal
+// directions share their transforms.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -21,59 +21,6 @@
 #include "fft_reg.cuh"
 
 namespace dgfs {
-
-// F = FFT(f)/n for a batch of slots (one cluster per slot, FP64).
-struct Fft3Args {
-  const void* f;
-  int f_double;
-  const int32_t* slots;
-  int base;
-  double2* out;        // [nevals][n]
-};
-
-template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT, 1)
-fft3_forward_kernel(Fft3Args a) {
-  using G = Geo<N, C>;
-  using T = double2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);
-  const int t = threadIdx.x;
-  const unsigned rank = cluster_rank();
-  const int e = blockIdx.y;
-  const int yl = t / N, z = t % N, y = rank * G::P + yl;
-  const int slot = a.slots ? a.slots[e] : a.base + e;
-  const size_t fb = (size_t)slot * G::n;
-  T v[N];
-#pragma unroll
-  for (int x = 0; x < N; ++x) {
-    v[x].x = a.f_double ? static_cast<const double*>(a.f)[fb + ((size_t)x * N + y) * N + z]
-                        : (double)static_cast<const float*>(a.f)[fb + ((size_t)x * N + y) * N + z];
-    v[x].y = 0.0;
-  }
-  fft<double, N, -1>(v);
-  push_pencils_to_xslab<double, N, C>(A, t, rank, v);
-  cluster_sync_all();
-  {
-    T w[N];
-    slab_col_load_fft<double, N, C, -1>(A, t, w);
-    const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-    for (int k = 0; k < N; ++k) A[base + k * G::ROW] = w[k];
-  }
-  __syncthreads();
-  slab_row_pass<double, N, C, -1>(A, t);
-  __syncthreads();
-  const double inv_n = 1.0 / (double)G::n;
-  T* out = a.out + (size_t)e * G::n + (size_t)rank * G::P * N * N;
-  for (int j = t; j < G::P * N * N; j += G::NT) {
-    T w = A[slab_index<N, C>(j)];
-    w.x *= inv_n;
-    w.y *= inv_n;
-    out[j] = w;
-  }
-  cluster_sync_all();  // no CTA leaves while peers may still write into it
-}
 
 // Weights of one pair (vss.mako:51-93, launch loop bi/scattering.py:185-204):
 //   b_rm(l) = sum_k B_mk fac_b(r) e^{-i mpq s_r sigma'_k . l}
@@ -205,178 +152,6 @@ __global__ void vss_sum_c_kernel(const double2* cpart, int Nrho, size_t n,
   c[l] = s;
 }
 
-struct VssPairArgs {
-  const double2* Fp;       // [nevals][n]  FFT(f_p)/n
-  const double2* Fq;       // [nevals][n]  FFT(f_q)/n
-  const double2* b;        // [Nrho][M][n]
-  const double2* c;        // [n]
-  const double2* ph;       // [Nrho][M][2][3][N]: e^{+i a mq'}, e^{-i a mp'} factors
-  const double* w;         // [Nrho] w_r s_w / n
-  const void* fp;          // f_p (for the loss product)
-  int f_double;
-  const int32_t* src_slots;
-  int src_base;
-  void* Q;                 // Q_p output (+=)
-  int q_double;
-  const int32_t* dst_slots;
-  int dst_base;
-  double prefac;
-  int Nrho, M;
-};
-
-template <int N, int C>
-__device__ __forceinline__ void vss_zpass_inverse(double2* A, const double2* Frow0,
-                                                  const double2* tb, int t,
-                                                  unsigned rank) {
-  using G = Geo<N, C>;
-  const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-  const double2 bxy = cmul(tb[lx], tb[N + ly]);
-  const double2* row = Frow0 + ((size_t)lx * N + ly) * N;
-  double2 v[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = cmul(row[k], cmul(bxy, tb[2 * N + k]));
-  fft<double, N, +1>(v);
-  const int base = pl * G::PLANE + ly * G::ROW;
-#pragma unroll
-  for (int k = 0; k < N; ++k) A[base + k] = v[k];
-}
-
-template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT, 1)
-vss_pair_kernel(VssPairArgs a) {
-  using G = Geo<N, C>;
-  using T = double2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);   // X-slab work buffer
-  T* Rb = A + G::SLAB;                     // Y-slab receive buffer
-  T* U = Rb + G::SLAB;                     // Y-slab: u pencils / loss
-  T* Qh = U + G::SLAB;                     // X-slab spectral accumulator
-  T* tab = Qh + G::SLAB;                   // [2][3][N] phase factors
-  const int t = threadIdx.x;
-  const unsigned rank = cluster_rank();
-  const int e = blockIdx.y;
-  const int yl = t / N, zz = t % N;
-  const int ybase = yl * G::PLANE + zz;    // thread's pencil in a Y-slab
-  const T* Fp = a.Fp + (size_t)e * G::n;
-  const T* Fq = a.Fq + (size_t)e * G::n;
-  bool pending = false;  // an arrive is outstanding (receive buffer in use)
-
-  // exchange this thread's y-pass column into the owners' receive buffers
-  auto exchange_cols = [&](const T* v) {
-    if (pending) cluster_wait();
-    push_cols_to_yslab<double, N, C>(Rb, t, rank, v);
-    cluster_arrive();
-    cluster_wait();
-  };
-  auto release_receive = [&]() {
-    cluster_arrive();
-    pending = true;
-  };
-  // inverse 3-D FFT of F * tables; result pencil (x) left in v
-  auto inverse = [&](const T* F, const T* tb, T* v) {
-    vss_zpass_inverse<N, C>(A, F, tb, t, rank);
-    __syncthreads();
-    slab_col_load_fft<double, N, C, +1>(A, t, v);
-    exchange_cols(v);
-    yslab_load_pencil<double, N, C>(Rb, t, v);
-    release_receive();
-    fft<double, N, +1>(v);
-  };
-
-  for (int j = t; j < G::SLAB; j += G::NT) Qh[j] = T{0, 0};
-  const int T_terms = a.Nrho * a.M;
-#pragma unroll 1
-  for (int term = 0; term < T_terms; ++term) {
-    const int r = term / a.M;
-    __syncthreads();
-    for (int i = t; i < 6 * N; i += G::NT) tab[i] = a.ph[(size_t)term * 6 * N + i];
-    __syncthreads();
-    T v[N];
-    inverse(Fp, tab, v);                       // u = IFFT(e^{+i a mq'} F)
-#pragma unroll
-    for (int x = 0; x < N; ++x) U[ybase + x * G::ROW] = v[x];
-    inverse(Fq, tab + 3 * N, v);               // v = IFFT(e^{-i a mp'} G)
-#pragma unroll
-    for (int x = 0; x < N; ++x) v[x] = cmul(U[ybase + x * G::ROW], v[x]);
-    fft<double, N, -1>(v);                     // forward: x pass
-    if (pending) cluster_wait();
-    push_pencils_to_xslab<double, N, C>(A, t, rank, v);
-    cluster_arrive();
-    cluster_wait();
-    pending = false;
-    {
-      T w[N];
-      slab_col_load_fft<double, N, C, -1>(A, t, w);
-      const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-      for (int k = 0; k < N; ++k) A[base + k * G::ROW] = w[k];
-    }
-    __syncthreads();
-    {
-      // z pass (rows) and accumulation W_r b_rm (*) FFT(h) into Qhat
-      const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-      const int base = pl * G::PLANE + ly * G::ROW;
-      T w[N];
-#pragma unroll
-      for (int k = 0; k < N; ++k) w[k] = A[base + k];
-      fft<double, N, -1>(w);
-      const T* brow = a.b + (size_t)term * G::n + ((size_t)lx * N + ly) * N;
-      const double wr = a.w[r];
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const T bb = brow[k];
-        const T pr = cmul(w[k], bb);
-        Qh[base + k].x += wr * pr.x;
-        Qh[base + k].y += wr * pr.y;
-      }
-    }
-  }
-
-  // loss: Re IFFT(c (*) G) -> U (real parts), then the gain IFFT(Qhat)
-  {
-    __syncthreads();
-    const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-    const T* row = Fq + ((size_t)lx * N + ly) * N;
-    const T* crow = a.c + ((size_t)lx * N + ly) * N;
-    T w[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) w[k] = cmul(crow[k], row[k]);
-    fft<double, N, +1>(w);
-    const int base = pl * G::PLANE + ly * G::ROW;
-#pragma unroll
-    for (int k = 0; k < N; ++k) A[base + k] = w[k];
-  }
-  __syncthreads();
-  T v[N];
-  slab_col_load_fft<double, N, C, +1>(A, t, v);
-  exchange_cols(v);
-  yslab_load_pencil<double, N, C>(Rb, t, v);
-  release_receive();
-  fft<double, N, +1>(v);
-#pragma unroll
-  for (int x = 0; x < N; ++x) U[ybase + x * G::ROW] = v[x];
-  slab_row_pass<double, N, C, +1>(Qh, t);
-  __syncthreads();
-  slab_col_load_fft<double, N, C, +1>(Qh, t, v);
-  exchange_cols(v);
-  yslab_load_pencil<double, N, C>(Rb, t, v);
-  release_receive();
-  fft<double, N, +1>(v);
-  const int y = rank * G::P + yl;
-  const size_t fb = (size_t)(a.src_slots ? a.src_slots[e] : a.src_base + e) * G::n;
-  const size_t qb = (size_t)(a.dst_slots ? a.dst_slots[e] : a.dst_base + e) * G::n;
-#pragma unroll
-  for (int x = 0; x < N; ++x) {
-    const size_t idx = ((size_t)x * N + y) * N + zz;
-    const double fv = a.f_double ? static_cast<const double*>(a.fp)[fb + idx]
-                                 : (double)static_cast<const float*>(a.fp)[fb + idx];
-    const double qv = a.prefac * (v[x].x - fv * U[ybase + x * G::ROW].x);
-    if (a.q_double) static_cast<double*>(a.Q)[qb + idx] += qv;
-    else static_cast<float*>(a.Q)[qb + idx] += (float)qv;
-  }
-  if (pending) cluster_wait();
-}
-
 // ---------------------------------------------------------------------------
 // FP32 mode (no counterpart in the reference, which is FP64 only): the
 // Maxwellian split of the VHS operator carried over to a pair.  With
@@ -431,232 +206,384 @@ __global__ void vss_tables_kernel(VssTablesArgs a) {
   for (int l = 0; l < N; ++l) hh[l] = u[l];
 }
 
-// GM[e][l] = sum_r w_r sum_m b_rm(l) prod_a H_a,rm(l_a)   (FP64)
-// grid (ceil(n/256), E), one thread per wavenumber l.
+// GM[e][l] = sum_r w_r sum_d b_rd(l) prod_a H_a,rd(l_a)   (FP64), d over the
+// pair's direction list (merged antipodes share H and add their b).
+// Grid (N [lx], N / NYB, ceil(E / EP)), block N NYB: a thread owns the
+// wavenumber (lx, ly, lz) of EP points, so that every weight b is read once
+// for EP points (one point per thread read b, 32 MB per pair at N=24, from L2
+// for each point: 163 us per pair at 18 points).  The 1-D factors of a chunk
+// of terms are staged in shared memory, hx hy folded once per (term, ly).
 struct VssGainArgs {
   const double2* hh;       // [E][T][3][N]
   const double2* b;        // [T][n]
   const double* w;         // [Nrho]
   double2* GM;             // out [E][n]
-  int Nrho, M;
+  const int2* dirs;
+  int nd, Nrho, M, nevals;
+};
+template <int N> struct VssGainGeo {
+  static constexpr int NYB = N == 16 ? 16 : 8;   // ly rows per CTA
+  static constexpr int NT = N * NYB;
+  static constexpr int EP = 3;                   // points per thread
+  static constexpr int CH = 12;                  // terms per staged chunk
 };
 
 template <int N>
-__global__ void __launch_bounds__(256) vss_maxwell_gain_kernel(VssGainArgs a) {
-  constexpr int n = N * N * N;
-  const int l = blockIdx.x * 256 + threadIdx.x, e = blockIdx.y;
-  if (l >= n) return;
-  const int lx = l / (N * N), ly = (l / N) % N, lz = l % N;
-  const int T = a.Nrho * a.M;
-  const double2* hh = a.hh + (size_t)e * T * 3 * N;
-  double2 G = make_double2(0, 0);
-  for (int r = 0; r < a.Nrho; ++r) {
-    double2 acc = make_double2(0, 0);
-    for (int m = 0; m < a.M; ++m) {
-      const int term = r * a.M + m;
-      const double2* h = hh + (size_t)term * 3 * N;
-      const double2 x = cmul(cmul(h[lx], h[N + ly]), h[2 * N + lz]);
-      const double2 p = cmul(x, a.b[(size_t)term * n + l]);
-      acc.x += p.x;
-      acc.y += p.y;
+__global__ void __launch_bounds__(VssGainGeo<N>::NT) vss_maxwell_gain_kernel(VssGainArgs a) {
+  using GG = VssGainGeo<N>;
+  constexpr int n = N * N * N, EP = GG::EP, CH = GG::CH, NYB = GG::NYB;
+  __shared__ double2 hz[CH][EP][N];
+  __shared__ double2 hxy[CH][EP][NYB];
+  const int lx = blockIdx.x, ly0 = blockIdx.y * NYB, e0 = blockIdx.z * EP;
+  const int t = threadIdx.x, yl = t / N, lz = t % N;
+  const size_t l = ((size_t)lx * N + ly0 + yl) * N + lz;
+  const int T = a.Nrho * a.M, total = a.Nrho * a.nd;
+  double2 acc[EP];
+#pragma unroll
+  for (int p = 0; p < EP; ++p) acc[p] = make_double2(0, 0);
+  for (int c0 = 0; c0 < total; c0 += CH) {
+    const int nc = min(CH, total - c0);
+    __syncthreads();
+    for (int i = t; i < nc * EP * (N + NYB); i += GG::NT) {
+      const int j = i % (N + NYB), p = (i / (N + NYB)) % EP, k = i / (EP * (N + NYB));
+      const int e = min(e0 + p, a.nevals - 1), r = (c0 + k) / a.nd;
+      const int term = r * a.M + a.dirs[(c0 + k) % a.nd].x;
+      const double2* h = a.hh + ((size_t)e * T + term) * 3 * N;
+      if (j < N) {
+        hz[k][p][j] = h[2 * N + j];
+      } else {
+        const double2 x = cmul(h[lx], h[N + ly0 + j - N]);
+        const double w = a.w[r];
+        hxy[k][p][j - N] = make_double2(w * x.x, w * x.y);
+      }
     }
-    G.x += a.w[r] * acc.x;
-    G.y += a.w[r] * acc.y;
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < nc; ++k) {
+      const int r = (c0 + k) / a.nd;
+      const int2 dir = a.dirs[(c0 + k) % a.nd];
+      double2 b = a.b[(size_t)(r * a.M + dir.x) * n + l];
+      if (dir.y >= 0) {
+        const double2 q = a.b[(size_t)(r * a.M + dir.y) * n + l];
+        b.x += q.x; b.y += q.y;
+      }
+#pragma unroll
+      for (int p = 0; p < EP; ++p) {
+        const double2 x = cmul(hxy[k][p][yl], hz[k][p][lz]);
+        acc[p].x += x.x * b.x; acc[p].x -= x.y * b.y;
+        acc[p].y += x.x * b.y; acc[p].y += x.y * b.x;
+      }
+    }
   }
-  a.GM[(size_t)e * n + l] = G;
+#pragma unroll
+  for (int p = 0; p < EP; ++p)
+    if (e0 + p < a.nevals) a.GM[(size_t)(e0 + p) * n + l] = acc[p];
 }
 
 // Pointers of one species pair; a launch covers npair pairs, grid z =
 // npair * nevals (pair major).
-struct VssTerms32Pair {
-  const float2* Fgp;       // [E][n] F_gp
-  const float2* Fgq;       // [E][n] F_gq
-  const float2* ph;        // [T][2][3][N] FP32 phase factors
-  const float2* uv;        // [E][T][2][3][N] u_M,a, v_M,a
-  const float2* b;         // [T][n] FP32 weights
-  float2* H;               // out [E][Nrho][n]
+struct VssTermsPair {
+  const void* Fp;          // [E][n] F_p (FP32 mode: F_gp)
+  const void* Fq;          // [E][n]
+  const void* ph;          // [T][2][3][N] phase factors of u and v
+  const float2* uv;        // FP32: [E][T][2][3][N] u_M,a, v_M,a
+  const void* b;           // [T][n] weights
+  const void* Fnyp;        // [E][3][N][N] Nyquist planes of F_p, F_q
+  const void* Fnyq;
+  void* rho;               // [E][T][3][N][N] plane transforms (u_i, v_i)
+  void* H;                 // out [E][NS][n]
+  const int2* dirs;        // [nd] direction and its merged antipode (or -1)
+  int nd;
 };
-struct VssTerms32Args {
-  VssTerms32Pair pr[16];
+struct VssTermsArgs {
+  VssTermsPair pr[4];
   const double* w;         // [Nrho]
   int Nrho, M, nevals;
+  int NS;                  // radial slices (blockIdx.y): r in [y Nrho/NS, ...)
 };
 
-// z-pass of an inverse transform: rows of F (global, FP32) times the phase.
-template <int N, int C>
-__device__ __forceinline__ void vss32_zpass(float2* A, const float2* F,
-                                            const float2* tb, int t,
-                                            unsigned rank) {
-  using G = Geo<N, C>;
-  const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-  const float2 bxy = cmul(tb[lx], tb[N + ly]);
-  const float2* row = F + ((size_t)lx * N + ly) * N;
-  float2 v[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = cmul(row[k], cmul(bxy, tb[2 * N + k]));
-  fft<float, N, +1>(v);
-  const int base = pl * G::PLANE + ly * G::ROW;
-#pragma unroll
-  for (int k = 0; k < N; ++k) A[base + k] = v[k];
+// exp(i N alpha_a) from the phase at the Nyquist index, exp(-i alpha_a N/2)
+template <typename T> __device__ __forceinline__ T vss_nu(T ph) {
+  T c; c.x = ph.x; c.y = -ph.y;
+  return cmul(c, c);
 }
 
-// One cluster per (pair, point, radial point r); per direction m three
-// transforms, each with one cluster barrier (arrive after the stores into
-// the peers, wait before reading):
-//   T1 = IFFT3(phi_p F_gp) -> receive buffer R0 -> X_u (registers)
-//   T2 = IFFT3(phi_q F_gq) -> R1 -> X_v, combined with X_u into h
-//   T3 = FFT3(h) -> X-slab B -> b_rm (*) FFT(h) added into Qhat (shared)
-// The z-pass of T2 runs while T1's stores land, and the z-pass of T1 of the
-// next direction while T2's do.  Five slabs: A (z/y passes of T1 and T2),
-// B (T3), R0, R1, Qhat; the direction tables sit in a two-slot ring.
-template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT, 1)
-vss_terms32_kernel(VssTerms32Args a) {
-  using G = Geo<N, C>;
-  using T = float2;
+// Plane transforms of one term.  With E the phase factor and f_S as in the
+// packed VHS transforms, E F splits on the Nyquist planes into
+// E (1 + f_S)/2 F, whose inverse transform is real, and E (1 - f_S)/2 F, whose
+// inverse transform is i u_i (i v_i).  This kernel forms u_i + i v_i, the
+// inverse transform of -i E_u (1 - f_u)/2 F_p + E_v (1 - f_v)/2 F_q, as three
+// 2-D transforms (rows and planes as in vhs_nyq_planes64_kernel).
+// Grid (terms of the list, 1, npair nevals), 3N threads, one pencil each.
+template <typename R, int N>
+__global__ void __launch_bounds__(3 * N) vss_planes_kernel(VssTermsArgs a) {
+  using T = c2_t<R>;
+  constexpr int ROW = N + 1, H = N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);   // X-slab work buffer (inverse)
-  T* B = A + G::SLAB;                      // X-slab receive (forward)
-  T* R0 = B + G::SLAB;                     // Y-slab receive buffers R0, R1
-  T* Qh = R0 + 2 * G::SLAB;                // X-slab spectral accumulator
-  T* tab = Qh + G::SLAB;                   // [2][12N]: phases p, q | u_M | v_M
-  const int t = threadIdx.x;
+  T* pls = reinterpret_cast<T*>(smem_raw);   // [3][N][ROW] planes of F_p
+  T* plq = pls + 3 * N * ROW;                 // of F_q
+  T* tb = plq + 3 * N * ROW;                  // [6N] phases
+  const int e = blockIdx.z % a.nevals, t = threadIdx.x;
+  const VssTermsPair& Pr = a.pr[blockIdx.z / a.nevals];
+  const int r = blockIdx.x / a.M, d = blockIdx.x % a.M;
+  if (d >= Pr.nd) return;
+  const int term = r * a.M + Pr.dirs[d].x;
+  const int P = t / N, i = t % N;
+  const T* Fp = static_cast<const T*>(Pr.Fnyp) + (size_t)e * 3 * N * N;
+  const T* Fq = static_cast<const T*>(Pr.Fnyq) + (size_t)e * 3 * N * N;
+#pragma unroll 4
+  for (int j = t; j < 3 * N * N; j += 3 * N) {
+    pls[(j / N) * ROW + j % N] = Fp[j];
+    plq[(j / N) * ROW + j % N] = Fq[j];
+  }
+  for (int j = t; j < 6 * N; j += 3 * N)
+    tb[j] = static_cast<const T*>(Pr.ph)[(size_t)term * 6 * N + j];
+  __syncthreads();
+  T v[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = T{R(0), R(0)};
+  T* rowp = pls + (P * N + i) * ROW;
+  const T* rowq = plq + (P * N + i) * ROW;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const T* tt = tb + 3 * N * s;
+    const T nx = vss_nu(tt[H]), ny = vss_nu(tt[N + H]), nz = vss_nu(tt[2 * N + H]);
+    T rowc, f_row, f_rowH;
+    const T* tk;
+    if (P == 0) {
+      rowc = cmul(tt[H], tt[N + i]);
+      f_row = (i == H) ? cmul(nx, ny) : nx;
+      f_rowH = cmul(f_row, nz);
+      tk = tt + 2 * N;
+    } else if (P == 1) {
+      rowc = cmul(tt[i], tt[N + H]);
+      f_row = ny;
+      f_rowH = cmul(ny, nz);
+      tk = tt + 2 * N;
+    } else {
+      rowc = cmul(tt[i], tt[2 * N + H]);
+      f_row = nz;
+      f_rowH = nz;
+      tk = tt + N;
+    }
+    if (P >= 1 && i == H) rowc = T{R(0), R(0)};
+    // (1 - f)/2 rowc
+    const T g = cmul(T{R(0.5) * (R(1) - f_row.x), R(-0.5) * f_row.y}, rowc);
+    const T gH = (P == 2) ? T{R(0), R(0)}
+                          : cmul(T{R(0.5) * (R(1) - f_rowH.x), R(-0.5) * f_rowH.y}, rowc);
+    const T* row = s == 0 ? rowp : rowq;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const T x = cmul(cmul(k == H ? gH : g, tk[k]), row[k]);
+      if (s == 0) { v[k].x += x.y; v[k].y -= x.x; }   // -i x
+      else { v[k].x += x.x; v[k].y += x.y; }
+    }
+  }
+  fft<R, N, +1>(v);
+#pragma unroll
+  for (int k = 0; k < N; ++k) rowp[k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = pls[(P * N + k) * ROW + i];
+  fft<R, N, +1>(v);
+  T* rho = static_cast<T*>(Pr.rho) +
+           (((size_t)e * a.Nrho * a.M + term) * 3 + P) * N * N;
+#pragma unroll
+  for (int k = 0; k < N; ++k) rho[(size_t)k * N + i] = v[k];
+}
+
+// Terms: one cluster per (pair, point, radial slice), two lanes per pencil
+// (half_pencil.cuh), one transform slab A and one receive slab R as in
+// vhs_termsh_kernel, whose bound (the exchange through distributed shared
+// memory) it shares: two exchanges per term.  Per direction:
+//   Z = M_u F_p + i M_v F_q elementwise into A (coalesced reads of F; the row
+//   factors of M in a table), z pass, y pass -> exchange into R -> x pass:
+//   u_r + i v_r, with the plane transforms u_i + i v_i -> the product h
+//   (FP32: u_M X_v + X_u (v_M + X_v)) -> x pass of FFT(h) -> exchange into A
+//   -> z pass, y pass, weighted by b into the lane's spectral sums, which stay
+//   in registers over all directions of the slice.
+// R is free again when the second exchange's barrier completes, and A when
+// the first one's does, so a term needs two cluster barriers.
+template <typename R, int N, int C> struct VssHGeo {
+  using G = HalfGeo<N, C>;
+  static constexpr bool SPLIT = sizeof(R) == 4;
+  static constexpr int RT = 4 * G::P * N;          // row factors of M_u, M_v
+  static constexpr size_t smem =
+      (size_t)(G::SLAB + G::P * N * N + RT + (SPLIT ? 6 * N : 0)) * sizeof(c2_t<R>);
+  static constexpr int by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
+  // threads per SM by the registers of three arrays of N/2 complex values
+  static constexpr int max_threads =
+      SPLIT ? (N <= 16 ? 768 : N == 24 ? 576 : 512) : (N <= 16 ? 512 : N == 24 ? 384 : 256);
+  static constexpr int by_regs = max_threads / G::NT;
+  static constexpr int per_sm =
+      by_smem < by_regs ? (by_smem > 0 ? by_smem : 1) : (by_regs > 0 ? by_regs : 1);
+};
+
+template <typename R, int N, int C>
+__global__ void __launch_bounds__(HalfGeo<N, C>::NT, VssHGeo<R, N, C>::per_sm)
+vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
+  using G = HalfGeo<N, C>;
+  using T = c2_t<R>;
+  constexpr int H = G::H, P = G::P, NT = G::NT;
+  constexpr bool SPLIT = sizeof(R) == 4;
+  constexpr uint32_t ES = (uint32_t)sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* A = reinterpret_cast<T*>(smem_raw);
+  T* Rb = A + G::SLAB;                 // [P][N x][N z]
+  T* rt = Rb + P * N * N;              // [u, v][lz != H, lz == H][P N]
+  T* uvt = rt + 4 * P * N;             // u_M [3N], v_M [3N] (SPLIT)
+  const int t = threadIdx.x, pp = half_pencil(t), h = half_lane(t);
   const unsigned rank = cluster_rank();
-  const int r = blockIdx.y, e = blockIdx.z % a.nevals;
-  const VssTerms32Pair& P = a.pr[blockIdx.z / a.nevals];
-  const int yl = t / N, zz = t % N, yy = rank * G::P + yl;
-  const T* Fp = P.Fgp + (size_t)e * G::n;
-  const T* Fq = P.Fgq + (size_t)e * G::n;
-  const int Tt = a.Nrho * a.M;
-  auto load_tables = [&](int m) {
-    T* dst = tab + (m & 1) * 12 * N;
-    const int term = r * a.M + m;
-    for (int i = t; i < 6 * N; i += G::NT) {
-      dst[i] = P.ph[(size_t)term * 6 * N + i];
-      dst[6 * N + i] = P.uv[((size_t)e * Tt + term) * 6 * N + i];
+  const int e = blockIdx.z % a.nevals;
+  const VssTermsPair& Pr = a.pr[blockIdx.z / a.nevals];
+  const int r0 = blockIdx.y * a.Nrho / a.NS, r1 = (blockIdx.y + 1) * a.Nrho / a.NS;
+  const int nd = Pr.nd, Tt = a.Nrho * a.M;
+  const size_t slab0 = (size_t)rank * P * N * N;
+  const T* Fp = static_cast<const T*>(Pr.Fp) + (size_t)e * G::n + slab0;
+  const T* Fq = static_cast<const T*>(Pr.Fq) + (size_t)e * G::n + slab0;
+  const int pl = pp / N, c = pp % N;
+  const int lx = rank * P + pl, yy = lx;
+  const int rowb = pl * G::PLANE + c * G::ROW, colb = pl * G::PLANE + c;
+  const int colr = pl * N * N + c;
+  uint32_t rdst[G::GRP];
+#pragma unroll
+  for (int g = 0; g < G::GRP; ++g)
+    rdst[g] = mapa_u32(smem_u32(Rb), (uint32_t)((h * H) / P + g)) +
+              ES * (uint32_t)((P > H ? ((h * H) % P) * N * N : 0) + lx * N + c);
+  const R sy = (yy & 1) ? R(-1) : R(1), sz = (c & 1) ? R(-1) : R(1);
+  const int ez = t % N;                // this thread's lz in the elementwise pass
+  T Qh[H];
+#pragma unroll
+  for (int m = 0; m < H; ++m) Qh[m] = T{R(0), R(0)};
+  // the row factors of a term: one (field, row) per thread
+  auto row_tables = [&](int term) {
+    const int f = t / (P * N), row = t % (P * N);
+    const int x = rank * P + row / N, y = row % N;
+    const T* ph = static_cast<const T*>(Pr.ph) + (size_t)term * 6 * N + f * 3 * N;
+    const T E = cmul(ph[x], ph[N + y]);
+    T fx = T{R(1), R(0)};
+    if (x == H) fx = vss_nu(ph[H]);
+    if (y == H) fx = cmul(fx, vss_nu(ph[N + H]));
+    const T fz = cmul(fx, vss_nu(ph[2 * N + H]));
+    rt[f * 2 * P * N + row] = cmul(E, T{R(0.5) * (R(1) + fx.x), R(0.5) * fx.y});
+    rt[f * 2 * P * N + P * N + row] = cmul(E, T{R(0.5) * (R(1) + fz.x), R(0.5) * fz.y});
+    if constexpr (SPLIT) {
+      const T* uv = Pr.uv + ((size_t)e * Tt + term) * 6 * N;
+      for (int i = t; i < 6 * N; i += NT) uvt[i] = uv[i];
     }
   };
-  uint32_t rb[C], bb[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    rb[c] = mapa_u32(smem_u32(R0), (uint32_t)c);
-    bb[c] = mapa_u32(smem_u32(B), (uint32_t)c);
-  }
-  // y-pass stores of an inverse transform into the peers' receive buffer buf
-  auto push_y = [&](int buf, const T* v) {
-    const int lx = rank * G::P + t / N, z = t % N;
-    const uint32_t off = (uint32_t)(buf * G::SLAB + lx * G::ROW + z) * 8u;
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-      for (int j = 0; j < G::P; ++j)
-        st_cluster(rb[c] + off + (uint32_t)(j * G::PLANE) * 8u, v[c * G::P + j]);
-  };
-  auto col_load = [&](const T* S, T* v) {
-    const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = S[base + k * G::ROW];
-  };
-  for (int j = t; j < G::SLAB; j += G::NT) Qh[j] = T{0.f, 0.f};
-  load_tables(0);
-  __syncthreads();
-  vss32_zpass<N, C>(A, Fp, tab, t, rank);
-  __syncthreads();
 #pragma unroll 1
-  for (int m = 0; m < a.M; ++m) {
-    const T* tb = tab + (m & 1) * 12 * N;
-    const int term = r * a.M + m;
-    T v[N], Xu[N];
-    // T1: y-pass, stores into R0; the z-pass of T2 overlaps them
-    col_load(A, v);
-    __syncthreads();                 // A read; ring slot (m+1)&1 free
-    if (m + 1 < a.M) load_tables(m + 1);
-    fft<float, N, +1>(v);
-    push_y(0, v);
-    cluster_arrive();
-    vss32_zpass<N, C>(A, Fq, tb + 3 * N, t, rank);
+  for (int r = r0; r < r1; ++r)
+#pragma unroll 1
+  for (int d = 0; d < nd; ++d) {
+    const int2 dir = Pr.dirs[d];
+    const int term = r * a.M + dir.x;
+    const T* ph = static_cast<const T*>(Pr.ph) + (size_t)term * 6 * N;
+    row_tables(term);
+    __syncthreads();                   // tables are in place; A is read
+    {
+      const T eu = ph[2 * N + ez], ev = ph[5 * N + ez];
+      const T* gu = rt + (ez == H ? P * N : 0);
+      const T* gv = gu + 2 * P * N;
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const int i = j * NT + t, row = i / N;    // i % N == ez
+        const T u = cmul(cmul(gu[row], eu), Fp[i]);
+        const T w = cmul(cmul(gv[row], ev), Fq[i]);
+        A[row * G::ROW + ez] = T{u.x - w.y, u.y + w.x};
+      }
+    }
     __syncthreads();
-    cluster_wait();
-    {
-      const T* R = R0 + yl * G::PLANE + zz;
+    T v[H];
 #pragma unroll
-      for (int x = 0; x < N; ++x) Xu[x] = R[x * G::ROW];
-    }
-    fft<float, N, +1>(Xu);
-    // T2: y-pass, stores into R1; the z-pass of T1 of the next direction
-    // overlaps them
-    col_load(A, v);
-    __syncthreads();                 // A read; the tables of m+1 are stored
-    fft<float, N, +1>(v);
-    push_y(1, v);
+    for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+    fft_half_dit<R, N, +1>(v, h);
+#pragma unroll
+    for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+    fft_half_dit<R, N, +1>(v, h);
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+      st_cluster(rdst[P > H ? 0 : m / P] + ES * (uint32_t)((P > H ? m : m % P) * N * N),
+                 v[m]);
     cluster_arrive();
-    if (m + 1 < a.M) vss32_zpass<N, C>(A, Fp, tab + ((m + 1) & 1) * 12 * N, t, rank);
-    cluster_wait();
+    // u_i + i v_i of this lane's points while the exchange completes
+    T pi[H];
     {
-      const T* R = R0 + G::SLAB + yl * G::PLANE + zz;
+      const T* rp = static_cast<const T*>(Pr.rho) + ((size_t)e * Tt + term) * 3 * N * N;
+      const T rx = rp[yy * N + c];
+      const T* rY = rp + N * N + c + h * H * N;
+      const T* rZ = rp + 2 * N * N + yy + h * H * N;
 #pragma unroll
-      for (int x = 0; x < N; ++x) v[x] = R[x * G::ROW];
+      for (int m = 0; m < H; ++m) {
+        const T ry = rY[m * N], rz = rZ[m * N];
+        const R xs = (m & 1) ? R(-1) : R(1);
+        pi[m].x = sz * rz.x + (sy * ry.x + xs * rx.x);
+        pi[m].y = sz * rz.y + (sy * ry.y + xs * rx.y);
+      }
     }
-    fft<float, N, +1>(v);            // X_v
-    {
-      const T* ut = tb + 6 * N;
-      const T* vt = tb + 9 * N;
-      const T uyz = cmul(ut[N + yy], ut[2 * N + zz]);
-      const T vyz = cmul(vt[N + yy], vt[2 * N + zz]);
+    cluster_wait();
 #pragma unroll
-      for (int x = 0; x < N; ++x) {
-        const T uM = cmul(ut[x], uyz), vM = cmul(vt[x], vyz);
-        const T Xv = v[x];
+    for (int m = 0; m < H; ++m) v[m] = Rb[colr + (2 * m + h) * N];
+    fft_half_dit<R, N, +1>(v, h);
+    if constexpr (SPLIT) {
+      const T uyz = cmul(uvt[N + yy], uvt[2 * N + c]);
+      const T vyz = cmul(uvt[4 * N + yy], uvt[5 * N + c]);
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const T uM = cmul(uvt[h * H + m], uyz), vM = cmul(uvt[3 * N + h * H + m], vyz);
+        const T Xu = T{v[m].x, pi[m].x}, Xv = T{v[m].y, pi[m].y};
         const T a1 = cmul(uM, Xv);
-        const T a2 = cmul(Xu[x], make_float2(vM.x + Xv.x, vM.y + Xv.y));
-        v[x] = make_float2(a1.x + a2.x, a1.y + a2.y);
+        const T a2 = cmul(Xu, T{vM.x + Xv.x, vM.y + Xv.y});
+        v[m] = T{a1.x + a2.x, a1.y + a2.y};
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < H; ++m)
+        v[m] = cmul(T{v[m].x, pi[m].x}, T{v[m].y, pi[m].y});
+    }
+    fft_half_dif<R, N, -1>(v, h);
+    {
+      const uint32_t a0 = smem_u32(A) + ES * (uint32_t)(yy * G::ROW + c);
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const int l = 2 * m + h;
+        st_cluster(mapa_u32(a0, (uint32_t)(l / P)) + ES * (uint32_t)((l % P) * G::PLANE), v[m]);
       }
     }
-    // T3: forward x-pass, stores into the peers' B, then y- and z-passes
-    // on B and the weighted accumulation into Qhat
-    fft<float, N, -1>(v);
-    {
-      const uint32_t off = (uint32_t)(yy * G::ROW + zz) * 8u;
+    cluster_sync_all();
 #pragma unroll
-      for (int c = 0; c < C; ++c)
+    for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+    fft_half_dit<R, N, -1>(v, h);
 #pragma unroll
-        for (int j = 0; j < G::P; ++j)
-          st_cluster(bb[c] + off + (uint32_t)(j * G::PLANE) * 8u, v[c * G::P + j]);
-    }
-    cluster_arrive();
-    cluster_wait();
-    {
-      T w2[N];
-      col_load(B, w2);
-      fft<float, N, -1>(w2);
-      const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-      for (int k = 0; k < N; ++k) B[base + k * G::ROW] = w2[k];
-    }
+    for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
     __syncthreads();
-    {
-      const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
-      const int base = pl * G::PLANE + ly * G::ROW;
-      T w2[N];
 #pragma unroll
-      for (int k = 0; k < N; ++k) w2[k] = B[base + k];
-      fft<float, N, -1>(w2);
-      const T* brow = P.b + (size_t)term * G::n + ((size_t)lx * N + ly) * N;
+    for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+    fft_half_dit<R, N, -1>(v, h);
+    // lane's points (lx, ly = h H + m, lz = c)
+    const size_t o = slab0 + (size_t)pl * N * N + (size_t)h * H * N + c;
+    const T* b1 = static_cast<const T*>(Pr.b) + (size_t)term * G::n + o;
+    const T* b2 = dir.y >= 0
+        ? static_cast<const T*>(Pr.b) + (size_t)(r * a.M + dir.y) * G::n + o : nullptr;
+    const R wr = SPLIT ? R(1) : (R)a.w[r];
 #pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const T pr = cmul(w2[k], brow[k]);
-        Qh[base + k].x += pr.x;
-        Qh[base + k].y += pr.y;
-      }
+    for (int m = 0; m < H; ++m) {
+      T b = b1[(size_t)m * N];
+      if (b2) { const T q = b2[(size_t)m * N]; b.x += q.x; b.y += q.y; }
+      const T x = cmul(v[m], b);
+      Qh[m].x += wr * x.x;
+      Qh[m].y += wr * x.y;
     }
   }
-  __syncthreads();
-  const float wr = (float)a.w[r];
-  T* H = P.H + ((size_t)e * a.Nrho + r) * G::n + (size_t)rank * G::P * N * N;
-  for (int j = t; j < G::P * N * N; j += G::NT) {
-    const T q = Qh[slab_index<N, C>(j)];
-    H[j] = make_float2(wr * q.x, wr * q.y);
-  }
+  const R wo = SPLIT ? (R)a.w[r0] : R(1);
+  T* Ho = static_cast<T*>(Pr.H) + ((size_t)e * a.NS + blockIdx.y) * G::n + slab0 +
+          (size_t)pl * N * N + (size_t)h * H * N + c;
+#pragma unroll
+  for (int m = 0; m < H; ++m) Ho[(size_t)m * N] = T{wo * Qh[m].x, wo * Qh[m].y};
+  cluster_sync_all();  // no CTA leaves while peers may still write into it
 }
 
 }  // namespace dgfs
