@@ -31,7 +31,7 @@ struct DgAdvectArgs {
   const double* c0;         // [N] velocity grid; c_x of v = c0[v / (N*N)]
   const double* invjac;     // [Ne]
   const double* f0[2];      // [Nv] boundary Maxwellians (left, right)
-  const double* nden;       // [2] wall densities (from dg_wall_final_kernel)
+  const double* nden;       // [2] wall densities (from dg_wall_kernel)
   int bc[2];                // boundary kinds (left, right)
   double bc_ux[2];          // wall x-velocities
   double nl[2];             // outward normals (-1, +1)
@@ -173,12 +173,14 @@ __device__ __forceinline__ double wall_expr_maxwellian(const DgAdvectArgs& a,
 // (updateBC of dgfs-wall-diffuse.mako with the two gpuarray.sum of
 // std/bc.py:63-76), in a deterministic order.
 // Grid (kWallCh chunks of the velocity grid, 2 sides): partial sums
-// [2][kWallCh][2]; then one thread per side adds them in a fixed order (one
-// CTA per side would leave the reduction latency-bound on two SMs).
+// [2][kWallCh][2]; the last CTA to finish adds them in a fixed order (one CTA
+// per side would leave the reduction latency-bound on two SMs; a second
+// launch for the sum of 64 numbers cost 3.5 us).  `done` counts CTAs and is
+// zero again afterwards.
 constexpr int kWallCh = 32;
-__global__ void __launch_bounds__(256) dg_wall_partial_kernel(DgAdvectArgs a,
-                                                              double cw,
-                                                              double* part) {
+__global__ void __launch_bounds__(256) dg_wall_kernel(DgAdvectArgs a, double cw,
+                                                      double* part, double* nden,
+                                                      unsigned* done) {
   const int ch = blockIdx.x, side = blockIdx.y, t = threadIdx.x;
   __shared__ double rn[256], rd[256];
   double sn = 0, sd = 0;
@@ -206,22 +208,24 @@ __global__ void __launch_bounds__(256) dg_wall_partial_kernel(DgAdvectArgs a,
     if (t < s2) { rn[t] += rn[t + s2]; rd[t] += rd[t + s2]; }
     __syncthreads();
   }
+  __shared__ bool last;
   if (t == 0) {
     part[(side * kWallCh + ch) * 2] = rn[0];
     part[(side * kWallCh + ch) * 2 + 1] = rd[0];
+    __threadfence();
+    last = atomicAdd(done, 1u) == 2 * kWallCh - 1;
   }
-}
-
-__global__ void dg_wall_final_kernel(DgAdvectArgs a, const double* part,
-                                     double* nden) {
-  const int side = threadIdx.x;
-  if (side >= 2) return;
-  double rn = 0, rd = 0;
-  for (int c = 0; c < kWallCh; ++c) {
-    rn += part[(side * kWallCh + c) * 2];
-    rd += part[(side * kWallCh + c) * 2 + 1];
+  __syncthreads();
+  if (last && t < 2) {
+    __threadfence();
+    double n = 0, d = 0;
+    for (int c = 0; c < kWallCh; ++c) {
+      n += __ldcg(part + (t * kWallCh + c) * 2);
+      d += __ldcg(part + (t * kWallCh + c) * 2 + 1);
+    }
+    nden[t] = (a.bc[t] == kBcWall || a.bc[t] == kBcWallExpr) ? -(n / d) : 0.0;
+    if (t == 0) *done = 0;
   }
-  nden[side] = (a.bc[side] == kBcWall || a.bc[side] == kBcWallExpr) ? -(rn / rd) : 0.0;
 }
 
 __device__ __forceinline__ double dg_ghost(const DgAdvectArgs& a, int side,
@@ -249,17 +253,23 @@ __device__ __forceinline__ double dg_ghost(const DgAdvectArgs& a, int side,
 // ux[k][e][v] = ((D u)[k] * (-c) - jL[e+1] gRD[k] + jR[e] gLD[k]) * invjac[e]
 // with jL = 0.5|c|(uL-uR) + 0.5c(uR-uL), jR = 0.5|c|(uL-uR) + 0.5c(uL-uR)
 // at each face (uL: state on its left, uR: on its right).  One thread per
-// velocity point walks the elements.
+// velocity point walks the elements [blockIdx.y len, + len) and reads one
+// element more on either side for the traces.  Bound: HBM; the elements are
+// split so that every SM holds enough threads to keep its share of the
+// bandwidth in flight (N=48, Ne=32, K=3: 39.7 us with one walk over all 32
+// elements, 432 CTAs on 148 SMs).
 template <int K>
-__global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a) {
+__global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a, int len) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= a.Nv) return;
   const int Ne = a.Ne, Nv = a.Nv;
+  const int e0 = blockIdx.y * len, e1 = min(Ne, e0 + len);
   const double cx = a.c0[v / (a.N * a.N)];
   const double ac = 0.5 * fabs(cx), hc = 0.5 * cx;
   double ue[K], un[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) ue[k] = ld(a.u, a.f_double, ((size_t)k * Ne) * Nv + v);
+  for (int k = 0; k < K; ++k)
+    ue[k] = ld(a.u, a.f_double, ((size_t)k * Ne + e0) * Nv + v);
   auto tl = [&](const double* w) {
     double s = 0;
 #pragma unroll
@@ -276,19 +286,24 @@ __global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a) {
   const double* Dv = (a.upwind == 1 && cx < 0) ? a.D2 : a.D;
   // traces at the two ends of the domain, for the swapped (periodic) ghosts
   double uEnd0 = 0, uEnd1 = 0;
-  if (a.swap) {
+  auto trace_of = [&](int e, bool right) {
     double ul[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      ul[k] = ld(a.u, a.f_double, ((size_t)k * Ne + Ne - 1) * Nv + v);
-    uEnd1 = tr(ul);
-    uEnd0 = tl(ue);
+    for (int k = 0; k < K; ++k) ul[k] = ld(a.u, a.f_double, ((size_t)k * Ne + e) * Nv + v);
+    return right ? tr(ul) : tl(ul);
+  };
+  if (a.swap) {
+    if (e0 == 0) uEnd1 = trace_of(Ne - 1, true);
+    if (e1 == Ne) uEnd0 = trace_of(0, false);
   }
-  // face 0: ghost on the left, element 0 on the right
+  // face e0: the ghost or the previous element on its left
   double uRf = tl(ue);
-  double uLf = dg_ghost(a, 0, v, cx, a.swap ? uEnd1 : uRf);
-  double jR = ac * (uLf - uRf) + hc * (uLf - uRf);
-  for (int e = 0; e < Ne; ++e) {
+  double uLf = e0 == 0 ? dg_ghost(a, 0, v, cx, a.swap ? uEnd1 : uRf)
+                       : trace_of(e0 - 1, true);
+  const double jd0 = ac * (uLf - uRf);
+  double jR = jd0 + hc * (uLf - uRf);
+#pragma unroll 2
+  for (int e = e0; e < e1; ++e) {
     // face e+1
     const double uL1 = tr(ue);
     double uR1;
@@ -339,19 +354,60 @@ struct AxnpbyArgs {
   size_t n;
 };
 
+__device__ __forceinline__ double axnpby_one(const AxnpbyArgs& a, double x0,
+                                             const double* x) {
+  double s = 0.0;
+  for (int j = 0; j < a.nterms; ++j) s = (j == 0) ? a.a[0] * x[0] : s + a.a[j] * x[j];
+  if (a.a0 == 0.0) return s;
+  if (a.a0 == 1.0) return x0 + s;
+  return a.a0 * x0 + s;
+}
+
+// Any size and alignment: one element per thread and step.
 __global__ void axnpby_kernel(AxnpbyArgs a) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (size_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < a.nterms; ++j) {
-      const double v = ld(a.x[j], a.f_double, i);
-      s = (j == 0) ? a.a[0] * v : s + a.a[j] * v;
+    double x[kAxMax];
+    for (int j = 0; j < a.nterms; ++j) x[j] = ld(a.x[j], a.f_double, i);
+    st(a.x0, a.f_double, i,
+       axnpby_one(a, a.a0 == 0.0 ? 0.0 : ld(a.x0, a.f_double, i), x));
+  }
+}
+
+// 16-byte aligned operands, a whole number of 16-byte groups: two groups per
+// thread and operand, all loads in flight before the first sum.  Bound: HBM
+// (two terms into a third array of 10.6 M doubles: 56 us with 8-byte loads).
+template <typename T, int NTERMS>
+__global__ void __launch_bounds__(256) axnpby_vec_kernel(AxnpbyArgs a) {
+  constexpr int VE = 16 / sizeof(T), U = 2;
+  struct alignas(16) V { T v[VE]; };
+  const size_t nv = a.n / VE, i0 = (size_t)blockIdx.x * (256 * U) + threadIdx.x;
+  V x[U][NTERMS], y[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const size_t i = i0 + u * 256;
+    if (i < nv) {
+#pragma unroll
+      for (int j = 0; j < NTERMS; ++j) x[u][j] = static_cast<const V*>(a.x[j])[i];
+      if (a.a0 != 0.0) y[u] = static_cast<const V*>(a.x0)[i];
     }
-    double r;
-    if (a.a0 == 0.0) r = s;
-    else if (a.a0 == 1.0) r = ld(a.x0, a.f_double, i) + s;
-    else r = a.a0 * ld(a.x0, a.f_double, i) + s;
-    st(a.x0, a.f_double, i, r);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const size_t i = i0 + u * 256;
+    if (i < nv) {
+      V r;
+#pragma unroll
+      for (int e = 0; e < VE; ++e) {
+        double s = a.a[0] * (double)x[u][0].v[e];
+#pragma unroll
+        for (int j = 1; j < NTERMS; ++j) s = s + a.a[j] * (double)x[u][j].v[e];
+        if (a.a0 == 1.0) s = (double)y[u].v[e] + s;
+        else if (a.a0 != 0.0) s = a.a0 * (double)y[u].v[e] + s;
+        r.v[e] = (T)s;
+      }
+      static_cast<V*>(a.x0)[i] = r;
+    }
   }
 }
 

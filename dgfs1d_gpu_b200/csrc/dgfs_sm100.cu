@@ -231,9 +231,9 @@ template <int N> struct VhsClusters;
 // per CTA and a 16-CTA epilogue cluster 34 KB, so two (four) CTAs share an SM
 // and a 24-point batch runs in one wave of each.
 template <> struct VhsClusters<8> { static constexpr int c64 = 1, ch32 = 1, c32 = 1, cpro = 1, cepi = 1; };
-template <> struct VhsClusters<16> { static constexpr int c64 = 2, ch32 = 1, c32 = 1, cpro = 2, cepi = 2; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 6, ch32 = 2, c32 = 3, cpro = 4, cepi = 4; };
-template <> struct VhsClusters<32> { static constexpr int c64 = 16, ch32 = 8, c32 = 4, cpro = 8, cepi = 16; };
+template <> struct VhsClusters<16> { static constexpr int c64 = 2, ch32 = 1, c32 = 1, cpro = 4, cepi = 4; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 6, ch32 = 2, c32 = 3, cpro = 6, cepi = 6; };
+template <> struct VhsClusters<32> { static constexpr int c64 = 16, ch32 = 8, c32 = 4, cpro = 16, cepi = 16; };
 // N=48: 16-CTA clusters of 3 planes
 template <> struct VhsClusters<48> { static constexpr int c64 = 16, ch32 = 16, c32 = 16, cpro = 16, cepi = 16; };
 
@@ -609,9 +609,6 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
   constexpr int C32 = VhsClusters<N>::c32;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
-  using GPRO = Geo<N, CPRO>;
-  using GEPI = Geo<N, CEPI>;
-  using G32 = Geo<N, C32>;
   const bool fp32 = h->precision == DGFS_PREC_FP32;
   int rc;
   int evi = 0;
@@ -630,7 +627,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     if (bl) { a.g = bl->g; a.alpha = bl->alpha; a.beta = bl->beta; }
     const size_t smem = prologue_smem<N, CPRO>();
     if ((rc = launch_cluster(vhs_prologue_kernel<N, CPRO>, dim3(CPRO, nevals),
-                             dim3(GPRO::NT), CPRO, smem, st, a)))
+                             dim3(HalfGeo<N, CPRO>::NT), CPRO, smem, st, a)))
       return rc;
   }
   mark();
@@ -731,7 +728,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     if (bl) { a.bilinear = 1; a.cg = bl->cg; a.cl = bl->cl; }
     const size_t smem = epilogue_smem<N, CEPI>();
     if ((rc = launch_cluster(vhs_epilogue_kernel<N, CEPI>, dim3(CEPI, nevals),
-                             dim3(GEPI::NT), CEPI, smem, st, a)))
+                             dim3(HalfGeo<N, CEPI>::NT), CEPI, smem, st, a)))
       return rc;
   }
   mark();
@@ -1179,6 +1176,7 @@ struct dgfs_dg_s {
   double* part = nullptr;  // residual partials
   double* part_h = nullptr;
   double* wpart = nullptr;  // wall-density partials [2][kWallCh][2]
+  unsigned* wdone = nullptr;  // finished CTAs of the wall kernel
   double* lim = nullptr;    // limiter tables: wavg [K] | wdr [K] | dx [K][Ne] | h [Ne]
   double* mpart = nullptr;  // penalty-moment partials [mpts][kPmCh][<= 14]
   int mpts = 0;
@@ -1186,7 +1184,7 @@ struct dgfs_dg_s {
 
 static void free_dg(dgfs_dg_s* h) {
   void* ptrs[] = {h->c0, h->invjac, h->f0[0], h->f0[1], h->nden, h->im, h->part,
-                  h->wpart, h->mpart, h->lim};
+                  h->wpart, h->wdone, h->mpart, h->lim};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->part_h) cudaFreeHost(h->part_h);
@@ -1242,6 +1240,9 @@ extern "C" int dgfs_dg_create(const dgfs_dg_desc* d, dgfs_dg_handle* out) {
   if (e1 == cudaSuccess) e1 = cudaMalloc(&h->part, 2 * 1024 * sizeof(double));
   if (e1 == cudaSuccess) e1 = cudaMallocHost(&h->part_h, 2 * 1024 * sizeof(double));
   if (e1 == cudaSuccess) e1 = cudaMalloc(&h->wpart, 2 * kWallCh * 2 * sizeof(double));
+  if (e1 == cudaSuccess) e1 = cudaMalloc(&h->wdone, sizeof(unsigned));
+  if (e1 == cudaSuccess) e1 = cudaMemset(h->wdone, 0, sizeof(unsigned));
+  if (e1 == cudaSuccess) e1 = cudaMemset(h->nden, 0, 2 * sizeof(double));
   h->mpts = std::max(K, d->Nqr) * Ne;
   if (e1 == cudaSuccess)
     e1 = cudaMalloc(&h->mpart, (size_t)h->mpts * kPmCh * kPmMaxNa * sizeof(double));
@@ -1272,19 +1273,24 @@ extern "C" int dgfs_dg_advect(dgfs_dg_handle h, const void* u, void* ux,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   DgAdvectArgs a = h->base;
   a.u = u; a.ux = ux; a.f_double = dtype == DGFS_F64;
-  dg_wall_partial_kernel<<<dim3(kWallCh, 2), 256, 0, st>>>(a, h->cw, h->wpart);
-  dg_wall_final_kernel<<<1, 32, 0, st>>>(a, h->wpart, h->nden);
-  DGFS_CUDA(cudaGetLastError());
-  const dim3 grid((a.Nv + 255) / 256), block(256);
+  auto is_wall = [&](int s) { return a.bc[s] == kBcWall || a.bc[s] == kBcWallExpr; };
+  if (is_wall(0) || is_wall(1)) {   // else the densities stay zero
+    dg_wall_kernel<<<dim3(kWallCh, 2), 256, 0, st>>>(a, h->cw, h->wpart, h->nden, h->wdone);
+    DGFS_CUDA(cudaGetLastError());
+  }
+  // split the element walk until about 1536 threads per SM are in flight
+  const int want = (148 * 1536 + a.Nv - 1) / a.Nv;
+  const int len = std::max(1, a.Ne / std::max(1, std::min(a.Ne, want)));
+  const dim3 grid((a.Nv + 255) / 256, (a.Ne + len - 1) / len), block(256);
   switch (a.K) {
-    case 1: dg_advect_kernel<1><<<grid, block, 0, st>>>(a); break;
-    case 2: dg_advect_kernel<2><<<grid, block, 0, st>>>(a); break;
-    case 3: dg_advect_kernel<3><<<grid, block, 0, st>>>(a); break;
-    case 4: dg_advect_kernel<4><<<grid, block, 0, st>>>(a); break;
-    case 5: dg_advect_kernel<5><<<grid, block, 0, st>>>(a); break;
-    case 6: dg_advect_kernel<6><<<grid, block, 0, st>>>(a); break;
-    case 7: dg_advect_kernel<7><<<grid, block, 0, st>>>(a); break;
-    default: dg_advect_kernel<8><<<grid, block, 0, st>>>(a); break;
+    case 1: dg_advect_kernel<1><<<grid, block, 0, st>>>(a, len); break;
+    case 2: dg_advect_kernel<2><<<grid, block, 0, st>>>(a, len); break;
+    case 3: dg_advect_kernel<3><<<grid, block, 0, st>>>(a, len); break;
+    case 4: dg_advect_kernel<4><<<grid, block, 0, st>>>(a, len); break;
+    case 5: dg_advect_kernel<5><<<grid, block, 0, st>>>(a, len); break;
+    case 6: dg_advect_kernel<6><<<grid, block, 0, st>>>(a, len); break;
+    case 7: dg_advect_kernel<7><<<grid, block, 0, st>>>(a, len); break;
+    default: dg_advect_kernel<8><<<grid, block, 0, st>>>(a, len); break;
   }
   DGFS_CUDA(cudaGetLastError());
   return DGFS_OK;
@@ -1367,12 +1373,30 @@ extern "C" int dgfs_axnpby(void* x0, int64_t n, int32_t dtype, double a0,
     a.a[i] = as[i];
   }
   if (n == 0) return DGFS_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int es = dtype == DGFS_F64 ? 8 : 4;
+  uintptr_t align = (uintptr_t)x0 | (uintptr_t)(n * es);
+  for (int i = 0; i < nterms; ++i) align |= (uintptr_t)xs[i];
+  if (align % 16 == 0) {
+    const unsigned blocks = (unsigned)(((size_t)n * es / 16 + 511) / 512);
+#define DGFS_AX(T)                                                        \
+  switch (nterms) {                                                       \
+    case 1: axnpby_vec_kernel<T, 1><<<blocks, 256, 0, st>>>(a); break;    \
+    case 2: axnpby_vec_kernel<T, 2><<<blocks, 256, 0, st>>>(a); break;    \
+    case 3: axnpby_vec_kernel<T, 3><<<blocks, 256, 0, st>>>(a); break;    \
+    default: axnpby_vec_kernel<T, 4><<<blocks, 256, 0, st>>>(a); break;   \
+  }
+    if (es == 8) { DGFS_AX(double) } else { DGFS_AX(float) }
+#undef DGFS_AX
+    DGFS_CUDA(cudaGetLastError());
+    return DGFS_OK;
+  }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t want = ((size_t)n + 255) / 256;
   const unsigned blocks = (unsigned)std::min<size_t>(want, (size_t)sms * 16);
-  axnpby_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  axnpby_kernel<<<blocks, 256, 0, st>>>(a);
   DGFS_CUDA(cudaGetLastError());
   return DGFS_OK;
 }
@@ -1699,7 +1723,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
       a.Fny64 = static_cast<double2*>(h->Fny[s]);
     }
     if ((rc = launch_cluster(vhs_prologue_kernel<N, CPRO>, dim3(CPRO, nevals),
-                             dim3(Geo<N, CPRO>::NT), CPRO, prologue_smem<N, CPRO>(), st,
+                             dim3(HalfGeo<N, CPRO>::NT), CPRO, prologue_smem<N, CPRO>(), st,
                              a)))
       return rc;
   }
@@ -1770,7 +1794,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
     ea.ReLft[k] = ReLf(k); ea.pref[k] = pair(k).prefac;
   }
   return launch_cluster(vhs_epilogue_kernel<N, CEPI>, dim3(CEPI, nevals),
-                        dim3(Geo<N, CEPI>::NT), CEPI, epilogue_smem<N, CEPI>(), st, ea);
+                        dim3(HalfGeo<N, CEPI>::NT), CEPI, epilogue_smem<N, CEPI>(), st, ea);
 }
 
 // Every point of a call, max_evals at a time.

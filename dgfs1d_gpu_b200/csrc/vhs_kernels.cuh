@@ -154,138 +154,148 @@ __device__ __forceinline__ double load_real(const void* p, int is_double,
 }
 
 // ---------------------------------------------------------------------------
-// Prologue: one cluster (C CTAs, FP64) per eval.  Up to N=32 one slab per CTA
-// serves both transforms (the exchange of the inverse transform waits for
-// every CTA to have read its slab), which keeps a 24-point batch in one wave.
+// Prologue: one cluster (C CTAs, FP64) per eval, two lanes per pencil, one
+// slab per CTA that serves both transforms (the exchange of the inverse
+// transform waits until every CTA has read its slab).  Bound: latency (loads,
+// two exchanges, FP64 passes of few warps); two lanes per pencil double the
+// warps, and the moment sums are shuffle trees.
 // ---------------------------------------------------------------------------
-// Whether the prologue and epilogue keep one slab per CTA (exchange after a
-// cluster barrier) or a separate receive slab.  One slab pays off where it
-// lets more CTAs share an SM (N <= 32); at N=48 registers allow one CTA per
-// SM either way and the second slab saves the barrier.
-template <int N> struct OneSlab { static constexpr bool value = N <= 32; };
-
-// Shared memory: the slab(s), the moment partials [5][NT] + [5] and the 1-D
-// Maxwellian factors [3N] (doubles; with two slabs they borrow the receive
-// slab, which peers write only two cluster barriers later), the Maxwellian
-// spectra [3][N] (complex) and the moments [8].
+// Shared memory: the slab, per-warp moment partials [32][5] + totals, the 1-D
+// Maxwellian factors [3N], spectra [3][N] (complex) and the N twiddles of
+// their direct transform.
 template <int N, int C>
 constexpr size_t prologue_smem() {
-  // ... + the N twiddles of the 1-D spectra (double2)
-  return OneSlab<N>::value
-             ? (size_t)Geo<N, C>::SLAB * sizeof(double2) +
-                   (size_t)(6 * Geo<N, C>::NT + 8 + 3 * N) * sizeof(double) +
-                   (size_t)3 * N * sizeof(double2) + 8 * sizeof(double) +
-                   (size_t)N * sizeof(double2)
-             : (size_t)2 * Geo<N, C>::SLAB * sizeof(double2) +
-                   (size_t)3 * N * sizeof(double2) + 8 * sizeof(double) +
-                   (size_t)N * sizeof(double2);
+  return (size_t)(HalfGeo<N, C>::SLAB + 4 * N) * sizeof(double2) +
+         (size_t)(3 * N + 32 * 5 + 24) * sizeof(double);
 }
 template <int N, int C>
 constexpr size_t epilogue_smem() {
-  return (size_t)(OneSlab<N>::value ? 1 : 2) * Geo<N, C>::SLAB * sizeof(double2);
+  return (size_t)HalfGeo<N, C>::SLAB * sizeof(double2) + (32 * 5 + 8) * sizeof(double);
+}
+// CTAs per SM by the registers of a lane's N/2 FP64 values
+template <int N, int C> constexpr int fp64_per_sm() {
+  constexpr int thr = N <= 16 ? 512 : N <= 32 ? 384 : 288;
+  constexpr int r = thr / HalfGeo<N, C>::NT;
+  constexpr int sm = (int)((size_t)(227 * 1024) / (prologue_smem<N, C>() + 1024));
+  return r < 1 ? 1 : r < sm ? r : sm < 1 ? 1 : sm;
+}
+
+// Cluster-wide sums of five values per thread, in a fixed order (shuffle tree,
+// warps in order, CTAs in order), so that every CTA gets the same bits.
+// red: [32][5] partials, [5] this CTA's totals (read by the peers).
+template <int NT, int C>
+__device__ __forceinline__ void cluster_sum5(const double* s, double* red, double* tot) {
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  constexpr int NW = (NT + 31) / 32;
+  static_assert(NT % 32 == 0, "whole warps");
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    double v = s[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[w * 5 + k] = v;
+  }
+  __syncthreads();
+  if (t < 5) {
+    double v = 0;
+    for (int i = 0; i < NW; ++i) v += red[i * 5 + t];
+    red[160 + t] = v;
+  }
+  cluster_sync_all();
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    double v = 0;
+    for (int c = 0; c < C; ++c) v += peer_ptr(red, (unsigned)c)[160 + k];
+    tot[k] = v;
+  }
+}
+
+// y pencils of an inverse transform (column in v, y = h H + m) into the
+// owners' slabs, dense Y layout [P][N x][N z].
+template <int N, int C>
+__device__ __forceinline__ void half_push_y(double2* A, int lx, int c, int h,
+                                            const double2* v) {
+  using G = HalfGeo<N, C>;
+  constexpr int H = G::H, P = G::P;
+#pragma unroll
+  for (int m = 0; m < H; ++m) {
+    const int y = h * H + m;
+    st_cluster(mapa_u32(smem_u32(A), (uint32_t)(y / P)) +
+                   16u * (uint32_t)((y % P) * N * N + lx * N + c),
+               v[m]);
+  }
 }
 
 template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT)
+__global__ void __launch_bounds__(HalfGeo<N, C>::NT, fp64_per_sm<N, C>())
 vhs_prologue_kernel(VhsPrologueArgs a) {
-  using G = Geo<N, C>;
+  using G = HalfGeo<N, C>;
   using T = double2;
+  constexpr int H = G::H, P = G::P, NT = G::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool OS = OneSlab<N>::value;
   T* A = reinterpret_cast<T*>(smem_raw);
-  T* Rb = OS ? A : A + G::SLAB;                             // Y-slab receive
-  double* red = OS ? reinterpret_cast<double*>(A + G::SLAB)  // [6 NT + 8 + 3N]
-                   : reinterpret_cast<double*>(Rb);
-  T* mh = OS ? reinterpret_cast<T*>(red + 6 * G::NT + 8 + 3 * N)
-             : A + 2 * G::SLAB;                              // [3][N]
-  double* mom = reinterpret_cast<double*>(mh + 3 * N);      // [8]
-  T* tws = reinterpret_cast<T*>(mom + 8);                   // [N] twiddles
-
-  const int t = threadIdx.x;
+  T* mh = A + G::SLAB;                                  // [3][N]
+  T* tws = mh + 3 * N;                                  // [N] twiddles
+  double* mv = reinterpret_cast<double*>(tws + N);      // [3N] 1-D Maxwellian
+  double* red = mv + 3 * N;                             // [32][5] + [24]
+  const int t = threadIdx.x, pp = half_pencil(t), h = half_lane(t);
   const unsigned rank = cluster_rank();
   const int e = blockIdx.y;
-  const int yl = t / N, z = t % N, y = rank * G::P + yl;
+  const int pl = pp / N, c = pp % N, y = rank * P + pl, lx = y;
+  const int rowb = pl * G::PLANE + c * G::ROW, colb = pl * G::PLANE + c;
   const size_t fbase = (size_t)slot_of(a.src_slots, a.src_base, e) * G::n;
   const void* fin = a.f_list ? a.f_list[e] : a.f;
 
-  T v[N];
+  T v[H];
 #pragma unroll
-  for (int x = 0; x < N; ++x) {
-    const size_t idx = fbase + ((size_t)x * N + y) * N + z;
-    v[x].x = a.g ? a.alpha * load_real(fin, a.f_double, idx) +
+  for (int m = 0; m < H; ++m) {
+    const size_t idx = fbase + ((size_t)(h * H + m) * N + y) * N + c;
+    v[m].x = a.g ? a.alpha * load_real(fin, a.f_double, idx) +
                        a.beta * load_real(a.g, a.f_double, idx)
                  : load_real(fin, a.f_double, idx);
-    v[x].y = 0.0;
+    v[m].y = 0.0;
   }
 
   if (a.split) {
-    // moments of f on the grid (sum f, sum f c, sum f |c|^2); deterministic
-    // two-level reduction: per-thread partials -> CTA -> cluster.
-    double s[5] = {0, 0, 0, 0, 0};
-    const double cy = a.c0[y], cz = a.c0[z];
+    // moments of f on the grid (sum f, sum f c, sum f |c|^2)
+    double s[5] = {0, 0, 0, 0, 0}, mom[5];
+    const double cy = a.c0[y], cz = a.c0[c];
 #pragma unroll
-    for (int x = 0; x < N; ++x) {
-      const double cx = a.c0[x], fv = v[x].x;
+    for (int m = 0; m < H; ++m) {
+      const double cx = a.c0[h * H + m], fv = v[m].x;
       s[0] += fv;
       s[1] += fv * cx;
       s[2] += fv * cy;
       s[3] += fv * cz;
       s[4] += fv * (cx * cx + cy * cy + cz * cz);
     }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) red[k * G::NT + t] = s[k];
     // the spectra's twiddles into shared memory (read below with a
     // different index on every lane, which constant memory serialises)
-    for (int i = t; i < N; i += G::NT) tws[i] = c_tw64[tw_offset(N) + i];
-    __syncthreads();
-    // this CTA's partial of moment k = t / 8: eight lanes each sum a strided
-    // eighth of the thread partials, then a three-step xor tree inside the
-    // eight-lane group (a fixed order: every run adds the same operands)
-    if (t < 40) {
-      const int k = t >> 3, sub = t & 7;
-      double acc = 0;
-      for (int i = sub; i < G::NT; i += 8) acc += red[k * G::NT + i];
-      const unsigned grp = t < 32 ? 0xFFFFFFFFu : 0xFFu;  // lanes in this branch
-      acc += __shfl_xor_sync(grp, acc, 4, 8);
-      acc += __shfl_xor_sync(grp, acc, 2, 8);
-      acc += __shfl_xor_sync(grp, acc, 1, 8);
-      if (sub == 0) red[5 * G::NT + k] = acc;
+    for (int i = t; i < N; i += NT) tws[i] = c_tw64[tw_offset(N) + i];
+    cluster_sum5<NT, C>(s, red, mom);
+    double rho = mom[0] * a.cw, u[3] = {0, 0, 0}, Tm = 1;
+    if (rho > 1e-300) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) u[k] = mom[1 + k] * a.cw / rho;
+      Tm = (2.0 / 3.0) * (mom[4] * a.cw / rho - (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]));
+      if (!(Tm > 1e-6)) { rho = 0; Tm = 1; }  // no useful Maxwellian
+    } else {
+      rho = 0;
     }
-    cluster_sync_all();
-    if (t < 5) {
-      double acc = 0;
-      for (int c = 0; c < C; ++c)
-        acc += peer_ptr(red, (unsigned)c)[5 * G::NT + t];
-      mom[t] = acc;
+    if (t == 0 && rank == 0 && a.moments) {
+      double* out = a.moments + (size_t)e * 5;
+      out[0] = rho; out[1] = u[0]; out[2] = u[1]; out[3] = u[2]; out[4] = Tm;
     }
-    __syncthreads();
-    if (t == 0) {
-      double rho = mom[0] * a.cw, ux = 0, uy = 0, uz = 0, Tm = 1;
-      if (rho > 1e-300) {
-        ux = mom[1] * a.cw / rho; uy = mom[2] * a.cw / rho; uz = mom[3] * a.cw / rho;
-        Tm = (2.0 / 3.0) * (mom[4] * a.cw / rho - (ux * ux + uy * uy + uz * uz));
-        if (!(Tm > 1e-6)) { rho = 0; Tm = 1; }  // no useful Maxwellian
-      } else {
-        rho = 0;
-      }
-      mom[0] = rho; mom[1] = ux; mom[2] = uy; mom[3] = uz; mom[4] = Tm;
-      if (rank == 0 && a.moments)
-        for (int k = 0; k < 5; ++k) a.moments[(size_t)e * 5 + k] = mom[k];
-    }
-    __syncthreads();
-    // 1-D Maxwellian factors (3N values, each computed once; past the moment
-    // partials, which peers read only below offset 5 NT + 5) and their
+    // 1-D Maxwellian factors (3N values, each computed once) and their
     // spectra (direct DFT, table twiddles)
-    double* mv = red + 6 * G::NT + 8;
-    for (int i = t; i < 3 * N; i += G::NT) {
+    for (int i = t; i < 3 * N; i += NT) {
       const int ax = i / N, j = i % N;
-      const double rho = mom[0], Tm = mom[4], u = mom[1 + ax];
       const double amp = (ax == 0) ? rho / pow(M_PI * Tm, 1.5) : 1.0;
-      const double d = a.c0[j] - u;
+      const double d = a.c0[j] - (ax == 0 ? u[0] : ax == 1 ? u[1] : u[2]);
       mv[i] = amp * exp(-d * d / Tm);
     }
     __syncthreads();
-    for (int i = t; i < 3 * N; i += G::NT) {
+    for (int i = t; i < 3 * N; i += NT) {
       const int ax = i / N, k = i % N;
       double re = 0, im = 0;
 #pragma unroll 8
@@ -298,85 +308,98 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
       mh[ax * N + k] = make_double2(re / N, im / N);
     }
     // (visibility of mh is ensured by the barriers below)
+  } else {
+    cluster_sync_all();  // every CTA of the cluster runs before remote stores
   }
 
   // forward x-pass and exchange into X-slabs
-  fft<double, N, -1>(v);
-  push_pencils_to_xslab<double, N, C>(A, t, rank, v);
-  cluster_sync_all();
+  fft_half_dif<double, N, -1>(v, h);
   {
-    T w[N];
-    slab_col_load_fft<double, N, C, -1>(A, t, w);
-    const int base = (t / N) * G::PLANE + (t % N);
+    const uint32_t a0 = smem_u32(A) + 16u * (uint32_t)(y * G::ROW + c);
 #pragma unroll
-    for (int k = 0; k < N; ++k) A[base + k * G::ROW] = w[k];
+    for (int m = 0; m < H; ++m) {
+      const int l = 2 * m + h;
+      st_cluster(mapa_u32(a0, (uint32_t)(l / P)) + 16u * (uint32_t)((l % P) * G::PLANE), v[m]);
+    }
   }
+  cluster_sync_all();
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+  fft_half_dit<double, N, -1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[colb + (h * H + m) * G::ROW] = v[m];
   __syncthreads();
-  slab_row_pass<double, N, C, -1>(A, t);
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+  fft_half_dit<double, N, -1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
   __syncthreads();
 
   // F = FFT(f)/n; write F (FP64) or F_g = F - mhat (FP32); then A <- b2 F
   const double inv_n = 1.0 / (double)G::n;
-  const size_t gbase = (size_t)e * G::n + (size_t)rank * G::P * N * N;
+  const size_t lbase = (size_t)rank * P * N * N, gbase = (size_t)e * G::n + lbase;
 #pragma unroll 4
-  for (int j = t; j < G::P * N * N; j += G::NT) {
-    const int si = slab_index<N, C>(j);
+  for (int j = t; j < P * N * N; j += NT) {
+    const int si = (j / N) * G::ROW + j % N;
+    const int fx = rank * P + j / (N * N), ly = (j / N) % N, lz = j % N;
     T Fv = A[si];
     Fv.x *= inv_n;
     Fv.y *= inv_n;
     if (a.split) {
-      const int lx = rank * G::P + j / (N * N), ly = (j / N) % N, lz = j % N;
-      const T mm = cmul(cmul(mh[lx], mh[N + ly]), mh[2 * N + lz]);
+      const T mm = cmul(cmul(mh[fx], mh[N + ly]), mh[2 * N + lz]);
       float2 g;
       g.x = (float)(Fv.x - mm.x);
       g.y = (float)(Fv.y - mm.y);
       if (a.Fg) static_cast<float2*>(a.Fg)[gbase + j] = g;
       if (a.Fny) {
         float2* ny = a.Fny + (size_t)e * 3 * N * N;
-        if (lx == N / 2) ny[ly * N + lz] = g;
-        if (ly == N / 2) ny[N * N + lx * N + lz] = g;
-        if (lz == N / 2) ny[2 * N * N + lx * N + ly] = g;
+        if (fx == N / 2) ny[ly * N + lz] = g;
+        if (ly == N / 2) ny[N * N + fx * N + lz] = g;
+        if (lz == N / 2) ny[2 * N * N + fx * N + ly] = g;
       }
     } else {
       static_cast<double2*>(a.Fg)[gbase + j] = Fv;
       if (a.Fny64) {
-        const int lx = rank * G::P + j / (N * N), ly = (j / N) % N, lz = j % N;
         double2* ny = a.Fny64 + (size_t)e * 3 * N * N;
-        if (lx == N / 2) ny[ly * N + lz] = Fv;
-        if (ly == N / 2) ny[N * N + lx * N + lz] = Fv;
-        if (lz == N / 2) ny[2 * N * N + lx * N + ly] = Fv;
+        if (fx == N / 2) ny[ly * N + lz] = Fv;
+        if (ly == N / 2) ny[N * N + fx * N + lz] = Fv;
+        if (lz == N / 2) ny[2 * N * N + fx * N + ly] = Fv;
       }
     }
+    if (!a.ReLf) continue;
     if (a.b2c) {
-      Fv = cmul(Fv, a.b2c[(size_t)rank * G::P * N * N + j]);
+      Fv = cmul(Fv, a.b2c[lbase + j]);
     } else {
-      const double b = a.b2[(size_t)rank * G::P * N * N + j];
+      const double b = a.b2[lbase + j];
       Fv.x *= b;
       Fv.y *= b;
     }
     A[si] = Fv;
   }
-  if (a.split && rank == 0)
-    if (a.mhat)
-      for (int i = t; i < 3 * N; i += G::NT) a.mhat[(size_t)e * 3 * N + i] = mh[i];
+  if (a.split && rank == 0 && a.mhat)
+    for (int i = t; i < 3 * N; i += NT) a.mhat[(size_t)e * 3 * N + i] = mh[i];
   if (!a.ReLf) return;   // (no CTA writes to a peer past this point)
   __syncthreads();
-  // loss: Re IFFT(b2 F); the Y-slab exchange reuses the slab once every CTA
-  // of the cluster has read its own
-  slab_row_pass<double, N, C, +1>(A, t);
-  __syncthreads();
-  {
-    T w[N];
-    slab_col_load_fft<double, N, C, +1>(A, t, w);
-    if (OS) cluster_sync_all();
-    push_cols_to_yslab<double, N, C>(Rb, t, rank, w);
-  }
-  cluster_sync_all();
-  yslab_load_pencil<double, N, C>(Rb, t, v);
-  fft<double, N, +1>(v);
+  // loss: Re IFFT(b2 F)
 #pragma unroll
-  for (int x = 0; x < N; ++x)
-    a.ReLf[(size_t)e * G::n + ((size_t)x * N + y) * N + z] = v[x].x;
+  for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+  fft_half_dit<double, N, +1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+  fft_half_dit<double, N, +1>(v, h);
+  cluster_sync_all();    // every CTA has read its slab: exchange into it
+  half_push_y<N, C>(A, lx, c, h, v);
+  cluster_sync_all();
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[pl * N * N + (2 * m + h) * N + c];
+  fft_half_dit<double, N, +1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m)
+    a.ReLf[(size_t)e * G::n + ((size_t)(h * H + m) * N + y) * N + c] = v[m].x;
 }
 
 // ---------------------------------------------------------------------------
@@ -1631,6 +1654,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
             (size_t)rank * P * N * N;
   R* stash = reinterpret_cast<R*>(Hout);
 
+  cluster_arrive();                      // (this CTA is running)
   load_phases(0);
   copy_slab();
   cp_async_wait_all();
@@ -1649,7 +1673,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     }
     if constexpr (SPLIT) load_uv(k);
     fft_half_dit<R, N, +1>(v, h);
-    if (k) cluster_wait();               // every CTA has read its R
+    cluster_wait();                      // every CTA runs and has read its R
 #pragma unroll
     for (int m = 0; m < H; ++m)
       st_cluster(rdst[P > H ? 0 : m / P] + ES * (uint32_t)((P > H ? m : m % P) * N * N),
@@ -1815,216 +1839,127 @@ __global__ void __launch_bounds__(3 * N) vhs_nyq_planes64_kernel(VhsTermsArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// Epilogue: one cluster (FP64) per eval.
+// Epilogue: one cluster (FP64) per eval, two lanes per pencil, one slab per
+// CTA as in the prologue.  Bound: latency; the sum over the radial spectra is
+// a coalesced pass with 16 loads of a thread in flight.
 // ---------------------------------------------------------------------------
+// sum over count spectra of one wavenumber block: acc[u] += src[p][j0 + u NT]
+template <int U, typename TS>
+__device__ __forceinline__ void epi_sum(double2* acc, const TS* src, size_t n, int count,
+                                        int stride) {
+#pragma unroll 4
+  for (int p = 0; p < count; ++p) {
+    TS h[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) h[u] = src[(size_t)p * n + u * stride];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      acc[u].x += (double)h[u].x;
+      acc[u].y += (double)h[u].y;
+    }
+  }
+}
+
 template <int N, int C>
-__global__ void __launch_bounds__(Geo<N, C>::NT, 1)
-vhs_epilogue_kernel(VhsEpilogueArgs a) {
-  using G = Geo<N, C>;
+__global__ void __launch_bounds__(HalfGeo<N, C>::NT, fp64_per_sm<N, C>())
+vhs_epilogue_kernel(const __grid_constant__ VhsEpilogueArgs a) {
+  using G = HalfGeo<N, C>;
   using T = double2;
+  constexpr int H = G::H, P = G::P, NT = G::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool OS = OneSlab<N>::value;
   T* A = reinterpret_cast<T*>(smem_raw);
-  T* Rb = OS ? A : A + G::SLAB;  // Y-slab receive
-  const int t = threadIdx.x;
+  double* red = reinterpret_cast<double*>(A + G::SLAB);
+  const int t = threadIdx.x, pp = half_pencil(t), h = half_lane(t);
   const unsigned rank = cluster_rank();
   const int e = blockIdx.y;
-  const size_t off = (size_t)rank * G::P * N * N;
-  // Ghat = Ghat_M + sum_p H_p over this CTA's slab: elements in pairs,
-  // UNR pairs per thread in flight per p so that the loads overlap
-  constexpr int TOT2 = G::P * N * N / 2;
-  constexpr int UNR = 8;
-  for (int b0 = t; b0 < TOT2 && a.nt > 0; b0 += G::NT * UNR) {
-    T acc[UNR][2];
+  const int pl = pp / N, c = pp % N, y = rank * P + pl, lx = y;
+  const int rowb = pl * G::PLANE + c * G::ROW, colb = pl * G::PLANE + c;
+  const size_t off = (size_t)rank * P * N * N;
+  // Ghat = Ghat_M + sum_p H_p (or the weighted sum over pairs) over this
+  // CTA's slab
+  constexpr int U = 4;
+  static_assert(H % U == 0, "elements per thread");
+#pragma unroll 1
+  for (int j0 = 0; j0 < H; j0 += U) {
+    const size_t o = off + (size_t)j0 * NT + t;
+    T acc[U];
+    const int nt = a.nt > 0 ? a.nt : 1;
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      acc[u][0] = T{0, 0};
-      acc[u][1] = T{0, 0};
-    }
-    for (int it = 0; it < a.nt; ++it) {
-      const double w = a.pref[it];
+    for (int u = 0; u < U; ++u) acc[u] = T{0, 0};
+#pragma unroll 1
+    for (int it = 0; it < nt; ++it) {
+      const void* Hs = a.nt > 0 ? a.Ht[it] : a.H;
+      const T* GM = a.nt > 0 ? a.GMt[it] : a.GM;
+      T g[U];
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const int j2 = b0 + u * G::NT;
-        if (j2 < TOT2) {
-          T g0 = T{0, 0}, g1 = T{0, 0};
-          if (a.GMt[it]) {
-            g0 = a.GMt[it][(size_t)e * G::n + off + 2 * j2];
-            g1 = a.GMt[it][(size_t)e * G::n + off + 2 * j2 + 1];
-          }
-          if (a.h_double) {
-            for (int p = 0; p < a.Nrho; ++p) {
-              const double2* h = static_cast<const double2*>(a.Ht[it]) +
-                                 ((size_t)e * a.Nrho + p) * G::n + off + 2 * j2;
-              const double2 h0 = h[0], h1 = h[1];
-              g0.x += h0.x; g0.y += h0.y; g1.x += h1.x; g1.y += h1.y;
-            }
-          } else for (int p = 0; p < a.Nrho; ++p) {
-            const float4 h = reinterpret_cast<const float4*>(
-                static_cast<const float2*>(a.Ht[it]) +
-                ((size_t)e * a.Nrho + p) * G::n + off)[j2];
-            g0.x += (double)h.x; g0.y += (double)h.y;
-            g1.x += (double)h.z; g1.y += (double)h.w;
-          }
-          acc[u][0].x += w * g0.x; acc[u][0].y += w * g0.y;
-          acc[u][1].x += w * g1.x; acc[u][1].y += w * g1.y;
-        }
-      }
-    }
+      for (int u = 0; u < U; ++u)
+        g[u] = GM ? GM[(size_t)e * G::n + o + u * NT] : T{0, 0};
+      const size_t hb = (size_t)e * a.Nrho * G::n + o;
+      if (a.h_double) epi_sum<U>(g, static_cast<const double2*>(Hs) + hb, G::n, a.Nrho, NT);
+      else epi_sum<U>(g, static_cast<const float2*>(Hs) + hb, G::n, a.Nrho, NT);
+      if (a.nt > 0) {
+        const double w = a.pref[it];
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      const int j2 = b0 + u * G::NT;
-      if (j2 < TOT2) {
-        const int si = slab_index<N, C>(2 * j2);
-        A[si] = acc[u][0];
-        A[si + 1] = acc[u][1];
-      }
-    }
-  }
-  // FP64 spectra (FP64 mode: one per radial point): UNR pairs per thread,
-  // two radial points' loads in flight per step
-  for (int b0 = t; b0 < TOT2 && a.nt == 0 && a.h_double; b0 += G::NT * UNR) {
-    T acc[UNR][2];
-#pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      const int j2 = b0 + u * G::NT;
-      if (a.GM && j2 < TOT2) {
-        acc[u][0] = a.GM[(size_t)e * G::n + off + 2 * j2];
-        acc[u][1] = a.GM[(size_t)e * G::n + off + 2 * j2 + 1];
+        for (int u = 0; u < U; ++u) { acc[u].x += w * g[u].x; acc[u].y += w * g[u].y; }
       } else {
-        acc[u][0] = T{0, 0};
-        acc[u][1] = T{0, 0};
-      }
-    }
-#pragma unroll 2
-    for (int p = 0; p < a.Nrho; ++p) {
-      const size_t hb = ((size_t)e * a.Nrho + p) * G::n + off;
-      const double2* Hp = static_cast<const double2*>(a.H) + hb;
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const int j2 = b0 + u * G::NT;
-        if (j2 < TOT2) {
-          const double2 h0 = Hp[2 * j2], h1 = Hp[2 * j2 + 1];
-          acc[u][0].x += h0.x; acc[u][0].y += h0.y;
-          acc[u][1].x += h1.x; acc[u][1].y += h1.y;
-        }
+        for (int u = 0; u < U; ++u) acc[u] = g[u];
       }
     }
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) {
-      const int j2 = b0 + u * G::NT;
-      if (j2 < TOT2) {
-        const int si = slab_index<N, C>(2 * j2);
-        A[si] = acc[u][0];
-        A[si + 1] = acc[u][1];
-      }
-    }
-  }
-  // packed FP32 spectra (FP32 mode: one per radial pair, eight at Nrho=16):
-  // UNR32 pairs per thread with eight radial pairs' loads in flight per step,
-  // so that a thread's whole share of a step's loads overlaps
-  constexpr int UNR32 = 4;
-  for (int b0 = t; b0 < TOT2 && a.nt == 0 && !a.h_double; b0 += G::NT * UNR32) {
-    T acc[UNR32][2];
-#pragma unroll
-    for (int u = 0; u < UNR32; ++u) {
-      const int j2 = b0 + u * G::NT;
-      if (a.GM && j2 < TOT2) {
-        acc[u][0] = a.GM[(size_t)e * G::n + off + 2 * j2];
-        acc[u][1] = a.GM[(size_t)e * G::n + off + 2 * j2 + 1];
-      } else {
-        acc[u][0] = T{0, 0};
-        acc[u][1] = T{0, 0};
-      }
-    }
-#pragma unroll 8
-    for (int p = 0; p < a.Nrho; ++p) {
-      const size_t hb = ((size_t)e * a.Nrho + p) * G::n + off;
-      const float4* Hp =
-          reinterpret_cast<const float4*>(static_cast<const float2*>(a.H) + hb);
-#pragma unroll
-      for (int u = 0; u < UNR32; ++u) {
-        const int j2 = b0 + u * G::NT;
-        if (j2 < TOT2) {
-          const float4 h = Hp[j2];
-          acc[u][0].x += (double)h.x; acc[u][0].y += (double)h.y;
-          acc[u][1].x += (double)h.z; acc[u][1].y += (double)h.w;
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < UNR32; ++u) {
-      const int j2 = b0 + u * G::NT;
-      if (j2 < TOT2) {
-        const int si = slab_index<N, C>(2 * j2);
-        A[si] = acc[u][0];
-        A[si + 1] = acc[u][1];
-      }
+    for (int u = 0; u < U; ++u) {
+      const int j = (j0 + u) * NT + t;
+      A[(j / N) * G::ROW + j % N] = acc[u];
     }
   }
   __syncthreads();
-  slab_row_pass<double, N, C, +1>(A, t);
+  T v[H];
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];
+  fft_half_dit<double, N, +1>(v, h);
+#pragma unroll
+  for (int m = 0; m < H; ++m) A[rowb + h * H + m] = v[m];
   __syncthreads();
-  {
-    T w[N];
-    slab_col_load_fft<double, N, C, +1>(A, t, w);
-    if (OS) cluster_sync_all();  // every CTA has read its slab: exchange into it
-    push_cols_to_yslab<double, N, C>(Rb, t, rank, w);
-  }
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[colb + (2 * m + h) * G::ROW];
+  fft_half_dit<double, N, +1>(v, h);
+  cluster_sync_all();    // every CTA has read its slab: exchange into it
+  half_push_y<N, C>(A, lx, c, h, v);
   cluster_sync_all();
-  T v[N];
-  yslab_load_pencil<double, N, C>(Rb, t, v);
-  fft<double, N, +1>(v);
-  const int yl = t / N, z = t % N, y = rank * G::P + yl;
+#pragma unroll
+  for (int m = 0; m < H; ++m) v[m] = A[pl * N * N + (2 * m + h) * N + c];
+  fft_half_dit<double, N, +1>(v, h);
   const size_t fb = (size_t)slot_of(a.src_slots, a.src_base, e) * G::n;
   const size_t qb = (size_t)slot_of(a.dst_slots, a.dst_base, e) * G::n;
   const void* fin = a.f_list ? a.f_list[e] : a.f;
   void* qout = a.q_list ? a.q_list[e] : a.Q;
 #pragma unroll
-  for (int x = 0; x < N; ++x) {
-    const size_t idx = ((size_t)x * N + y) * N + z;
+  for (int m = 0; m < H; ++m) {
+    const size_t idx = ((size_t)(h * H + m) * N + y) * N + c;
     const double fv = load_real(fin, a.f_double, fb + idx);
     if (a.nt > 0) {
       double lf = 0;
       for (int it = 0; it < a.nt; ++it)
         lf += a.pref[it] * a.ReLft[it][(size_t)e * G::n + idx];
-      v[x].y = v[x].x - fv * lf;
-      continue;
+      v[m].y = v[m].x - fv * lf;
+    } else {
+      const double lf = a.ReLf[(size_t)e * G::n + idx];
+      v[m].y = a.bilinear ? a.prefac * (a.cg * v[m].x - a.cl * fv * lf)
+                          : a.prefac * (v[m].x - fv * lf);
     }
-    const double lf = a.ReLf[(size_t)e * G::n + idx];
-    v[x].y = a.bilinear ? a.prefac * (a.cg * v[x].x - a.cl * fv * lf)
-                        : a.prefac * (v[x].x - fv * lf);
   }
   double lam[5] = {0, 0, 0, 0, 0};
   if (a.project) {
-    // moments of this point's Q (FP64): thread -> CTA -> cluster, in a
-    // fixed order so every CTA derives the same multipliers
-    double* red = reinterpret_cast<double*>(A);  // A is free again
-    const double cy = a.c0[y], cz = a.c0[z];
-    double m[5] = {0, 0, 0, 0, 0};
+    // moments of this point's Q (FP64), the same bits in every CTA
+    const double cy = a.c0[y], cz = a.c0[c];
+    double s[5] = {0, 0, 0, 0, 0}, tot[5];
 #pragma unroll
-    for (int x = 0; x < N; ++x) {
-      const double cx = a.c0[x], q = v[x].y * a.cw;
-      m[0] += q; m[1] += q * cx; m[2] += q * cy; m[3] += q * cz;
-      m[4] += q * (cx * cx + cy * cy + cz * cz);
+    for (int m = 0; m < H; ++m) {
+      const double cx = a.c0[h * H + m], q = v[m].y * a.cw;
+      s[0] += q; s[1] += q * cx; s[2] += q * cy; s[3] += q * cz;
+      s[4] += q * (cx * cx + cy * cy + cz * cz);
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 5; ++k) red[k * G::NT + t] = m[k];
-    __syncthreads();
-    if (t < 5) {
-      double acc = 0;
-      for (int i = 0; i < G::NT; ++i) acc += red[t * G::NT + i];
-      red[5 * G::NT + t] = acc;
-    }
-    cluster_sync_all();
-    double tot[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      double acc = 0;
-      for (int c = 0; c < C; ++c) acc += peer_ptr(red, (unsigned)c)[5 * G::NT + k];
-      tot[k] = acc;
-    }
+    cluster_sum5<NT, C>(s, red, tot);
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
       double l = 0;
@@ -2035,11 +1970,12 @@ vhs_epilogue_kernel(VhsEpilogueArgs a) {
     cluster_sync_all();  // peers have read this CTA's partial sums
   }
 #pragma unroll
-  for (int x = 0; x < N; ++x) {
-    const size_t idx = ((size_t)x * N + y) * N + z;
-    double qv = v[x].y;
+  for (int m = 0; m < H; ++m) {
+    const int x = h * H + m;
+    const size_t idx = ((size_t)x * N + y) * N + c;
+    double qv = v[m].y;
     if (a.project) {
-      const double cx = a.c0[x], cy = a.c0[y], cz = a.c0[z];
+      const double cx = a.c0[x], cy = a.c0[y], cz = a.c0[c];
       qv -= lam[0] + lam[1] * cx + lam[2] * cy + lam[3] * cz +
             lam[4] * (cx * cx + cy * cy + cz * cz);
     }

@@ -472,6 +472,7 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
       for (int i = t; i < 6 * N; i += NT) uvt[i] = uv[i];
     }
   };
+  cluster_sync_all();                  // every CTA runs before remote stores
 #pragma unroll 1
   for (int r = r0; r < r1; ++r)
 #pragma unroll 1
