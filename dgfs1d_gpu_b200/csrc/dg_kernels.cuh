@@ -254,22 +254,28 @@ __device__ __forceinline__ double dg_ghost(const DgAdvectArgs& a, int side,
 // with jL = 0.5|c|(uL-uR) + 0.5c(uR-uL), jR = 0.5|c|(uL-uR) + 0.5c(uL-uR)
 // at each face (uL: state on its left, uR: on its right).  One thread per
 // velocity point walks the elements [blockIdx.y len, + len) and reads one
-// element more on either side for the traces.  Bound: HBM; the elements are
-// split so that every SM holds enough threads to keep its share of the
-// bandwidth in flight (N=48, Ne=32, K=3: 39.7 us with one walk over all 32
-// elements, 432 CTAs on 148 SMs).
+// element more on either side for the traces.  Bound: HBM; element e + 2 is
+// loaded while e is computed.  Small velocity grids split the walk (see
+// dgfs_dg_advect); large ones do not: four walks of eight elements instead of
+// one of 32 took 59.6 instead of 39.7 us at N=48, K=3.
+// (Three CTAs per SM: at 94 registers, i.e. two, the 432 CTAs of N=48 ran in
+// a wave and a half, 64 us.)
 template <int K>
-__global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a, int len) {
+__global__ void __launch_bounds__(256, K <= 4 ? 3 : 2)
+dg_advect_kernel(DgAdvectArgs a, int len) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= a.Nv) return;
   const int Ne = a.Ne, Nv = a.Nv;
   const int e0 = blockIdx.y * len, e1 = min(Ne, e0 + len);
   const double cx = a.c0[v / (a.N * a.N)];
   const double ac = 0.5 * fabs(cx), hc = 0.5 * cx;
-  double ue[K], un[K];
+  double ue[K], un[K], u2[K];
 #pragma unroll
   for (int k = 0; k < K; ++k)
     ue[k] = ld(a.u, a.f_double, ((size_t)k * Ne + e0) * Nv + v);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    un[k] = e0 + 1 < Ne ? ld(a.u, a.f_double, ((size_t)k * Ne + e0 + 1) * Nv + v) : 0.;
   auto tl = [&](const double* w) {
     double s = 0;
 #pragma unroll
@@ -304,17 +310,14 @@ __global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a, int len)
   double jR = jd0 + hc * (uLf - uRf);
 #pragma unroll 2
   for (int e = e0; e < e1; ++e) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      u2[k] = e + 2 < Ne && e + 1 < e1
+                  ? ld(a.u, a.f_double, ((size_t)k * Ne + e + 2) * Nv + v) : 0.;
     // face e+1
     const double uL1 = tr(ue);
-    double uR1;
-    if (e + 1 < Ne) {
-#pragma unroll
-      for (int k = 0; k < K; ++k)
-        un[k] = ld(a.u, a.f_double, ((size_t)k * Ne + e + 1) * Nv + v);
-      uR1 = tl(un);
-    } else {
-      uR1 = dg_ghost(a, 1, v, cx, a.swap ? uEnd0 : uL1);
-    }
+    const double uR1 =
+        e + 1 < Ne ? tl(un) : dg_ghost(a, 1, v, cx, a.swap ? uEnd0 : uL1);
     const double jd = ac * (uL1 - uR1);
     const double jL1 = jd + hc * (uR1 - uL1);
     const double ij = a.invjac[e];
@@ -337,7 +340,7 @@ __global__ void __launch_bounds__(256) dg_advect_kernel(DgAdvectArgs a, int len)
     }
     jR = jd + hc * (uL1 - uR1);  // jR of face e+1 for element e+1
 #pragma unroll
-    for (int k = 0; k < K; ++k) ue[k] = un[k];
+    for (int k = 0; k < K; ++k) { ue[k] = un[k]; un[k] = u2[k]; }
   }
 }
 

@@ -188,7 +188,8 @@ struct dgfs_vhs_s {
   double2* Fny64 = nullptr;  //   allocation-free entry), and exp(i N kappa_a)
   double2* nyq64 = nullptr;
   void* Fg = nullptr;        // [E][n] complex R
-  void* H = nullptr;         // [E][Nrho][n] complex R
+  void* H = nullptr;         // [hslots][n] complex R: spectra of radial pairs
+  size_t hslots = 0;
   double* ReLf = nullptr;    // [E][n]
   double2* mhat = nullptr;   // [E][3][N]
   double* moments = nullptr; // [E][5]
@@ -225,17 +226,16 @@ static int c32_of(int N) {
   }
 }
 template <int N> struct VhsClusters;
-// c64, ch32: terms kernel with two lanes per pencil (vhs_termsh_kernel), FP64
-// and FP32 (the default there); c32: FP32 terms kernel with one thread per pencil; cpro / cepi: prologue / epilogue (FP64,
-// one slab per CTA up to N=32).  At N=32 an 8-CTA prologue cluster needs 75 KB
-// per CTA and a 16-CTA epilogue cluster 34 KB, so two (four) CTAs share an SM
-// and a 24-point batch runs in one wave of each.
-template <> struct VhsClusters<8> { static constexpr int c64 = 1, ch32 = 1, c32 = 1, cpro = 1, cepi = 1; };
-template <> struct VhsClusters<16> { static constexpr int c64 = 2, ch32 = 1, c32 = 1, cpro = 4, cepi = 4; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 6, ch32 = 2, c32 = 3, cpro = 6, cepi = 6; };
-template <> struct VhsClusters<32> { static constexpr int c64 = 16, ch32 = 8, c32 = 4, cpro = 16, cepi = 16; };
+// c64: FP64 terms kernel with two lanes per pencil (vhs_termsh_kernel; up to
+// N=16 vhs_terms1_kernel runs); c32: FP32 terms kernel with one thread per
+// pencil; cpro / cepi: prologue / epilogue (FP64, two lanes per pencil, one slab
+// per CTA), small enough that a 24-point batch runs in one wave up to N=32.
+template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = 1, cepi = 1; };
+template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = 4, cepi = 4; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 6, c32 = 3, cpro = 6, cepi = 6; };
+template <> struct VhsClusters<32> { static constexpr int c64 = 16, c32 = 4, cpro = 16, cepi = 16; };
 // N=48: 16-CTA clusters of 3 planes
-template <> struct VhsClusters<48> { static constexpr int c64 = 16, ch32 = 16, c32 = 16, cpro = 16, cepi = 16; };
+template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = 16, cepi = 16; };
 
 static size_t slab_bytes(int N, int C, size_t elem) {
   return (size_t)(N / C) * N * (N + 1) * elem;
@@ -404,7 +404,10 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   alloc((void**)&h->err, sizeof(int));
   if (ce_ == cudaSuccess) ce_ = cudaMemset(h->err, 0, sizeof(int));
   alloc(&h->Fg, E * n * ce);
-  alloc(&h->H, E * ((Nrho + 1) / 2) * n * ce);  // packed radial pairs
+  // packed radial pairs; at least 64 spectra, for the direction slices of
+  // small batches
+  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), 64);
+  alloc(&h->H, h->hslots * n * ce);
   alloc((void**)&h->ReLf, E * n * sizeof(double));
   if (fp32) {
     alloc((void**)&h->mhat, E * 3 * N * sizeof(double2));
@@ -515,8 +518,16 @@ static int launch_terms32_c(const VhsTermsArgs& a, int nevals, int Nrho,
 template <typename R, int N, int C>
 static int launch_termsh_c(const VhsTermsArgs& a, int nevals, int Nrho,
                            cudaStream_t st) {
-  return launch_cluster(vhs_termsh_kernel<R, N, C>, dim3(C, (Nrho + 1) / 2, nevals),
+  return launch_cluster(vhs_termsh_kernel<R, N, C>, dim3(C, (Nrho + 1) / 2 * a.NS, nevals),
                         dim3(HalfGeo<N, C>::NT), C, TermsHGeo<R, N, C>::smem, st, a);
+}
+
+// Terms kernel with the whole cube in one CTA (vhs_terms1_kernel).
+template <typename R, int N>
+static int launch_terms1(const VhsTermsArgs& a, int nevals, int Nrho, cudaStream_t st) {
+  using G = Terms1Geo<R, N>;
+  return launch_plain(vhs_terms1_kernel<R, N>, dim3((Nrho + 1) / 2 * a.NS, nevals),
+                      dim3(G::NT), G::smem, st, a);
 }
 
 // Split-pencil terms kernel (two threads per pencil), same shared memory.
@@ -536,26 +547,41 @@ static int launch_terms32s_c(const VhsTermsArgs& a, int nevals, int Nrho,
 // Variant codes: the cluster size C for the one-thread-per-pencil kernel,
 // 100 + C for the split-pencil kernel, 500 + C for the one-thread kernel
 // whose F_g slab and plane transforms arrive by TMA and bulk copies, 600 + C
-// for the kernel with two lanes (l, l ^ 16) per pencil.
+// for the kernel with two lanes (l, l ^ 16) per pencil, 700 for the cube in one
+// CTA.
 template <int N> struct Terms32Variants;
-template <> struct Terms32Variants<8> { static constexpr int v[4] = {1, 2, 501, 601}; };
-template <> struct Terms32Variants<16> { static constexpr int v[5] = {1, 2, 501, 601, 602}; };
-template <> struct Terms32Variants<24> { static constexpr int v[7] = {3, 4, 6, 503, 602, 604, 606}; };
+template <> struct Terms32Variants<8> { static constexpr int v[5] = {1, 2, 501, 601, 700}; };
+template <> struct Terms32Variants<16> { static constexpr int v[7] = {1, 2, 501, 601, 602, 604, 700}; };
+template <> struct Terms32Variants<24> { static constexpr int v[8] = {3, 4, 6, 503, 602, 604, 606, 700}; };
 template <> struct Terms32Variants<32> { static constexpr int v[8] = {4, 8, 104, 108, 504, 604, 608, 616}; };
 template <> struct Terms32Variants<48> { static constexpr int v[4] = {16, 116, 516, 616}; };
 
-// Default variant: two lanes per pencil where two CTAs of different clusters
-// fit an SM and so hide each other's exchanges (N=24: 275 against 329 us for a
-// 24-point evaluation; N=48: 42.3 against 63.9 ms for 96 points); below, the
-// one-thread kernel with TMA staging (N=32: 666 against 719 us).
-template <int N> static int default_terms32(bool tma) {
-  if (N == 24 || N == 48) return 600 + VhsClusters<N>::ch32;
-  return (tma ? 500 : 0) + VhsClusters<N>::c32;
+// Direction slices of a terms launch: the two radial points of a CTA or cluster
+// of `ctas` CTAs share its 2 Mu serial transforms; while they leave SMs idle,
+// the directions are split (each slice has its own spectrum, summed in FP64 by
+// the epilogue).
+static int dir_slices(const dgfs_vhs_s* h, int nevals, int ctas) {
+  const int npairs = (h->Nrho + 1) / 2, base = nevals * npairs;
+  const int fit = std::min(148 / (base * ctas), (int)(h->hslots / base));
+  return std::max(1, std::min(fit, h->Mu));
+}
+
+// Default variant: the cube in one CTA where it fits (N=24: 225 us for a
+// 24-point evaluation against 257 with clusters of two), else two lanes per
+// pencil with two or three CTAs of different clusters on an SM, which hide each
+// other's exchanges (N=32: 639 against 659 us for the one-thread kernel with
+// TMA staging; N=48: 42.3 against 63.9 ms for 96 points).
+template <int N> constexpr int default_terms32() {
+  return N <= 24 ? 700 : 616;
 }
 
 template <int N>
 static int launch_terms32(int c, const VhsTermsArgs& a, int nevals, int Nrho,
                           cudaStream_t st, const CUtensorMap* map = nullptr) {
+  if constexpr (N <= 24)
+    if (c == 700) return launch_terms1<float, N>(a, nevals, Nrho, st);
+  if constexpr (N == 16)
+    if (c == 604) return launch_termsh_c<float, N, 4>(a, nevals, Nrho, st);
   if constexpr (N <= 16)
     if (c == 601) return launch_termsh_c<float, N, 1>(a, nevals, Nrho, st);
   if constexpr (N == 16 || N == 24)
@@ -610,7 +636,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
   const bool fp32 = h->precision == DGFS_PREC_FP32;
-  int rc;
+  int rc, nslices = 1;
   int evi = 0;
   auto mark = [&]() {
     if (h->profile) cudaEventRecord(h->ev[evi++], st);
@@ -650,8 +676,10 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.b1w = h->b1w32; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq32; a.rho = h->rho; a.Fny = h->Fny; a.err = h->err;
     // default: the two-lanes-per-pencil kernel (its own plane format)
-    const int c = h->c32 ? h->c32 : default_terms32<N>(h->fg_map_ok);
+    const int c = h->c32 ? h->c32 : default_terms32<N>();
     a.pm = c >= 600;
+    a.NS = c >= 600 ? dir_slices(h, nevals, c >= 700 ? 1 : c - 600) : 1;
+    nslices = a.NS;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
                            dim3((h->Mu + 1) / 2, h->Nrho, nevals), dim3(6 * N),
@@ -698,7 +726,10 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
                              dim3(3 * N), psmem, st, a)))
         return rc;
       mark(); mark();  // no Maxwellian-gain stage in FP64 mode
-      if ((rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st))) return rc;
+      a.NS = nslices = dir_slices(h, nevals, N <= 16 ? 1 : C64);
+      if constexpr (N <= 16) rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
+      else rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
+      if (rc) return rc;
     } else if constexpr (N == 8 || N == 16 || N == 32) {
       // allocation-free entry: its fixed scratch has no room for the plane
       // transforms, so each term takes a cosine and a sine transform
@@ -722,7 +753,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.dst_slots = dst_slots; a.dst_base = dst_base;
     a.prefac = h->prefac;
     // packed radial pairs, except in the allocation-free entry
-    a.Nrho = (fp32 || h->rho64) ? (h->Nrho + 1) / 2 : h->Nrho;
+    a.Nrho = (fp32 || h->rho64) ? (h->Nrho + 1) / 2 * nslices : h->Nrho;
     a.project = h->project; a.c0 = h->c0; a.cw = h->cw;
     for (int i = 0; i < 25; ++i) a.Ginv[i] = h->Ginv[i];
     if (bl) { a.bilinear = 1; a.cg = bl->cg; a.cl = bl->cl; }
@@ -1278,8 +1309,9 @@ extern "C" int dgfs_dg_advect(dgfs_dg_handle h, const void* u, void* ux,
     dg_wall_kernel<<<dim3(kWallCh, 2), 256, 0, st>>>(a, h->cw, h->wpart, h->nden, h->wdone);
     DGFS_CUDA(cudaGetLastError());
   }
-  // split the element walk until about 1536 threads per SM are in flight
-  const int want = (148 * 1536 + a.Nv - 1) / a.Nv;
+  // one walk per velocity point from N=48 on; below, the walk is split until
+  // about 512 threads per SM are in flight (N=24, Ne=8: 11.4 -> 7.6 us)
+  const int want = (148 * 512 + a.Nv - 1) / a.Nv;
   const int len = std::max(1, a.Ne / std::max(1, std::min(a.Ne, want)));
   const dim3 grid((a.Nv + 255) / 256, (a.Ne + len - 1) / len), block(256);
   switch (a.K) {
@@ -1488,17 +1520,11 @@ __global__ void vss_to_fp32_kernel(const double2* in, float2* out, size_t n) {
   if (i < n) out[i] = make_float2((float)in[i].x, (float)in[i].y);
 }
 
-// cluster sizes of the terms kernel (vss_terms_kernel), FP64 and FP32
+// cluster sizes of vss_terms_kernel, FP64 and FP32 (1: vss_terms1_kernel runs)
 template <int N> struct VssClusters;
 template <> struct VssClusters<8> { static constexpr int c64 = 1, c32 = 1; };
-template <> struct VssClusters<16> { static constexpr int c64 = 2, c32 = 2; };
-#ifndef VC64
-#define VC64 6
-#endif
-#ifndef VC32
-#define VC32 6
-#endif
-template <> struct VssClusters<24> { static constexpr int c64 = VC64, c32 = VC32; };
+template <> struct VssClusters<16> { static constexpr int c64 = 1, c32 = 1; };
+template <> struct VssClusters<24> { static constexpr int c64 = 6, c32 = 6; };
 template <> struct VssClusters<32> { static constexpr int c64 = 16, c32 = 8; };
 
 template <int N>
@@ -1765,9 +1791,13 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
   if ((rc = launch_plain(vss_planes_kernel<R, N>, dim3((unsigned)Tt, 1, nevals * c.nq),
                          dim3(3 * N), psmem, st, tt)))
     return rc;
-  if ((rc = launch_cluster(vss_terms_kernel<R, N, C>, dim3(C, tt.NS, nevals * c.nq),
-                           dim3(HalfGeo<N, C>::NT), C, VssHGeo<R, N, C>::smem, st, tt)))
-    return rc;
+  if constexpr (N <= (FP32 ? 24 : 16))
+    rc = launch_plain(vss_terms1_kernel<R, N>, dim3(1, tt.NS, nevals * c.nq),
+                      dim3(Vss1Geo<R, N>::NT), Vss1Geo<R, N>::smem, st, tt);
+  else
+    rc = launch_cluster(vss_terms_kernel<R, N, C>, dim3(C, tt.NS, nevals * c.nq),
+                        dim3(HalfGeo<N, C>::NT), C, VssHGeo<R, N, C>::smem, st, tt);
+  if (rc) return rc;
   if (FP32) {
     for (int k = 0; k < c.nq; ++k) {
       VssGainArgs ga{};

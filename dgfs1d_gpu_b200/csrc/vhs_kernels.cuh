@@ -81,6 +81,9 @@ struct VhsTermsArgs {
   int Nrho;
   int* err;                   // device error flag (a bounded wait gave up)
   int pm;                     // FP32 plane transforms: 1 stores (Re+Im, Re-Im)
+  int NS;                     // direction slices (termsh, terms1 kernels): slice
+                              // s sums q in [s Mu/NS, (s+1) Mu/NS) and has its
+                              // own H, [nevals][ceil(Nrho/2)][NS][n]
 };
 
 struct VhsTablesArgs {
@@ -174,7 +177,7 @@ constexpr size_t epilogue_smem() {
 }
 // CTAs per SM by the registers of a lane's N/2 FP64 values
 template <int N, int C> constexpr int fp64_per_sm() {
-  constexpr int thr = N <= 16 ? 512 : N <= 32 ? 384 : 288;
+  constexpr int thr = N <= 16 ? 512 : N == 24 ? 384 : N == 32 ? 512 : 288;
   constexpr int r = thr / HalfGeo<N, C>::NT;
   constexpr int sm = (int)((size_t)(227 * 1024) / (prologue_smem<N, C>() + 1024));
   return r < 1 ? 1 : r < sm ? r : sm < 1 ? 1 : sm;
@@ -1575,9 +1578,10 @@ vhs_termsh_kernel(VhsTermsArgs a) {
   T* ut = tb + 3 * N + 4;              // u [3N], v [3N] (SPLIT)
   const int t = threadIdx.x, pp = half_pencil(t), h = half_lane(t);
   const unsigned rank = cluster_rank();
-  const int pair = blockIdx.y, e = blockIdx.z;
+  const int pair = blockIdx.y / a.NS, e = blockIdx.z, sl = blockIdx.y % a.NS;
   const int Mu = a.Mu, p0 = 2 * pair;
-  const int npass = (p0 + 1 < a.Nrho ? 2 : 1) * Mu;
+  const int q0 = sl * Mu / a.NS, nq = (sl + 1) * Mu / a.NS - q0;
+  const int npass = (p0 + 1 < a.Nrho ? 2 : 1) * nq;
   const int npairs = (a.Nrho + 1) / 2;
   const T* Fg = static_cast<const T*>(a.Fg) + (size_t)e * G::n +
                 (size_t)rank * P * N * N;
@@ -1587,7 +1591,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
   // pencil pp: plane pl, row / column c of the X-slab; (yl, z) of the Y-slab
   const int pl = pp / N, c = pp % N;
   const int lx = rank * P + pl, yy = lx;
-  auto term = [&](int k) { return (size_t)(p0 + k / Mu) * Mu + k % Mu; };
+  auto term = [&](int k) { return (size_t)(p0 + k / nq) * Mu + q0 + k % nq; };
   auto load_phases = [&](int k) {      // read by zpass(k)
     const size_t pq = term(k);
     for (int i = t; i < 3 * N; i += NT) tb[i] = phb[pq * 3 * N + i];
@@ -1650,7 +1654,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
 #pragma unroll
   for (int m = 0; m < H; ++m) S[m] = R(0);
   // the first radial point's sums wait in this CTA's own block of H
-  T* Hout = static_cast<T*>(a.H) + ((size_t)e * npairs + pair) * G::n +
+  T* Hout = static_cast<T*>(a.H) + (((size_t)e * npairs + pair) * a.NS + sl) * G::n +
             (size_t)rank * P * N * N;
   R* stash = reinterpret_cast<R*>(Hout);
 
@@ -1689,7 +1693,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     const T rx = rp[yy * N + c];
     const T* rY = rp + N * N + c + h * H * N;
     const T* rZ = rp + 2 * N * N + yy + h * H * N;
-    const R mq = SPLIT ? R(1) : (R)a.mult[k % Mu];
+    const R mq = SPLIT ? R(1) : (R)a.mult[q0 + k % nq];
     T uyz{}, vyz{};
     if constexpr (SPLIT) {
       uyz = cmul(ut[N + yy], ut[2 * N + c]);
@@ -1729,7 +1733,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
         S[m] += mq * (gp * gm);
       }
     }
-    if (k == Mu - 1 && npass > Mu) {
+    if (k == nq - 1 && npass > nq) {
 #pragma unroll
       for (int m = 0; m < H; ++m) { stash[m * NT + t] = S[m]; S[m] = R(0); }
     }
@@ -1738,7 +1742,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
   T v[H];
 #pragma unroll
   for (int m = 0; m < H; ++m)
-    v[m] = npass > Mu ? T{stash[m * NT + t], S[m]} : T{S[m], R(0)};
+    v[m] = npass > nq ? T{stash[m * NT + t], S[m]} : T{S[m], R(0)};
   fft_half_dif<R, N, -1>(v, h);
   cluster_wait();                        // every CTA is past its last y pass
   {
@@ -1764,12 +1768,202 @@ vhs_termsh_kernel(VhsTermsArgs a) {
   __syncthreads();
   const R* b1a = static_cast<const R*>(a.b1w) + (size_t)p0 * G::n +
                  (size_t)rank * P * N * N;
-  const R* b1b = npass > Mu ? b1a + G::n : nullptr;
+  const R* b1b = npass > nq ? b1a + G::n : nullptr;
 #pragma unroll 4
   for (int j = t; j < P * N * N; j += NT) {
     const T hv = A[(j / N) * G::ROW + j % N];
     const R w0 = b1a[j], w1 = b1b ? b1b[j] : R(0);
     Hout[j] = T{hv.x * w0 + hv.y * w1, hv.y * w0 - hv.x * w1};
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Terms in a single CTA: the whole cube in one SM's shared memory (transform
+// slab A, padded, and the resident F), for grids that fit (FP32 up to N=24,
+// FP64 up to N=16).  No exchange and no cluster barrier: three CTA barriers
+// per transform.  Passes along x (from F, coalesced), y and z in place, so that
+// a lane ends with a z-pencil of its (x, y); the forward transform runs z, y, x
+// and stores H coalesced.  HP: two lanes per pencil (N <= 16), else one thread.
+// Same algebra and plane format as vhs_termsh_kernel.
+// ---------------------------------------------------------------------------
+template <typename R, int N> struct Terms1Geo {
+  static constexpr bool SPLIT = sizeof(R) == 4;
+  static constexpr bool HP = N <= 16;
+  static constexpr int V = HP ? N / 2 : N;         // values per thread
+  static constexpr int NT = HP ? 2 * N * N : N * N;
+  static constexpr int ROW = N + 1, PLANE = N * ROW, n = N * N * N;
+  static constexpr size_t smem =
+      (size_t)(N * PLANE + n + N * ROW + 3 * N + 4 + (SPLIT ? 6 * N : 0)) * sizeof(c2_t<R>);
+  static constexpr int by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
+  static constexpr int by_regs = (HP ? (SPLIT ? 1024 : 512) : 576) / NT;
+  static constexpr int per_sm =
+      by_smem < by_regs ? (by_smem > 0 ? by_smem : 1) : (by_regs > 0 ? by_regs : 1);
+};
+
+template <typename R, int N>
+__global__ void __launch_bounds__(Terms1Geo<R, N>::NT, Terms1Geo<R, N>::per_sm)
+vhs_terms1_kernel(VhsTermsArgs a) {
+  using G = Terms1Geo<R, N>;
+  using T = c2_t<R>;
+  constexpr int V = G::V, NT = G::NT, ROW = G::ROW, PLANE = G::PLANE, H = N / 2;
+  constexpr bool HP = G::HP, SPLIT = G::SPLIT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* A = reinterpret_cast<T*>(smem_raw);     // [N x][N y][ROW z]
+  T* Fs = A + N * PLANE;                      // [N][N][N]
+  T* rxs = Fs + G::n;                         // r_x of the term [N y][ROW]
+  T* tb = rxs + N * ROW;                      // phases [3N], nu [3]
+  T* ut = tb + 3 * N + 4;                     // u, v [6N] (SPLIT)
+  const int t = threadIdx.x, pp = HP ? half_pencil(t) : t, h = HP ? half_lane(t) : 0;
+  const int p = pp / N, q = pp % N;           // the two fixed indices of a pass
+  const int pair = blockIdx.x / a.NS, e = blockIdx.y, sl = blockIdx.x % a.NS;
+  const int Mu = a.Mu, p0 = 2 * pair;
+  const int q0 = sl * Mu / a.NS, nq = (sl + 1) * Mu / a.NS - q0;
+  const int npass = (p0 + 1 < a.Nrho ? 2 : 1) * nq;
+  const int npairs = (a.Nrho + 1) / 2;
+  const T* Fg = static_cast<const T*>(a.Fg) + (size_t)e * G::n;
+  auto in = [&](int m) { return HP ? 2 * m + h : m; };
+  auto out = [&](int m) { return HP ? h * H + m : m; };
+  auto inv = [&](T* v) {
+    if constexpr (HP) fft_half_dit<R, N, +1>(v, h);
+    else fft<R, N, +1>(v);
+  };
+  auto fwd = [&](T* v) {                      // in() -> out()
+    if constexpr (HP) fft_half_dit<R, N, -1>(v, h);
+    else fft<R, N, -1>(v);
+  };
+  auto term = [&](int k) { return (size_t)(p0 + k / nq) * Mu + q0 + k % nq; };
+  auto rho_of = [&](int k) {
+    return static_cast<const T*>(a.rho) + ((size_t)e * a.Nrho * Mu + term(k)) * 3 * N * N;
+  };
+  auto copy = [&](T* dst, const T* src) {     // one element, asynchronous
+    if constexpr (SPLIT)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n"
+                   :: "r"(smem_u32(dst)), "l"(src) : "memory");
+    else
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n"
+                   :: "r"(smem_u32(dst)), "l"(src) : "memory");
+  };
+  auto load_phases = [&](int k) {             // read by the x pass of term k
+    const size_t pq = term(k);
+    for (int i = t; i < 3 * N + 3; i += NT)
+      copy(tb + i, i < 3 * N ? static_cast<const T*>(a.ph) + pq * 3 * N + i
+                             : static_cast<const T*>(a.nyq) + pq * 3 + i - 3 * N);
+  };
+  auto load_comb = [&](int k) {               // read by the combine of term k
+    const T* rx = rho_of(k);
+    for (int i = t; i < N * N; i += NT) copy(rxs + (i / N) * ROW + i % N, rx + i);
+    if constexpr (SPLIT) {
+      const T* uv = static_cast<const T*>(a.uv) + ((size_t)e * a.Nrho * Mu + term(k)) * 6 * N;
+      for (int i = t; i < 6 * N; i += NT) copy(ut + i, uv + i);
+    }
+  };
+  R S[V];
+#pragma unroll
+  for (int m = 0; m < V; ++m) S[m] = R(0);
+  T* Hout = static_cast<T*>(a.H) + (((size_t)e * npairs + pair) * a.NS + sl) * G::n;
+  R* stash = reinterpret_cast<R*>(Hout);      // the first radial point's sums
+  for (int i = t; i < G::n; i += NT) copy(Fs + i, Fg + i);
+  load_phases(0);
+#pragma unroll 1
+  for (int k = 0; k < npass; ++k) {
+    T v[V];
+    cp_async_wait_all();
+    __syncthreads();      // the phases are in place; z pencils of k - 1 are read
+    {  // x pass, (ly, lz) = (p, q): multiplier, inverse transform
+      const T* nu = tb + 3 * N;
+      const T byz = cmul(tb[N + p], tb[2 * N + q]);
+      T fyz = T{R(1), R(0)};
+      if (p == H) fyz = nu[1];
+      if (q == H) fyz = cmul(fyz, nu[2]);
+      const T gb = cmul(nyq_mul(fyz, R(1)), byz);
+      const T gbx = cmul(nyq_mul(cmul(fyz, nu[0]), R(1)), byz);
+#pragma unroll
+      for (int m = 0; m < V; ++m) {
+        const T bx = tb[in(m)];
+        const T f = Fs[in(m) * N * N + pp];
+        // lx = in(m) is the Nyquist index H
+        const T g = (HP ? (2 * m == H && h == 0) : m == H) ? gbx : gb;
+        const R w = g.x * bx.x - g.y * bx.y;
+        v[m] = T{f.x * w, f.y * w};
+      }
+      inv(v);
+#pragma unroll
+      for (int m = 0; m < V; ++m) A[out(m) * PLANE + p * ROW + q] = v[m];
+    }
+    __syncthreads();
+    if (k + 1 < npass) load_phases(k + 1);
+    load_comb(k);
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + in(m) * ROW + q];   // (x, z)
+    inv(v);
+#pragma unroll
+    for (int m = 0; m < V; ++m) A[p * PLANE + out(m) * ROW + q] = v[m];
+    // r_y, r_z of (x, y) = (p, q)
+    const T* rp = rho_of(k);
+    const T* rY = rp + N * N + p * N;
+    const T rz = rp[2 * N * N + p * N + q];
+    cp_async_wait_all();
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + q * ROW + in(m)];   // (x, y)
+    inv(v);
+    const R sx = (p & 1) ? R(-1) : R(1), sy = (q & 1) ? R(-1) : R(1);
+    T uxy{}, vxy{};
+    if constexpr (SPLIT) {
+      uxy = cmul(ut[p], ut[N + q]);
+      vxy = cmul(ut[3 * N + p], ut[4 * N + q]);
+    }
+    const R mq = SPLIT ? R(1) : (R)a.mult[q0 + k % nq];
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int z = out(m);
+      const T rx = rxs[q * ROW + z], ry = rY[z];
+      const R zs = (m & 1) ? R(-1) : R(1);    // (-1)^z, H is even
+      const R wp = sx * rx.x + (sy * ry.x + zs * rz.x);
+      const R wm = sx * rx.y + (sy * ry.y + zs * rz.y);
+      const R gp = v[m].x + v[m].y, gm = v[m].x - v[m].y;
+      if constexpr (SPLIT) {
+        const T um = cmul(uxy, ut[2 * N + z]), vm = cmul(vxy, ut[5 * N + z]);
+        S[m] += gp * (gm + um.x);
+        S[m] += vm.x * gm;
+        S[m] += wm * (wp + um.y);
+        S[m] -= vm.y * wp;
+      } else {
+        S[m] += mq * (gp * gm + wm * wp);
+      }
+    }
+    if (k == nq - 1 && npass > nq) {
+#pragma unroll
+      for (int m = 0; m < V; ++m) { stash[m * NT + t] = S[m]; S[m] = R(0); }
+    }
+  }
+  // forward transform of S_p0 + i S_p1: z (in registers), y, x
+  T v[V];
+#pragma unroll
+  for (int m = 0; m < V; ++m)
+    v[m] = npass > nq ? T{stash[m * NT + t], S[m]} : T{S[m], R(0)};
+  if constexpr (HP) fft_half_dif<R, N, -1>(v, h);    // out() -> in()
+  else fft<R, N, -1>(v);
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < V; ++m) A[p * PLANE + q * ROW + in(m)] = v[m];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + in(m) * ROW + q];
+  fwd(v);
+#pragma unroll
+  for (int m = 0; m < V; ++m) A[p * PLANE + out(m) * ROW + q] = v[m];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < V; ++m) v[m] = A[in(m) * PLANE + p * ROW + q];
+  fwd(v);
+  const R* b1a = static_cast<const R*>(a.b1w) + (size_t)p0 * G::n;
+  const R* b1b = npass > nq ? b1a + G::n : nullptr;
+#pragma unroll
+  for (int m = 0; m < V; ++m) {
+    const int j = out(m) * N * N + pp;
+    const R w0 = b1a[j], w1 = b1b ? b1b[j] : R(0);
+    Hout[j] = T{v[m].x * w0 + v[m].y * w1, v[m].y * w0 - v[m].x * w1};
   }
 }
 

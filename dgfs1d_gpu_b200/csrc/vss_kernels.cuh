@@ -587,4 +587,176 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
   cluster_sync_all();  // no CTA leaves while peers may still write into it
 }
 
+// Terms with the whole cube in one CTA, for grids that fit (FP32 up to N=24,
+// FP64 up to N=16): transform slab A (padded) and the spectral sums Qh in shared
+// memory, no exchange.  Passes x (from F_p and F_q, coalesced), y, z; the
+// product of a z-pencil and its forward z pass in registers; y; x, weighted by
+// b into Qh.  A thread's x pencils of the last pass of a term and the first of
+// the next are the same, so a term takes four CTA barriers.  HP: two lanes per
+// pencil (N <= 16).
+template <typename R, int N> struct Vss1Geo {
+  static constexpr bool SPLIT = sizeof(R) == 4;
+  static constexpr bool HP = N <= 16;
+  static constexpr int V = HP ? N / 2 : N;
+  static constexpr int NT = HP ? 2 * N * N : N * N;
+  static constexpr int ROW = N + 1, PLANE = N * ROW, n = N * N * N;
+  // A, Qh, r_x of the term, u_M and v_M
+  static constexpr size_t smem =
+      (size_t)(N * PLANE + n + N * ROW + (SPLIT ? 6 * N : 0)) * sizeof(c2_t<R>);
+  static constexpr int by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
+  static constexpr int by_regs = (HP ? (SPLIT ? 1024 : 512) : 576) / NT;
+  static constexpr int per_sm =
+      by_smem < by_regs ? (by_smem > 0 ? by_smem : 1) : (by_regs > 0 ? by_regs : 1);
+};
+
+template <typename R, int N>
+__global__ void __launch_bounds__(Vss1Geo<R, N>::NT, Vss1Geo<R, N>::per_sm)
+vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
+  using G = Vss1Geo<R, N>;
+  using T = c2_t<R>;
+  constexpr int V = G::V, NT = G::NT, ROW = G::ROW, PLANE = G::PLANE, H = N / 2;
+  constexpr bool HP = G::HP, SPLIT = G::SPLIT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* A = reinterpret_cast<T*>(smem_raw);     // [N x][N y][ROW z]
+  T* Qh = A + N * PLANE;                      // [N][N][N]
+  T* rxs = Qh + G::n;                         // [N y][ROW]
+  T* uvt = rxs + N * ROW;                     // u_M [3N], v_M [3N] (SPLIT)
+  const int t = threadIdx.x, pp = HP ? half_pencil(t) : t, h = HP ? half_lane(t) : 0;
+  const int p = pp / N, q = pp % N;
+  const int e = blockIdx.z % a.nevals;
+  const VssTermsPair& Pr = a.pr[blockIdx.z / a.nevals];
+  const int r0 = blockIdx.y * a.Nrho / a.NS, r1 = (blockIdx.y + 1) * a.Nrho / a.NS;
+  const int nd = Pr.nd, Tt = a.Nrho * a.M;
+  const T* Fp = static_cast<const T*>(Pr.Fp) + (size_t)e * G::n + pp;
+  const T* Fq = static_cast<const T*>(Pr.Fq) + (size_t)e * G::n + pp;
+  auto in = [&](int m) { return HP ? 2 * m + h : m; };
+  auto out = [&](int m) { return HP ? h * H + m : m; };
+  auto inv = [&](T* v) {
+    if constexpr (HP) fft_half_dit<R, N, +1>(v, h);
+    else fft<R, N, +1>(v);
+  };
+  auto fwd = [&](T* v) {
+    if constexpr (HP) fft_half_dit<R, N, -1>(v, h);
+    else fft<R, N, -1>(v);
+  };
+  for (int i = t; i < G::n; i += NT) Qh[i] = T{R(0), R(0)};
+  __syncthreads();
+#pragma unroll 1
+  for (int r = r0; r < r1; ++r)
+#pragma unroll 1
+  for (int d = 0; d < nd; ++d) {
+    const int2 dir = Pr.dirs[d];
+    const int term = r * a.M + dir.x;
+    const T* rp = static_cast<const T*>(Pr.rho) + ((size_t)e * Tt + term) * 3 * N * N;
+    T v[V];
+    {  // x pass, (ly, lz) = (p, q): Z = M_u F_p + i M_v F_q
+      T g[2], gx[2];
+      const T* ph = static_cast<const T*>(Pr.ph) + (size_t)term * 6 * N;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const T* f = ph + 3 * N * s;
+        const T E = cmul(f[N + p], f[2 * N + q]);
+        T fy = T{R(1), R(0)};
+        if (p == H) fy = vss_nu(f[N + H]);
+        if (q == H) fy = cmul(fy, vss_nu(f[2 * N + H]));
+        const T fx = cmul(fy, vss_nu(f[H]));
+        g[s] = cmul(E, T{R(0.5) * (R(1) + fy.x), R(0.5) * fy.y});
+        gx[s] = cmul(E, T{R(0.5) * (R(1) + fx.x), R(0.5) * fx.y});
+      }
+#pragma unroll
+      for (int m = 0; m < V; ++m) {
+        const int x = in(m);
+        const bool nyq = HP ? (2 * m == H && h == 0) : m == H;
+        const T u = cmul(cmul(nyq ? gx[0] : g[0], ph[x]), Fp[x * N * N]);
+        const T w = cmul(cmul(nyq ? gx[1] : g[1], ph[3 * N + x]), Fq[x * N * N]);
+        v[m] = T{u.x - w.y, u.y + w.x};
+      }
+      inv(v);
+#pragma unroll
+      for (int m = 0; m < V; ++m) A[out(m) * PLANE + p * ROW + q] = v[m];
+    }
+    __syncthreads();
+    // tables of the product, read two barriers later at the earliest
+    for (int i = t; i < N * N; i += NT) rxs[(i / N) * ROW + i % N] = rp[i];
+    if constexpr (SPLIT) {
+      const T* uv = Pr.uv + ((size_t)e * Tt + term) * 6 * N;
+      for (int i = t; i < 6 * N; i += NT) uvt[i] = uv[i];
+    }
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + in(m) * ROW + q];   // (x, z)
+    inv(v);
+#pragma unroll
+    for (int m = 0; m < V; ++m) A[p * PLANE + out(m) * ROW + q] = v[m];
+    const T rz = rp[2 * N * N + p * N + q];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + q * ROW + in(m)];   // (x, y)
+    inv(v);
+    {
+      const R sx = (p & 1) ? R(-1) : R(1), sy = (q & 1) ? R(-1) : R(1);
+      const T* rY = rp + N * N + p * N;
+      T uxy{}, vxy{};
+      if constexpr (SPLIT) {
+        uxy = cmul(uvt[p], uvt[N + q]);
+        vxy = cmul(uvt[3 * N + p], uvt[4 * N + q]);
+      }
+#pragma unroll
+      for (int m = 0; m < V; ++m) {
+        const int z = out(m);
+        const T rx = rxs[q * ROW + z], ry = rY[z];
+        const R zs = (m & 1) ? R(-1) : R(1);
+        const T Xu = T{v[m].x, sx * rx.x + (sy * ry.x + zs * rz.x)};
+        const T Xv = T{v[m].y, sx * rx.y + (sy * ry.y + zs * rz.y)};
+        if constexpr (SPLIT) {
+          const T uM = cmul(uxy, uvt[2 * N + z]), vM = cmul(vxy, uvt[5 * N + z]);
+          const T a1 = cmul(uM, Xv);
+          const T a2 = cmul(Xu, T{vM.x + Xv.x, vM.y + Xv.y});
+          v[m] = T{a1.x + a2.x, a1.y + a2.y};
+        } else {
+          v[m] = cmul(Xu, Xv);
+        }
+      }
+    }
+    if constexpr (HP) fft_half_dif<R, N, -1>(v, h);    // out() -> in()
+    else fft<R, N, -1>(v);
+#pragma unroll
+    for (int m = 0; m < V; ++m) A[p * PLANE + q * ROW + in(m)] = v[m];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[p * PLANE + in(m) * ROW + q];
+    fwd(v);
+#pragma unroll
+    for (int m = 0; m < V; ++m) A[p * PLANE + out(m) * ROW + q] = v[m];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = A[in(m) * PLANE + p * ROW + q];
+    fwd(v);
+    const T* b1 = static_cast<const T*>(Pr.b) + (size_t)term * G::n + pp;
+    const T* b2 = dir.y >= 0
+        ? static_cast<const T*>(Pr.b) + (size_t)(r * a.M + dir.y) * G::n + pp : nullptr;
+    const R wr = SPLIT ? R(1) : (R)a.w[r];
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int j = out(m) * N * N;
+      T b = b1[j];
+      if (b2) { const T c = b2[j]; b.x += c.x; b.y += c.y; }
+      const T x = cmul(v[m], b);
+      T s = Qh[j + pp];
+      s.x += wr * x.x;
+      s.y += wr * x.y;
+      Qh[j + pp] = s;
+    }
+    // (HP: the pencil's other lane still reads A[in()] of this pass, and both
+    // lanes' next stores follow the shuffles of the next transform)
+  }
+  const R wo = SPLIT ? (R)a.w[r0] : R(1);
+  T* Ho = static_cast<T*>(Pr.H) + ((size_t)e * a.NS + blockIdx.y) * G::n + pp;
+#pragma unroll
+  for (int m = 0; m < V; ++m) {
+    const int j = out(m) * N * N;
+    const T s = Qh[j + pp];
+    Ho[j] = T{wo * s.x, wo * s.y};
+  }
+}
+
 }  // namespace dgfs
