@@ -48,14 +48,20 @@ class DGFSIntegratorAstd:
         self.dt, self.nsub = dt, nsub
 
     def _z(self):
+        """Zeros, for what the explicit part writes (it may accumulate)."""
         return torch.zeros(self.shape, dtype=self.dtype, device=self.device)
 
-    def _zm(self):
-        return torch.zeros((self.npts, self._sm.nalph), dtype=torch.float64,
+    def _e(self):
+        """Uninitialised, for what the native updates and the penalty model
+        write in full (a fill of the state costs as much as one of them)."""
+        return torch.empty(self.shape, dtype=self.dtype, device=self.device)
+
+    def _em(self):
+        return torch.empty((self.npts, self._sm.nalph), dtype=torch.float64,
                            device=self.device)
 
     def _mom(self, x):
-        U = self._zm()
+        U = self._em()
         self._sm.moment(0.0, x, U)
         return U
 
@@ -68,10 +74,10 @@ class Bdf111IntegratorAstd(DGFSIntegratorAstd):
         L0 = self._z()
         self._explicit(t, f, L0)
         LU0 = self._mom(L0)
-        U = self._zm()
+        U = self._em()
         _lin(U, [(1.0, U0), (dt, LU0)])
         self._sm.relax(U, 1.0, dt)
-        rhs = self._z()
+        rhs = self._e()
         _lin(rhs, [(1.0, f), (dt, L0)])
         self._sm.implicit(U, rhs, f, 1.0, dt)
 
@@ -101,15 +107,15 @@ class _StageIMEXIntegratorAstd(DGFSIntegratorAstd):
     def _stage(self, t, dt, F0, Ls, Ps, q_expl, q_impl, U):
         """F_q from the explicit weights over Ls, implicit weights over the
         earlier stages' penalties Ps and the implicit weight of stage q."""
-        rhs = self._z()
+        rhs = self._e()
         _lin(rhs, [(1.0, F0)] + [(dt * a, L) for a, L in zip(q_expl, Ls)]
              + [(dt * a, P) for a, P in zip(q_impl, Ps)])
-        f = self._z()
+        f = self._e()
         self._sm.implicit(U, rhs, f, 1.0, self._aqq * dt)
         return f
 
     def _penalty(self, t, U, f):
-        P = self._z()
+        P = self._e()
         self._sm.collide(t, U, f, P)
         return P
 
@@ -129,7 +135,7 @@ class ARSIntegratorAstd(_StageIMEXIntegratorAstd):
             Ls.append(L)
             LUs.append(self._mom(L))
             ex = self._A[i + 1][0:i + 1]
-            U = self._zm()
+            U = self._em()
             _lin(U, [(1.0, U0)] + [(dt * a, LU) for a, LU in zip(ex, LUs)])
             Us.append(U)
             self._aqq = self.A[i + 1][i + 1]
@@ -184,7 +190,7 @@ class SSPLIntegratorAstd(_StageIMEXIntegratorAstd):
             Ls.append(L)
             LUs.append(self._mom(L))
             ex = self._A[i][0:i]
-            U = self._zm()
+            U = self._em()
             _lin(U, [(1.0, U0)] + [(dt * a, LU) for a, LU in zip(ex, LUs)])
             Us.append(U)
             self._aqq = self.A[i][i]
@@ -226,7 +232,7 @@ class BoltzARS111IntegratorAstd(DGFSIntegratorAstd):
 
     def integrate(self, t, dt, nacptsteps, f):
         U0 = self._mom(f)
-        P0 = self._z()
+        P0 = self._e()
         self._sm.collide(t, U0, f, P0)
         L0 = self._z()
         self._explicit(t, f, L0)
@@ -234,10 +240,10 @@ class BoltzARS111IntegratorAstd(DGFSIntegratorAstd):
         if self._Q is not None:
             self._Q(t, f, L0)             # accumulates Q(f)
         axnpby(L0, 1.0, -1.0, P0)
-        U = self._zm()
+        U = self._em()
         _lin(U, [(1.0, U0), (dt, LU0)])
         self._sm.relax(U, 1.0, dt)
-        rhs = self._z()
+        rhs = self._e()
         _lin(rhs, [(1.0, f), (dt, L0)])
         self._sm.implicit(U, rhs, f, 1.0, dt)
 
@@ -270,11 +276,11 @@ class BdfIntegratorAstd(DGFSIntegratorAstd):
             self.hist.append(self._state(t + dt, f))
             return
         hs = self.hist
-        U = self._zm()
+        U = self._em()
         _lin(U, [p for i in range(k) for p in (
             (-A[i] / A[k], hs[i]['U']), (G[i] * dt / A[k], hs[i]['LU']))])
         self._sm.relax(U, A[k], B * dt)
-        rhs = self._z()
+        rhs = self._e()
         _lin(rhs, [p for i in range(k) for p in (
             (-A[i], hs[i]['F']), (G[i] * dt, hs[i]['L']))])
         self._sm.implicit(U, rhs, f, A[k], B * dt)
@@ -323,7 +329,7 @@ class IMEXLMIntegratorAstd(DGFSIntegratorAstd):
 
     def _state(self, t, f):
         U = self._mom(f)
-        P = self._z()
+        P = self._e()
         self._sm.collide(t, U, f, P)
         E = self._z()
         self._explicit(t, f, E)
@@ -340,16 +346,16 @@ class IMEXLMIntegratorAstd(DGFSIntegratorAstd):
             f.copy_(self.starts[nacptsteps])
             return
         hs = self.hist
-        U = self._zm()
+        U = self._em()
         _lin(U, [p for i in range(s) for p in (
             (-A[s - i - 1], hs[i]['U']), (dt * B[s - i - 1], hs[i]['LU']),
             (dt * C[s - i], hs[i]['LM']))])
-        rhs = self._z()
+        rhs = self._e()
         _lin(rhs, [p for i in range(s) for p in (
             (-A[s - i - 1], hs[i]['F']), (dt * B[s - i - 1], hs[i]['L']),
             (dt * C[s - i], hs[i]['P']))])
         self._sm.relax(U, 1.0, C[0] * dt)
-        P = self._z()
+        P = self._e()
         self._sm.implicit(U, rhs, f, 1.0, C[0] * dt, P=P)
         E = self._z()
         self._explicit(t + dt, f, E)

@@ -232,7 +232,7 @@ template <int N> struct VhsClusters;
 // per CTA), small enough that a 24-point batch runs in one wave up to N=32.
 template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = 1, cepi = 1; };
 template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = 4, cepi = 4; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 6, c32 = 3, cpro = 6, cepi = 6; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 12, c32 = 3, cpro = 6, cepi = 6; };
 template <> struct VhsClusters<32> { static constexpr int c64 = 16, c32 = 4, cpro = 16, cepi = 16; };
 // N=48: 16-CTA clusters of 3 planes
 template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = 16, cepi = 16; };
@@ -404,9 +404,9 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   alloc((void**)&h->err, sizeof(int));
   if (ce_ == cudaSuccess) ce_ = cudaMemset(h->err, 0, sizeof(int));
   alloc(&h->Fg, E * n * ce);
-  // packed radial pairs; at least 64 spectra, for the direction slices of
-  // small batches
-  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), 64);
+  // packed radial pairs; at least 32 MB (FP64: 64 MB) of spectra, for the
+  // direction slices of small batches
+  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), ((size_t)4 << 20) / n);
   alloc(&h->H, h->hslots * n * ce);
   alloc((void**)&h->ReLf, E * n * sizeof(double));
   if (fp32) {
@@ -554,16 +554,41 @@ template <> struct Terms32Variants<8> { static constexpr int v[5] = {1, 2, 501, 
 template <> struct Terms32Variants<16> { static constexpr int v[7] = {1, 2, 501, 601, 602, 604, 700}; };
 template <> struct Terms32Variants<24> { static constexpr int v[8] = {3, 4, 6, 503, 602, 604, 606, 700}; };
 template <> struct Terms32Variants<32> { static constexpr int v[8] = {4, 8, 104, 108, 504, 604, 608, 616}; };
-template <> struct Terms32Variants<48> { static constexpr int v[4] = {16, 116, 516, 616}; };
+template <> struct Terms32Variants<48> { static constexpr int v[5] = {16, 116, 516, 608, 616}; };
 
 // Direction slices of a terms launch: the two radial points of a CTA or cluster
-// of `ctas` CTAs share its 2 Mu serial transforms; while they leave SMs idle,
-// the directions are split (each slice has its own spectrum, summed in FP64 by
-// the epilogue).
-static int dir_slices(const dgfs_vhs_s* h, int nevals, int ctas) {
-  const int npairs = (h->Nrho + 1) / 2, base = nevals * npairs;
-  const int fit = std::min(148 / (base * ctas), (int)(h->hslots / base));
+// share its 2 Mu serial transforms; while fewer than `resident` CTAs or
+// clusters run, the directions are split (each slice has its own spectrum,
+// summed in FP64 by the epilogue).
+static int dir_slices(const dgfs_vhs_s* h, int nevals, int resident) {
+  const int base = nevals * ((h->Nrho + 1) / 2);
+  const int fit = std::min(resident / base, (int)(h->hslots / base));
   return std::max(1, std::min(fit, h->Mu));
+}
+// CTAs (vhs_terms1_kernel) or clusters (vhs_termsh_kernel) of a kernel that the
+// GPU holds at once; clusters stay inside a GPC, which leaves about a quarter of
+// the SMs unused at 16 CTAs (measured: 7 clusters of 16 at one CTA per SM).
+template <typename R, int N> constexpr int terms1_resident() {
+  return 148 * Terms1Geo<R, N>::per_sm;
+}
+template <typename R, int N, int C> constexpr int termsh_resident() {
+  return 148 * TermsHGeo<R, N, C>::per_sm * 3 / (4 * C);
+}
+template <int N> static int resident32(int code) {
+  if (code == 700) {
+    if constexpr (N <= 24) return terms1_resident<float, N>();
+  }
+  if constexpr (N >= 16 && N <= 24)
+    if (code == 602) return termsh_resident<float, N, 2>();
+  if constexpr (N >= 16 && N <= 32)
+    if (code == 604) return termsh_resident<float, N, 4>();
+  if constexpr (N == 24)
+    if (code == 606) return termsh_resident<float, N, 6>();
+  if constexpr (N >= 32) {
+    if (code == 608) return termsh_resident<float, N, 8>();
+    if (code == 616) return termsh_resident<float, N, 16>();
+  }
+  return 148;
 }
 
 // Default variant: the cube in one CTA where it fits (N=24: 225 us for a
@@ -590,7 +615,7 @@ static int launch_terms32(int c, const VhsTermsArgs& a, int nevals, int Nrho,
     if (c == 604) return launch_termsh_c<float, N, 4>(a, nevals, Nrho, st);
   if constexpr (N == 24)
     if (c == 606) return launch_termsh_c<float, N, 6>(a, nevals, Nrho, st);
-  if constexpr (N == 32)
+  if constexpr (N == 32 || N == 48)
     if (c == 608) return launch_termsh_c<float, N, 8>(a, nevals, Nrho, st);
   if constexpr (N == 32 || N == 48)
     if (c == 616) return launch_termsh_c<float, N, 16>(a, nevals, Nrho, st);
@@ -632,7 +657,6 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
                    const void* const* f_list = nullptr,
                    void* const* q_list = nullptr) {
   constexpr int C64 = VhsClusters<N>::c64;
-  constexpr int C32 = VhsClusters<N>::c32;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
   const bool fp32 = h->precision == DGFS_PREC_FP32;
@@ -664,9 +688,9 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     VhsTablesArgs t{};
     t.mhat = h->mhat; t.mult = h->mult; t.kappa = h->kappa; t.uv = h->uv;
     t.hh = h->hh;
-    t.Mu = h->Mu; t.Nrho = h->Nrho; t.nevals = nevals; t.uv_double = 0;
+    t.Mu = h->Mu; t.Nrho = h->Nrho; t.nevals = nevals;
     const int total = nevals * h->Nrho * h->Mu * 3;
-    if ((rc = launch_plain(vhs_tables_kernel<N>, dim3((total + 95) / 96),
+    if ((rc = launch_plain(vhs_tables_kernel<N>, dim3((total + 47) / 48),
                            dim3(96), 0, h->aux, t)))
       return rc;
     DGFS_CUDA(cudaEventRecord(h->tab, h->aux));
@@ -678,7 +702,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     // default: the two-lanes-per-pencil kernel (its own plane format)
     const int c = h->c32 ? h->c32 : default_terms32<N>();
     a.pm = c >= 600;
-    a.NS = c >= 600 ? dir_slices(h, nevals, c >= 700 ? 1 : c - 600) : 1;
+    a.NS = c >= 600 ? dir_slices(h, nevals, resident32<N>(c)) : 1;
     nslices = a.NS;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
@@ -726,9 +750,13 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
                              dim3(3 * N), psmem, st, a)))
         return rc;
       mark(); mark();  // no Maxwellian-gain stage in FP64 mode
-      a.NS = nslices = dir_slices(h, nevals, N <= 16 ? 1 : C64);
-      if constexpr (N <= 16) rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
-      else rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
+      if constexpr (N <= 16) {
+        a.NS = nslices = dir_slices(h, nevals, terms1_resident<double, N>());
+        rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
+      } else {
+        a.NS = nslices = dir_slices(h, nevals, termsh_resident<double, N, C64>());
+        rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
+      }
       if (rc) return rc;
     } else if constexpr (N == 8 || N == 16 || N == 32) {
       // allocation-free entry: its fixed scratch has no room for the plane
@@ -2273,7 +2301,8 @@ struct dgfs_fno_s {
   std::vector<void*> owned;
 };
 
-static constexpr int kFnoWgradGrid = 296;
+// CTAs of the backward kernels: two (projection) or three (layers) per SM
+static constexpr int kFnoWgradGrid = 296, kFnoLayerGrid = 444;
 
 static void fno_free(dgfs_fno_s* h) {
   for (void* p : h->owned)
@@ -2605,7 +2634,7 @@ template <int MODE>
 static int fno_layer_bwd(dgfs_fno_s* h, const fno::LayerBwdArgs& a, long off,
                          cudaStream_t st) {
   constexpr int n = MODE == 2 ? fno::CIN * fno::WD + fno::WD : fno::kLayerPart;
-  const int grid = (int)std::min<long>((a.R + fno::LBT - 1) / fno::LBT, kFnoWgradGrid);
+  const int grid = (int)std::min<long>((a.R + fno::LBT - 1) / fno::LBT, kFnoLayerGrid);
   DGFS_CUDA(cudaFuncSetAttribute(fno::fno_layer_bwd_kernel<MODE>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)fno::kLayerBwdSmem));

@@ -81,6 +81,7 @@ struct VhsTermsArgs {
   int Nrho;
   int* err;                   // device error flag (a bounded wait gave up)
   int pm;                     // FP32 plane transforms: 1 stores (Re+Im, Re-Im)
+                              // and r_z as [y][x]
   int NS;                     // direction slices (termsh, terms1 kernels): slice
                               // s sums q in [s Mu/NS, (s+1) Mu/NS) and has its
                               // own H, [nevals][ceil(Nrho/2)][NS][n]
@@ -90,12 +91,11 @@ struct VhsTablesArgs {
   const double2* mhat;        // [nevals][3][N]
   const float* mult;          // [Mu] (FP32 tables carry sqrt(mult) on axis x)
   const double* kappa;        // [Nrho][Mu][3] kappa_a = (pi/L)(rho_p/2) sigma_qa
-  void* uv;                   // out [nevals][Nrho][Mu][2][3][N] precision R
+  void* uv;                   // out [nevals][Nrho][Mu][2][3][N] FP32
   double2* hh;                // out [nevals][Nrho][Mu][3][N] FFT(u_a v_a)
   int Mu;
   int Nrho;
   int nevals;
-  int uv_double;              // 1: uv stored as double2
 };
 
 struct VhsGainArgs {
@@ -407,54 +407,54 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
 
 // ---------------------------------------------------------------------------
 // Tables: per (eval, p, q, axis) u_a = IFFT(e^{+i k l} mhat_a),
-// v_a = IFFT(e^{-i k l} mhat_a), hh_a = FFT(u_a v_a)  (FP64, one thread each).
+// v_a = IFFT(e^{-i k l} mhat_a), hh_a = FFT(u_a v_a)  (FP64, two lanes each).
+// Bound: the latency of one lane's chain of N/2 sincos and three transforms
+// (one thread each: 54 us at N=48 for a single point, 10 us at N=16).
 // ---------------------------------------------------------------------------
 template <int N>
-__global__ void vhs_tables_kernel(VhsTablesArgs a) {
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(96) vhs_tables_kernel(VhsTablesArgs a) {
+  constexpr int H = N / 2;
+  const int gid = blockIdx.x * (blockDim.x / 2) + half_pencil(threadIdx.x);
+  const int h = half_lane(threadIdx.x);
   const int total = a.nevals * a.Nrho * a.Mu * 3;
-  if (gid >= total) return;
-  const int ax = gid % 3;
-  const int q = (gid / 3) % a.Mu;
-  const int p = (gid / (3 * a.Mu)) % a.Nrho;
-  const int e = gid / (3 * a.Mu * a.Nrho);
+  const bool live = gid < total;          // (whole warps take part in shuffles)
+  const int g = live ? gid : total - 1;
+  const int ax = g % 3;
+  const int q = (g / 3) % a.Mu;
+  const int p = (g / (3 * a.Mu)) % a.Nrho;
+  const int e = g / (3 * a.Mu * a.Nrho);
   const double kap = a.kappa[((size_t)p * a.Mu + q) * 3 + ax];
   const double2* mh = a.mhat + (size_t)e * 3 * N + ax * N;
-  double2 u[N], w[N];
+  double2 u[H], w[H];
 #pragma unroll
-  for (int l = 0; l < N; ++l) {
-    const int rl = (l < N / 2) ? l : l - N;
+  for (int m = 0; m < H; ++m) {
+    const int l = 2 * m + h, rl = (l < H) ? l : l - N;
     double s, c;
     sincos(kap * (double)rl, &s, &c);
-    const double2 m = mh[l];
-    u[l] = cmul(m, make_double2(c, s));
-    w[l] = cmul(m, make_double2(c, -s));
+    const double2 f = mh[l];
+    u[m] = cmul(f, make_double2(c, s));
+    w[m] = cmul(f, make_double2(c, -s));
   }
-  fft<double, N, +1>(u);
-  fft<double, N, +1>(w);
+  fft_half_dit<double, N, +1>(u, h);      // values h H + m
+  fft_half_dit<double, N, +1>(w, h);
   const size_t tb = (((size_t)e * a.Nrho + p) * a.Mu + q);
-  if (a.uv_double) {
-    double2* uv = static_cast<double2*>(a.uv) + tb * 6 * N;
-#pragma unroll
-    for (int l = 0; l < N; ++l) {
-      uv[ax * N + l] = u[l];
-      uv[(3 + ax) * N + l] = w[l];
-    }
-  } else {
-    float2* uv = static_cast<float2*>(a.uv) + tb * 6 * N;
+  if (live) {
+    float2* uv = static_cast<float2*>(a.uv) + tb * 6 * N + ax * N + h * H;
     const double sc = (ax == 0) ? sqrt((double)a.mult[q]) : 1.0;
 #pragma unroll
-    for (int l = 0; l < N; ++l) {
-      uv[ax * N + l] = make_float2((float)(sc * u[l].x), (float)(sc * u[l].y));
-      uv[(3 + ax) * N + l] = make_float2((float)(sc * w[l].x), (float)(sc * w[l].y));
+    for (int m = 0; m < H; ++m) {
+      uv[m] = make_float2((float)(sc * u[m].x), (float)(sc * u[m].y));
+      uv[3 * N + m] = make_float2((float)(sc * w[m].x), (float)(sc * w[m].y));
     }
   }
 #pragma unroll
-  for (int l = 0; l < N; ++l) u[l] = cmul(u[l], w[l]);
-  fft<double, N, -1>(u);
-  double2* hh = a.hh + tb * 3 * N + ax * N;
+  for (int m = 0; m < H; ++m) u[m] = cmul(u[m], w[m]);
+  fft_half_dif<double, N, -1>(u, h);      // bins 2 m + h
+  if (live) {
+    double2* hh = a.hh + tb * 3 * N + ax * N;
 #pragma unroll
-  for (int l = 0; l < N; ++l) hh[l] = u[l];
+    for (int m = 0; m < H; ++m) hh[2 * m + h] = u[m];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -544,8 +544,8 @@ vhs_maxwell_gain_kernel(VhsGainArgs a) {
         for (int k = 0; k < GG::KY; ++k) {
           const int ly = min(ly0 + GG::NYB * k, N - 1);
           const double2 hxy = hj[q * 2 * N + ly];
-          acc[k].x += hxy.x * hz.x - hxy.y * hz.y;
-          acc[k].y += hxy.x * hz.y + hxy.y * hz.x;
+          acc[k].x += hxy.x * hz.x; acc[k].x -= hxy.y * hz.y;
+          acc[k].y += hxy.x * hz.y; acc[k].y += hxy.y * hz.x;
         }
       }
 #pragma unroll
@@ -920,7 +920,7 @@ vhs_nyq_planes_kernel(VhsTermsArgs a) {
                   ((((size_t)e * a.Nrho + p) * Mu + q) * 3 + P) * N * N;
 #pragma unroll
     for (int r = 0; r < N; ++r)
-      rho[(size_t)r * N + i] =
+      rho[a.pm && P == 2 ? (size_t)i * N + r : (size_t)r * N + i] =
           a.pm ? make_float2(v[r].x + v[r].y, v[r].x - v[r].y) : v[r];
   }
 }
@@ -1555,7 +1555,7 @@ template <typename R, int N, int C> struct TermsHGeo {
   // registers that a lane's N/2 values and sums need
   static constexpr int by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
   static constexpr int max_threads =
-      SPLIT ? (N <= 32 ? 768 : 576)
+      SPLIT ? (N <= 24 ? 768 : N == 32 ? 768 : 576)
             : (N <= 16 ? 640 : N == 24 ? 512 : 384);
   static constexpr int by_regs = max_threads / G::NT;
   static constexpr int per_sm =
@@ -1692,7 +1692,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
                   ((size_t)e * a.Nrho * Mu + term(k)) * 3 * N * N;
     const T rx = rp[yy * N + c];
     const T* rY = rp + N * N + c + h * H * N;
-    const T* rZ = rp + 2 * N * N + yy + h * H * N;
+    const T* rZ = rp + 2 * N * N + yy * N + h * H;   // [y][x]
     const R mq = SPLIT ? R(1) : (R)a.mult[q0 + k % nq];
     T uyz{}, vyz{};
     if constexpr (SPLIT) {
@@ -1701,7 +1701,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     }
 #pragma unroll
     for (int m = 0; m < H; ++m) {
-      const T ry = rY[m * N], rz = rZ[m * N];
+      const T ry = rY[m * N], rz = rZ[m];
       const R xs = (m & 1) ? R(-1) : R(1);   // (-1)^x, H is even
       const R wp = sz * rz.x + (sy * ry.x + xs * rx.x);
       const R wm = sz * rz.y + (sy * ry.y + xs * rx.y);
@@ -1901,7 +1901,7 @@ vhs_terms1_kernel(VhsTermsArgs a) {
     // r_y, r_z of (x, y) = (p, q)
     const T* rp = rho_of(k);
     const T* rY = rp + N * N + p * N;
-    const T rz = rp[2 * N * N + p * N + q];
+    const T rz = rp[2 * N * N + q * N + p];   // [y][x]
     cp_async_wait_all();
     __syncthreads();
 #pragma unroll
@@ -1970,7 +1970,8 @@ vhs_terms1_kernel(VhsTermsArgs a) {
 // Plane transforms of the FP64 terms kernel: as vhs_nyq_planes_kernel, one
 // direction per CTA (3N threads, one pencil each) with the planes transformed
 // in place in shared memory; stores (Re + Im, Re - Im), the combinations
-// s_R + c_I and s_R - c_I the terms kernel multiplies.
+// s_R + c_I and s_R - c_I the terms kernel multiplies, and r_z as [y][x], so
+// that a lane's x values are adjacent.
 template <int N>
 __global__ void __launch_bounds__(3 * N) vhs_nyq_planes64_kernel(VhsTermsArgs a) {
   constexpr int ROW = N + 1, H = N / 2;
@@ -2029,7 +2030,8 @@ __global__ void __launch_bounds__(3 * N) vhs_nyq_planes64_kernel(VhsTermsArgs a)
                  (((size_t)e * a.Nrho * Mu + pq) * 3 + P) * N * N;
 #pragma unroll
   for (int r = 0; r < N; ++r)
-    rho[(size_t)r * N + i] = make_double2(v[r].x + v[r].y, v[r].x - v[r].y);
+    rho[P == 2 ? (size_t)i * N + r : (size_t)r * N + i] =
+        make_double2(v[r].x + v[r].y, v[r].x - v[r].y);
 }
 
 // ---------------------------------------------------------------------------
