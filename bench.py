@@ -38,6 +38,16 @@ def make_inputs(rank=0):
     return prm, f
 
 
+def terms_kernel_name(code):
+    """The FP32 N=32 terms kernel of a variant code (0: the default, 616)."""
+    code = int(code) or 616
+    c = code % 100
+    return {0: f'vhs_terms_fp32_kernel<32,{c}>',
+            1: f'vhs_terms_fp32s_kernel<32,{c}>',
+            5: f'vhs_terms_fp32_kernel<32,{c},TMA>',
+            6: f'vhs_termsh_kernel<float,32,{c}>'}[code // 100]
+
+
 def max_over_ranks(torch, dist, value, world, device):
     """The maximum of a per-rank float over all ranks (the job's time)."""
     t = torch.tensor([float(value)], device=device, dtype=torch.float64)
@@ -772,8 +782,8 @@ def main():
                         'ms_per_step': ms_e2e_seq}},
             'roofline': {
                 'bound': 'fp32-fma',
-                'kernel': f'vhs_terms_fp32_kernel<32,{op32.variant}> '
-                          '(dominant) within the whole operator',
+                'kernel': terms_kernel_name(op32.variant) +
+                          ' (dominant) within the whole operator',
                 'achieved': achieved, 'peak': fma_peak, 'unit': 'TFLOP/s',
                 'frac': achieved / fma_peak,
                 'flops_per_eval_minimal_algorithm': min_flops_eval,

@@ -64,7 +64,7 @@ class VHSOperator:
         nat.check(nat.lib().dgfs_vhs_create(ctypes.byref(d), ctypes.byref(h)))
         self._h = h
         self.Nrho, self.M = d.Nrho, d.M
-        self.variant = 0          # 0: the library's default cluster size
+        self.variant = 0          # 0: the library's default terms kernel
 
     def _nevals(self, f, Q, src, dst, src_base, dst_base, nevals):
         """Check the arrays and slot ranges; return the evaluation count."""

@@ -171,7 +171,7 @@ struct dgfs_vhs_s {
   int device = 0;
   int project = 0;
   double Ginv[25] = {};
-  int c32 = 0;  // cluster size of the FP32 terms kernel (autotuner choice)
+  int c32 = 0;  // variant code of the FP32 terms kernel (autotuner choice)
   // constant tables
   double* c0 = nullptr;      // [N]
   double* b2 = nullptr;      // [n]
@@ -214,7 +214,8 @@ struct dgfs_vhs_s {
   cudaEvent_t join_hi = nullptr, join_aux = nullptr;
 };
 
-// FP32-terms cluster size per N (0: grid not compiled in)
+// cluster size of the one-thread-per-pencil FP32 terms kernel per N (0: grid
+// not compiled in)
 static int c32_of(int N) {
   switch (N) {
     case 8: return 1;
@@ -763,10 +764,10 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
       // transforms, so each term takes a cosine and a sine transform
       constexpr int CN = N == 32 ? 8 : N / 8;
       mark(); mark();
-      if ((rc = launch_cluster(vhs_terms_kernel<double, N, CN, false>,
+      if ((rc = launch_cluster(vhs_terms_kernel<N, CN>,
                                dim3(CN, h->Nrho, nevals), dim3(Geo<N, CN>::NT), CN,
                                3 * (size_t)Geo<N, CN>::SLAB * sizeof(double2) +
-                                   9 * N * sizeof(double2), st, a)))
+                                   3 * N * sizeof(double2), st, a)))
         return rc;
     }
     mark();
@@ -2235,7 +2236,7 @@ extern "C" int dgfs_penalty_model_relax(dgfs_dg_handle h, int32_t kind,
   return DGFS_OK;
 }
 
-// Variants of the FP32 terms kernel (cluster sizes) for the autotuner.
+// Variants of the FP32 terms kernel (codes, see launch_terms32) for the autotuner.
 extern "C" int dgfs_vhs_variants(int32_t N, int32_t* out, int32_t max) {
   if (!out || max <= 0) return fail(DGFS_ERR_INVALID, "bad output buffer");
   const int* v = nullptr;
@@ -2252,15 +2253,15 @@ extern "C" int dgfs_vhs_variants(int32_t N, int32_t* out, int32_t max) {
   return std::min(n, (int)max);
 }
 
-extern "C" int dgfs_vhs_set_variant(dgfs_vhs_handle h, int32_t cluster) {
+extern "C" int dgfs_vhs_set_variant(dgfs_vhs_handle h, int32_t variant) {
   if (!h) return fail(DGFS_ERR_INVALID, "null handle");
   int buf[8];
   const int n = dgfs_vhs_variants(h->N, buf, 8);
   if (n < 0) return n;
   for (int i = 0; i < n; ++i)
-    if (buf[i] == cluster) { h->c32 = cluster; return DGFS_OK; }
-  if (cluster == 0) { h->c32 = 0; return DGFS_OK; }
-  return fail(DGFS_ERR_INVALID, "cluster size not a variant for this N");
+    if (buf[i] == variant) { h->c32 = variant; return DGFS_OK; }
+  if (variant == 0) { h->c32 = 0; return DGFS_OK; }
+  return fail(DGFS_ERR_INVALID, "code is not a variant for this N");
 }
 
 // ---------------------------------------------------------------------------
@@ -2279,7 +2280,7 @@ struct dgfs_fno_s {
   float* grad = nullptr;
   float* am = nullptr;
   float* av = nullptr;
-  float2 *tF = nullptr, *tG = nullptr, *tFs = nullptr, *tGs = nullptr;
+  float2 *tF = nullptr, *tG = nullptr;
   __nv_bfloat16* x0 = nullptr;
   __nv_bfloat16* v[5] = {};
   __nv_bfloat16* y[4] = {};
@@ -2370,16 +2371,14 @@ extern "C" int dgfs_fno_create(const dgfs_fno_desc* d, dgfs_fno_handle* out) {
       for (int s = 0; s < 5; ++s) h->Ginv[r * 5 + s] = (double)G[r][5 + s];
   }
   // DFT tables: modes k = 0..K/2-1, -K/2..-1
-  std::vector<float2> tF(K * N), tG(N * K), tFs(K * N), tGs(N * K);
+  std::vector<float2> tF(K * N), tG(N * K);
   for (int kk = 0; kk < K; ++kk) {
     const int k = kk < K / 2 ? kk : kk - K;
     for (int x = 0; x < N; ++x) {
       const double a = -2.0 * M_PI * (double)k * x / N;
       const double c = std::cos(a), s = std::sin(a);
       tF[kk * N + x] = make_float2((float)c, (float)s);
-      tFs[kk * N + x] = make_float2((float)(c / N), (float)(s / N));
       tG[x * K + kk] = make_float2((float)(c / N), (float)(-s / N));
-      tGs[x * K + kk] = make_float2((float)c, (float)(-s));
     }
   }
   cudaError_t e = cudaSuccess;
@@ -2389,7 +2388,7 @@ extern "C" int dgfs_fno_create(const dgfs_fno_desc* d, dgfs_fno_handle* out) {
   A(&h->c0, N);
   A(&h->p32, h->L.total); A(&h->p16, h->L.total); A(&h->grad, h->L.total);
   A(&h->am, h->L.total); A(&h->av, h->L.total);
-  A(&h->tF, K * N); A(&h->tG, K * N); A(&h->tFs, K * N); A(&h->tGs, K * N);
+  A(&h->tF, K * N); A(&h->tG, K * N);
   A(&h->x0, B * n * fno::CIN);
   for (int l = 0; l < 5; ++l) A(&h->v[l], B * n * fno::WD);
   for (int l = 0; l < 4; ++l) A(&h->y[l], B * n * fno::WD);
@@ -2414,8 +2413,6 @@ extern "C" int dgfs_fno_create(const dgfs_fno_desc* d, dgfs_fno_handle* out) {
   if (e == cudaSuccess) e = cudaMemcpy(h->c0, c0.data(), N * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(h->tF, tF.data(), K * N * sizeof(float2), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(h->tG, tG.data(), K * N * sizeof(float2), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(h->tFs, tFs.data(), K * N * sizeof(float2), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(h->tGs, tGs.data(), K * N * sizeof(float2), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(h->p32, 0, h->L.total * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(h->p16, 0, h->L.total * sizeof(__nv_bfloat16));
   if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));

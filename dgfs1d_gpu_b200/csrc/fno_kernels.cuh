@@ -265,9 +265,7 @@ __global__ void __launch_bounds__(256) fno_features_kernel(FeatArgs a) {
 // ---------------------------------------------------------------------------
 // Truncated DFT along one axis: in [outer][LIN][inner] -> out [outer][LOUT][inner],
 // out[k] = sum_j T[k][j] in[j] with a complex table T [LOUT][LIN].
-// IN: 0 BF16 real, 1 FP32 real, 2 complex FP32.
-// OUT: 0 complex FP32, 1 Re -> FP32 store, 2 Re -> FP32 accumulate,
-//      3 Re -> BF16 store.
+// IN: 0 BF16 real, 2 complex FP32.  OUT: 0 complex FP32, 3 Re -> BF16 store.
 // One thread per two adjacent (outer, inner) pencils (inner is even):
 // consecutive threads take consecutive inner pairs, so loads and stores are
 // coalesced and every table entry read from shared memory serves two pencils.
@@ -291,10 +289,6 @@ fno_dft_kernel(const void* in, void* out, const float2* table, long outer,
     if (IN == 0) {
       const float2 v = __bfloat1622float2(
           *reinterpret_cast<const __nv_bfloat162*>(static_cast<const __nv_bfloat16*>(in) + idx));
-      x0[j] = make_float2(v.x, 0.f);
-      x1[j] = make_float2(v.y, 0.f);
-    } else if (IN == 1) {
-      const float2 v = *reinterpret_cast<const float2*>(static_cast<const float*>(in) + idx);
       x0[j] = make_float2(v.x, 0.f);
       x1[j] = make_float2(v.y, 0.f);
     } else {
@@ -328,12 +322,6 @@ fno_dft_kernel(const void* in, void* out, const float2* table, long outer,
     const long idx = (o * LOUT + k) * inner + i;
     if (OUT == 0) {
       *reinterpret_cast<float4*>(static_cast<float2*>(out) + idx) = make_float4(r0, i0, r1, i1);
-    } else if (OUT == 1) {
-      *reinterpret_cast<float2*>(static_cast<float*>(out) + idx) = make_float2(r0, r1);
-    } else if (OUT == 2) {
-      float2* q = reinterpret_cast<float2*>(static_cast<float*>(out) + idx);
-      const float2 c = *q;
-      *q = make_float2(c.x + r0, c.y + r1);
     } else {
       *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(out) + idx) =
           __floats2bfloat162_rn(r0, r1);
@@ -528,8 +516,9 @@ fno_proj_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w16, Layout L,
 // Bound: FP32 FMAs and shared-memory reads, about equal.  Against separate
 // kernels for dz, its products and its column sums (which moved 2 x 4 B x PJ
 // per point through global memory twice) a step's projection backward went
-// from 2.0 to 0.5 ms on 24 samples at N=32, and the four layers' pointwise
-// parts from 2.5 to 0.6 ms.
+// from 2.0 to 0.61 ms on 24 samples at N=32, and the four layers' pointwise
+// parts from 2.5 to 0.86 ms (the lift's weight gradient, 1.4 ms before, is in
+// the last one).
 // ---------------------------------------------------------------------------
 constexpr int PBT = 64;                    // points per tile (projection)
 constexpr int PBX = WD + 4, PBZ = PJ + 4;  // row pitches (floats)
@@ -1131,8 +1120,9 @@ __global__ void __launch_bounds__(128) fno_tc_kernel(TcArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Evaluation path with fused spectral passes (inference; training keeps the
-// per-axis passes above, whose intermediates its backward pass reuses).
+// Forward path with fused spectral passes, for evaluation and training (a
+// training step also stores each layer's mode spectra Vh and pre-activation y
+// for its backward pass).
 // With Y[b][x][ky][kz][c] = the yz spectra of v_l (complex FP32):
 //   fno_xmix_kernel        one CTA per (ky, kz): FFT over x, keep K modes, mix
 //                          with W_l, inverse FFT over x (1/N)

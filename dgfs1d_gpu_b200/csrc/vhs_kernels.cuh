@@ -23,8 +23,9 @@
 //              F_g = F - M_hat, Re IFFT(b2 F)
 //   tables     (FP64): per (eval,p,q) 1-D u_a, v_a and FFT(u_a v_a)
 //   maxwell_gain (FP64): Ghat_M = sum_p W_p b1_p sum_q m_q prod_a FFT(u_a v_a)
-//   terms      (cluster per (eval,p), precision R): H_p = W_p b1_p FFT(S_p)
-//   epilogue   (cluster per eval, FP64): Ghat = Ghat_M + sum_p H_p,
+//   nyq_planes: 2-D transforms of the Nyquist planes, for packed transforms
+//   terms      (CTA or cluster per (eval, radial pair)): H = b1 FFT(S)
+//   epilogue   (cluster per eval, FP64): Ghat = Ghat_M + sum H,
 //              Q += prefac (Re IFFT(Ghat) - f Re IFFT(b2 F))
 #pragma once
 #include <cuda_runtime.h>
@@ -565,52 +566,37 @@ vhs_maxwell_gain_kernel(VhsGainArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Terms: one cluster per (eval, p).  Precision R; SPLIT selects the
-// Maxwellian-split combine.  FP32 keeps the running S_p in registers and the
-// F slab resident in shared memory; FP64 keeps S_p in shared memory and
-// streams F rows from global memory.
+// Terms, FP64, a cosine and a sine transform per term: one cluster per (eval,
+// p), the running sums S_p in shared memory, F rows streamed from global
+// memory.  Serves the allocation-free entry, whose fixed scratch has no room
+// for the plane transforms that packed transforms need (with a handle, N=32,
+// 24 points, the packed kernel takes 1.0 ms against 3.0 ms here).
 // ---------------------------------------------------------------------------
-template <typename R, int N, int C, bool SPLIT>
+template <int N, int C>
 __global__ void __launch_bounds__(Geo<N, C>::NT, 1)
 vhs_terms_kernel(VhsTermsArgs a) {
   using G = Geo<N, C>;
-  using T = c2_t<R>;
-  constexpr bool S_REG = (sizeof(R) == 4);
+  using R = double;
+  using T = double2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* A = reinterpret_cast<T*>(smem_raw);
   T* Rb = A + G::SLAB;
-  T* F = Rb + G::SLAB;              // S_REG: resident F slab; else S slab
-  T* tab = F + G::SLAB;             // [3][N] phase + [6][N] u,v
+  T* Ss = Rb + G::SLAB;             // running sums S_p
+  T* tab = Ss + G::SLAB;            // [3][N] phase
   const int t = threadIdx.x;
   const unsigned rank = cluster_rank();
   const int p = blockIdx.y, e = blockIdx.z;
   const T* Fg = static_cast<const T*>(a.Fg) + (size_t)e * G::n;
   const T* ph = static_cast<const T*>(a.ph);
-  const T* uvg = static_cast<const T*>(a.uv);
-
-  T S[S_REG ? N : 1];
-  if constexpr (S_REG) {
+  const int yl = t / N, zz = t % N;
+  const int ybase = yl * G::PLANE + zz;   // this thread's pencil of a Y-slab
 #pragma unroll
-    for (int x = 0; x < N; ++x) S[x] = T{0, 0};
-    for (int j = t; j < G::P * N * N; j += G::NT)
-      F[slab_index<N, C>(j)] = Fg[(size_t)rank * G::P * N * N + j];
-  } else {
-    const int base = (t / N) * G::PLANE + (t % N);
-#pragma unroll
-    for (int x = 0; x < N; ++x) F[base + x * G::ROW] = T{0, 0};
-  }
-
-  const int yl = t / N, zz = t % N, yy = rank * G::P + yl;
-  bool first = true;
+  for (int x = 0; x < N; ++x) Ss[ybase + x * G::ROW] = T{0, 0};
+  cluster_arrive();                 // (this CTA is running)
   for (int q = 0; q < a.Mu; ++q) {
     __syncthreads();  // previous term's table readers are done
     for (int i = t; i < 3 * N; i += G::NT)
       tab[i] = ph[((size_t)p * a.Mu + q) * 3 * N + i];
-    if constexpr (SPLIT) {
-      for (int i = t; i < 6 * N; i += G::NT)
-        tab[3 * N + i] =
-            uvg[((((size_t)e * a.Nrho) + p) * a.Mu + q) * 6 * N + i];
-    }
     __syncthreads();
     const R mq = (R)a.mult[q];
 #pragma unroll 1
@@ -620,15 +606,9 @@ vhs_terms_kernel(VhsTermsArgs a) {
         const int pl = t / N, ly = t % N, lx = rank * G::P + pl;
         const T bxy = cmul(tab[lx], tab[N + ly]);
         T v[N];
-        if constexpr (S_REG) {
-          const int base = pl * G::PLANE + ly * G::ROW;
+        const T* row = Fg + ((size_t)lx * N + ly) * N;
 #pragma unroll
-          for (int k = 0; k < N; ++k) v[k] = F[base + k];
-        } else {
-          const T* row = Fg + ((size_t)lx * N + ly) * N;
-#pragma unroll
-          for (int k = 0; k < N; ++k) v[k] = row[k];
-        }
+        for (int k = 0; k < N; ++k) v[k] = row[k];
 #pragma unroll
         for (int k = 0; k < N; ++k) {
           const T ph3 = cmul(bxy, tab[2 * N + k]);
@@ -642,70 +622,32 @@ vhs_terms_kernel(VhsTermsArgs a) {
         for (int k = 0; k < N; ++k) A[base + k] = v[k];
       }
       __syncthreads();
-      {
-        T v[N];
-        slab_col_load_fft<R, N, C, +1>(A, t, v);
-        if (!first) cluster_wait();  // receive buffers are free
-        push_cols_to_yslab<R, N, C>(Rb, t, rank, v);
-      }
-      first = false;
+      T v[N];
+      slab_col_load_fft<R, N, C, +1>(A, t, v);
+      cluster_wait();    // every CTA runs and its receive buffer is free
+      push_cols_to_yslab<R, N, C>(Rb, t, rank, v);
       cluster_arrive();
       cluster_wait();
-      T v[N];
       yslab_load_pencil<R, N, C>(Rb, t, v);
       cluster_arrive();  // done reading the receive buffer
       fft<R, N, +1>(v);
-      T sv[N];
-      if constexpr (!S_REG) {
-        const int base = yl * G::PLANE + zz;
 #pragma unroll
-        for (int x = 0; x < N; ++x) sv[x] = F[base + x * G::ROW];
-      }
-      if constexpr (SPLIT) {
-        const T* ut = tab + 3 * N;
-        const T* vt = tab + 6 * N;
-        const T uyz = cmul(ut[N + yy], ut[2 * N + zz]);
-        const T vyz = cmul(vt[N + yy], vt[2 * N + zz]);
-#pragma unroll
-        for (int x = 0; x < N; ++x) {
-          const T um = cmul(ut[x], uyz), vm = cmul(vt[x], vyz);
-          T XM;
-          if (s == 0) { XM.x = R(0.5) * (um.x + vm.x); XM.y = R(0.5) * (um.y + vm.y); }
-          else        { XM.x = R(0.5) * (um.y - vm.y); XM.y = R(-0.5) * (um.x - vm.x); }
-          // h_rest = 2 XM X + X^2 = X (2 XM + X)
-          T w; w.x = R(2) * XM.x + v[x].x; w.y = R(2) * XM.y + v[x].y;
-          const T h = cmul(v[x], w);
-          if constexpr (S_REG) { S[x].x += mq * h.x; S[x].y += mq * h.y; }
-          else { sv[x].x += mq * h.x; sv[x].y += mq * h.y; }
-        }
-      } else {
-#pragma unroll
-        for (int x = 0; x < N; ++x) {
-          const T h = cmul(v[x], v[x]);
-          if constexpr (S_REG) { S[x].x += mq * h.x; S[x].y += mq * h.y; }
-          else { sv[x].x += mq * h.x; sv[x].y += mq * h.y; }
-        }
-      }
-      if constexpr (!S_REG) {
-        const int base = yl * G::PLANE + zz;
-#pragma unroll
-        for (int x = 0; x < N; ++x) F[base + x * G::ROW] = sv[x];
+      for (int x = 0; x < N; ++x) {
+        const T h = cmul(v[x], v[x]);
+        T sv = Ss[ybase + x * G::ROW];
+        sv.x += mq * h.x;
+        sv.y += mq * h.y;
+        Ss[ybase + x * G::ROW] = sv;
       }
     }
   }
 
   // forward FFT of S_p: x-pass, exchange into X-slabs, y-pass, z-pass
   T v[N];
-  if constexpr (S_REG) {
 #pragma unroll
-    for (int x = 0; x < N; ++x) v[x] = S[x];
-  } else {
-    const int base = yl * G::PLANE + zz;
-#pragma unroll
-    for (int x = 0; x < N; ++x) v[x] = F[base + x * G::ROW];
-  }
+  for (int x = 0; x < N; ++x) v[x] = Ss[ybase + x * G::ROW];
   fft<R, N, -1>(v);
-  if (!first) cluster_wait();
+  cluster_wait();
   push_pencils_to_xslab<R, N, C>(A, t, rank, v);
   cluster_arrive();
   cluster_wait();

@@ -148,8 +148,8 @@ class FNOSurrogate:
         nat.check(nat.lib().dgfs_fno_set_tensor_cores(self._h, int(bool(enable))))
 
     def set_fused(self, enable=True):
-        """Evaluation with the fused spectral kernels (default) or with the
-        per-axis DFT passes that training uses."""
+        """Evaluation and the training forward with the fused spectral kernels
+        (default) or with the per-axis DFT passes."""
         nat.check(nat.lib().dgfs_fno_set_fused(self._h, int(bool(enable))))
 
     def device_error(self):

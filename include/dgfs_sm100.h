@@ -133,11 +133,12 @@ int dgfs_vhs_fs2(dgfs_vhs_handle h, const void* f, const void* g, void* Q,
 int dgfs_vhs_set_projection(dgfs_vhs_handle h, int32_t enable);
 
 /* Autotuning (no reference counterpart): the FP32 terms kernel comes in
- * several thread-block-cluster sizes per N.  dgfs_vhs_variants writes the
- * compiled cluster sizes for N into out (up to max) and returns their count;
+ * several variants per N (kinds and thread-block-cluster sizes).
+ * dgfs_vhs_variants writes the codes of the variants compiled for N into out
+ * (up to max) and returns their count;
  * dgfs_vhs_set_variant selects one for a handle (0 = built-in default). */
 int dgfs_vhs_variants(int32_t N, int32_t* out, int32_t max);
-int dgfs_vhs_set_variant(dgfs_vhs_handle h, int32_t cluster);
+int dgfs_vhs_set_variant(dgfs_vhs_handle h, int32_t variant);
 
 /* Device error flag of the handle's kernels (no reference counterpart):
  * nonzero when a bounded wait (the TMA copies of the TMA terms variant)
@@ -213,10 +214,10 @@ int dgfs_vss_eval(dgfs_vss_handle h, int32_t p, int32_t q, const void* f_p,
 /* Every pair of one species in one call (the species loop of the
  * reference's mixture right-hand side, bi/bi.py:336-342, which calls fs once
  * per partner q):  Q_p[dst(i)] += sum_q Q_pq(f_p[src(i)], f_q[src(i)]).
- * f is a host array of nspcs device pointers (f[q] holds species q).  In
- * the FP32 mode one launch per stage covers every pair (prologues once per
- * input species, the FP64 Maxwellian gain beside the FP32 terms kernel, one
- * epilogue summing the pairs); in the FP64 mode the pairs run one by one. */
+ * f is a host array of nspcs device pointers (f[q] holds species q).  One
+ * launch per stage covers every pair in both precisions (prologues once per
+ * input species, one epilogue summing the pairs; in the FP32 mode the FP64
+ * Maxwellian gain runs beside the FP32 terms kernel). */
 int dgfs_vss_eval_species(dgfs_vss_handle h, int32_t p, const void* const* f,
                           int32_t f_dtype, void* Q_p, int32_t q_dtype,
                           const int32_t* src_slots, int32_t src_base,
@@ -489,8 +490,9 @@ int dgfs_fno_last_loss(dgfs_fno_handle h, double* host, int32_t B);
 int dgfs_fno_set_tensor_cores(dgfs_fno_handle h, int32_t enable);
 /* Evaluation with the fused spectral kernels (default, 1: per layer an x-mix
  * launch and a yz-inverse + tensor-core dense launch, yz spectra by register
- * FFTs) or with the per-axis DFT passes that training uses (0).  The fused
- * path needs the tensor cores; with them disabled eval uses the passes. */
+ * FFTs) or with the per-axis DFT passes (0); the training forward follows
+ * the same choice.  The fused path needs the tensor cores; with them disabled
+ * the passes run. */
 int dgfs_fno_set_fused(dgfs_fno_handle h, int32_t enable);
 /* Device error flag of the tensor-core kernels (1: an MMA completion wait
  * timed out and the kernel stopped); synchronous, resets the flag. */
