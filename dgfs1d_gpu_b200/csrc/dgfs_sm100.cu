@@ -227,6 +227,7 @@ static int c32_of(int N) {
   }
 }
 template <int N> struct VhsClusters;
+static size_t slots_resident(int N, bool fp32);
 // c64: FP64 terms kernel with two lanes per pencil (vhs_termsh_kernel; up to
 // N=16 vhs_terms1_kernel runs); c32: FP32 terms kernel with one thread per
 // pencil; cpro / cepi: prologue / epilogue (FP64, two lanes per pencil, one slab
@@ -405,9 +406,9 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   alloc((void**)&h->err, sizeof(int));
   if (ce_ == cudaSuccess) ce_ = cudaMemset(h->err, 0, sizeof(int));
   alloc(&h->Fg, E * n * ce);
-  // packed radial pairs; at least 32 MB (FP64: 64 MB) of spectra, for the
-  // direction slices of small batches
-  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), ((size_t)4 << 20) / n);
+  // packed radial pairs; at least what the GPU holds at once, for the direction
+  // slices of small batches
+  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), slots_resident(N, fp32));
   alloc(&h->H, h->hslots * n * ce);
   alloc((void**)&h->ReLf, E * n * sizeof(double));
   if (fp32) {
@@ -599,6 +600,27 @@ template <int N> static int resident32(int code) {
 // TMA staging; N=48: 42.3 against 63.9 ms for 96 points).
 template <int N> constexpr int default_terms32() {
   return N <= 24 ? 700 : 616;
+}
+
+// The largest grid (CTAs or clusters) that dir_slices fills, over the variants.
+template <int N> static size_t slots_resident_n(bool fp32) {
+  if (!fp32) {
+    if constexpr (N <= 16) return terms1_resident<double, N>();
+    else return termsh_resident<double, N, VhsClusters<N>::c64>();
+  }
+  int m = 1;
+  for (int c : Terms32Variants<N>::v)
+    if (c >= 600) m = std::max(m, resident32<N>(c));
+  return m;
+}
+static size_t slots_resident(int N, bool fp32) {
+  switch (N) {
+    case 8: return slots_resident_n<8>(fp32);
+    case 16: return slots_resident_n<16>(fp32);
+    case 24: return slots_resident_n<24>(fp32);
+    case 32: return slots_resident_n<32>(fp32);
+    default: return slots_resident_n<48>(fp32);
+  }
 }
 
 template <int N>
@@ -1244,7 +1266,7 @@ struct dgfs_dg_s {
 
 static void free_dg(dgfs_dg_s* h) {
   void* ptrs[] = {h->c0, h->invjac, h->f0[0], h->f0[1], h->nden, h->im, h->part,
-                  h->wpart, h->wdone, h->mpart, h->lim};
+                  h->mpart, h->lim};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->part_h) cudaFreeHost(h->part_h);
@@ -1296,13 +1318,14 @@ extern "C" int dgfs_dg_create(const dgfs_dg_desc* d, dgfs_dg_handle* out) {
       std::vector<double> f0(d->bc_f0[s], d->bc_f0[s] + Nv);
       if ((rc = upload(&h->f0[s], f0))) { free_dg(h); return rc; }
     }
-  cudaError_t e1 = cudaMalloc(&h->nden, 2 * sizeof(double));
+  // nden, wpart and wdone share one allocation, zeroed once
+  const size_t wall = (2 + 4 * kWallCh + 1) * sizeof(double);
+  cudaError_t e1 = cudaMalloc(&h->nden, wall);
+  if (e1 == cudaSuccess) e1 = cudaMemset(h->nden, 0, wall);
+  h->wpart = h->nden + 2;
+  h->wdone = reinterpret_cast<unsigned*>(h->wpart + 4 * kWallCh);
   if (e1 == cudaSuccess) e1 = cudaMalloc(&h->part, 2 * 1024 * sizeof(double));
   if (e1 == cudaSuccess) e1 = cudaMallocHost(&h->part_h, 2 * 1024 * sizeof(double));
-  if (e1 == cudaSuccess) e1 = cudaMalloc(&h->wpart, 2 * kWallCh * 2 * sizeof(double));
-  if (e1 == cudaSuccess) e1 = cudaMalloc(&h->wdone, sizeof(unsigned));
-  if (e1 == cudaSuccess) e1 = cudaMemset(h->wdone, 0, sizeof(unsigned));
-  if (e1 == cudaSuccess) e1 = cudaMemset(h->nden, 0, 2 * sizeof(double));
   h->mpts = std::max(K, d->Nqr) * Ne;
   if (e1 == cudaSuccess)
     e1 = cudaMalloc(&h->mpart, (size_t)h->mpts * kPmCh * kPmMaxNa * sizeof(double));
