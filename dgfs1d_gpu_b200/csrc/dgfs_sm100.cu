@@ -1534,6 +1534,7 @@ struct dgfs_vss_s {
   double* c0 = nullptr;                // [N]
   void* F[4] = {};                     // [E][n] complex R
   void* Fny[4] = {};                   // [E][3][N][N] complex R
+  double* norm2[4] = {};               // [E][cpro <= 16] partial sums |F|^2
   double2* mhat[4] = {};               // [E][3][N]
   double* mom[4] = {};                 // [E][5]
   double* ReLf = nullptr;              // [nspcs][E][n]
@@ -1556,7 +1557,8 @@ static void free_vss(dgfs_vss_s* h) {
     for (void* q : {(void*)p.b, (void*)p.c, (void*)p.ph, (void*)p.b32, (void*)p.ph32})
       if (q) cudaFree(q);
   for (int i = 0; i < 4; ++i)
-    for (void* q : {h->F[i], h->Fny[i], (void*)h->mhat[i], (void*)h->mom[i]})
+    for (void* q : {h->F[i], h->Fny[i], (void*)h->norm2[i], (void*)h->mhat[i],
+                    (void*)h->mom[i]})
       if (q) cudaFree(q);
   for (void* q : {(void*)h->w, (void*)h->dirs, (void*)h->dirsm, (void*)h->c0,
                   (void*)h->ReLf, h->rho, (void*)h->uv, (void*)h->hh, (void*)h->GM, h->H})
@@ -1700,6 +1702,7 @@ extern "C" int dgfs_vss_create(const dgfs_vss_desc* d, dgfs_vss_handle* out) {
     for (int s2 = 0; s2 < std::max(2, h->nspcs); ++s2) {
       A(&h->F[s2], E * n * ce);
       A(&h->Fny[s2], E * 3 * N * N * ce);
+      A(&h->norm2[s2], E * 16 * sizeof(double));
       if (fp32) {
         A(&h->mhat[s2], E * 3 * N * sizeof(double2));
         A(&h->mom[s2], E * 5 * sizeof(double));
@@ -1793,7 +1796,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
     a.f = c.fin[s]; a.f_list = c.fl[s]; a.f_double = f_double;
     a.src_slots = ss; a.src_base = sb; a.c0 = h->c0; a.cw = h->cw;
     a.b2c = pair(k < c.nq ? k : 0).c; a.ReLf = k < c.nq ? ReLf(k) : nullptr;
-    a.Fg = h->F[s];
+    a.Fg = h->F[s]; a.norm2 = h->norm2[s];
     if (FP32) {
       a.split = 1; a.Fny = static_cast<float2*>(h->Fny[s]);
       a.mhat = h->mhat[s]; a.moments = h->mom[s];
@@ -1806,7 +1809,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
       return rc;
   }
   VssTermsArgs tt{};
-  tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals;
+  tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals; tt.nc = CPRO;
   tt.NS = FP32 ? h->Nrho
                : (int)std::max<size_t>(1, std::min<size_t>(
                      h->Nrho, h->hslots / ((size_t)c.nq * nevals)));
@@ -1817,6 +1820,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
     VssTermsPair& pr = tt.pr[k];
     pr.Fp = h->F[c.sp]; pr.Fq = h->F[c.sq[k]];
     pr.Fnyp = h->Fny[c.sp]; pr.Fnyq = h->Fny[c.sq[k]];
+    pr.n2p = h->norm2[c.sp]; pr.n2q = h->norm2[c.sq[k]];
     pr.ph = FP32 ? (const void*)P.ph32 : (const void*)P.ph;
     pr.b = FP32 ? (const void*)P.b32 : (const void*)P.b;
     pr.uv = FP32 ? h->uv + k * E * Tt * 6 * N : nullptr;

@@ -65,6 +65,8 @@ struct VhsPrologueArgs {
                               // F_g: [0][ly][lz] at lx=N/2, [1][lx][lz] at
                               // ly=N/2, [2][lx][ly] at lz=N/2
   double2* Fny64;             // out (not split, may be null): those of F
+  double* norm2;              // out (may be null) [nevals][C] sum |Fg|^2 of
+                              // each CTA's slab
 };
 
 struct VhsTermsArgs {
@@ -343,6 +345,7 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
   // F = FFT(f)/n; write F (FP64) or F_g = F - mhat (FP32); then A <- b2 F
   const double inv_n = 1.0 / (double)G::n;
   const size_t lbase = (size_t)rank * P * N * N, gbase = (size_t)e * G::n + lbase;
+  double nrm = 0;
 #pragma unroll 4
   for (int j = t; j < P * N * N; j += NT) {
     const int si = (j / N) * G::ROW + j % N;
@@ -356,6 +359,7 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
       g.x = (float)(Fv.x - mm.x);
       g.y = (float)(Fv.y - mm.y);
       if (a.Fg) static_cast<float2*>(a.Fg)[gbase + j] = g;
+      nrm += (double)g.x * g.x + (double)g.y * g.y;
       if (a.Fny) {
         float2* ny = a.Fny + (size_t)e * 3 * N * N;
         if (fx == N / 2) ny[ly * N + lz] = g;
@@ -364,6 +368,7 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
       }
     } else {
       static_cast<double2*>(a.Fg)[gbase + j] = Fv;
+      nrm += Fv.x * Fv.x + Fv.y * Fv.y;
       if (a.Fny64) {
         double2* ny = a.Fny64 + (size_t)e * 3 * N * N;
         if (fx == N / 2) ny[ly * N + lz] = Fv;
@@ -383,6 +388,16 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
   }
   if (a.split && rank == 0 && a.mhat)
     for (int i = t; i < 3 * N; i += NT) a.mhat[(size_t)e * 3 * N + i] = mh[i];
+  if (a.norm2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+    if ((t & 31) == 0) red[t >> 5] = nrm;   // (peers read red[160 + k] only)
+    __syncthreads();
+    if (t == 0) {
+      for (int i = 1; i < NT / 32; ++i) nrm += red[i];
+      a.norm2[(size_t)e * C + rank] = nrm;
+    }
+  }
   if (!a.ReLf) return;   // (no CTA writes to a peer past this point)
   __syncthreads();
   // loss: Re IFFT(b2 F)

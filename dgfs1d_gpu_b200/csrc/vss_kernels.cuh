@@ -294,10 +294,13 @@ struct VssTermsPair {
   void* H;                 // out [E][NS][n]
   const int2* dirs;        // [nd] direction and its merged antipode (or -1)
   int nd;
+  const double* n2p;       // [E][nc] sums |F_p|^2, |F_q|^2 of the prologue's CTAs
+  const double* n2q;
 };
 struct VssTermsArgs {
   VssTermsPair pr[4];
   const double* w;         // [Nrho]
+  int nc;                  // CTAs per point of the prologue
   int Nrho, M, nevals;
   int NS;                  // radial slices (blockIdx.y): r in [y Nrho/NS, ...)
 };
@@ -308,12 +311,36 @@ template <typename T> __device__ __forceinline__ T vss_nu(T ph) {
   return cmul(c, c);
 }
 
+// Powers of two that bring F_p and F_q of a point to the same norm.  u and v
+// share one complex transform, whose rounding is relative to the larger of the
+// two; unscaled, the smaller one (a trace species, or in the FP32 mode the
+// species nearer to its Maxwellian) would carry the larger one's absolute
+// error.  The smaller is scaled up, by su or sv, and the factor leaves the
+// spectral sums through back = 1 / (su sv): every step is exact.  back = 0 if
+// either is zero everywhere (u v = 0).
+template <typename R> struct VssScale { R su, sv, back; };
+template <typename R>
+__device__ __forceinline__ VssScale<R> vss_scale(const VssTermsPair& Pr, int e, int nc) {
+  double sp = 0, sq = 0;
+  for (int c = 0; c < nc; ++c) {
+    sp += Pr.n2p[(size_t)e * nc + c];
+    sq += Pr.n2q[(size_t)e * nc + c];
+  }
+  if (sp == 0 || sq == 0) return {R(1), R(1), R(0)};
+  constexpr int KMAX = sizeof(R) == 4 ? 60 : 400;
+  int k = 0;                       // (a sum that is not finite: unscaled)
+  if (isfinite(sp) && isfinite(sq)) k = (ilogb(sq) - ilogb(sp)) / 2;
+  k = max(-KMAX, min(KMAX, k));
+  return {(R)ldexp(1.0, max(k, 0)), (R)ldexp(1.0, max(-k, 0)), (R)ldexp(1.0, -abs(k))};
+}
+
 // Plane transforms of one term.  With E the phase factor and f_S as in the
 // packed VHS transforms, E F splits on the Nyquist planes into
 // E (1 + f_S)/2 F, whose inverse transform is real, and E (1 - f_S)/2 F, whose
 // inverse transform is i u_i (i v_i).  This kernel forms u_i + i v_i, the
 // inverse transform of -i E_u (1 - f_u)/2 F_p + E_v (1 - f_v)/2 F_q, as three
-// 2-D transforms (rows and planes as in vhs_nyq_planes64_kernel).
+// 2-D transforms (rows and planes as in vhs_nyq_planes64_kernel), scaled as
+// the terms are (vss_scale).
 // Grid (terms of the list, 1, npair nevals), 3N threads, one pencil each.
 template <typename R, int N>
 __global__ void __launch_bounds__(3 * N) vss_planes_kernel(VssTermsArgs a) {
@@ -331,6 +358,7 @@ __global__ void __launch_bounds__(3 * N) vss_planes_kernel(VssTermsArgs a) {
   const int P = t / N, i = t % N;
   const T* Fp = static_cast<const T*>(Pr.Fnyp) + (size_t)e * 3 * N * N;
   const T* Fq = static_cast<const T*>(Pr.Fnyq) + (size_t)e * 3 * N * N;
+  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
 #pragma unroll 4
   for (int j = t; j < 3 * N * N; j += 3 * N) {
     pls[(j / N) * ROW + j % N] = Fp[j];
@@ -367,6 +395,9 @@ __global__ void __launch_bounds__(3 * N) vss_planes_kernel(VssTermsArgs a) {
       tk = tt + N;
     }
     if (P >= 1 && i == H) rowc = T{R(0), R(0)};
+    const R ss = s == 0 ? sc.su : sc.sv;
+    rowc.x *= ss;
+    rowc.y *= ss;
     // (1 - f)/2 rowc
     const T g = cmul(T{R(0.5) * (R(1) - f_row.x), R(-0.5) * f_row.y}, rowc);
     const T gH = (P == 2) ? T{R(0), R(0)}
@@ -455,12 +486,16 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
   T Qh[H];
 #pragma unroll
   for (int m = 0; m < H; ++m) Qh[m] = T{R(0), R(0)};
-  // the row factors of a term: one (field, row) per thread
+  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
+  // the row factors of a term, scaled: one (field, row) per thread
   auto row_tables = [&](int term) {
     const int f = t / (P * N), row = t % (P * N);
     const int x = rank * P + row / N, y = row % N;
     const T* ph = static_cast<const T*>(Pr.ph) + (size_t)term * 6 * N + f * 3 * N;
-    const T E = cmul(ph[x], ph[N + y]);
+    T E = cmul(ph[x], ph[N + y]);
+    const R ss = f == 0 ? sc.su : sc.sv;
+    E.x *= ss;
+    E.y *= ss;
     T fx = T{R(1), R(0)};
     if (x == H) fx = vss_nu(ph[H]);
     if (y == H) fx = cmul(fx, vss_nu(ph[N + H]));
@@ -530,8 +565,10 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
     for (int m = 0; m < H; ++m) v[m] = Rb[colr + (2 * m + h) * N];
     fft_half_dit<R, N, +1>(v, h);
     if constexpr (SPLIT) {
-      const T uyz = cmul(uvt[N + yy], uvt[2 * N + c]);
-      const T vyz = cmul(uvt[4 * N + yy], uvt[5 * N + c]);
+      T uyz = cmul(uvt[N + yy], uvt[2 * N + c]);
+      T vyz = cmul(uvt[4 * N + yy], uvt[5 * N + c]);
+      uyz.x *= sc.su; uyz.y *= sc.su;
+      vyz.x *= sc.sv; vyz.y *= sc.sv;
 #pragma unroll
       for (int m = 0; m < H; ++m) {
         const T uM = cmul(uvt[h * H + m], uyz), vM = cmul(uvt[3 * N + h * H + m], vyz);
@@ -579,7 +616,7 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
       Qh[m].y += wr * x.y;
     }
   }
-  const R wo = SPLIT ? (R)a.w[r0] : R(1);
+  const R wo = SPLIT ? (R)a.w[r0] * sc.back : sc.back;
   T* Ho = static_cast<T*>(Pr.H) + ((size_t)e * a.NS + blockIdx.y) * G::n + slab0 +
           (size_t)pl * N * N + (size_t)h * H * N + c;
 #pragma unroll
@@ -639,6 +676,7 @@ vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
     if constexpr (HP) fft_half_dit<R, N, -1>(v, h);
     else fft<R, N, -1>(v);
   };
+  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
   for (int i = t; i < G::n; i += NT) Qh[i] = T{R(0), R(0)};
   __syncthreads();
 #pragma unroll 1
@@ -655,7 +693,10 @@ vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const T* f = ph + 3 * N * s;
-        const T E = cmul(f[N + p], f[2 * N + q]);
+        T E = cmul(f[N + p], f[2 * N + q]);
+        const R ss = s == 0 ? sc.su : sc.sv;
+        E.x *= ss;
+        E.y *= ss;
         T fy = T{R(1), R(0)};
         if (p == H) fy = vss_nu(f[N + H]);
         if (q == H) fy = cmul(fy, vss_nu(f[2 * N + H]));
@@ -699,6 +740,8 @@ vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
       if constexpr (SPLIT) {
         uxy = cmul(uvt[p], uvt[N + q]);
         vxy = cmul(uvt[3 * N + p], uvt[4 * N + q]);
+        uxy.x *= sc.su; uxy.y *= sc.su;
+        vxy.x *= sc.sv; vxy.y *= sc.sv;
       }
 #pragma unroll
       for (int m = 0; m < V; ++m) {
@@ -749,7 +792,7 @@ vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
     // (HP: the pencil's other lane still reads A[in()] of this pass, and both
     // lanes' next stores follow the shuffles of the next transform)
   }
-  const R wo = SPLIT ? (R)a.w[r0] : R(1);
+  const R wo = SPLIT ? (R)a.w[r0] * sc.back : sc.back;
   T* Ho = static_cast<T*>(Pr.H) + ((size_t)e * a.NS + blockIdx.y) * G::n + pp;
 #pragma unroll
   for (int m = 0; m < V; ++m) {

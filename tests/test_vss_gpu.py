@@ -128,3 +128,37 @@ def test_vss_species_sum_matches_oracle(built, N, precision):
                                  f[p][s], f[q][s])
             err = _rel(got[d], ref)
             assert err < tol, (N, p, s, precision, err)
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'fp32'])
+@pytest.mark.parametrize('N', [16, 24, 32])
+def test_vss_species_of_unequal_density(built, N, precision):
+    """A trace species: every pair's Q keeps its own relative accuracy, in both
+    orders, on the one-CTA and the cluster kernels; an absent one has none."""
+    from dgfs1d_gpu_b200.collision import VSSOperator
+    masses = [1.0, 2.0]
+    vm = om.VelocityMeshBi(Nv=N, M=6, masses=masses, Nrho=3, dev=5.0)
+    szpre = om.sphere_design(32)
+    rng = np.random.default_rng(11)
+    f = []
+    for T in (1.0, 1.2):
+        m = 0.5 * np.exp(-np.sum(vm.cv ** 2, axis=0) / T) / (np.pi * T) ** 1.5
+        f.append(m * (1 + 0.02 * rng.uniform(-1, 1, m.shape)))
+    one = np.ones((2, 2))
+    op = VSSOperator(N, vm.L, vm.qz, vm.qw, vm.sz, vm.sw, szpre, masses, 0.38 * one,
+                     0.4 * one, 0.1 * one, max_evals=4, precision=precision)
+    ratios = [1e-2, 1e-4, 1e-6, 0.0]
+    many = torch.tensor(np.stack([f[0]] * 4), device='cuda')
+    few = torch.tensor(np.stack([r * f[1] for r in ratios]), device='cuda')
+    tol = FP64_TOL if precision == 'fp64' else FP32_TOL
+    for p, q, fp, fq in ((0, 1, many, few), (1, 0, few, many)):
+        Q = torch.zeros_like(fp)
+        op.eval(p, q, fp, fq, Q)
+        got = Q.cpu().numpy()
+        tab = oc.VSSTables(N, vm.L, vm.qz, vm.qw, vm.sz, vm.sw, szpre, 0.38, 0.4,
+                           masses[q] / (masses[p] + masses[q]))
+        ref = oc.vss_fs(tab, 0.1, masses[p], masses[q], f[p], f[q])   # bilinear
+        for i, r in enumerate(ratios[:3]):
+            err = _rel(got[i], r * ref)
+            assert err < tol, (N, p, q, r, precision, err)
+        assert not got[3].any()
