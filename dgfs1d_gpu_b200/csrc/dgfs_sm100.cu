@@ -2599,10 +2599,10 @@ static int fno_forward(dgfs_fno_s* h, const void* f, int f_double,
 // Forward with the fused spectral passes (see fno_kernels.cuh): per layer one
 // x-mix launch and one yz-inverse + dense launch, and one yz-forward launch
 // for the next layer's spectra.  Training also keeps y_l and the spectra Vh.
-template <int N, int K>
+template <int N, int K, bool TRAIN>
 static int fno_forward_fused(dgfs_fno_s* h, const void* f, int f_double,
                              const int32_t* src_slots, int src_base, int B,
-                             cudaStream_t st, bool train = false) {
+                             cudaStream_t st) {
   using namespace fno;
   const long R = (long)B * h->n;
   FeatArgs fa{};
@@ -2617,27 +2617,27 @@ static int fno_forward_fused(dgfs_fno_s* h, const void* f, int f_double,
   const int fsm = N * K * WD * (int)sizeof(float2);
   const int xsm = 2 * K * K * WD * (int)sizeof(float2);
   const int ism = YzInvGeo<N, K>::SMEM;
-  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, __nv_bfloat16>,
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, TRAIN, __nv_bfloat16>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   DGFS_CUDA(cudaFuncSetAttribute(fno_xmix_kernel<N, K>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
-  DGFS_CUDA(cudaFuncSetAttribute(fno_yzinv_dense_kernel<N, K>,
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzinv_dense_kernel<N, K, TRAIN>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, ism));
   const dim3 pg(N, B);
-  fno_yzfwd_kernel<N, K, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[0], h->Yp);
+  fno_yzfwd_kernel<N, K, TRAIN, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[0], h->Yp);
   DGFS_CUDA(cudaGetLastError());
   for (int l = 0; l < 4; ++l) {
     fno_xmix_kernel<N, K><<<dim3(K * K, (B + K - 1) / K), K * 32, xsm, st>>>(
-        h->Yp, h->p16 + h->L.W[l], h->Sp, train ? h->Vh[l] : nullptr, B);
+        h->Yp, h->p16 + h->L.W[l], h->Sp, TRAIN ? h->Vh[l] : nullptr, B);
     YzInvArgs ya{};
     ya.S = h->Sp; ya.v = h->v[l]; ya.w16 = h->p16; ya.offD = h->L.D[l];
     ya.offd = h->L.d[l]; ya.vout = h->v[l + 1]; ya.act = l < 3 ? 1 : 0;
-    ya.y = train ? h->y[l] : nullptr;
+    ya.y = h->y[l];
     ya.err = h->err;
-    fno_yzinv_dense_kernel<N, K><<<dim3(N * YzInvGeo<N, K>::ZP, B),
-                                   YzInvGeo<N, K>::NT, ism, st>>>(ya);
+    fno_yzinv_dense_kernel<N, K, TRAIN><<<dim3(N * YzInvGeo<N, K>::ZP, B),
+                                          YzInvGeo<N, K>::NT, ism, st>>>(ya);
     if (l < 3)
-      fno_yzfwd_kernel<N, K, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[l + 1], h->Yp);
+      fno_yzfwd_kernel<N, K, TRAIN, __nv_bfloat16><<<pg, 256, fsm, st>>>(h->v[l + 1], h->Yp);
     DGFS_CUDA(cudaGetLastError());
   }
   TcArgs ta{};
@@ -2687,7 +2687,7 @@ static int fno_backward(dgfs_fno_s* h, int B, cudaStream_t st) {
   const int fsm = N * K * WD * (int)sizeof(float2);
   const int xsm = 2 * K * K * WD * (int)sizeof(float2);
   const int ism = YzInvGeo<N, K>::T_BYTES;
-  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, float>,
+  DGFS_CUDA(cudaFuncSetAttribute(fno_yzfwd_kernel<N, K, true, float>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   DGFS_CUDA(cudaFuncSetAttribute(fno_xmix_bwd_kernel<N, K>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
@@ -2699,7 +2699,7 @@ static int fno_backward(dgfs_fno_s* h, int B, cudaStream_t st) {
   la.dy = dy; la.v = h->v[3];
   if ((rc = fno_layer_bwd<0>(h, la, h->L.D[3], st))) return rc;
   for (int l = 3; l >= 0; --l) {
-    fno_yzfwd_kernel<N, K, float><<<dim3(N, B), 256, fsm, st>>>(dy, h->Yp);
+    fno_yzfwd_kernel<N, K, true, float><<<dim3(N, B), 256, fsm, st>>>(dy, h->Yp);
     fno_xmix_bwd_kernel<N, K><<<K * K, K * 32, xsm, st>>>(
         h->Yp, h->Vh[l], h->p16 + h->L.W[l], h->Sp,
         reinterpret_cast<float2*>(h->grad + h->L.W[l]), B);
@@ -2729,7 +2729,7 @@ static int fno_eval_t(dgfs_fno_s* h, const void* f, int f_double, void* Q,
     int rc;
     const int32_t* ss = src_slots ? src_slots + off : nullptr;
     if ((rc = (h->use_fused && h->use_tc)
-                  ? fno_forward_fused<N, K>(h, f, f_double, ss, src_base + off, B, st)
+                  ? fno_forward_fused<N, K, false>(h, f, f_double, ss, src_base + off, B, st)
                   : fno_forward<N, K>(h, f, f_double, ss, src_base + off, B, st, false)))
       return rc;
     fno::OutArgs oa{};
@@ -2773,7 +2773,7 @@ static int fno_train_t(dgfs_fno_s* h, const double* f, const double* Qt, int B,
                        float lr, int step, int update, cudaStream_t st) {
   int rc;
   if ((rc = (h->use_fused && h->use_tc)
-                ? fno_forward_fused<N, K>(h, f, 1, nullptr, 0, B, st, true)
+                ? fno_forward_fused<N, K, true>(h, f, 1, nullptr, 0, B, st)
                 : fno_forward<N, K>(h, f, 1, nullptr, 0, B, st)))
     return rc;
   fno::fno_loss_kernel<512><<<B, 512, 0, st>>>(h->out, Qt, h->qs, h->sQ, h->n,

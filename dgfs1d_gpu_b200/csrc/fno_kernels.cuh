@@ -1226,9 +1226,36 @@ __device__ __forceinline__ float2 chan2(const float* p) {
   return *reinterpret_cast<const float2*>(p);
 }
 
+// Two real pencils that share one complex transform, brought to one size.  The
+// transform's rounding is relative to the larger pencil, so a channel far below
+// its neighbour would carry the neighbour's absolute error, and a zero one would
+// not stay zero; training divides each gradient by its own size.  The smaller
+// pencil (largest magnitudes mx, my) is scaled up by a power of two, s, and the
+// results back by u; u = 0 for a pencil of zeros.  Training only: evaluation
+// rounds to BF16 in every layer.
+struct PairScale {
+  float sx = 1.f, sy = 1.f, ux = 1.f, uy = 1.f;
+};
+__device__ __forceinline__ PairScale pair_scale(float mx, float my) {
+  const int d = (__float_as_int(mx) >> 23) - (__float_as_int(my) >> 23);
+  const int k = max(-60, min(60, d));
+  PairScale p;
+  if (mx == 0.f) p.ux = 0.f;
+  if (my == 0.f) p.uy = 0.f;
+  if (mx == 0.f || my == 0.f) return p;
+  if (k > 0) {
+    p.sy = __int_as_float((127 + k) << 23);
+    p.uy = __int_as_float((127 - k) << 23);
+  } else {
+    p.sx = __int_as_float((127 - k) << 23);
+    p.ux = __int_as_float((127 + k) << 23);
+  }
+  return p;
+}
+
 // yz spectra of one (b, x) plane of a BF16 (activations) or FP32 (gradients)
-// field [B][N][N][N][WD].
-template <int N, int K, typename TV>
+// field [B][N][N][N][WD].  EQ: pairs of channels brought to one size.
+template <int N, int K, bool EQ, typename TV>
 __global__ void __launch_bounds__(256)
 fno_yzfwd_kernel(const TV* __restrict__ v, float2* __restrict__ Y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1244,6 +1271,19 @@ fno_yzfwd_kernel(const TV* __restrict__ v, float2* __restrict__ Y) {
 #pragma unroll
     for (int z = 0; z < N; ++z)
       c[z] = chan2(vp + ((long)y * N + z) * WD + 2 * cp);
+    PairScale ps;
+    if constexpr (EQ) {
+      float mx = 0.f, my = 0.f;
+#pragma unroll
+      for (int z = 0; z < N; ++z) {
+        mx = fmaxf(mx, fabsf(c[z].x));
+        my = fmaxf(my, fabsf(c[z].y));
+      }
+      ps = pair_scale(mx, my);
+#pragma unroll
+      for (int z = 0; z < N; ++z) { c[z].x *= ps.sx; c[z].y *= ps.sy; }
+    }
+    const float hx = 0.5f * ps.ux, hy = 0.5f * ps.uy;
     fft<float, N, -1>(c);
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
@@ -1251,8 +1291,8 @@ fno_yzfwd_kernel(const TV* __restrict__ v, float2* __restrict__ Y) {
       const float2 C = c[k], Cn = c[nk];
       // channel 2cp: (C + conj Cn)/2; channel 2cp+1: (C - conj Cn)/(2i)
       *reinterpret_cast<float4*>(T2 + (y * K + kk) * WD + 2 * cp) =
-          make_float4(0.5f * (C.x + Cn.x), 0.5f * (C.y - Cn.y),
-                      0.5f * (C.y + Cn.y), -0.5f * (C.x - Cn.x));
+          make_float4(hx * (C.x + Cn.x), hx * (C.y - Cn.y),
+                      hy * (C.y + Cn.y), -hy * (C.x - Cn.x));
     }
   }
   __syncthreads();
@@ -1275,7 +1315,7 @@ struct YzInvArgs {
   const __nv_bfloat16* w16;  // BF16 parameters
   long offD, offd;           // D_l [WD][WD], d_l [WD]
   __nv_bfloat16* vout;       // v_{l+1} [B][N^3][WD]
-  __nv_bfloat16* y;          // pre-activation out (training; may be null)
+  __nv_bfloat16* y;          // pre-activation out (training)
   int act;                   // GELU (layers 0..2) or identity (last layer)
   int* err;                  // device error flag
 };
@@ -1318,26 +1358,45 @@ __device__ __forceinline__ void yzinv_zpass(const float2* src, float2* T, int ky
 // Spectrum along y of two real pencils as one complex one: with sym(a)(k) =
 // (a(k) + conj a(-k))/2, c = sym(a) + i sym(b), so that IFFT(c) = Re IFFT(a) +
 // i Re IFFT(b).  src: the two channels' values at ky = 0, `pitch` apart per ky.
-template <int N, int K>
-__device__ __forceinline__ void yzinv_sym(const float2* src, int pitch, float2* c) {
+// EQ: the pencils brought to one size; the results are to be multiplied by the
+// returned ux, uy.
+template <int N, int K, bool EQ>
+__device__ __forceinline__ PairScale yzinv_sym(const float2* src, int pitch, float2* c) {
+  PairScale ps;
+  if constexpr (EQ) {
+    float mx = 0.f, my = 0.f;
+#pragma unroll
+    for (int ky = 0; ky < K; ++ky) {
+      const float4 ab = *reinterpret_cast<const float4*>(src + ky * pitch);
+      mx = fmaxf(mx, fmaxf(fabsf(ab.x), fabsf(ab.y)));
+      my = fmaxf(my, fmaxf(fabsf(ab.z), fabsf(ab.w)));
+    }
+    ps = pair_scale(mx, my);
+  }
 #pragma unroll
   for (int j = 0; j < N; ++j) c[j] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int ky = 0; ky < K; ++ky) {
-    const float4 ab = *reinterpret_cast<const float4*>(src + ky * pitch);
+    float4 ab = *reinterpret_cast<const float4*>(src + ky * pitch);
+    if constexpr (EQ) {
+      ab.x *= ps.sx; ab.y *= ps.sx;
+      ab.z *= ps.sy; ab.w *= ps.sy;
+    }
     const int k = fbin<N, K>(ky), nk = (N - k) % N;
     c[k].x += 0.5f * (ab.x - ab.w);
     c[k].y += 0.5f * (ab.y + ab.z);
     c[nk].x += 0.5f * (ab.x + ab.w);
     c[nk].y += 0.5f * (ab.z - ab.y);
   }
+  return ps;
 }
 
 // Grid (N ZP, B): blockIdx.x = x ZP + slab.  The rows' BF16 activations load
 // asynchronously while the CUDA cores run the kz -> z pass; the dense MMAs
 // are issued next, and U overwrites their A operand only after the MMA
-// completion barrier; the epilogue adds U to the accumulator.
-template <int N, int K>
+// completion barrier; the epilogue adds U to the accumulator.  TRAIN: pairs of
+// channels brought to one size (pair_scale), and y is stored.
+template <int N, int K, bool TRAIN>
 __global__ void __launch_bounds__(YzInvGeo<N, K>::NT, 2)
 fno_yzinv_dense_kernel(YzInvArgs a) {
   using G = YzInvGeo<N, K>;
@@ -1438,12 +1497,13 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
     for (int p = t; p < NZ * (WD / 2); p += NT) {
       const int zl = p / (WD / 2), cp = p % (WD / 2);
       float2 c[N];
-      yzinv_sym<N, K>(T + zl * WD + 2 * cp, NZ * WD, c);
+      const PairScale ps = yzinv_sym<N, K, TRAIN>(T + zl * WD + 2 * cp, NZ * WD, c);
+      const float ix = inv * ps.ux, iy = inv * ps.uy;
       fft<float, N, +1>(c);
 #pragma unroll
       for (int y = 0; y < N; ++y)
         *reinterpret_cast<__nv_bfloat162*>(Us + (long)(y * NZ + zl) * WD + 2 * cp) =
-            __floats2bfloat162_rn(c[y].x * inv, c[y].y * inv);
+            __floats2bfloat162_rn(c[y].x * ix, c[y].y * iy);
     }
   }
   __syncthreads();
@@ -1480,7 +1540,7 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
           const __nv_bfloat162 yy = __floats2bfloat162_rn(
               __uint_as_float(rg[j]) + ep[j] + uf.x,
               __uint_as_float(rg[j + 1]) + ep[j + 1] + uf.y);
-          reinterpret_cast<__nv_bfloat162*>(&yo[c4])[h] = yy;
+          if (TRAIN) reinterpret_cast<__nv_bfloat162*>(&yo[c4])[h] = yy;
           if (a.act) {
             const float2 yf = __bfloat1622float2(yy);
             o2[h] = __floats2bfloat162_rn(gelu(yf.x), gelu(yf.y));
@@ -1492,7 +1552,7 @@ fno_yzinv_dense_kernel(YzInvArgs a) {
       uint4* vd = reinterpret_cast<uint4*>(a.vout + (plane * N * N + pt) * WD);
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) vd[c4] = vo[c4];
-      if (a.y) {
+      if (TRAIN) {
         uint4* yd = reinterpret_cast<uint4*>(a.y + (plane * N * N + pt) * WD);
 #pragma unroll
         for (int c4 = 0; c4 < 4; ++c4) yd[c4] = yo[c4];
@@ -1629,11 +1689,13 @@ fno_yzinv_bwd_kernel(const float2* __restrict__ S, float* __restrict__ U) {
   for (int p = t; p < NZ * (WD / 2); p += 256) {
     const int zl = p / (WD / 2), cp = p % (WD / 2);
     float2 c[N];
-    yzinv_sym<N, K>(T + zl * WD + 2 * cp, NZ * WD, c);
+    const PairScale ps = yzinv_sym<N, K, true>(T + zl * WD + 2 * cp, NZ * WD, c);
     fft<float, N, +1>(c);
     float* dst = U + (plane * N * N + z0 + zl) * WD + 2 * cp;
 #pragma unroll
-    for (int y = 0; y < N; ++y) *reinterpret_cast<float2*>(dst + (long)y * N * WD) = c[y];
+    for (int y = 0; y < N; ++y)
+      *reinterpret_cast<float2*>(dst + (long)y * N * WD) =
+          make_float2(c[y].x * ps.ux, c[y].y * ps.uy);
   }
 }
 

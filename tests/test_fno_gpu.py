@@ -152,3 +152,44 @@ def test_fused_eval_matches_per_axis_passes(built):
         e = _rel(out[0], out[1])
         print(f'N={n_}: fused vs per-axis passes rel L2 {e:.2e}')
         assert e < 1e-2, e
+
+
+@pytest.mark.parametrize('fused', [True, False])
+def test_gradients_of_faint_and_unused_channels(built, fused):
+    """Channels far below their neighbours (lift columns and projection rows
+    times 2^-20, or zero): the transforms take two channels at a time, and each
+    channel's spectral-weight gradients keep their own relative accuracy; those
+    of an unused channel are exactly zero (Adam divides a gradient by its own
+    size)."""
+    from dgfs1d_gpu_b200.surrogate import FNOSurrogate, layout, init_params
+    lay = layout(K)
+    w = init_params(K, seed=3)
+    P = w[lay['P'][0]:][:128].reshape(4, 32)
+    pb = w[lay['p'][0]:][:32]
+    Q1 = w[lay['Q1'][0]:][:32 * 128].reshape(32, 128)
+    faint, unused = [5, 8], [14, 19]
+    for c in faint:
+        P[:, c] *= 2.0 ** -20
+        pb[c] *= 2.0 ** -20
+        Q1[c] *= 2.0 ** -20
+    for c in unused:
+        P[:, c] = pb[c] = Q1[c] = 0.0
+    net = FNOSurrogate(N, L, q_scale=SQ, max_batch=4, params=w)
+    net.set_fused(fused)
+    f, Qt = _data()
+    net.train_step(torch.tensor(f, device='cuda'), torch.tensor(Qt, device='cuda'),
+                   update=False)
+    g = net.grads()
+    ref = ofno.FNO(N, K, L, SQ, net.params(), emulate_bf16=True)
+    out, cache = ref.forward(f)
+    _, dout = ref.loss(out, Qt, cache['qs'])
+    gr = ref.backward(dout, cache)
+
+    def W(a, l):
+        o, s = lay[f'W{l}']
+        return np.asarray(a[o:o + s]).reshape(K ** 3, 32, 32, 2)
+    for c in faint:
+        assert _rel(W(g, 0)[:, c], W(gr, 0)[:, c]) < 2e-2, c    # v_0 is faint
+        assert _rel(W(g, 3)[:, :, c], W(gr, 3)[:, :, c]) < 2e-2, c  # dL/dv_4 is
+    for c in unused:
+        assert not W(g, 0)[:, c].any() and not W(g, 3)[:, :, c].any(), c
