@@ -173,7 +173,7 @@ struct dgfs_vhs_s {
   double Ginv[25] = {};
   int c32 = 0;  // variant code of the FP32 terms kernel (autotuner choice)
   // constant tables
-  double* c0 = nullptr;      // [N]
+  double* c0 = nullptr;      // [N], in the FP64 mode then multp [Nrho][Mu]
   double* b2 = nullptr;      // [n]
   double* b1w64 = nullptr;   // [Nrho][n]
   float* b1w32 = nullptr;    // [Nrho][n] (FP32 mode)
@@ -355,7 +355,19 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
           ph64[(((size_t)p * Mu + u) * 3 + a) * N + l] =
               make_double2(std::cos(k * l0[l]), std::sin(k * l0[l]));
       }
-  std::vector<double> c0(d->c0, d->c0 + N);
+  std::vector<double> c0(d->c0, d->c0 + N), ps(Nrho, 1.0);
+  // FP64 packed terms: each radial point's power of two within its pair (1 for
+  // the larger weight), on the multiplicities of its directions and off b1w;
+  // one allocation with the velocity grid
+  for (int p = 0; p < Nrho && !fp32; ++p) {
+    const double w = std::fabs(b1w[(size_t)p * n]), o = (p ^ 1) < Nrho
+        ? std::fabs(b1w[(size_t)(p ^ 1) * n]) : 0.0;
+    const int k = w > 0 ? std::max(-60, std::ilogb(w) - std::ilogb(o)) : -60;
+    const double s = o > w && std::isfinite(o) ? std::ldexp(1.0, k) : 1.0;
+    for (int u = 0; u < Mu; ++u) c0.push_back(s * mult[u]);
+    ps[p] = s;
+  }
+  for (size_t i = 0; i < b1w.size(); ++i) b1w[i] /= ps[i / n];
 
   int rc = DGFS_OK;
   if ((rc = upload(&h->c0, c0)) || (rc = upload(&h->b2, b2)) ||
@@ -764,7 +776,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
   } else {
     VhsTermsArgs a{};
     a.Fg = h->Fg; a.ph = h->ph; a.uv = nullptr; a.mult = h->mult;
-    a.b1w = h->b1w64; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
+    a.b1w = h->b1w64; a.multp = h->c0 ? h->c0 + N : nullptr; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq64; a.rho = h->rho64; a.Fny = h->Fny64;
     if (h->rho64) {
       // packed transforms: Nyquist-plane transforms, then the terms

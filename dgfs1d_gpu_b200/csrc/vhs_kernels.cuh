@@ -75,6 +75,8 @@ struct VhsTermsArgs {
   const void* uv;             // [nevals][Nrho][Mu][2][3][N] u_a, v_a (split)
   const float* mult;          // [Mu] multiplicity of each transformed direction
   const void* b1w;            // [Nrho][n] W_p b1_p(l), precision R
+  const double* multp;        // FP64 packed terms: [Nrho][Mu] multiplicity times
+                              // the radial point's power of two (off b1w)
   void* H;                    // out [nevals][Nrho][n] complex, precision R
                               // (FP32: [nevals][ceil(Nrho/2)][n], packed pairs)
   const void* nyq;            // FP32: [Nrho][Mu][3] exp(i N kappa_a)
@@ -718,7 +720,12 @@ vhs_terms_kernel(VhsTermsArgs a) {
 // packed as S = S_p0 + i S_p1 and forward-transformed together; since both
 // spectra are Hermitian, Re IFFT((b1_p0 - i b1_p1) FFT(S)) =
 // IFFT(b1_p0 FFT(S_p0) + b1_p1 FFT(S_p1)), so the epilogue sums the packed
-// spectra H = (b1_p0 - i b1_p1) FFT(S) unchanged.
+// spectra H = (b1_p0 - i b1_p1) FFT(S) unchanged.  The transform rounds
+// relative to the larger sum, and W grows steeply with the radius while S
+// falls, so that S_p0's rounding, weighted by b1_p1, would dominate the FP64
+// mode's error (N=24, radii 0.05 and 4: 1.3e-11 instead of 2.2e-12): there the
+// sum of the smaller weight is packed times the power of two nearest to the
+// weights' ratio (multp) and its b1 divided by it, both exact.
 //
 // Pipeline per transform k (term (p, q) = (p0 + k / Mu, k % Mu)):
 //   y-pass(k) -> exchange(k) into receive buffer k%2 -> arrive
@@ -1650,7 +1657,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     const T rx = rp[yy * N + c];
     const T* rY = rp + N * N + c + h * H * N;
     const T* rZ = rp + 2 * N * N + yy * N + h * H;   // [y][x]
-    const R mq = SPLIT ? R(1) : (R)a.mult[q0 + k % nq];
+    const R mq = SPLIT ? R(1) : (R)a.multp[term(k)];
     T uyz{}, vyz{};
     if constexpr (SPLIT) {
       uyz = cmul(ut[N + yy], ut[2 * N + c]);
@@ -1870,7 +1877,7 @@ vhs_terms1_kernel(VhsTermsArgs a) {
       uxy = cmul(ut[p], ut[N + q]);
       vxy = cmul(ut[3 * N + p], ut[4 * N + q]);
     }
-    const R mq = SPLIT ? R(1) : (R)a.mult[q0 + k % nq];
+    const R mq = SPLIT ? R(1) : (R)a.multp[term(k)];
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int z = out(m);

@@ -54,6 +54,24 @@ def test_direction_slices_and_radial_remainders(precision, N, M, full, Nrho, poi
         assert _rel(got[s], ref) < TOL[precision] + floor, (N, Nrho, s)
 
 
+@pytest.mark.parametrize('N', [16, 24])
+def test_radial_points_of_very_different_weight(N):
+    """Two radial points share a forward transform: the sum of the small radius
+    is large and its weight small, and its rounding must not enter with the
+    other's weight.  Bound: twice the error with a transform for each (1.2e-13
+    and 2.2e-12, from the cancellation of the far radius' sums); 6.9e-13 and
+    1.3e-11 unscaled.  N=16: one-CTA kernel, N=24: cluster kernel."""
+    from dgfs1d_gpu_b200.collision import VHSOperator
+    vm, prefac, gamma, f = vhs_case(N, 6, 2, 6.0, False)
+    vm.qz, vm.qw = np.array([0.05, 4.0]), np.array([1.0, 1.0])
+    op = VHSOperator(**op_kwargs(vm, prefac, gamma), precision='fp64', max_evals=1)
+    fd = torch.tensor(f, device='cuda')
+    Q = torch.zeros_like(fd)
+    op.eval(fd, Q)
+    ref = vhs_gll_fs(vhs_tables(vm, gamma), prefac, f[0])
+    assert _rel(Q[0].cpu().numpy(), ref) < {16: 2.5e-13, 24: 4.4e-12}[N]
+
+
 def test_sliced_and_unsliced_batches_agree():
     """A point evaluated alone (sliced directions) and within a batch."""
     from dgfs1d_gpu_b200.collision import VHSOperator
