@@ -175,8 +175,9 @@ __device__ __forceinline__ double wall_expr_maxwellian(const DgAdvectArgs& a,
 // Grid (kWallCh chunks of the velocity grid, 2 sides): partial sums
 // [2][kWallCh][2]; the last CTA to finish adds them in a fixed order (one CTA
 // per side would leave the reduction latency-bound on two SMs; a second
-// launch for the sum of 64 numbers cost 3.5 us).  `done` counts CTAs and is
-// zero again afterwards.
+// launch for the sum of 64 numbers cost 3.5 us).  `done` counts CTAs and wraps
+// by itself: were two calls on one handle to overlap, against the documented
+// order, their densities would be undefined, but those of later calls not.
 constexpr int kWallCh = 32;
 __global__ void __launch_bounds__(256) dg_wall_kernel(DgAdvectArgs a, double cw,
                                                       double* part, double* nden,
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(256) dg_wall_kernel(DgAdvectArgs a, double cw,
     part[(side * kWallCh + ch) * 2] = rn[0];
     part[(side * kWallCh + ch) * 2 + 1] = rd[0];
     __threadfence();
-    last = atomicAdd(done, 1u) == 2 * kWallCh - 1;
+    last = atomicInc(done, 2 * kWallCh - 1) == 2 * kWallCh - 1;
   }
   __syncthreads();
   if (last && t < 2) {
@@ -224,7 +225,6 @@ __global__ void __launch_bounds__(256) dg_wall_kernel(DgAdvectArgs a, double cw,
       d += __ldcg(part + (t * kWallCh + c) * 2 + 1);
     }
     nden[t] = (a.bc[t] == kBcWall || a.bc[t] == kBcWallExpr) ? -(n / d) : 0.0;
-    if (t == 0) *done = 0;
   }
 }
 

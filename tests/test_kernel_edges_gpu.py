@@ -183,6 +183,51 @@ def test_advection_split_over_elements(Ne, K, bc):
         assert _rel(ux.cpu().numpy(), ref) < 1e-13, (N, Ne, K, bc)
 
 
+def _wall_case(N, Ne, K, seed=0):
+    from dgfs1d_gpu_b200.basis import get_basis
+    from dgfs1d_gpu_b200.config import Config
+    from dgfs1d_gpu_b200.dg import DGOperator
+    L = 5.0
+    c0 = np.linspace(-L + L / N, L - L / N, N)
+    c2 = sum(x ** 2 for x in np.meshgrid(c0, c0, c0, indexing='ij')).ravel()
+    basis = get_basis(Config(f'[basis]\nkind = nodal-sem-gll\nK = {K}\nNqr = {K}\n'))
+    rng = np.random.default_rng(seed)
+    u = np.exp(-c2) * (1 + 0.1 * rng.uniform(-1, 1, (K, Ne, N ** 3)))
+    bc = ('dgfs-wall-diffuse', np.exp(-c2) / np.pi ** 1.5, 0.0)
+    dg = DGOperator(basis, np.full(Ne, 2.0 * Ne), c0, (2 * L / N) ** 3, [bc, bc])
+    return dg, torch.tensor(u, device='cuda')
+
+
+def test_wall_density_after_overlapping_calls():
+    """Calls that overlap on one handle (two streams, beside a kernel that makes
+    their CTAs trickle in) have undefined wall densities; the ordered calls after
+    them have their own."""
+    dg, u = _wall_case(32, 2, 3)
+    u3, ux, ref = 3.0 * u, torch.empty_like(u), torch.empty_like(u)
+    dg.advect(u3, ref)
+    nden = dg.wall_density()
+    load, first, second = [torch.cuda.Stream() for _ in range(3)]
+    junk = [torch.empty_like(u) for _ in range(2)]
+    big = torch.ones(1 << 27, device='cuda')
+    torch.cuda.synchronize()
+
+    def busy():
+        with torch.cuda.stream(load):
+            for _ in range(3):
+                big.sin_()
+    for i in range(100):
+        busy()
+        for _ in range(3):
+            dg.advect(u, junk[0], stream=first)
+            dg.advect(u, junk[1], stream=second)
+        torch.cuda.synchronize()
+        busy()
+        dg.advect(u3, ux)
+        torch.cuda.synchronize()
+        assert np.array_equal(dg.wall_density(), nden), i
+        assert torch.equal(ux, ref), i
+
+
 def _advect(basis, invjac, cx, bcl, bcr, u):
     """Strong-form nodal DG advection with upwind faces, straight from the
     operators."""
