@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -243,6 +244,16 @@ static size_t slab_bytes(int N, int C, size_t elem) {
   return (size_t)(N / C) * N * (N + 1) * elem;
 }
 
+// Points per pass of a handle whose scratch takes `bytes` per point: the packed
+// transforms' plane scratch is tens of MB per point on the large grids, and the
+// solvers pass K Ne points.  4 GiB hold tens of points of the largest rule, i.e.
+// thousands of CTAs; a call with more points runs in several passes.  (65535:
+// grid limit.)
+static int points_per_pass(int max_evals, size_t bytes, int grid_per_point) {
+  const size_t fit = std::max<size_t>(1, ((size_t)4 << 30) / bytes);
+  return (int)std::min<size_t>({(size_t)max_evals, fit, (size_t)(65535 / grid_per_point)});
+}
+
 static void free_handle(dgfs_vhs_s* h) {
   void* ptrs[] = {h->c0, h->b2, h->b1w64, h->b1w32, h->ph, h->kappa, h->mult,
                   h->Fg, h->H, h->ReLf, h->mhat, h->moments, h->uv, h->hh,
@@ -409,8 +420,13 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
     h->ph = p64;
   }
 
-  const size_t E = (size_t)d->max_evals;
   const size_t ce = fp32 ? sizeof(float2) : sizeof(double2);
+  if (!fp32)
+    h->max_evals = points_per_pass(
+        d->max_evals,
+        (n + (size_t)(Nrho + 1) / 2 * n + ((size_t)Nrho * Mu + 1) * 3 * N * N) * ce +
+            n * sizeof(double), 1);
+  const size_t E = (size_t)h->max_evals;
   cudaError_t ce_ = cudaSuccess;
   auto alloc = [&](void** p, size_t bytes) {
     if (ce_ == cudaSuccess) ce_ = cudaMalloc(p, bytes);
@@ -1530,7 +1546,8 @@ struct VssPair {
 };
 
 struct dgfs_vss_s {
-  int N = 0, Nrho = 0, M = 0, nspcs = 0, n = 0, max_evals = 0;
+  int N = 0, Nrho = 0, M = 0, nspcs = 0, n = 0;
+  int max_evals = 0;       // points per pass (points_per_pass)
   int precision = DGFS_PREC_FP64;
   double* w = nullptr;     // [Nrho] w_r s_w / n
   VssPair pair[16];
@@ -1705,8 +1722,16 @@ extern "C" int dgfs_vss_create(const dgfs_vss_desc* d, dgfs_vss_handle* out) {
   if (!rc) rc = upload(&h->dirsm, dirsm);
   const bool fp32 = h->precision == DGFS_PREC_FP32;
   if (!rc) {
-    const size_t E = h->max_evals, n = h->n, N = h->N, T = (size_t)h->Nrho * h->M;
+    const size_t n = h->n, N = h->N, T = (size_t)h->Nrho * h->M;
     const size_t ns = h->nspcs, ce = fp32 ? sizeof(float2) : sizeof(double2);
+    const size_t per_pair = (T * 3 * N * N + (fp32 ? h->Nrho : 1) * n) * ce +
+                            n * sizeof(double) +
+                            (fp32 ? T * 6 * N * sizeof(float2) +
+                                        (T * 3 * N + n) * sizeof(double2) : 0);
+    h->max_evals = points_per_pass(
+        h->max_evals, ns * per_pair + std::max<size_t>(2, ns) * (n + 3 * N * N) * ce,
+        h->nspcs);
+    const size_t E = h->max_evals;
     cudaError_t e1 = cudaSuccess;
     auto A = [&](auto** q, size_t bytes) {
       if (e1 == cudaSuccess) e1 = cudaMalloc((void**)q, bytes);

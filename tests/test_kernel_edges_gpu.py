@@ -120,6 +120,42 @@ def test_vss_merged_antipodes_and_radial_slices(N, precision):
         assert _rel(Qb[199].cpu().numpy(), ref) < tol
 
 
+def test_scratch_is_bounded():
+    """Handles for thousands of points of a large grid fit beside a solver's
+    state, and a call longer than a pass gives every point its value."""
+    from dgfs1d_gpu_b200.collision import VHSOperator, VSSOperator
+    masses = [1.0, 2.0]
+    vm = om.VelocityMeshBi(Nv=32, M=12, masses=masses, Nrho=16, dev=5.0)
+    one = np.ones((2, 2))
+    f = np.stack([np.exp(-np.sum(vm.cv ** 2, axis=0) / T) for T in (1.0, 1.2)])
+    fd = torch.tensor(f, device='cuda')
+    torch.cuda.synchronize()
+    for precision in ('fp64', 'fp32'):
+        free = torch.cuda.mem_get_info()[0]
+        op = VSSOperator(32, vm.L, vm.qz, vm.qw, vm.sz, vm.sw, om.sphere_design(32),
+                         masses, 0.38 * one, 0.4 * one, 0.1 * one, max_evals=6000,
+                         precision=precision)
+        assert free - torch.cuda.mem_get_info()[0] < 6 << 30, precision
+        many = 230 if precision == 'fp64' else 330
+        fp, fq = (x.expand(many, -1).contiguous() for x in (fd[:1], fd[1:]))
+        Q, Q1 = torch.zeros_like(fp), torch.zeros_like(fp[:1])
+        op.eval(0, 1, fp, fq, Q)
+        op.eval(0, 1, fp[:1], fq[:1], Q1)
+        for i in (0, many // 2, many - 1):
+            assert _rel(Q[i].cpu().numpy(), Q1[0].cpu().numpy()) < TOL[precision], i
+        op.close()
+    vm, prefac, gamma, f = vhs_case(48, 32, 24, 6.0, True)
+    free = torch.cuda.mem_get_info()[0]
+    op = VHSOperator(**op_kwargs(vm, prefac, gamma), precision='fp64', max_evals=3000)
+    assert free - torch.cuda.mem_get_info()[0] < 6 << 30
+    fb = torch.tensor(f, device='cuda').expand(70, -1).contiguous()
+    Q, Q1 = torch.zeros_like(fb), torch.zeros_like(fb[:1])
+    op.eval(fb, Q)
+    op.eval(fb[:1].contiguous(), Q1)
+    for i in (0, 69):
+        assert _rel(Q[i].cpu().numpy(), Q1[0].cpu().numpy()) < 1e-11, i
+
+
 @pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
 def test_axnpby_vector_and_scalar_routes(dtype):
     """Sizes around the vector kernel's groups, operands off 16-byte alignment
