@@ -228,7 +228,7 @@ static int c32_of(int N) {
   }
 }
 template <int N> struct VhsClusters;
-static size_t slots_resident(int N, bool fp32);
+static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu);
 // c64: FP64 terms kernel with two lanes per pencil (vhs_termsh_kernel; up to
 // N=16 vhs_terms1_kernel runs); c32: FP32 terms kernel with one thread per
 // pencil; cpro / cepi: prologue / epilogue (FP64, two lanes per pencil, one slab
@@ -434,9 +434,8 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   alloc((void**)&h->err, sizeof(int));
   if (ce_ == cudaSuccess) ce_ = cudaMemset(h->err, 0, sizeof(int));
   alloc(&h->Fg, E * n * ce);
-  // packed radial pairs; at least what the GPU holds at once, for the direction
-  // slices of small batches
-  h->hslots = std::max<size_t>(E * ((Nrho + 1) / 2), slots_resident(N, fp32));
+  // packed radial pairs, and the direction slices of small batches
+  h->hslots = spectra_slots(N, fp32, E * ((Nrho + 1) / 2), Mu);
   alloc(&h->H, h->hslots * n * ce);
   alloc((void**)&h->ReLf, E * n * sizeof(double));
   if (fp32) {
@@ -520,28 +519,31 @@ extern "C" int dgfs_vhs_device_error(dgfs_vhs_handle h, int32_t* out) {
   return DGFS_OK;
 }
 
+// Shared memory of the FP32 terms kernel with one thread per pencil: three slabs
+// (with TMA the transform slab has rows of N+2 elements and 128 bytes of
+// alignment slack), two table slots, the staged plane transforms of one term
+// (and the TMA mbarrier).
+template <int N, int C, bool TMA> static size_t terms32_smem() {
+  return (TMA ? (size_t)Geo<N, C>::P * N * (N + 2) * sizeof(float2) + 128
+              : slab_bytes(N, C, sizeof(float2))) +
+         2 * slab_bytes(N, C, sizeof(float2)) + 2 * (9 * N + 4) * sizeof(float2) +
+         (size_t)((TermsRyStaged<C>::value ? N * N : 0) + 2 * Geo<N, C>::P * N) *
+             sizeof(float2) +
+         (TMA ? sizeof(uint64_t) : 0);
+}
+
 // FP32 terms kernel at cluster size C (each C must divide N and fit three
 // slabs in shared memory).
 template <int N, int C, bool TMA = false>
 static int launch_terms32_c(const VhsTermsArgs& a, int nevals, int Nrho,
                             cudaStream_t st, const CUtensorMap* map = nullptr) {
   using G = Geo<N, C>;
-  // three slabs (with TMA the transform slab has rows of N+2 elements and
-  // 128 bytes of alignment slack), two table slots, the staged plane
-  // transforms of one term (and the TMA mbarrier)
-  const size_t smem = (TMA ? (size_t)G::P * N * (N + 2) * sizeof(float2) + 128
-                           : slab_bytes(N, C, sizeof(float2))) +
-                      2 * slab_bytes(N, C, sizeof(float2)) +
-                      2 * (9 * N + 4) * sizeof(float2) +
-                      (size_t)((TermsRyStaged<C>::value ? N * N : 0) +
-                               2 * G::P * N) * sizeof(float2) +
-                      (TMA ? sizeof(uint64_t) : 0);
   if (TMA && !map) return fail(DGFS_ERR_UNSUPPORTED, "no TMA map for this handle");
   CUtensorMap none;
   std::memset(&none, 0, sizeof(none));
   return launch_cluster2(vhs_terms_fp32_kernel<N, C, TMA>,
-                         dim3(C, (Nrho + 1) / 2, nevals), dim3(G::NT), C, smem,
-                         st, a, map ? *map : none);
+                         dim3(C, (Nrho + 1) / 2, nevals), dim3(G::NT), C,
+                         terms32_smem<N, C, TMA>(), st, a, map ? *map : none);
 }
 
 // Terms kernel with two lanes per pencil (vhs_termsh_kernel).
@@ -586,29 +588,58 @@ template <> struct Terms32Variants<24> { static constexpr int v[8] = {3, 4, 6, 5
 template <> struct Terms32Variants<32> { static constexpr int v[8] = {4, 8, 104, 108, 504, 604, 608, 616}; };
 template <> struct Terms32Variants<48> { static constexpr int v[5] = {16, 116, 516, 608, 616}; };
 
-// Direction slices of a terms launch: the two radial points of a CTA or cluster
-// share its 2 Mu serial transforms; while fewer than `resident` CTAs or
-// clusters run, the directions are split (each slice has its own spectrum,
-// summed in FP64 by the epilogue).
-static int dir_slices(const dgfs_vhs_s* h, int nevals, int resident) {
-  const int base = nevals * ((h->Nrho + 1) / 2);
-  const int fit = std::min(resident / base, (int)(h->hslots / base));
-  return std::max(1, std::min(fit, h->Mu));
+// CTAs or clusters of a kernel that the GPU holds at once (clusters stay inside a
+// GPC, which leaves SMs unused: 45 clusters of 16 at six CTAs per SM), asked of
+// the driver once per kernel.
+template <typename K>
+static int max_clusters(K kernel, int cluster, int threads, size_t smem) {
+  int n = 0, dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (cluster == 1) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+    n *= sms;
+  } else {
+    if (cluster > 8)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  }
+  cudaGetLastError();   // (an error leaves n = 0, and a launch reports it)
+  return n > 0 ? n : std::max(1, sms / cluster);
 }
-// CTAs (vhs_terms1_kernel) or clusters (vhs_termsh_kernel) of a kernel that the
-// GPU holds at once; clusters stay inside a GPC, which leaves about a quarter of
-// the SMs unused at 16 CTAs (measured: 7 clusters of 16 at one CTA per SM).
-template <typename R, int N> constexpr int terms1_resident() {
-  return 148 * Terms1Geo<R, N>::per_sm;
+template <typename R, int N> static int terms1_resident() {
+  static const int n =
+      max_clusters(vhs_terms1_kernel<R, N>, 1, Terms1Geo<R, N>::NT, Terms1Geo<R, N>::smem);
+  return n;
 }
-template <typename R, int N, int C> constexpr int termsh_resident() {
-  return 148 * TermsHGeo<R, N, C>::per_sm * 3 / (4 * C);
+template <typename R, int N, int C> static int termsh_resident() {
+  static const int n = max_clusters(vhs_termsh_kernel<R, N, C>, C, HalfGeo<N, C>::NT,
+                                    TermsHGeo<R, N, C>::smem);
+  return n;
+}
+template <int N, int C> static int terms32_tma_resident() {
+  static const int n = max_clusters(vhs_terms_fp32_kernel<N, C, true>, C, Geo<N, C>::NT,
+                                    terms32_smem<N, C, true>());
+  return n;
 }
 template <int N> static int resident32(int code) {
-  if (code == 700) {
-    if constexpr (N <= 24) return terms1_resident<float, N>();
-  }
-  if constexpr (N >= 16 && N <= 24)
+  if constexpr (N <= 24)
+    if (code == 700) return terms1_resident<float, N>();
+  if constexpr (N <= 16)
+    if (code == 601) return termsh_resident<float, N, 1>();
+  if constexpr (N == 16 || N == 24)
     if (code == 602) return termsh_resident<float, N, 2>();
   if constexpr (N >= 16 && N <= 32)
     if (code == 604) return termsh_resident<float, N, 4>();
@@ -618,37 +649,93 @@ template <int N> static int resident32(int code) {
     if (code == 608) return termsh_resident<float, N, 8>();
     if (code == 616) return termsh_resident<float, N, 16>();
   }
-  return 148;
+  return 1;
 }
 
-// Default variant: the cube in one CTA where it fits (N=24: 225 us for a
-// 24-point evaluation against 257 with clusters of two), else two lanes per
-// pencil with two or three CTAs of different clusters on an SM, which hide each
-// other's exchanges (N=32: 639 against 659 us for the one-thread kernel with
-// TMA staging; N=48: 42.3 against 63.9 ms for 96 points).
+// Direction slices of a terms launch.  The (one or two) radial points of a CTA or
+// cluster share its `rad` Mu serial transforms; a batch of `base` of them that
+// does not fill the GPU splits the directions into ns slices with a spectrum
+// each, summed in FP64 by the epilogue.  Estimate, in units of a transform while
+// `resident` run at once:
+//   waves (rad ceil(Mu / ns) + start) + 0.01 base (ns - 1),
+// `start` the start-up and the forward transform, the last term the spectra's
+// traffic.  A part-filled wave of x resident costs x plus latency (1 - x), since
+// a transform alone on its SM takes `latency` of its time among others; after
+// full waves the CTAs no longer run in step, and the next wave fills the gaps.
+// More slices of a cluster kernel have to win by 2%, since how many clusters fit
+// differs a little between GPUs.
+// Measured over N = 8..48, 1 to 48 points, 6 and 16 directions, both precisions,
+// every ns: the choice is on average 0.3 to 1.7% slower than the fastest ns (FP32
+// N=16: 4%, steps of 2 us); resident / base slices were 3% (FP32 N=32) and 4%
+// (FP64 N=24), and up to 13 and 28%, slower.
+struct SliceCost { double latency, start, margin; };
+constexpr SliceCost kCostOneCta{0.9, 2.0, 1.0}, kCostCluster{0.6, 3.0, 0.98};
+struct Slices { int ns; double cost; };
+static Slices dir_slices(const dgfs_vhs_s* h, int nevals, int resident, SliceCost k) {
+  const int base = nevals * ((h->Nrho + 1) / 2), rad = h->Nrho > 1 ? 2 : 1;
+  Slices best{1, 1e300};
+  for (int ns = 1; ns <= h->Mu && (ns == 1 || (size_t)ns * base <= h->hslots); ++ns) {
+    const int full = ns * base / resident;
+    const double x = (double)(ns * base % resident) / resident;
+    const double waves = full + (x > 0 ? x + (1 - x) * k.latency / (full + 1) : 0.0);
+    const double c =
+        waves * (rad * ((h->Mu + ns - 1) / ns) + k.start) + 0.01 * base * (ns - 1);
+    if (c < k.margin * best.cost) best = {ns, c};
+  }
+  return best;
+}
+
+// Default variant of the FP32 terms kernel and its slices.  The cube in one CTA
+// where it fits (N=24: 225 us for a 24-point evaluation against 257 with clusters
+// of two), else two lanes per pencil with CTAs of different clusters on an SM,
+// which hide each other's exchanges (N=48: 42.3 against 63.9 ms for 96 points).
+// At N=32 the kernel with one thread per pencil and TMA staging (504: 33
+// clusters of four at once, one CTA per SM, so that its waves run in step) takes
+// 1 / 1.28 of a transform of the two-lane kernel (616: 45 of 16, six CTAs per
+// SM) and is the faster one where its waves are full: 32 clusters 139 us against
+// 158, 64 clusters 498 against 516; 40 clusters 215 against 171, 192 clusters 629
+// against 611.
 template <int N> constexpr int default_terms32() {
   return N <= 24 ? 700 : 616;
 }
-
-// The largest grid (CTAs or clusters) that dir_slices fills, over the variants.
-template <int N> static size_t slots_resident_n(bool fp32) {
-  if (!fp32) {
-    if constexpr (N <= 16) return terms1_resident<double, N>();
-    else return termsh_resident<double, N, VhsClusters<N>::c64>();
-  }
-  int m = 1;
-  for (int c : Terms32Variants<N>::v)
-    if (c >= 600) m = std::max(m, resident32<N>(c));
-  return m;
+struct Terms32Choice { int code, ns; };
+template <int N> static Terms32Choice choose_terms32(const dgfs_vhs_s* h, int nevals) {
+  const int code = h->c32 ? h->c32 : default_terms32<N>();
+  if (code < 600) return {code, 1};
+  const Slices s = dir_slices(h, nevals, resident32<N>(code),
+                              code == 700 ? kCostOneCta : kCostCluster);
+  if constexpr (N == 32)
+    if (!h->c32 && h->fg_map_ok) {
+      const int base = nevals * ((h->Nrho + 1) / 2), r = terms32_tma_resident<N, 4>();
+      const double waves = (base + r - 1) / r;
+      if (waves * ((h->Nrho > 1 ? 2 : 1) * h->Mu + 2.0) < 1.28 * s.cost) return {504, 1};
+    }
+  return {code, s.ns};
 }
-static size_t slots_resident(int N, bool fp32) {
-  switch (N) {
-    case 8: return slots_resident_n<8>(fp32);
-    case 16: return slots_resident_n<16>(fp32);
-    case 24: return slots_resident_n<24>(fp32);
-    case 32: return slots_resident_n<32>(fp32);
-    default: return slots_resident_n<48>(fp32);
+
+// Spectra that dir_slices may ask for: the batch's own, or twice what the GPU
+// holds at once of any variant (more measured no faster).
+template <int N> static size_t spectra_slots_n(bool fp32) {
+  int m = 1;
+  if (!fp32) {
+    if constexpr (N <= 16) m = terms1_resident<double, N>();
+    else m = termsh_resident<double, N, VhsClusters<N>::c64>();
+  } else {
+    for (int c : Terms32Variants<N>::v)
+      if (c >= 600) m = std::max(m, resident32<N>(c));
   }
+  return 2 * (size_t)m;
+}
+static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu) {
+  size_t m;
+  switch (N) {
+    case 8: m = spectra_slots_n<8>(fp32); break;
+    case 16: m = spectra_slots_n<16>(fp32); break;
+    case 24: m = spectra_slots_n<24>(fp32); break;
+    case 32: m = spectra_slots_n<32>(fp32); break;
+    default: m = spectra_slots_n<48>(fp32); break;
+  }
+  return std::max(pairs, std::min(m, pairs * Mu));
 }
 
 template <int N>
@@ -750,11 +837,10 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.Fg = h->Fg; a.ph = h->ph; a.uv = h->uv; a.mult = h->mult;
     a.b1w = h->b1w32; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq32; a.rho = h->rho; a.Fny = h->Fny; a.err = h->err;
-    // default: the two-lanes-per-pencil kernel (its own plane format)
-    const int c = h->c32 ? h->c32 : default_terms32<N>();
-    a.pm = c >= 600;
-    a.NS = c >= 600 ? dir_slices(h, nevals, resident32<N>(c)) : 1;
-    nslices = a.NS;
+    const Terms32Choice tc = choose_terms32<N>(h, nevals);
+    const int c = tc.code;
+    a.pm = c >= 600;   // (the two-lane kernels have their own plane format)
+    a.NS = nslices = tc.ns;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
                            dim3((h->Mu + 1) / 2, h->Nrho, nevals), dim3(6 * N),
@@ -802,10 +888,12 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
         return rc;
       mark(); mark();  // no Maxwellian-gain stage in FP64 mode
       if constexpr (N <= 16) {
-        a.NS = nslices = dir_slices(h, nevals, terms1_resident<double, N>());
+        a.NS = nslices =
+            dir_slices(h, nevals, terms1_resident<double, N>(), kCostOneCta).ns;
         rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
       } else {
-        a.NS = nslices = dir_slices(h, nevals, termsh_resident<double, N, C64>());
+        a.NS = nslices =
+            dir_slices(h, nevals, termsh_resident<double, N, C64>(), kCostCluster).ns;
         rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
       }
       if (rc) return rc;

@@ -54,6 +54,46 @@ def test_direction_slices_and_radial_remainders(precision, N, M, full, Nrho, poi
         assert _rel(got[s], ref) < TOL[precision] + floor, (N, Nrho, s)
 
 
+@pytest.mark.parametrize('points', [1, 3, 6, 8, 10, 12, 16])
+def test_default_terms_kernel_by_batch_size(points):
+    """N=32, FP32: the default kernel and its direction slices follow the batch
+    size; at each the values of every variant, and (10% allowed for the timing)
+    no more time than the kernel of clusters of four, which a default fixed for
+    24 points once exceeded by 14% at 8 points."""
+    from dgfs1d_gpu_b200.collision import VHSOperator
+    vm, prefac, gamma, f = vhs_case(32, 12, 8, 6.0, True, nslots=points)
+    op = VHSOperator(**op_kwargs(vm, prefac, gamma), precision='fp32', max_evals=points)
+    fd = torch.tensor(f, device='cuda')
+    st = torch.cuda.Stream()
+
+    def run(code):
+        op.set_variant(code)
+        Q, T = torch.zeros_like(fd), torch.zeros_like(fd)
+        with torch.cuda.stream(st):
+            op.eval(fd, Q, stream=st)
+        st.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            for _ in range(5):
+                op.eval(fd, T, stream=st)
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        ms = []
+        for _ in range(8):
+            a.record()
+            g.replay()
+            b.record()
+            b.synchronize()
+            ms.append(a.elapsed_time(b))
+        del g
+        return Q.cpu().numpy(), min(ms)
+    ref, t504 = run(504)
+    for code in (0, 608, 616):
+        Q, t = run(code)
+        assert _rel(Q, ref) < 1e-6, code
+        if code == 0:
+            assert t < 1.1 * t504, (t, t504)
+
+
 @pytest.mark.parametrize('N', [16, 24])
 def test_radial_points_of_very_different_weight(N):
     """Two radial points share a forward transform: the sum of the small radius
