@@ -18,6 +18,11 @@
 
 namespace dgfs {
 
+// CTAs per point of the prologue kernel (its partial results are per CTA).
+__host__ __device__ constexpr int prologue_ctas(int N) {
+  return N == 8 ? 1 : N == 16 ? 4 : N == 24 ? 6 : 16;
+}
+
 template <int N, int C> struct Geo {
   static_assert(N % C == 0, "cluster size must divide N");
   static constexpr int P = N / C;         // planes per CTA

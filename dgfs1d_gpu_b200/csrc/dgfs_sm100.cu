@@ -233,12 +233,12 @@ static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu);
 // N=16 vhs_terms1_kernel runs); c32: FP32 terms kernel with one thread per
 // pencil; cpro / cepi: prologue / epilogue (FP64, two lanes per pencil, one slab
 // per CTA), small enough that a 24-point batch runs in one wave up to N=32.
-template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = 1, cepi = 1; };
-template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = 4, cepi = 4; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 12, c32 = 3, cpro = 6, cepi = 6; };
-template <> struct VhsClusters<32> { static constexpr int c64 = 16, c32 = 4, cpro = 16, cepi = 16; };
+template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = prologue_ctas(8), cepi = 1; };
+template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = prologue_ctas(16), cepi = 4; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 12, c32 = 3, cpro = prologue_ctas(24), cepi = 6; };
+template <> struct VhsClusters<32> { static constexpr int c64 = 16, c32 = 4, cpro = prologue_ctas(32), cepi = 16; };
 // N=48: 16-CTA clusters of 3 planes
-template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = 16, cepi = 16; };
+template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = prologue_ctas(48), cepi = 16; };
 
 static size_t slab_bytes(int N, int C, size_t elem) {
   return (size_t)(N / C) * N * (N + 1) * elem;
@@ -1664,7 +1664,7 @@ struct dgfs_vss_s {
                                        // points x radial slices
   double cw = 0;
   // the FP64 Maxwellian gain of the FP32 mode runs on `aux` (low priority)
-  // beside the terms kernel
+  // beside the plane transforms and the terms kernel
   cudaStream_t aux = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
@@ -1680,8 +1680,8 @@ static void free_vss(dgfs_vss_s* h) {
   for (void* q : {(void*)h->w, (void*)h->dirs, (void*)h->dirsm, (void*)h->c0,
                   (void*)h->ReLf, h->rho, (void*)h->uv, (void*)h->hh, (void*)h->GM, h->H})
     if (q) cudaFree(q);
-  if (h->fork) cudaEventDestroy(h->fork);
-  if (h->join) cudaEventDestroy(h->join);
+  for (cudaEvent_t ev : {h->fork, h->join})
+    if (ev) cudaEventDestroy(ev);
   if (h->aux) cudaStreamDestroy(h->aux);
   delete h;
 }
@@ -1850,8 +1850,8 @@ extern "C" int dgfs_vss_create(const dgfs_vss_desc* d, dgfs_vss_handle* out) {
         e1 = cudaDeviceGetStreamPriorityRange(&lo, &hi);
         if (e1 == cudaSuccess)
           e1 = cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, lo);
-        if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
-        if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming);
+        for (cudaEvent_t* ev : {&h->fork, &h->join})
+          if (e1 == cudaSuccess) e1 = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
       }
       for (int pq = 0; pq < h->nspcs * h->nspcs; ++pq) {
         A(&h->pair[pq].b32, T * n * sizeof(float2));
@@ -1899,8 +1899,8 @@ struct VssCall {
 // the loss of the pair), the plane transforms, one terms launch over every
 // pair and one epilogue that sums the pairs' spectra with their prefactors
 // before a single inverse transform (Re IFFT is linear); in the FP32 mode also
-// the 1-D tables per pair and the FP64 Maxwellian gain on the low-priority
-// stream beside the terms.
+// the pairs' 1-D tables, and the FP64 Maxwellian gain on the low-priority stream
+// beside the planes and the terms.
 template <typename R, int N>
 static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int q_double,
                    const int32_t* ss, int sb, const int32_t* ds, int db, int nevals,
@@ -1934,7 +1934,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
       return rc;
   }
   VssTermsArgs tt{};
-  tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals; tt.nc = CPRO;
+  tt.w = h->w; tt.Nrho = h->Nrho; tt.M = h->M; tt.nevals = nevals;
   tt.NS = FP32 ? h->Nrho
                : (int)std::max<size_t>(1, std::min<size_t>(
                      h->Nrho, h->hslots / ((size_t)c.nq * nevals)));
@@ -1956,16 +1956,15 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
   }
   const size_t psmem = (size_t)(6 * N * (N + 1) + 6 * N) * sizeof(T);
   if (FP32) {
-    for (int k = 0; k < c.nq; ++k) {
-      VssTablesArgs ta{};
-      ta.mhat_p = h->mhat[c.sp]; ta.mhat_q = h->mhat[c.sq[k]];
-      ta.ph = pair(k).ph; ta.uv = const_cast<float2*>(tt.pr[k].uv);
-      ta.hh = h->hh + k * E * Tt * 3 * N; ta.T = (int)Tt; ta.nevals = nevals;
-      if ((rc = launch_plain(vss_tables_kernel<N>,
-                             dim3((unsigned)((nevals * Tt * 3 + 127) / 128)), dim3(128), 0,
-                             st, ta)))
-        return rc;
-    }
+    VssTablesArgs ta{};
+    ta.mhat_p = h->mhat[c.sp]; ta.T = (int)Tt; ta.nevals = nevals;
+    for (int k = 0; k < c.nq; ++k)
+      ta.pr[k] = {h->mhat[c.sq[k]], pair(k).ph, const_cast<float2*>(tt.pr[k].uv),
+                  h->hh + k * E * Tt * 3 * N};
+    if ((rc = launch_plain(vss_tables_kernel<N>,
+                           dim3((unsigned)((nevals * Tt * 3 + 127) / 128), c.nq), dim3(128),
+                           0, st, ta)))
+      return rc;
     DGFS_CUDA(cudaEventRecord(h->fork, st));
     DGFS_CUDA(cudaStreamWaitEvent(h->aux, h->fork, 0));
   }
@@ -1980,15 +1979,23 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
                         dim3(HalfGeo<N, C>::NT), C, VssHGeo<R, N, C>::smem, st, tt);
   if (rc) return rc;
   if (FP32) {
-    for (int k = 0; k < c.nq; ++k) {
+    using GG = VssGainGeo<N>;
+    const int ep = std::min(nevals, 3), groups = (nevals + ep - 1) / ep;
+    auto* gain = ep == 1 ? vss_maxwell_gain_kernel<N, 1>
+               : ep == 2 ? vss_maxwell_gain_kernel<N, 2> : vss_maxwell_gain_kernel<N, 3>;
+    // one launch for the pairs of a few points or while they take at most a CTA
+    // per SM (N=32, one point: 572 against 612 us for both species); a larger one
+    // keeps the terms' CTAs from starting (N=32, 18 points: 2968 us against 2874
+    // with a launch each; N=16, 24 points, 256 CTAs: 370 against 360)
+    const int step = groups == 1 || N * (N / GG::NYB) * groups * c.nq <= 148 ? c.nq : 1;
+    for (int k0 = 0; k0 < c.nq; k0 += step) {
       VssGainArgs ga{};
-      ga.hh = h->hh + k * E * Tt * 3 * N; ga.b = pair(k).b; ga.w = h->w;
-      ga.GM = h->GM + k * E * n; ga.dirs = tt.pr[k].dirs; ga.nd = tt.pr[k].nd;
-      ga.Nrho = h->Nrho; ga.M = h->M; ga.nevals = nevals;
-      using GG = VssGainGeo<N>;
-      if ((rc = launch_plain(vss_maxwell_gain_kernel<N>,
-                             dim3(N, N / GG::NYB, (nevals + GG::EP - 1) / GG::EP),
-                             dim3(GG::NT), 0, h->aux, ga)))
+      ga.w = h->w; ga.Nrho = h->Nrho; ga.M = h->M; ga.nevals = nevals;
+      for (int k = k0; k < k0 + step; ++k)
+        ga.pr[k - k0] = {h->hh + k * E * Tt * 3 * N, pair(k).b, h->GM + k * E * n,
+                         tt.pr[k].dirs, tt.pr[k].nd};
+      if ((rc = launch_plain(gain, dim3(N, N / GG::NYB, step * groups), dim3(GG::NT), 0,
+                             h->aux, ga)))
         return rc;
     }
     DGFS_CUDA(cudaEventRecord(h->join, h->aux));

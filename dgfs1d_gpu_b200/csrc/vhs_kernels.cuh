@@ -394,14 +394,15 @@ vhs_prologue_kernel(VhsPrologueArgs a) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
     if ((t & 31) == 0) red[t >> 5] = nrm;   // (peers read red[160 + k] only)
-    __syncthreads();
-    if (t == 0) {
-      for (int i = 1; i < NT / 32; ++i) nrm += red[i];
-      a.norm2[(size_t)e * C + rank] = nrm;
-    }
+  } else if (!a.ReLf) {
+    return;              // (no CTA writes to a peer past this point)
   }
-  if (!a.ReLf) return;   // (no CTA writes to a peer past this point)
   __syncthreads();
+  if (a.norm2 && t == 0) {
+    for (int i = 1; i < NT / 32; ++i) nrm += red[i];
+    a.norm2[(size_t)e * C + rank] = nrm;
+  }
+  if (!a.ReLf) return;
   // loss: Re IFFT(b2 F)
 #pragma unroll
   for (int m = 0; m < H; ++m) v[m] = A[rowb + 2 * m + h];

@@ -167,24 +167,28 @@ __global__ void vss_sum_c_kernel(const double2* cpart, int Nrho, size_t n,
 // and the loss f_p Re IFFT(c G) run in FP64 (prologue and epilogue kernels
 // of the VHS operator, with the complex loss kernel c).
 // ---------------------------------------------------------------------------
+// Grid y: the pairs of the call.
 struct VssTablesArgs {
   const double2* mhat_p;   // [E][3][N]
-  const double2* mhat_q;   // [E][3][N]
-  const double2* ph;       // [T][2][3][N]
-  float2* uv;              // out [E][T][2][3][N]: u_M,a and v_M,a (FP32)
-  double2* hh;             // out [E][T][3][N]: FFT1(u_M,a v_M,a)
+  struct {
+    const double2* mhat_q; // [E][3][N]
+    const double2* ph;     // [T][2][3][N]
+    float2* uv;            // out [E][T][2][3][N]: u_M,a and v_M,a (FP32)
+    double2* hh;           // out [E][T][3][N]: FFT1(u_M,a v_M,a)
+  } pr[4];
   int T, nevals;
 };
 
 template <int N>
-__global__ void vss_tables_kernel(VssTablesArgs a) {
+__global__ void vss_tables_kernel(const __grid_constant__ VssTablesArgs a) {
+  const auto& Pr = a.pr[blockIdx.y];
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= a.nevals * a.T * 3) return;
   const int ax = gid % 3, term = (gid / 3) % a.T, e = gid / (3 * a.T);
   const double2* mp = a.mhat_p + (size_t)e * 3 * N + ax * N;
-  const double2* mq = a.mhat_q + (size_t)e * 3 * N + ax * N;
-  const double2* pu = a.ph + ((size_t)term * 6 + ax) * N;
-  const double2* pv = a.ph + ((size_t)term * 6 + 3 + ax) * N;
+  const double2* mq = Pr.mhat_q + (size_t)e * 3 * N + ax * N;
+  const double2* pu = Pr.ph + ((size_t)term * 6 + ax) * N;
+  const double2* pv = Pr.ph + ((size_t)term * 6 + 3 + ax) * N;
   double2 u[N], v[N];
 #pragma unroll
   for (int l = 0; l < N; ++l) {
@@ -193,7 +197,7 @@ __global__ void vss_tables_kernel(VssTablesArgs a) {
   }
   fft<double, N, +1>(u);
   fft<double, N, +1>(v);
-  float2* uv = a.uv + ((size_t)e * a.T + term) * 6 * N;
+  float2* uv = Pr.uv + ((size_t)e * a.T + term) * 6 * N;
 #pragma unroll
   for (int l = 0; l < N; ++l) {
     uv[ax * N + l] = make_float2((float)u[l].x, (float)u[l].y);
@@ -201,43 +205,50 @@ __global__ void vss_tables_kernel(VssTablesArgs a) {
     u[l] = cmul(u[l], v[l]);
   }
   fft<double, N, -1>(u);
-  double2* hh = a.hh + (((size_t)e * a.T + term) * 3 + ax) * N;
+  double2* hh = Pr.hh + (((size_t)e * a.T + term) * 3 + ax) * N;
 #pragma unroll
   for (int l = 0; l < N; ++l) hh[l] = u[l];
 }
 
 // GM[e][l] = sum_r w_r sum_d b_rd(l) prod_a H_a,rd(l_a)   (FP64), d over the
 // pair's direction list (merged antipodes share H and add their b).
-// Grid (N [lx], N / NYB, ceil(E / EP)), block N NYB: a thread owns the
+// Grid (N [lx], N / NYB, pairs ceil(E / EP)), block N NYB: a thread owns the
 // wavenumber (lx, ly, lz) of EP points, so that every weight b is read once
 // for EP points (one point per thread read b, 32 MB per pair at N=24, from L2
-// for each point: 163 us per pair at 18 points).  The 1-D factors of a chunk
-// of terms are staged in shared memory, hx hy folded once per (term, ly).
+// for each point: 163 us per pair at 18 points).  EP = 3, or the number of points
+// if that is less.  The 1-D factors of a chunk of terms are staged in shared
+// memory, hx hy folded once per (term, ly).
 struct VssGainArgs {
-  const double2* hh;       // [E][T][3][N]
-  const double2* b;        // [T][n]
+  struct {
+    const double2* hh;     // [E][T][3][N]
+    const double2* b;      // [T][n]
+    double2* GM;           // out [E][n]
+    const int2* dirs;
+    int nd;
+  } pr[4];
   const double* w;         // [Nrho]
-  double2* GM;             // out [E][n]
-  const int2* dirs;
-  int nd, Nrho, M, nevals;
+  int Nrho, M, nevals;
 };
 template <int N> struct VssGainGeo {
   static constexpr int NYB = N == 16 ? 16 : 8;   // ly rows per CTA
   static constexpr int NT = N * NYB;
-  static constexpr int EP = 3;                   // points per thread
   static constexpr int CH = 12;                  // terms per staged chunk
 };
 
-template <int N>
-__global__ void __launch_bounds__(VssGainGeo<N>::NT) vss_maxwell_gain_kernel(VssGainArgs a) {
+template <int N, int EP>
+__global__ void __launch_bounds__(VssGainGeo<N>::NT)
+vss_maxwell_gain_kernel(const __grid_constant__ VssGainArgs a) {
   using GG = VssGainGeo<N>;
-  constexpr int n = N * N * N, EP = GG::EP, CH = GG::CH, NYB = GG::NYB;
+  constexpr int n = N * N * N, CH = GG::CH, NYB = GG::NYB;
   __shared__ double2 hz[CH][EP][N];
   __shared__ double2 hxy[CH][EP][NYB];
-  const int lx = blockIdx.x, ly0 = blockIdx.y * NYB, e0 = blockIdx.z * EP;
+  const int groups = (a.nevals + EP - 1) / EP;
+  const auto& Pr = a.pr[blockIdx.z / groups];
+  const int nd = Pr.nd;
+  const int lx = blockIdx.x, ly0 = blockIdx.y * NYB, e0 = (blockIdx.z % groups) * EP;
   const int t = threadIdx.x, yl = t / N, lz = t % N;
   const size_t l = ((size_t)lx * N + ly0 + yl) * N + lz;
-  const int T = a.Nrho * a.M, total = a.Nrho * a.nd;
+  const int T = a.Nrho * a.M, total = a.Nrho * nd;
   double2 acc[EP];
 #pragma unroll
   for (int p = 0; p < EP; ++p) acc[p] = make_double2(0, 0);
@@ -246,9 +257,9 @@ __global__ void __launch_bounds__(VssGainGeo<N>::NT) vss_maxwell_gain_kernel(Vss
     __syncthreads();
     for (int i = t; i < nc * EP * (N + NYB); i += GG::NT) {
       const int j = i % (N + NYB), p = (i / (N + NYB)) % EP, k = i / (EP * (N + NYB));
-      const int e = min(e0 + p, a.nevals - 1), r = (c0 + k) / a.nd;
-      const int term = r * a.M + a.dirs[(c0 + k) % a.nd].x;
-      const double2* h = a.hh + ((size_t)e * T + term) * 3 * N;
+      const int e = min(e0 + p, a.nevals - 1), r = (c0 + k) / nd;
+      const int term = r * a.M + Pr.dirs[(c0 + k) % nd].x;
+      const double2* h = Pr.hh + ((size_t)e * T + term) * 3 * N;
       if (j < N) {
         hz[k][p][j] = h[2 * N + j];
       } else {
@@ -260,11 +271,11 @@ __global__ void __launch_bounds__(VssGainGeo<N>::NT) vss_maxwell_gain_kernel(Vss
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < nc; ++k) {
-      const int r = (c0 + k) / a.nd;
-      const int2 dir = a.dirs[(c0 + k) % a.nd];
-      double2 b = a.b[(size_t)(r * a.M + dir.x) * n + l];
+      const int r = (c0 + k) / nd;
+      const int2 dir = Pr.dirs[(c0 + k) % nd];
+      double2 b = Pr.b[(size_t)(r * a.M + dir.x) * n + l];
       if (dir.y >= 0) {
-        const double2 q = a.b[(size_t)(r * a.M + dir.y) * n + l];
+        const double2 q = Pr.b[(size_t)(r * a.M + dir.y) * n + l];
         b.x += q.x; b.y += q.y;
       }
 #pragma unroll
@@ -277,7 +288,7 @@ __global__ void __launch_bounds__(VssGainGeo<N>::NT) vss_maxwell_gain_kernel(Vss
   }
 #pragma unroll
   for (int p = 0; p < EP; ++p)
-    if (e0 + p < a.nevals) a.GM[(size_t)(e0 + p) * n + l] = acc[p];
+    if (e0 + p < a.nevals) Pr.GM[(size_t)(e0 + p) * n + l] = acc[p];
 }
 
 // Pointers of one species pair; a launch covers npair pairs, grid z =
@@ -294,13 +305,12 @@ struct VssTermsPair {
   void* H;                 // out [E][NS][n]
   const int2* dirs;        // [nd] direction and its merged antipode (or -1)
   int nd;
-  const double* n2p;       // [E][nc] sums |F_p|^2, |F_q|^2 of the prologue's CTAs
+  const double* n2p;       // [E][prologue CTAs] sums |F_p|^2, |F_q|^2
   const double* n2q;
 };
 struct VssTermsArgs {
   VssTermsPair pr[4];
   const double* w;         // [Nrho]
-  int nc;                  // CTAs per point of the prologue
   int Nrho, M, nevals;
   int NS;                  // radial slices (blockIdx.y): r in [y Nrho/NS, ...)
 };
@@ -319,19 +329,24 @@ template <typename T> __device__ __forceinline__ T vss_nu(T ph) {
 // spectral sums through back = 1 / (su sv): every step is exact.  back = 0 if
 // either is zero everywhere (u v = 0).
 template <typename R> struct VssScale { R su, sv, back; };
-template <typename R>
-__device__ __forceinline__ VssScale<R> vss_scale(const VssTermsPair& Pr, int e, int nc) {
+__device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+template <typename R, int N>
+__device__ __forceinline__ VssScale<R> vss_scale(const VssTermsPair& Pr, int e) {
+  constexpr int NC = prologue_ctas(N);
   double sp = 0, sq = 0;
-  for (int c = 0; c < nc; ++c) {
-    sp += Pr.n2p[(size_t)e * nc + c];
-    sq += Pr.n2q[(size_t)e * nc + c];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    sp += Pr.n2p[(size_t)e * NC + c];
+    sq += Pr.n2q[(size_t)e * NC + c];
   }
-  if (sp == 0 || sq == 0) return {R(1), R(1), R(0)};
+  // biased exponents; 0x7ff: a sum that is not finite, unscaled (no branches, so
+  // that the loads stay in flight under what follows)
   constexpr int KMAX = sizeof(R) == 4 ? 60 : 400;
-  int k = 0;                       // (a sum that is not finite: unscaled)
-  if (isfinite(sp) && isfinite(sq)) k = (ilogb(sq) - ilogb(sp)) / 2;
-  k = max(-KMAX, min(KMAX, k));
-  return {(R)ldexp(1.0, max(k, 0)), (R)ldexp(1.0, max(-k, 0)), (R)ldexp(1.0, -abs(k))};
+  const int ep = (__double2hiint(sp) >> 20) & 0x7ff, eq = (__double2hiint(sq) >> 20) & 0x7ff;
+  const bool none = ep == 0 || eq == 0;
+  int k = max(-KMAX, min(KMAX, (eq - ep) / 2));
+  k = none || ep == 0x7ff || eq == 0x7ff ? 0 : k;
+  return {(R)pow2(max(k, 0)), (R)pow2(max(-k, 0)), none ? R(0) : (R)pow2(-abs(k))};
 }
 
 // Plane transforms of one term.  With E the phase factor and f_S as in the
@@ -358,7 +373,7 @@ __global__ void __launch_bounds__(3 * N) vss_planes_kernel(VssTermsArgs a) {
   const int P = t / N, i = t % N;
   const T* Fp = static_cast<const T*>(Pr.Fnyp) + (size_t)e * 3 * N * N;
   const T* Fq = static_cast<const T*>(Pr.Fnyq) + (size_t)e * 3 * N * N;
-  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
+  const VssScale<R> sc = vss_scale<R, N>(Pr, e);
 #pragma unroll 4
   for (int j = t; j < 3 * N * N; j += 3 * N) {
     pls[(j / N) * ROW + j % N] = Fp[j];
@@ -486,14 +501,15 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
   T Qh[H];
 #pragma unroll
   for (int m = 0; m < H; ++m) Qh[m] = T{R(0), R(0)};
-  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
+  // (its third part is taken again at the end: it need not stay in registers)
+  const VssScale<R> sc = vss_scale<R, N>(Pr, e);
+  const R ss = t < P * N ? sc.su : sc.sv;
   // the row factors of a term, scaled: one (field, row) per thread
   auto row_tables = [&](int term) {
     const int f = t / (P * N), row = t % (P * N);
     const int x = rank * P + row / N, y = row % N;
     const T* ph = static_cast<const T*>(Pr.ph) + (size_t)term * 6 * N + f * 3 * N;
     T E = cmul(ph[x], ph[N + y]);
-    const R ss = f == 0 ? sc.su : sc.sv;
     E.x *= ss;
     E.y *= ss;
     T fx = T{R(1), R(0)};
@@ -616,7 +632,8 @@ vss_terms_kernel(const __grid_constant__ VssTermsArgs a) {
       Qh[m].y += wr * x.y;
     }
   }
-  const R wo = SPLIT ? (R)a.w[r0] * sc.back : sc.back;
+  const R back = vss_scale<R, N>(Pr, e).back;
+  const R wo = SPLIT ? (R)a.w[r0] * back : back;
   T* Ho = static_cast<T*>(Pr.H) + ((size_t)e * a.NS + blockIdx.y) * G::n + slab0 +
           (size_t)pl * N * N + (size_t)h * H * N + c;
 #pragma unroll
@@ -676,7 +693,7 @@ vss_terms1_kernel(const __grid_constant__ VssTermsArgs a) {
     if constexpr (HP) fft_half_dit<R, N, -1>(v, h);
     else fft<R, N, -1>(v);
   };
-  const VssScale<R> sc = vss_scale<R>(Pr, e, a.nc);
+  const VssScale<R> sc = vss_scale<R, N>(Pr, e);
   for (int i = t; i < G::n; i += NT) Qh[i] = T{R(0), R(0)};
   __syncthreads();
 #pragma unroll 1

@@ -196,6 +196,36 @@ def test_scratch_is_bounded():
         assert _rel(Q[i].cpu().numpy(), Q1[0].cpu().numpy()) < 1e-11, i
 
 
+@pytest.mark.parametrize('points', [1, 2, 3, 4, 7])
+def test_vss_gain_by_batch_size(points):
+    """FP32 mixture gain with one, two and three points per thread, the last group
+    part-filled, one launch for the pairs (up to three points at N=24) and one
+    each: the FP64 mode's values."""
+    from dgfs1d_gpu_b200.collision import VSSOperator
+    masses = [1.0, 1.7]
+    vm = om.VelocityMeshBi(Nv=24, M=6, masses=masses, Nrho=3, dev=5.0)
+    one = np.ones((2, 2))
+    rng = np.random.default_rng(9)
+    fs = []
+    for T in (1.0, 1.2):
+        m = 0.5 * np.exp(-np.sum(vm.cv ** 2, axis=0) / T) / (np.pi * T) ** 1.5
+        fs.append(torch.tensor(np.stack([
+            m * (1 + 0.02 * rng.uniform(-1, 1, m.shape)) for _ in range(points)]),
+            device='cuda'))
+    Q = {}
+    for precision in ('fp64', 'fp32'):
+        op = VSSOperator(24, vm.L, vm.qz, vm.qw, vm.sz, vm.sw, om.sphere_design(12),
+                         masses, 0.38 * one, 0.4 * one, 0.1 * one, max_evals=points,
+                         precision=precision)
+        Q[precision] = [torch.zeros_like(x) for x in fs]
+        for p in range(2):
+            op.eval_species(p, fs, Q[precision][p])
+    for p in range(2):
+        for i in range(points):
+            assert _rel(Q['fp32'][p][i].cpu().numpy(),
+                        Q['fp64'][p][i].cpu().numpy()) < TOL['fp32'], (p, i)
+
+
 @pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
 def test_axnpby_vector_and_scalar_routes(dtype):
     """Sizes around the vector kernel's groups, operands off 16-byte alignment
