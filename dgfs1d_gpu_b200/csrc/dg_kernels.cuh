@@ -254,15 +254,18 @@ __device__ __forceinline__ double dg_ghost(const DgAdvectArgs& a, int side,
 // with jL = 0.5|c|(uL-uR) + 0.5c(uR-uL), jR = 0.5|c|(uL-uR) + 0.5c(uL-uR)
 // at each face (uL: state on its left, uR: on its right).  One thread per
 // velocity point walks the elements [blockIdx.y len, + len) and reads one
-// element more on either side for the traces.  Bound: HBM; element e + 2 is
-// loaded while e is computed.  Small velocity grids split the walk (see
-// dgfs_dg_advect); large ones do not: four walks of eight elements instead of
-// one of 32 took 59.6 instead of 39.7 us at N=48, K=3.
-// (Three CTAs per SM: at 94 registers, i.e. two, the 432 CTAs of N=48 ran in
-// a wave and a half, 64 us.)
+// element more on either side for the traces.  Bound: HBM; up to K = 3 element
+// e + 2 is loaded while e is computed, above it only e + 1, in a loop that is not
+// unrolled: a third element's registers cost a CTA per SM (K=5, N=48, 48
+// elements with the update: 228 us with, 186 without; FP32 arrays 206 and 153).
+// Small velocity grids split the walk (see dgfs_dg_advect); large ones do not:
+// four walks of eight elements instead of one of 32 took 59.6 instead of 39.7 us
+// at N=48, K=3.  (Three CTAs per SM: at 94 registers, i.e. two, the 432 CTAs of
+// N=48 ran in a wave and a half, 64 us.)
 template <int K>
-__global__ void __launch_bounds__(256, K <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(256, K <= 6 ? 3 : 2)
 dg_advect_kernel(DgAdvectArgs a, int len) {
+  constexpr bool AHEAD2 = K <= 3;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= a.Nv) return;
   const int Ne = a.Ne, Nv = a.Nv;
@@ -273,9 +276,12 @@ dg_advect_kernel(DgAdvectArgs a, int len) {
 #pragma unroll
   for (int k = 0; k < K; ++k)
     ue[k] = ld(a.u, a.f_double, ((size_t)k * Ne + e0) * Nv + v);
+  auto load = [&](double* w, int e, bool in) {
 #pragma unroll
-  for (int k = 0; k < K; ++k)
-    un[k] = e0 + 1 < Ne ? ld(a.u, a.f_double, ((size_t)k * Ne + e0 + 1) * Nv + v) : 0.;
+    for (int k = 0; k < K; ++k)
+      w[k] = in ? ld(a.u, a.f_double, ((size_t)k * Ne + e) * Nv + v) : 0.;
+  };
+  if (AHEAD2) load(un, e0 + 1, e0 + 1 < Ne);
   auto tl = [&](const double* w) {
     double s = 0;
 #pragma unroll
@@ -308,12 +314,10 @@ dg_advect_kernel(DgAdvectArgs a, int len) {
                        : trace_of(e0 - 1, true);
   const double jd0 = ac * (uLf - uRf);
   double jR = jd0 + hc * (uLf - uRf);
-#pragma unroll 2
+#pragma unroll (AHEAD2 ? 2 : 1)
   for (int e = e0; e < e1; ++e) {
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      u2[k] = e + 2 < Ne && e + 1 < e1
-                  ? ld(a.u, a.f_double, ((size_t)k * Ne + e + 2) * Nv + v) : 0.;
+    if (AHEAD2) load(u2, e + 2, e + 2 < Ne && e + 1 < e1);
+    else load(un, e + 1, e + 1 < Ne);
     // face e+1
     const double uL1 = tr(ue);
     const double uR1 =
@@ -340,7 +344,10 @@ dg_advect_kernel(DgAdvectArgs a, int len) {
     }
     jR = jd + hc * (uL1 - uR1);  // jR of face e+1 for element e+1
 #pragma unroll
-    for (int k = 0; k < K; ++k) { ue[k] = un[k]; un[k] = u2[k]; }
+    for (int k = 0; k < K; ++k) {
+      ue[k] = un[k];
+      if (AHEAD2) un[k] = u2[k];
+    }
   }
 }
 
