@@ -1,8 +1,9 @@
-// Fused fast-spectral VSS collision operator of a binary mixture, one
-// species pair (p, q) per call.  Reference: DGFSBiVSSScatteringModel
-// (dgfs1D/bi/scattering.py:47-321) and dgfs1D/bi/kernels/scattering/vss.mako.
+// Fused fast-spectral VSS collision operator of a mixture: one species pair
+// (p, q), or every pair of a species, per call.  Reference:
+// DGFSBiVSSScatteringModel (dgfs1D/bi/scattering.py:47-321) and
+// dgfs1D/bi/kernels/scattering/vss.mako.
 //
-// Per point the reference computes, with F = FFT(f_p)/n, G = FFT(f_q)/n and
+// Per point and pair the reference computes, with F = FFT(f_p)/n, G = FFT(f_q)/n and
 // a_rm(l) = (pi/L) rho_r sigma_m . l:
 //   t1 = e^{+i a m_q/(m_p+m_q)} F,  t2 = e^{-i a m_p/(m_p+m_q)} G,
 //   Qhat = sum_{r,m} (w_r s_w / n) b_{pq,rm}(l) FFT(IFFT(t1) IFFT(t2)),
@@ -162,8 +163,8 @@ __global__ void vss_sum_c_kernel(const double2* cpart, int Nrho, size_t n,
 // and the product splits into u_M v_M, whose 3-D transform is the product of
 // the 1-D FP64 transforms H_a = FFT1(u_M,a v_M,a) (vss_maxwell_gain_kernel),
 // and the remainder u_M X_v + X_u (v_M + X_v), transformed in FP32
-// (vss_terms32_kernel, one cluster per (pair, point, radial point), summed
-// over the directions in shared memory).  The radial sum, the final transform
+// (vss_terms1_kernel or vss_terms_kernel, one CTA or cluster per (pair, point,
+// radial point), summed over the directions in FP32).  The radial sum, the final transform
 // and the loss f_p Re IFFT(c G) run in FP64 (prologue and epilogue kernels
 // of the VHS operator, with the complex loss kernel c).
 // ---------------------------------------------------------------------------
@@ -243,8 +244,11 @@ vss_maxwell_gain_kernel(const __grid_constant__ VssGainArgs a) {
   __shared__ double2 hz[CH][EP][N];
   __shared__ double2 hxy[CH][EP][NYB];
   const int groups = (a.nevals + EP - 1) / EP;
-  const auto& Pr = a.pr[blockIdx.z / groups];
-  const int nd = Pr.nd;
+  const int pi = blockIdx.z / groups, nd = a.pr[pi].nd;
+  const double2* hh = a.pr[pi].hh;
+  const double2* bw = a.pr[pi].b;
+  double2* GM = a.pr[pi].GM;
+  const int2* dirs = a.pr[pi].dirs;
   const int lx = blockIdx.x, ly0 = blockIdx.y * NYB, e0 = (blockIdx.z % groups) * EP;
   const int t = threadIdx.x, yl = t / N, lz = t % N;
   const size_t l = ((size_t)lx * N + ly0 + yl) * N + lz;
@@ -258,8 +262,8 @@ vss_maxwell_gain_kernel(const __grid_constant__ VssGainArgs a) {
     for (int i = t; i < nc * EP * (N + NYB); i += GG::NT) {
       const int j = i % (N + NYB), p = (i / (N + NYB)) % EP, k = i / (EP * (N + NYB));
       const int e = min(e0 + p, a.nevals - 1), r = (c0 + k) / nd;
-      const int term = r * a.M + Pr.dirs[(c0 + k) % nd].x;
-      const double2* h = Pr.hh + ((size_t)e * T + term) * 3 * N;
+      const int term = r * a.M + dirs[(c0 + k) % nd].x;
+      const double2* h = hh + ((size_t)e * T + term) * 3 * N;
       if (j < N) {
         hz[k][p][j] = h[2 * N + j];
       } else {
@@ -272,10 +276,10 @@ vss_maxwell_gain_kernel(const __grid_constant__ VssGainArgs a) {
 #pragma unroll 4
     for (int k = 0; k < nc; ++k) {
       const int r = (c0 + k) / nd;
-      const int2 dir = Pr.dirs[(c0 + k) % nd];
-      double2 b = Pr.b[(size_t)(r * a.M + dir.x) * n + l];
+      const int2 dir = dirs[(c0 + k) % nd];
+      double2 b = bw[(size_t)(r * a.M + dir.x) * n + l];
       if (dir.y >= 0) {
-        const double2 q = Pr.b[(size_t)(r * a.M + dir.y) * n + l];
+        const double2 q = bw[(size_t)(r * a.M + dir.y) * n + l];
         b.x += q.x; b.y += q.y;
       }
 #pragma unroll
@@ -288,7 +292,7 @@ vss_maxwell_gain_kernel(const __grid_constant__ VssGainArgs a) {
   }
 #pragma unroll
   for (int p = 0; p < EP; ++p)
-    if (e0 + p < a.nevals) Pr.GM[(size_t)(e0 + p) * n + l] = acc[p];
+    if (e0 + p < a.nevals) GM[(size_t)(e0 + p) * n + l] = acc[p];
 }
 
 // Pointers of one species pair; a launch covers npair pairs, grid z =
@@ -339,14 +343,15 @@ __device__ __forceinline__ VssScale<R> vss_scale(const VssTermsPair& Pr, int e) 
     sp += Pr.n2p[(size_t)e * NC + c];
     sq += Pr.n2q[(size_t)e * NC + c];
   }
-  // biased exponents; 0x7ff: a sum that is not finite, unscaled (no branches, so
-  // that the loads stay in flight under what follows)
+  // biased exponents; 0x7ff: a sum that is not finite, unscaled.  (The early
+  // return also keeps the result in registers: without it the one-CTA kernel at
+  // N=24, 18 points, took 517 us instead of 495.)
   constexpr int KMAX = sizeof(R) == 4 ? 60 : 400;
   const int ep = (__double2hiint(sp) >> 20) & 0x7ff, eq = (__double2hiint(sq) >> 20) & 0x7ff;
-  const bool none = ep == 0 || eq == 0;
+  if (ep == 0 || eq == 0) return {R(1), R(1), R(0)};
   int k = max(-KMAX, min(KMAX, (eq - ep) / 2));
-  k = none || ep == 0x7ff || eq == 0x7ff ? 0 : k;
-  return {(R)pow2(max(k, 0)), (R)pow2(max(-k, 0)), none ? R(0) : (R)pow2(-abs(k))};
+  if (ep == 0x7ff || eq == 0x7ff) k = 0;
+  return {(R)pow2(max(k, 0)), (R)pow2(max(-k, 0)), (R)pow2(-abs(k))};
 }
 
 // Plane transforms of one term.  With E the phase factor and f_S as in the
