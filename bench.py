@@ -39,7 +39,8 @@ def make_inputs(rank=0):
 
 
 def terms_kernel_name(code):
-    """The FP32 N=32 terms kernel of a variant code (0: the default, 616)."""
+    """The FP32 N=32 terms kernel of a variant code (0: the default, at 24
+    points 616)."""
     code = int(code) or 616
     c = code % 100
     return {0: f'vhs_terms_fp32_kernel<32,{c}>',

@@ -136,7 +136,8 @@ class VHSOperator:
             nevals, _stream_ptr(stream)))
 
     def variants(self):
-        """Cluster sizes of the FP32 terms kernel compiled for this N."""
+        """Codes of the FP32 terms kernel's variants compiled for this N (see
+        dgfs_vhs_variants; 0 selects by batch size)."""
         buf = (ctypes.c_int32 * 8)()
         n = nat.lib().dgfs_vhs_variants(self.N, buf, 8)
         if n < 0:

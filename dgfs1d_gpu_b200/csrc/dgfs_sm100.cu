@@ -161,6 +161,8 @@ static int launch_plain(K kernel, dim3 grid, dim3 block, size_t smem,
   return DGFS_OK;
 }
 
+constexpr int kSms = 148;   // SMs of a B200 (sm_100a code runs on nothing else)
+
 // ---------------------------------------------------------------------------
 // VHS handle
 // ---------------------------------------------------------------------------
@@ -230,15 +232,17 @@ static int c32_of(int N) {
 template <int N> struct VhsClusters;
 static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu);
 // c64: FP64 terms kernel with two lanes per pencil (vhs_termsh_kernel; up to
-// N=16 vhs_terms1_kernel runs); c32: FP32 terms kernel with one thread per
-// pencil; cpro / cepi: prologue / epilogue (FP64, two lanes per pencil, one slab
-// per CTA), small enough that a 24-point batch runs in one wave up to N=32.
-template <> struct VhsClusters<8> { static constexpr int c64 = 1, c32 = 1, cpro = prologue_ctas(8), cepi = 1; };
-template <> struct VhsClusters<16> { static constexpr int c64 = 2, c32 = 1, cpro = prologue_ctas(16), cepi = 4; };
-template <> struct VhsClusters<24> { static constexpr int c64 = 12, c32 = 3, cpro = prologue_ctas(24), cepi = 6; };
-template <> struct VhsClusters<32> { static constexpr int c64 = 16, c32 = 4, cpro = prologue_ctas(32), cepi = 16; };
-// N=48: 16-CTA clusters of 3 planes
-template <> struct VhsClusters<48> { static constexpr int c64 = 16, c32 = 16, cpro = prologue_ctas(48), cepi = 16; };
+// N=16 vhs_terms1_kernel runs).  Over 1 to 48 points, each size with its best
+// slices, evaluations are 3% (N=24, 12 against 6 CTAs), 16% (12 against 4) and
+// 18% (N=32, 16 against 8) shorter: more CTAs of other clusters on an SM hide
+// the exchange.  N=48: only 16 fit.  cpro / cepi: prologue / epilogue (FP64, two
+// lanes per pencil, one slab per CTA), small enough that a 24-point batch runs
+// in one wave up to N=32.
+template <> struct VhsClusters<8> { static constexpr int cpro = prologue_ctas(8), cepi = 1; };
+template <> struct VhsClusters<16> { static constexpr int cpro = prologue_ctas(16), cepi = 4; };
+template <> struct VhsClusters<24> { static constexpr int c64 = 12, cpro = prologue_ctas(24), cepi = 6; };
+template <> struct VhsClusters<32> { static constexpr int c64 = 16, cpro = prologue_ctas(32), cepi = 16; };
+template <> struct VhsClusters<48> { static constexpr int c64 = 16, cpro = prologue_ctas(48), cepi = 16; };
 
 static size_t slab_bytes(int N, int C, size_t elem) {
   return (size_t)(N / C) * N * (N + 1) * elem;
@@ -366,19 +370,20 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
           ph64[(((size_t)p * Mu + u) * 3 + a) * N + l] =
               make_double2(std::cos(k * l0[l]), std::sin(k * l0[l]));
       }
-  std::vector<double> c0(d->c0, d->c0 + N), ps(Nrho, 1.0);
+  std::vector<double> c0(d->c0, d->c0 + N);
   // FP64 packed terms: each radial point's power of two within its pair (1 for
   // the larger weight), on the multiplicities of its directions and off b1w;
   // one allocation with the velocity grid
+  std::vector<double> w0;   // the weights at l = 0, their largest
+  for (int p = 0; p < Nrho; ++p) w0.push_back(std::fabs(b1w[(size_t)p * n]));
   for (int p = 0; p < Nrho && !fp32; ++p) {
-    const double w = std::fabs(b1w[(size_t)p * n]), o = (p ^ 1) < Nrho
-        ? std::fabs(b1w[(size_t)(p ^ 1) * n]) : 0.0;
+    const double w = w0[p], o = (p ^ 1) < Nrho ? w0[p ^ 1] : 0.0;
     const int k = w > 0 ? std::max(-60, std::ilogb(w) - std::ilogb(o)) : -60;
     const double s = o > w && std::isfinite(o) ? std::ldexp(1.0, k) : 1.0;
     for (int u = 0; u < Mu; ++u) c0.push_back(s * mult[u]);
-    ps[p] = s;
+    if (s != 1.0)
+      for (int l = 0; l < n; ++l) b1w[(size_t)p * n + l] *= 1.0 / s;
   }
-  for (size_t i = 0; i < b1w.size(); ++i) b1w[i] /= ps[i / n];
 
   int rc = DGFS_OK;
   if ((rc = upload(&h->c0, c0)) || (rc = upload(&h->b2, b2)) ||
@@ -457,7 +462,7 @@ extern "C" int dgfs_vhs_create(const dgfs_vhs_desc* d, dgfs_vhs_handle* out) {
   }
   if (fp32) {
     // TMA map of F_g for the TMA terms variant at the default cluster size
-    // (P = N / c32 planes per CTA): dims (lz, ly, lx, eval), 8-byte elements
+    // (P = N / c32_of(N) planes per CTA): dims (lz, ly, lx, eval), 8-byte elements
     // (one complex float), box (N+2, N, P, 1): the two elements past each
     // row are out of bounds and arrive as zeros (the row padding)
     void* fn = nullptr;
@@ -593,13 +598,11 @@ template <> struct Terms32Variants<48> { static constexpr int v[5] = {16, 116, 5
 // the driver once per kernel.
 template <typename K>
 static int max_clusters(K kernel, int cluster, int threads, size_t smem) {
-  int n = 0, dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int n = 0;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (cluster == 1) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
-    n *= sms;
+    n *= kSms;
   } else {
     if (cluster > 8)
       cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -617,7 +620,7 @@ static int max_clusters(K kernel, int cluster, int threads, size_t smem) {
     cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   }
   cudaGetLastError();   // (an error leaves n = 0, and a launch reports it)
-  return n > 0 ? n : std::max(1, sms / cluster);
+  return n > 0 ? n : std::max(1, kSms / cluster);
 }
 template <typename R, int N> static int terms1_resident() {
   static const int n =
@@ -794,7 +797,6 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
                    cudaStream_t st, const VhsBilin* bl = nullptr,
                    const void* const* f_list = nullptr,
                    void* const* q_list = nullptr) {
-  constexpr int C64 = VhsClusters<N>::c64;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
   const bool fp32 = h->precision == DGFS_PREC_FP32;
@@ -892,6 +894,7 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
             dir_slices(h, nevals, terms1_resident<double, N>(), kCostOneCta).ns;
         rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
       } else {
+        constexpr int C64 = VhsClusters<N>::c64;
         a.NS = nslices =
             dir_slices(h, nevals, termsh_resident<double, N, C64>(), kCostCluster).ns;
         rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
@@ -1479,7 +1482,7 @@ extern "C" int dgfs_dg_advect(dgfs_dg_handle h, const void* u, void* ux,
   }
   // one walk per velocity point from N=48 on; below, the walk is split until
   // about 512 threads per SM are in flight (N=24, Ne=8: 11.4 -> 7.6 us)
-  const int want = (148 * 512 + a.Nv - 1) / a.Nv;
+  const int want = (kSms * 512 + a.Nv - 1) / a.Nv;
   const int len = std::max(1, a.Ne / std::max(1, std::min(a.Ne, want)));
   const dim3 grid((a.Nv + 255) / 256, (a.Ne + len - 1) / len), block(256);
   switch (a.K) {
@@ -1591,11 +1594,8 @@ extern "C" int dgfs_axnpby(void* x0, int64_t n, int32_t dtype, double a0,
     DGFS_CUDA(cudaGetLastError());
     return DGFS_OK;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t want = ((size_t)n + 255) / 256;
-  const unsigned blocks = (unsigned)std::min<size_t>(want, (size_t)sms * 16);
+  const unsigned blocks = (unsigned)std::min<size_t>(want, (size_t)kSms * 16);
   axnpby_kernel<<<blocks, 256, 0, st>>>(a);
   DGFS_CUDA(cudaGetLastError());
   return DGFS_OK;
@@ -1691,12 +1691,13 @@ __global__ void vss_to_fp32_kernel(const double2* in, float2* out, size_t n) {
   if (i < n) out[i] = make_float2((float)in[i].x, (float)in[i].y);
 }
 
-// cluster sizes of vss_terms_kernel, FP64 and FP32 (1: vss_terms1_kernel runs)
-template <int N> struct VssClusters;
-template <> struct VssClusters<8> { static constexpr int c64 = 1, c32 = 1; };
-template <> struct VssClusters<16> { static constexpr int c64 = 1, c32 = 1; };
-template <> struct VssClusters<24> { static constexpr int c64 = 6, c32 = 6; };
-template <> struct VssClusters<32> { static constexpr int c64 = 16, c32 = 8; };
+// cluster sizes of vss_terms_kernel, for the grids that vss_terms1_kernel does
+// not take.  FP64 N=24: 6, 9 points, both species 886 us against 927 with 12
+// CTAs; FP32 N=32: 8, 18 points 2.85 ms against 2.85 with 16; FP64 N=32: only 16
+// fit
+template <typename R, int N> constexpr int vss_cluster() {
+  return N == 24 ? 6 : sizeof(R) == 4 ? 8 : 16;
+}
 
 template <int N>
 static int vss_setup_pair(dgfs_vss_s* h, const dgfs_vss_desc* d, int p, int q,
@@ -1908,7 +1909,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
   constexpr bool FP32 = sizeof(R) == 4;
   constexpr int CPRO = VhsClusters<N>::cpro;
   constexpr int CEPI = VhsClusters<N>::cepi;
-  constexpr int C = FP32 ? VssClusters<N>::c32 : VssClusters<N>::c64;
+  constexpr int C = vss_cluster<R, N>();
   using T = c2_t<R>;
   const size_t E = h->max_evals, n = h->n, Tt = (size_t)h->Nrho * h->M;
   auto ReLf = [&](int k) { return h->ReLf + k * E * n; };
@@ -1987,7 +1988,7 @@ static int vss_run(dgfs_vss_s* h, const VssCall& c, int f_double, void* Qp, int 
     // per SM (N=32, one point: 572 against 612 us for both species); a larger one
     // keeps the terms' CTAs from starting (N=32, 18 points: 2968 us against 2874
     // with a launch each; N=16, 24 points, 256 CTAs: 370 against 360)
-    const int step = groups == 1 || N * (N / GG::NYB) * groups * c.nq <= 148 ? c.nq : 1;
+    const int step = groups == 1 || N * (N / GG::NYB) * groups * c.nq <= kSms ? c.nq : 1;
     for (int k0 = 0; k0 < c.nq; k0 += step) {
       VssGainArgs ga{};
       ga.w = h->w; ga.Nrho = h->Nrho; ga.M = h->M; ga.nevals = nevals;
@@ -2668,7 +2669,7 @@ static int fno_tc(dgfs_fno_s* h, const fno::TcArgs& a, cudaStream_t st) {
   // the 512 TMEM columns); NC=32: 16 CTAs x 32 columns fit
   const size_t pad = NC == 128 ? 40 * 1024 : 0;
   const int per_sm = NC == 128 ? 3 : 8;
-  const unsigned grid = (unsigned)std::min<long>(ntiles, 148L * per_sm);
+  const unsigned grid = (unsigned)std::min<long>(ntiles, (long)kSms * per_sm);
   if (pad)
     DGFS_CUDA(cudaFuncSetAttribute(fno::fno_tc_kernel<NC, EPI>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -1494,8 +1494,9 @@ vhs_terms_fp32s_kernel(VhsTermsArgs a) {
 // a barrier costs 800-1000 clocks, so a lone CTA waits most of the time.  The
 // kernel therefore keeps only the transform slab A (z and y passes in place)
 // and one receive slab R in shared memory, and half the values per lane, so
-// that two or three CTAs of different clusters share an SM and one's exchange
-// runs under another's transforms.  One receive slab needs two cluster
+// that two to six CTAs of different clusters share an SM (FP64 N=48: one, and
+// nothing hides its exchange) and one's exchange runs under another's
+// transforms.  One receive slab needs two cluster
 // barriers per transform (data arrived; buffer read), each split into arrive
 // and wait around a pass that does not depend on it.
 // ---------------------------------------------------------------------------

@@ -66,7 +66,9 @@ typedef struct {
   double cw;
   const double* c0;        /* [N] host */
   int32_t precision;       /* DGFS_PREC_* */
-  int32_t max_evals;       /* evaluations per launch batch (scratch size) */
+  int32_t max_evals;       /* evaluations per pass (scratch size); in the FP64 mode
+                              at most what 4 GiB of scratch hold.  Longer calls
+                              run in several passes */
 } dgfs_vhs_desc;
 
 /* Replaces DGFSVHSGLLScatteringModelStd.__init__/perform_precomputation
@@ -136,7 +138,7 @@ int dgfs_vhs_set_projection(dgfs_vhs_handle h, int32_t enable);
  * several variants per N (kinds and thread-block-cluster sizes).
  * dgfs_vhs_variants writes the codes of the variants compiled for N into out
  * (up to max) and returns their count;
- * dgfs_vhs_set_variant selects one for a handle (0 = built-in default). */
+ * dgfs_vhs_set_variant selects one for a handle (0 = by grid and batch size). */
 int dgfs_vhs_variants(int32_t N, int32_t* out, int32_t max);
 int dgfs_vhs_set_variant(dgfs_vhs_handle h, int32_t variant);
 
@@ -191,7 +193,8 @@ typedef struct {
   const double* gamma;     /* [nspcs*nspcs] host */
   const double* eta;       /* [nspcs*nspcs] host */
   const double* prefac;    /* [nspcs*nspcs] host */
-  int32_t max_evals;
+  int32_t max_evals;       /* evaluations per pass; at most what 4 GiB of scratch
+                              hold.  Longer calls run in several passes */
   int32_t precision;       /* DGFS_PREC_FP64 (reference) or DGFS_PREC_FP32:
                               FP32 transforms of f - M with the Maxwellian
                               parts and the radial sum, final transform and
