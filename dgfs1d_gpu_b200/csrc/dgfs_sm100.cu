@@ -175,8 +175,12 @@ struct dgfs_vhs_s {
   int project = 0;
   double Ginv[25] = {};
   int c32 = 0;  // variant code of the FP32 terms kernel (autotuner choice)
+  // the last call's batch size, variant setting, chosen terms kernel and slices
+  // (choosing anew costs 0.5 us)
+  int plan_evals = 0, plan_c32 = 0, plan_code = 0, plan_ns = 0;
   // constant tables
-  double* c0 = nullptr;      // [N], in the FP64 mode then multp [Nrho][Mu]
+  double* c0 = nullptr;      // [N], in the FP64 mode then the scaled
+                             //   multiplicities [Nrho][Mu]
   double* b2 = nullptr;      // [n]
   double* b1w64 = nullptr;   // [Nrho][n]
   float* b1w32 = nullptr;    // [Nrho][n] (FP32 mode)
@@ -716,8 +720,9 @@ template <int N> static Terms32Choice choose_terms32(const dgfs_vhs_s* h, int ne
   return {code, s.ns};
 }
 
-// Spectra that dir_slices may ask for: the batch's own, or twice what the GPU
-// holds at once of any variant (more measured no faster).
+// Spectra that dir_slices may use: the batch's own, or what the GPU holds at once
+// of any variant; twice that where a full batch leaves the GPU part-empty (more
+// measured no faster).
 template <int N> static size_t spectra_slots_n(bool fp32) {
   int m = 1;
   if (!fp32) {
@@ -738,6 +743,7 @@ static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu) {
     case 32: m = spectra_slots_n<32>(fp32); break;
     default: m = spectra_slots_n<48>(fp32); break;
   }
+  if (pairs >= m / 2) m /= 2;
   return std::max(pairs, std::min(m, pairs * Mu));
 }
 
@@ -839,10 +845,14 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
     a.Fg = h->Fg; a.ph = h->ph; a.uv = h->uv; a.mult = h->mult;
     a.b1w = h->b1w32; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq32; a.rho = h->rho; a.Fny = h->Fny; a.err = h->err;
-    const Terms32Choice tc = choose_terms32<N>(h, nevals);
-    const int c = tc.code;
+    if (h->plan_evals != nevals || h->plan_c32 != h->c32) {
+      const Terms32Choice tc = choose_terms32<N>(h, nevals);
+      h->plan_evals = nevals; h->plan_c32 = h->c32;
+      h->plan_code = tc.code; h->plan_ns = tc.ns;
+    }
+    const int c = h->plan_code;
     a.pm = c >= 600;   // (the two-lane kernels have their own plane format)
-    a.NS = nslices = tc.ns;
+    a.NS = nslices = h->plan_ns;
     const size_t psmem = (size_t)(9 * N * (N + 1) + 2 * (3 * N + 3)) * sizeof(float2);
     if ((rc = launch_plain(vhs_nyq_planes_kernel<N>,
                            dim3((h->Mu + 1) / 2, h->Nrho, nevals), dim3(6 * N),
@@ -880,7 +890,8 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
   } else {
     VhsTermsArgs a{};
     a.Fg = h->Fg; a.ph = h->ph; a.uv = nullptr; a.mult = h->mult;
-    a.b1w = h->b1w64; a.multp = h->c0 ? h->c0 + N : nullptr; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
+    if (h->rho64) a.mult = h->c0 + N;
+    a.b1w = h->b1w64; a.H = h->H; a.Mu = h->Mu; a.Nrho = h->Nrho;
     a.nyq = h->nyq64; a.rho = h->rho64; a.Fny = h->Fny64;
     if (h->rho64) {
       // packed transforms: Nyquist-plane transforms, then the terms
@@ -890,13 +901,20 @@ static int vhs_run(dgfs_vhs_s* h, const void* f, int f_double, void* Q,
         return rc;
       mark(); mark();  // no Maxwellian-gain stage in FP64 mode
       if constexpr (N <= 16) {
-        a.NS = nslices =
-            dir_slices(h, nevals, terms1_resident<double, N>(), kCostOneCta).ns;
+        if (h->plan_evals != nevals) {
+          h->plan_evals = nevals;
+          h->plan_ns = dir_slices(h, nevals, terms1_resident<double, N>(), kCostOneCta).ns;
+        }
+        a.NS = nslices = h->plan_ns;
         rc = launch_terms1<double, N>(a, nevals, h->Nrho, st);
       } else {
         constexpr int C64 = VhsClusters<N>::c64;
-        a.NS = nslices =
-            dir_slices(h, nevals, termsh_resident<double, N, C64>(), kCostCluster).ns;
+        if (h->plan_evals != nevals) {
+          h->plan_evals = nevals;
+          h->plan_ns =
+              dir_slices(h, nevals, termsh_resident<double, N, C64>(), kCostCluster).ns;
+        }
+        a.NS = nslices = h->plan_ns;
         rc = launch_termsh_c<double, N, C64>(a, nevals, h->Nrho, st);
       }
       if (rc) return rc;

@@ -73,10 +73,10 @@ struct VhsTermsArgs {
   const void* Fg;             // [nevals][n] complex, precision R
   const void* ph;             // [Nrho][Mu][3][N] exp(i kappa_a rep(l)), precision R
   const void* uv;             // [nevals][Nrho][Mu][2][3][N] u_a, v_a (split)
-  const float* mult;          // [Mu] multiplicity of each transformed direction
+  const void* mult;           // [Mu] multiplicity (float); FP64 packed terms: double
+                              // [Nrho][Mu], times the radial point's power of two
+                              // (off b1w)
   const void* b1w;            // [Nrho][n] W_p b1_p(l), precision R
-  const double* multp;        // FP64 packed terms: [Nrho][Mu] multiplicity times
-                              // the radial point's power of two (off b1w)
   void* H;                    // out [nevals][Nrho][n] complex, precision R
                               // (FP32: [nevals][ceil(Nrho/2)][n], packed pairs)
   const void* nyq;            // FP32: [Nrho][Mu][3] exp(i N kappa_a)
@@ -616,7 +616,7 @@ vhs_terms_kernel(VhsTermsArgs a) {
     for (int i = t; i < 3 * N; i += G::NT)
       tab[i] = ph[((size_t)p * a.Mu + q) * 3 * N + i];
     __syncthreads();
-    const R mq = (R)a.mult[q];
+    const R mq = (R)static_cast<const float*>(a.mult)[q];
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
       // z-pass: multiplier cos/sin of a(l), inverse FFT along z
@@ -726,7 +726,8 @@ vhs_terms_kernel(VhsTermsArgs a) {
 // falls, so that S_p0's rounding, weighted by b1_p1, would dominate the FP64
 // mode's error (N=24, radii 0.05 and 4: 1.3e-11 instead of 2.2e-12): there the
 // sum of the smaller weight is packed times the power of two nearest to the
-// weights' ratio (multp) and its b1 divided by it, both exact.
+// weights' ratio (in its directions' multiplicities) and its b1 divided by it,
+// both exact.
 //
 // Pipeline per transform k (term (p, q) = (p0 + k / Mu, k % Mu)):
 //   y-pass(k) -> exchange(k) into receive buffer k%2 -> arrive
@@ -1659,7 +1660,7 @@ vhs_termsh_kernel(VhsTermsArgs a) {
     const T rx = rp[yy * N + c];
     const T* rY = rp + N * N + c + h * H * N;
     const T* rZ = rp + 2 * N * N + yy * N + h * H;   // [y][x]
-    const R mq = SPLIT ? R(1) : (R)a.multp[term(k)];
+    const R mq = SPLIT ? R(1) : static_cast<const R*>(a.mult)[term(k)];
     T uyz{}, vyz{};
     if constexpr (SPLIT) {
       uyz = cmul(ut[N + yy], ut[2 * N + c]);
@@ -1879,7 +1880,7 @@ vhs_terms1_kernel(VhsTermsArgs a) {
       uxy = cmul(ut[p], ut[N + q]);
       vxy = cmul(ut[3 * N + p], ut[4 * N + q]);
     }
-    const R mq = SPLIT ? R(1) : (R)a.multp[term(k)];
+    const R mq = SPLIT ? R(1) : static_cast<const R*>(a.mult)[term(k)];
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int z = out(m);
