@@ -740,7 +740,10 @@ static size_t spectra_slots(int N, bool fp32, size_t pairs, int Mu) {
     case 8: m = spectra_slots_n<8>(fp32); break;
     case 16: m = spectra_slots_n<16>(fp32); break;
     case 24: m = spectra_slots_n<24>(fp32); break;
-    case 32: m = spectra_slots_n<32>(fp32); break;
+    case 32:
+      m = spectra_slots_n<32>(fp32);
+      if (fp32) terms32_tma_resident<32, 4>();   // (asked at create, not in a capture)
+      break;
     default: m = spectra_slots_n<48>(fp32); break;
   }
   if (pairs >= m / 2) m /= 2;
